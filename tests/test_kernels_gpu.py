@@ -242,6 +242,23 @@ def test_gemm_simt_rows_independent(ops):
     assert torch.equal(whole[5:6], one)
 
 
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 16, 17, 33, 65, 129, 700])
+@pytest.mark.parametrize("N,K", [(1, 4), (65, 33), (129, 256), (200, 2052), (1030, 260)])
+def test_gemm_simt_one_order_of_sums(ops, M, N, K):
+    """Every tile and every split of K (they follow M, N and K), and the form for rows that are no 16-byte pieces, give a
+    row the same bits; its error is that of eight chains of K/8 (each at most K/8 roundings of its partial sums)."""
+    a = rnd(700, K, seed=44)
+    w = rnd(N, K, scale=0.05, seed=45)
+    one = ops.gemm_simt(a[:1], w, torch.empty(1, N, device="cuda"))
+    got = ops.gemm_simt(a[:M], w, torch.full((M, N), float("nan"), device="cuda"))
+    wide = torch.zeros(M, K + 1, device="cuda")        # the same rows at a stride of no 16-byte pieces
+    wide[:, :K] = a[:M]
+    assert torch.equal(got[:1], one)
+    assert torch.equal(ops.gemm_simt(wide[:, :K], w, torch.empty(M, N, device="cuda")), got)
+    bound = (K / 8 + 4) * 2.0 ** -24 * (a[:M].double().abs() @ w.double().abs().T)
+    assert ((got.double() - a[:M].double() @ w.double().T).abs() <= bound + 1e-30).all()
+
+
 @pytest.mark.parametrize("R,V", [(1, 331), (5, 151936), (3, 1000), (64, 4097)])
 def test_argmax(ops, R, V):
     lg = rnd(R, V, seed=50)
