@@ -221,6 +221,47 @@ def test_attention_generic_far_key(ops, dtype):
         torch.testing.assert_close(o1, o2, **tol(dtype))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("q_lens", [(1, 1, 1), (63,), (64,), (1, 64, 1, 1), (65, 2, 1, 33), (1, 130, 1)])
+@pytest.mark.parametrize("NH,NKV,D,DV,window,keep", [(3, 3, 64, 64, 0, 0), (4, 2, 128, 64, 33, 5), (9, 3, 20, 36, 0, 0), (16, 2, 32, 256, 40, 70),
+                                                    (5, 1, 136, 132, 31, 0)])
+def test_attention_generic_options(ops, dtype, q_lens, NH, NKV, D, DV, window, keep):
+    """Steps of one-token requests, of portions and of both, around the edges of the kernels' tiles (64 tokens, 32 keys),
+    with every option, against float64; a value that no query sees is not a number and must not reach a result."""
+    page, B = 8, len(q_lens)
+    lens = [q + (0 if i % 3 == 1 else 37 * (i + 1)) for i, q in enumerate(q_lens)]
+    n_pages = sum(-(-l // page) for l in lens) + 2
+    perm = torch.randperm(n_pages, generator=torch.Generator().manual_seed(3)).tolist()
+    table = torch.full((B, max(-(-l // page) for l in lens)), -1, dtype=torch.int32)
+    kp, vp = rnd(n_pages, NKV, page, D, dtype=dtype, seed=50), rnd(n_pages, NKV, page, DV, dtype=dtype, seed=51)
+    for b, l in enumerate(lens):
+        for i in range(-(-l // page)):
+            table[b, i] = perm.pop()
+        if l % page:
+            vp[int(table[b, l // page]), :, l % page:] = float("nan")      # behind the request's last key
+    table = table.cuda()
+    T = sum(q_lens)
+    pos = torch.cat([torch.arange(l - q, l) for l, q in zip(lens, q_lens)]).to(torch.int32).cuda()
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(q_lens)).to(torch.int32).cuda()
+    q, gate = rnd(T, NH * D + 4, dtype=dtype, seed=52)[:, :NH * D], rnd(T, NH * DV, dtype=dtype, seed=53)
+    sinks, slopes = rnd(NH, seed=54), rnd(NH, seed=55).abs() * 0.1
+    out = torch.full((T, NH * DV), float("nan"), device="cuda", dtype=dtype)
+    ops.attention_generic(q, out, kp, vp, pos, seq, table, NH, NKV, D, D ** -0.5, window, value_dim=DV if DV != D else 0, keep_first=keep,
+                          sinks=sinks, slopes=slopes, gate=gate)
+    want, at = torch.empty(T, NH, DV, dtype=torch.float64, device="cuda"), 0
+    for b, (l, n) in enumerate(zip(lens, q_lens)):
+        j = torch.arange(l, device="cuda")
+        k, v = (x[table[b, j // page].long(), :, j % page].double().repeat_interleave(NH // NKV, 1) for x in (kp, vp))
+        d = pos[at:at + n, None].long() - j
+        hidden = (d < 0) | ((d >= window) & (j[None] >= keep) if window else torch.zeros_like(d, dtype=torch.bool))
+        s = torch.einsum("qhd,khd->hqk", q[at:at + n].double().view(n, NH, D), k) * D ** -0.5 - slopes.double()[:, None, None] * d
+        s = torch.cat([s.masked_fill(hidden, -float("inf")), sinks.double()[:, None, None].expand(NH, n, 1)], -1).softmax(-1)[:, :, :-1]
+        want[at:at + n] = torch.einsum("hqk,khd->qhd", s, v)
+        at += n
+    want = want.reshape(T, NH * DV) * torch.sigmoid(gate.double())
+    torch.testing.assert_close(out.double(), want, **tol(dtype))
+
+
 @pytest.mark.parametrize("in_dtype,out_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32),
                                                 (torch.bfloat16, torch.bfloat16)])
 @pytest.mark.parametrize("M,N,K", [(1, 331, 80), (7, 100, 72), (65, 130, 200), (3, 1000, 4096), (128, 64, 16)])
