@@ -39,6 +39,61 @@
 #define AT_HALF 64                   // keys of a half tile
 #define AT_LAZY 8.0f                 // a row's maximum may lag by this much (log2 units) before O is rescaled
 
+// Two floats that one instruction works on.
+typedef unsigned long long at_f2;
+__device__ __forceinline__ at_f2 at_pack(float a, float b) {
+    at_f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void at_split(at_f2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
+__device__ __forceinline__ at_f2 at_fma(at_f2 a, at_f2 b, at_f2 c) {
+    at_f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ at_f2 at_add(at_f2 a, at_f2 b) {
+    at_f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ at_f2 at_mul(at_f2 a, at_f2 b) {
+    at_f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ at_f2 at_both(float x) { return at_pack(x, x); }
+
+// 2^y for two y on the multiply-add pipes: y = n + f, n the nearest whole number (the low bits of y + 1.5 2^23), f in
+// [-1/2, 1/2], 2^f by a polynomial of degree five fitted here for the least largest relative error (7.5e-8 in exact
+// arithmetic; the special-function unit's is 1.2e-7), times 2^n.  y below -126 counts as -126 (1.2e-38 where the exact
+// value is smaller still); a y that is no number stays none.
+__device__ __forceinline__ at_f2 at_exp2_poly(at_f2 y) {
+    float a, b;
+    at_split(y, a, b);
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(-126.f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(b) : "f"(-126.f));
+    y = at_pack(a, b);
+    const at_f2 z = at_add(y, at_both(12582912.f));
+    const at_f2 f = at_fma(at_add(z, at_both(-12582912.f)), at_both(-1.f), y);
+    at_f2 q = at_fma(at_both(1.32764701e-3f), f, at_both(9.67554096e-3f));
+    q = at_fma(q, f, at_both(5.55071346e-2f));
+    q = at_fma(q, f, at_both(2.40221202e-1f));
+    q = at_fma(q, f, at_both(6.93146944e-1f));
+    q = at_fma(q, f, at_both(1.00000012f));
+    at_split(z, a, b);
+    const float s0 = __uint_as_float((__float_as_uint(a) << 23) + 0x3f800000u), s1 = __uint_as_float((__float_as_uint(b) << 23) + 0x3f800000u);
+    return at_mul(q, at_pack(s0, s1));
+}
+
+// Of eight pairs of columns the first AT_POLY take their exponentials on the multiply-add pipes, the others on the
+// special-function unit (4 lanes a clock and sub-partition: a half tile's 64 columns of the two warps there take it 1024
+// clocks, as long as the half's products take the tensor core).  A pair costs ten packed instructions (20 clocks of the
+// multiply-add pipe, which the rest leaves three quarters idle) in place of 16 clocks of that unit, so three of eight
+// come out even.  Measured, microseconds with one exponential at a time, then 0, 2, 3, 4 of eight pairs: 2048 tokens 49.7, 47.9,
+// 46.5, 45.8, 47.0 (32 heads on 8); 2048 behind 6144 263, 252, 240, 232, 246; 1000 behind 5000 (40 heads) 188, 180, 172, 174, 178.
+#define AT_POLY 3
+
 struct AttnTcParams {
     bf16* out;
     int out_stride;
@@ -318,18 +373,31 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             TL_PHASE(2);
             // second pass, on the scores still in registers: P = 2^(s * scale - m) as packed bfloat16 into the first 32
             // columns of S_x
+            // (pairs of columns: two floats to an instruction; the sums are those of columns 0, 1, 2, 3 modulo 4)
+            const at_f2 scale2 = at_both(scale_log2), m2 = at_both(-m_use);
             auto exp_of = [&](uint32_t (&raw)[32], int c0) {
-                float part[4] = {0.f, 0.f, 0.f, 0.f};
+                at_f2 part[2] = {0ull, 0ull};
                 uint32_t pk[16];
 #pragma unroll
                 for (int c = 0; c < 32; c += 2) {
-                    const float e0 = tc_exp2(fmaf(__uint_as_float(raw[c]), scale_log2, -m_use));
-                    const float e1 = tc_exp2(fmaf(__uint_as_float(raw[c + 1]), scale_log2, -m_use));
-                    part[c & 3] += e0;
-                    part[(c + 1) & 3] += e1;
+                    const at_f2 y = at_fma(at_pack(__uint_as_float(raw[c]), __uint_as_float(raw[c + 1])), scale2, m2);
+                    at_f2 e;
+                    if ((c >> 1) % 8 < AT_POLY) {
+                        e = at_exp2_poly(y);
+                    } else {
+                        float y0, y1;
+                        at_split(y, y0, y1);
+                        e = at_pack(tc_exp2(y0), tc_exp2(y1));
+                    }
+                    part[(c >> 1) & 1] = at_add(part[(c >> 1) & 1], e);
+                    float e0, e1;
+                    at_split(e, e0, e1);
                     pk[c >> 1] = pack_bf16x2(e0, e1);
                 }
-                l_run += (part[0] + part[1]) + (part[2] + part[3]);
+                float s0, s1, s2, s3;
+                at_split(part[0], s0, s1);
+                at_split(part[1], s2, s3);
+                l_run += (s0 + s1) + (s2 + s3);
                 tc_st16_nowait(tmem_sx + (c0 >> 1), pk);
             };
             exp_of(ra, 0);
@@ -350,7 +418,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (!failed && !abort_s && mbar_wait(o_full + 8 * hs, 0, &abort_s)) {
             tc_fence_after();
             if (p.sinks && m_run != -INFINITY) l_run += exp2f(p.sinks[head] * AT_LOG2E - m_run);
-            const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+            const float inv = l_run > 0.f && m_run != -INFINITY ? 1.f / l_run : 0.f;      // (a row that sees no key: zeros)
             bf16* dst = p.out + (size_t)(tok0 + r) * p.out_stride + (size_t)(h0 + hs) * D;
 #pragma unroll
             for (int c0 = 0; c0 < D; c0 += 32) {

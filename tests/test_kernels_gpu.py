@@ -373,6 +373,27 @@ def test_attention_chunk_kernel(ops, NH, NKV, D, page):
     torch.testing.assert_close(o1, o2, **tol(torch.bfloat16))
 
 
+@pytest.mark.parametrize("D,spread", [(128, 0.0), (128, 1.0), (128, 40.0), (128, 4000.0), (64, 40.0)])
+def test_prompt_attention_exponentials_of_every_size(ops, D, spread):
+    """Scores that are all equal, that differ by a few units and that differ by thousands (exponentials of which almost all
+    vanish, far below where the smallest float lies), each column of a tile by whichever unit takes its exponential."""
+    NH, NKV, page, n = 2, 1, 64, 256
+    kp, vp = torch.zeros(4, NKV, page, D, device="cuda", dtype=torch.bfloat16), rnd(4, NKV, page, D, dtype=torch.bfloat16, seed=56)
+    kp[..., 0] = rnd(4, NKV, page, dtype=torch.bfloat16, seed=57)
+    q = torch.zeros(n, (NH + 2 * NKV) * D, device="cuda", dtype=torch.bfloat16)
+    q[:, 0:NH * D:D] = spread
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    call = lambda q: ops.attention_tc(q, torch.full((n, NH * D), 7.0, device="cuda", dtype=torch.bfloat16), kp, vp, i32([0, 0]), i32([128, 0]), 2,
+                                      i32([0, n]), i32([n]), i32([[0, 1, 2, 3]]), NH, NKV, D, 1.0, 0)
+    got = call(q)
+    s = spread * kp[:, 0, :, 0].reshape(1, n).double() + torch.full((n, n), -float("inf"), device="cuda", dtype=torch.float64).triu(1)
+    want = (s.softmax(-1) @ vp[:, 0].reshape(n, D).double()).repeat(1, NH)
+    torch.testing.assert_close(got.double(), want, **tol(torch.bfloat16))
+    q[70, :D] = float("nan")            # a query that is no number stays none, and alone
+    bad = call(q).isnan()
+    assert bad[70, :D].all() and int(bad.sum()) == D
+
+
 @pytest.mark.parametrize("window", [1, 7, 64, 100])
 def test_tensor_core_attention_window_and_mixed_batch(ops, window):
     o1, o2 = _tc_case(ops, 8, 2, 128, 16, lens=[150, 90, 300, 17, 64], q_lens=[150, 1, 70, 1, 2], window=window, seed=62)
