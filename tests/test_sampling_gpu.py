@@ -46,6 +46,37 @@ def test_sample_matches_plain(V):
             assert abs(lps[i] - float(torch.log_softmax(scaled, -1)[got[i]])) < 1e-3
 
 
+@pytest.mark.parametrize("V", [16384, 16389, 40000])
+@pytest.mark.parametrize("kind", ["equal", "two", "spread", "negative", "holes"])
+def test_wide_rows_cut_where_the_plain_sampler_cuts(V, kind):
+    """Rows for which the cut's bits are all of one kind: one value, two values, magnitudes from 1e-30 to 1e3, all below
+    zero, -inf in places; a top-k at a tie keeps every equal value."""
+    g = torch.Generator().manual_seed(V)
+    row = {"equal": lambda: torch.full((V,), 1.5), "two": lambda: torch.where(torch.rand(V, generator=g) < 0.5, 1.0, 1.0000001),
+           "spread": lambda: torch.randn(V, generator=g) * 10.0 ** (torch.rand(V, generator=g) * 33 - 30),
+           "negative": lambda: -torch.rand(V, generator=g) * 20 - 1e-3,
+           "holes": lambda: torch.randn(V, generator=g).masked_fill(torch.rand(V, generator=g) < 0.7, float("-inf"))}[kind]()
+    cases = [(1.0, 7, 1.0, 0.0), (1.0, 0, 0.5, 0.0), (0.7, 1000, 0.9, 0.0), (1.0, V - 1, 0.99, 0.001), (1.0, 1, 0.3, 0.0)]
+    R = len(cases)
+    got, _ = run_sample(row.repeat(R, 1).cuda(), *[[c[j] for c in cases] for j in (0, 1, 2, 3)], list(range(R)), [3] * R)
+    for i, (temp, k, p, mp) in enumerate(cases):
+        x = (row / temp).double()
+        weight = (x - x.max()).exp()
+        keep = x >= x.topk(k).values[-1] if 0 < k < V else torch.ones(V, dtype=torch.bool)
+        keep &= weight >= mp
+        values, at = torch.unique(x[keep], return_inverse=True)         # ascending; equal values stay or go together
+        mass = torch.zeros(len(values), dtype=torch.float64).index_add_(0, at, weight[keep])
+        above = mass.flip(0).cumsum(0).flip(0) - mass
+        if p < 1.0:         # a value goes when the mass above it exceeds p
+            keep &= x >= values[above <= p * mass.sum() * (1 + 1e-6)][0]
+        assert keep[got[i]], f"case {i}: a dropped token was drawn"
+        # (where the draw falls between two tokens by less than the sums' rounding either may come)
+        cdf = torch.where(keep, weight, 0.0).cumsum(0) / weight[keep].sum()
+        u = plain_qwen3.philox_uniform(i, 3)
+        before = float(cdf[got[i]] - weight[got[i]] / weight[keep].sum())
+        assert before - 1e-4 <= u <= float(cdf[got[i]]) + 1e-4, f"case {i}"
+
+
 def test_draws_follow_the_distribution():
     """Many counters on one row: the empirical frequencies approach the kept probabilities."""
     V = 50
