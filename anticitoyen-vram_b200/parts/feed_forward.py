@@ -285,7 +285,10 @@ class RoutedExperts(FeedForward):
         if self.router_linear is not None:
             # many tokens against a few dozen router rows: one column of tiles, so the reduction is split eight ways
             # to put more than a ninth of the SMs to work
-            plan = (0, 128, 8, 4, 0) if h.dtype == torch.bfloat16 and T >= 512 and H >= 2048 and self.router_linear.out_features <= 128 else None
+            # (a few tokens: that column is one tile, whose k-blocks a cluster of eight shares instead of four)
+            plan = None
+            if h.dtype == torch.bfloat16 and H >= 2048 and self.router_linear.out_features <= 128:
+                plan = (0, 128, 8, 4, 0) if T >= 512 else (1, 16, 8, 8) if T <= 16 else None
             logits = self.router_linear(h, out_dtype=torch.float32, plan=plan)
             ops.moe_route(h, None, None, top, self.scoring == "softmax", self.renormalize, ids, weights, gate, logits=logits,
                           experts=E, **route)

@@ -324,3 +324,51 @@ def test_dense_unit_with_gelu_in_the_product(T, H, F, dtype):
     part.load({n: torch.as_tensor(v) for n, v in W.items()}, Runtime(torch.device(DEV), DT[dtype]))
     h = bf(rng.standard_normal((T, H)))
     close(part.forward(dev(h, DT[dtype]), None), pz.dense(h, W, "m."), 3e-5 if dtype == "float32" else 3e-2, "dense unit")
+
+
+# --------------------------------------------------------------------------- the experts' outputs, summed; rows grouped
+@pytest.mark.parametrize("out_dtype,d_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("H,ld,top", [(8, 8, 1), (520, 520, 6), (1032, 1048, 8), (4096, 4096, 9), (4100, 4100, 17), (516, 517, 3), (30, 30, 4)])
+@pytest.mark.parametrize("shared", [False, True])
+def test_combine_sums_in_the_order_of_the_choices(out_dtype, d_dtype, H, ld, top, shared):
+    """Rows of whole 16-byte pieces and others, more choices than are loaded at a time, choices without a row: the same
+    sum, term by term, in float."""
+    from acvram_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(H + top)
+    T, rows = 3, 40
+    d = torch.randn(rows, ld, device="cuda", generator=g).to(d_dtype)[:, :H]
+    place = torch.randint(0, rows, (T * top,), device="cuda", generator=g, dtype=torch.int32)
+    place[1] = -1 if top > 1 else place[1]
+    s = torch.randn(T, ld, device="cuda", generator=g).to(out_dtype)[:, :H] if shared else None
+    gate = torch.rand(T, device="cuda", generator=g) if shared else None
+    out = torch.full((T, ld), 7.0, device="cuda", dtype=out_dtype)[:, :H]
+    ops.moe_combine(d, place, top, s, gate, out)
+    want = torch.zeros(T, H, device="cuda")
+    for t in range(T):
+        for j in range(top):
+            at = int(place[t * top + j])
+            if at >= 0:
+                want[t] += d[at].float()
+        if shared:      # (one multiply-add in the kernel)
+            want[t] = (want[t].double() + gate[t].double() * s[t].double()).float()
+    assert torch.equal(out, want.to(out_dtype))
+
+
+@pytest.mark.parametrize("E", [1, 31, 32, 33, 64, 257])
+@pytest.mark.parametrize("tile", [64, 128])
+def test_grouped_rows_start_at_tiles(E, tile):
+    """Experts' tiles lie one behind the other in the experts' order, whatever their number."""
+    from acvram_b200.kernels import ops
+    N = 700
+    ids = torch.randint(0, E, (N,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(E), dtype=torch.int32)
+    if E > 2:
+        ids[ids == 1] = 2       # an expert without rows
+    tiles = ops.moe_max_tiles(N, E, tile)
+    grouped = torch.full((tiles * tile,), -7, device="cuda", dtype=torch.int32)
+    place, expert, used = (torch.empty(n, device="cuda", dtype=torch.int32) for n in (N, tiles, 1))
+    ops.moe_group(ids, E, grouped, place, expert, tile, used)
+    counts = torch.bincount(ids.long(), minlength=E).tolist()
+    want = [e for e in range(E) for _ in range(-(-counts[e] // tile))]
+    assert int(used) == len(want) and expert.tolist() == want + [-1] * (tiles - len(want))
+    assert (grouped[place.long()] == torch.arange(N, device="cuda")).all()
+    assert (expert[(place // tile).long()] == ids).all() and int((grouped[:len(want) * tile] >= 0).sum()) == N
