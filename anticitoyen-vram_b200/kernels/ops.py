@@ -412,22 +412,45 @@ def sm_count(device=None) -> int:
 
 
 # Split and pipeline depth of the products with few tokens (weight rows on the tensor core's M side), as measured
-# on a B200 with layer sizes from 0.6B to 32B models: the first row that fits decides.  Splits of K are the CTAs
-# of one cluster (summed through its shared memory).  Columns: tiles per SM from (inclusive) to (exclusive),
-# k-blocks of 64 from to, tokens per tile (bn) from to (inclusive), then what to do: splits, stages.
-#   many tiles: no split, several CTAs share an SM; few tiles: 2..4 splits fill the SMs
+# on a B200 with layer sizes from 0.6B to 32B models, whole feed-forwards and steps one product behind the other: the first row
+# that fits decides.  Splits of K are the CTAs of one cluster (summed through its shared memory).  Columns: tiles per SM
+# from (inclusive) to (exclusive), k-blocks of 64 from to, tokens per tile (bn) from to (inclusive), then what to do:
+# splits, stages.
+#   What decides is that the CTAs come in one wave.  With a deep pipeline a CTA has its SM to itself, and clusters of s CTAs
+#   lie inside a part of the chip: 148, 74, 45, 33, 26, 22, 15, 15 clusters of 1..8 fit at once (0.304, 0.223, 0.176, 0.149,
+#   0.101 tiles per SM for s = 3, 4, 5, 6, 7), not 148 / s.  So few tiles take the most splits that fit: 20 tiles (2560 x 9728)
+#   6 instead of 4, three feed-forwards of 5 tokens 102.5 -> 94.5 us; 40 tiles (5120 x 17408) 3 instead of 4, two of
+#   32 tokens 211 -> 178.  Between a half and one tile per SM two shallower CTAs share an SM (the 96 tiles of 12288 x 2048:
+#   six feed-forwards of 12 tokens 154 -> 132 us with 3 splits of 3 stages, of 64 tokens 258 -> 188 unsplit), and from 1.5
+#   tiles on one CTA a tile with 3 or 4 stages, as many to an SM as its share of the tiles.
 INF = float("inf")
 GEMM_FEW_TOKENS_RULES = (
+    (2.2,    3.0,    0,   INF, 16, 16,  1, 3),
+    (2.0,    2.2,    0,   INF, 16, 64,  1, 4),
     (2.0,    INF,    0,   INF, 16, 128, 1, 8),
+    (1.5,    2.0,    0,   INF, 16, 16,  1, 4),
     (1.0,    2.0,    0,   INF, 16, 16,  2, 3),
     (1.0,    2.0,    0,   INF, 32, 128, 1, 4),
     (0.0,    1.0,    0,   16,  16, 128, 1, 8),
+    (0.0,    0.1014, 32,  INF, 16, 16,  7, 6),
+    (0.0,    0.1014, 48,  INF, 32, 32,  7, 6),
+    (0.1014, 0.149,  32,  INF, 16, 16,  6, 8),
+    (0.1014, 0.1149, 32,  INF, 32, 32,  5, 6),
+    (0.1149, 0.149,  32,  INF, 32, 32,  6, 6),
+    (0.149,  0.176,  128, INF, 32, 32,  5, 8),
+    (0.0,    0.2231, 48,  INF, 64, 64,  4, 6),
+    (0.2231, 0.3041, 128, INF, 16, 64,  3, 8),
+    (0.3041, 0.5,    16,  INF, 64, 64,  2, 8),
+    (0.5,    1.0,    16,  INF, 64, 64,  1, 8),
+    (0.5,    1.0,    16,  128, 32, 32,  2, 4),
+    (0.5,    0.75,   16,  128, 16, 16,  3, 3),
+    (0.75,   1.0,    16,  128, 16, 16,  2, 4),
     (0.0,    1.0,    128, INF, 16, 32,  4, 8),
     (0.0,    1.0,    128, INF, 64, 128, 4, 6),
-    (0.2501, 1.0,    16,  128, 16, 16,  4, 4),
+    (0.2501, 0.5,    16,  128, 16, 16,  4, 4),
     (0.0,    0.2501, 16,  128, 16, 16,  4, 6),
     (0.0,    0.2196, 16,  128, 32, 32,  4, 6),
-    (0.2196, 1.0,    16,  128, 32, 32,  2, 6),
+    (0.2196, 0.5,    16,  128, 32, 32,  2, 6),
     (0.0,    1.0,    16,  128, 64, 128, 3, 6),
 )
 
