@@ -427,11 +427,11 @@ INF = float("inf")
 GEMM_FEW_TOKENS_RULES = (
     (2.2,    3.0,    0,   INF, 16, 16,  1, 3),
     (2.0,    2.2,    0,   INF, 16, 64,  1, 4),
-    (2.0,    INF,    0,   INF, 16, 128, 1, 8),
+    (2.0,    INF,    0,   INF, 16, 64,  1, 8),
     (1.5,    2.0,    0,   INF, 16, 16,  1, 4),
     (1.0,    2.0,    0,   INF, 16, 16,  2, 3),
-    (1.0,    2.0,    0,   INF, 32, 128, 1, 4),
-    (0.0,    1.0,    0,   16,  16, 128, 1, 8),
+    (1.0,    2.0,    0,   INF, 32, 64,  1, 4),
+    (0.0,    1.0,    0,   16,  16, 64,  1, 8),
     (0.0,    0.1014, 32,  INF, 16, 16,  7, 6),
     (0.0,    0.1014, 48,  INF, 32, 32,  7, 6),
     (0.1014, 0.149,  32,  INF, 16, 16,  6, 8),
@@ -446,12 +446,11 @@ GEMM_FEW_TOKENS_RULES = (
     (0.5,    0.75,   16,  128, 16, 16,  3, 3),
     (0.75,   1.0,    16,  128, 16, 16,  2, 4),
     (0.0,    1.0,    128, INF, 16, 32,  4, 8),
-    (0.0,    1.0,    128, INF, 64, 128, 4, 6),
     (0.2501, 0.5,    16,  128, 16, 16,  4, 4),
     (0.0,    0.2501, 16,  128, 16, 16,  4, 6),
     (0.0,    0.2196, 16,  128, 32, 32,  4, 6),
     (0.2196, 0.5,    16,  128, 32, 32,  2, 6),
-    (0.0,    1.0,    16,  128, 64, 128, 3, 6),
+    (0.0,    0.3041, 16,  128, 64, 64,  3, 6),
 )
 
 
@@ -462,10 +461,10 @@ GEMM_FEW_TOKENS_RULES = (
 # 69 us at 256, 63 us at 160).  The width is chosen so that rounds x (width + overhead) comes out least.
 GEMM_TILE_WIDTHS = (256, 224, 192, 160, 128)
 GEMM_TILE_OVERHEAD = 120
-# Pairs of CTAs on tiles of 256 tokens by 256 features (cta_group::2): a round of such tiles takes about 0.92 of a round
-# of 128 x 256 tiles (measured at 2048 and 8192 tokens with the layer sizes of 8B and 14B models: 4 to 11 % less), and
-# there are half as many places for them.
-GEMM_PAIR_ROUND = 0.92
+# Pairs of CTAs on tiles of 256 tokens by 256 features (cta_group::2): a round of such tiles takes about 0.9 of a round
+# of 128 x 256 tiles (measured at 512 to 8192 tokens with the layer sizes of 4B to 14B models: 4 to 13 % less), and there
+# are half as many places for them.
+GEMM_PAIR_ROUND = 0.905
 GEMM_PAIR = 4               # fifth element of a plan: the flag that asks for the pair kernel
 
 
@@ -474,23 +473,47 @@ def gemm_tc_plan(M: int, N: int, K: int, sms: int | None = None, bn_multiple: in
 
     Up to 128 tokens the weight rows fill the tensor core's M = 128 and the tokens are the narrow
     side (weights stream once whatever the batch); splits of K are chosen so that the work items fill
-    whole waves of the SMs (``GEMM_FEW_TOKENS_RULES``).  Above, tokens are the M side and a tile is 128
+    one wave of the SMs (``GEMM_FEW_TOKENS_RULES``).  Above, and where 65 tokens or more meet more tiles of weight rows
+    than SMs, tokens are the M side and a tile is 128
     tokens by 128..256 features: the width that needs the least rounds x width (``GEMM_TILE_WIDTHS``;
-    ``bn_multiple``: widths that are multiples of this only, for an epilogue that wants whole heads),
+    ``bn_multiple``: widths that are multiples of this only, for an epilogue that wants whole heads; over 128 tokens any
+    but 16 also means tokens on the rows and no split of K),
     or, where that comes out cheaper, 256 x 256 on a pair of CTAs (``mode`` = ``GEMM_PAIR``)."""
     n_kb = -(-K // 64)
-    if M <= 128:
-        sms = sms or sm_count()
-        bn = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
-        tiles = -(-N // 128) * -(-M // bn)
-        per_sm = tiles / sms
+    sms = sms or sm_count()
+    wide = -(-N // 128)
+    if M <= 64:
+        bn = 16 if M <= 16 else 32 if M <= 32 else 64
+        per_sm = wide / sms
         for t0, t1, k0, k1, b0, b1, splits, stages in GEMM_FEW_TOKENS_RULES:
             if t0 <= per_sm < t1 and k0 <= n_kb < k1 and b0 <= bn <= b1:
                 return 1, bn, splits, stages
         return 1, bn, 1, 8
+    if M <= 128 and wide > 3 * sms:         # (a vocabulary: many rounds, each weight row read once either way)
+        return 1, 128, 1, 8
+    if M <= 128 and wide <= sms:
+        # two tiles of 64 tokens with as many splits as come in one wave of clusters (see above), one tile of 128 where there
+        # are too many for that: its partial tile, 64 KB, leaves room for two splits (128 tokens, microseconds with one tile and 3
+        # or 4 splits before: 4096 x 4096 29.1 -> 17.6, 2560 x 9728 35.9 -> 22.8, 7168 x 5120 53 -> 24, 12288 x 2048 40.5 -> 18.5)
+        if n_kb < 16:
+            return 1, 128, 1, 8
+        per_sm = 2 * wide / sms
+        if per_sm <= 0.5:
+            return 1, 64, (4 if per_sm < 0.2231 else 3 if per_sm < 0.3041 else 2), 8
+        return (1, 128, 2, 6) if wide <= 0.5 * sms else (1, 128, 1, 6)
     if N < 256:
         return 0, (128 if N > 64 else 64), 1, 8
-    sms = sms or sm_count()
+    if M > 128 and bn_multiple == 16 and n_kb >= 48:
+        # half of the SMs or fewer would have a tile: two CTAs of a cluster share one (256 tokens, microseconds: 4096 x 12288 63 -> 41,
+        # 2560 x 9728 50 -> 34, 4096 x 4096 24.5 -> 20.6), or with a long K and somewhat more tiles two CTAs through the
+        # workspace share a wider one (256 x 5120 x 17408 91 -> 61, 300 x 4096 x 12288 65 -> 49)
+        rows = -(-M // 128)
+        if rows * wide <= 0.5 * sms:
+            return 1, 128, 2, 6
+        if n_kb >= 128:
+            for bn in (160, 192):
+                if rows * -(-N // bn) <= 0.5 * sms:
+                    return 0, bn, 2, 8
     best, best_cost = 256, None
     for bn in GEMM_TILE_WIDTHS:
         if bn % bn_multiple:
@@ -499,7 +522,7 @@ def gemm_tc_plan(M: int, N: int, K: int, sms: int | None = None, bn_multiple: in
         cost = -(-tiles // sms) * (bn + GEMM_TILE_OVERHEAD)
         if best_cost is None or cost < 0.97 * best_cost:       # a narrower tile has to win clearly
             best, best_cost = bn, cost
-    if sms >= 2 and 256 % bn_multiple == 0:
+    if M > 128 and sms >= 2 and 256 % bn_multiple == 0:
         pair_tiles = -(-M // 256) * -(-N // 256)
         if -(-pair_tiles // (sms // 2)) * (256 + GEMM_TILE_OVERHEAD) * GEMM_PAIR_ROUND < best_cost:
             return 0, 256, 1, 6, GEMM_PAIR
@@ -1381,7 +1404,7 @@ def linear_bf16_glu(x: torch.Tensor, w_pairs: torch.Tensor, out: torch.Tensor, l
     N = w_pairs.shape[0]
     if out.shape != (M, N // 2) or out.dtype != torch.bfloat16 or out.stride(1) != 1 or w_pairs.shape[1] != K:
         raise KernelError(f"linear_bf16_glu: shapes {tuple(x.shape)} x {tuple(w_pairs.shape)} -> {tuple(out.shape)} do not fit")
-    plan = gemm_tc_plan(M, N, K)
+    plan = gemm_tc_plan(M, N, K, bn_multiple=32)        # (an epilogue for tokens on the rows, without splits of K)
     if plan[0]:
         raise KernelError("linear_bf16_glu: tokens must lie on the rows (more than 128 of them)")
     bn, stages = plan[1], plan[3] if len(plan) > 3 else 8

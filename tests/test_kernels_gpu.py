@@ -531,6 +531,46 @@ def test_gemm_tc_every_tile_shape_and_split(ops, plan):
         torch.testing.assert_close(out.double(), x.double() @ w.double().T, **t)
 
 
+@pytest.mark.parametrize("M,N,K", [
+    # one shape for every way that the plans split and share a product: few tokens with 7, 6, 5, 4, 3 and 2 splits and with two or
+    # three CTAs an SM, 65 to 128 tokens in tiles of 64 and 128 or on the rows, more tokens with two CTAs to a tile
+    (3, 1024, 3072), (9, 2560, 4096), (20, 2048, 3072), (30, 2560, 3072), (25, 3072, 8192), (33, 1024, 3072), (64, 2560, 9728), (40, 5120, 8192),
+    (50, 6144, 1024), (60, 12288, 1088), (12, 12288, 1088), (20, 12288, 1088), (5, 16384, 1088), (16, 34816, 512), (7, 41472, 256), (65, 1024, 1032),
+    (100, 2560, 2048), (128, 4096, 1024), (128, 7168, 1088), (80, 12288, 1024), (70, 19456, 640), (127, 24576, 512), (66, 256, 512),
+    (129, 4096, 3072), (200, 2560, 4104), (300, 2056, 3080), (257, 5120, 8192), (300, 4096, 8200), (512, 24576, 512)])
+@pytest.mark.parametrize("form", ["float", "bias", "unary", "swiglu"])
+def test_gemm_tc_as_planned(ops, M, N, K, form):
+    """Every epilogue behind every plan, with rows and a K that fill no tile; rows that lie further apart than they are long."""
+    x = rnd(M, K + 8, dtype=torch.bfloat16, seed=58)[:, :K]
+    w = rnd(N, K, dtype=torch.bfloat16, scale=0.05, seed=59)
+    bias = rnd(N, seed=60)
+    want = x.double() @ w.double().T
+    if form == "float":
+        out = ops.gemm_tc(x, w, torch.full((M, N), 7.0, device="cuda"))
+        torch.testing.assert_close(out.double(), want, rtol=1e-4, atol=1e-3)
+    elif form == "swiglu":
+        out = ops.gemm_tc(x, w, torch.full((M, N // 2), 7.0, device="cuda", dtype=torch.bfloat16), swiglu_pairs=True, bias=bias)
+        want = (want + bias.double()).bfloat16().double()
+        gate = want[:, ::2]
+        torch.testing.assert_close(out.double(), (gate * torch.sigmoid(gate)).bfloat16().double() * want[:, 1::2], rtol=2.4e-2, atol=2.4e-2)
+    else:
+        out = ops.gemm_tc(x, w, torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16), bias=bias, unary="silu" if form == "unary" else None)
+        want = want + bias.double()
+        torch.testing.assert_close(out.double(), want * torch.sigmoid(want) if form == "unary" else want, **tol(torch.bfloat16))
+    assert ops.gemm_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 3072, 4096), (200, 512, 4096), (256, 5120, 8192)])
+def test_clamped_unit_keeps_its_tokens_on_the_rows(ops, M, N, K):
+    """The product with the clamped gated unit has no form for shared tiles: sizes for which a plain product takes one."""
+    assert ops.gemm_tc_plan(M, N, K, 148)[:3] != ops.gemm_tc_plan(M, N, K, 148, bn_multiple=32)[:3]
+    x, w = rnd(M, K, dtype=torch.bfloat16, seed=61), rnd(N, K, dtype=torch.bfloat16, scale=0.02, seed=62)
+    out = ops.linear_bf16_glu(x, w, torch.empty(M, N // 2, device="cuda", dtype=torch.bfloat16), 2.0, 1.7)
+    z = x.double() @ w.double().T
+    g, u = z[:, ::2].clamp(max=2.0), z[:, 1::2].clamp(-2.0, 2.0)
+    torch.testing.assert_close(out.double(), g * torch.sigmoid(1.7 * g) * (u + 1), **tol(torch.bfloat16))
+
+
 @pytest.mark.parametrize("M,plan", [(8, None), (8, (1, 16, 4, 4, 0)), (300, None), (300, (0, 256, 1, 4, 4))])
 def test_gemm_tc_wait_that_runs_out_leaves_its_code_and_returns(ops, M, plan):
     """A bounded wait made to run out, without a fault: the product is told to poll each barrier a few thousand
