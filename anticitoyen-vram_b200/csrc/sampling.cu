@@ -370,11 +370,11 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
 // on shared memory; what a pass counts is added up over the cluster through the CTAs' shared memory (every CTA
 // writes its part into every CTA's table, one cluster barrier, every CTA adds the parts in rank order, so all take
 // the same decision).  The arithmetic is sample_kernel's; sums are formed slice by slice.
+#define SMPC_CTAS 8
 #define SMPC_THREADS 1024
 
-template <int CTAS>
 struct ClusterSum {
-    float* parts;          // [2][CTAS] in this CTA's shared memory
+    float* parts;          // [2][SMPC_CTAS] in this CTA's shared memory
     float* warps;          // [32]
     float* table;          // [32][17]
     int turn;
@@ -382,8 +382,7 @@ struct ClusterSum {
 };
 
 // every thread gets the sum over the cluster of `v` (a float; counts up to 2^24 are exact)
-template <int CTAS>
-__device__ __forceinline__ float cluster_all_sum(ClusterSum<CTAS>& c, float v) {
+__device__ __forceinline__ float cluster_all_sum(ClusterSum& c, float v) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     v = warp_sum(v);
     if (lane == 0) c.warps[warp] = v;
@@ -391,18 +390,17 @@ __device__ __forceinline__ float cluster_all_sum(ClusterSum<CTAS>& c, float v) {
     if (warp == 0) {
         float t = lane < (int)(blockDim.x >> 5) ? c.warps[lane] : 0.f;
         t = warp_sum(t);
-        if (lane < CTAS)
-            cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(c.parts + c.turn * CTAS + c.rank), lane), t);
+        if (lane < SMPC_CTAS)
+            cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(c.parts + c.turn * SMPC_CTAS + c.rank), lane), t);
     }
     cluster_sync_all();
     float total = 0.f;
 #pragma unroll
-    for (int r = 0; r < CTAS; ++r) total += c.parts[c.turn * CTAS + r];
+    for (int r = 0; r < SMPC_CTAS; ++r) total += c.parts[c.turn * SMPC_CTAS + r];
     c.turn ^= 1;
     return total;
 }
-template <int CTAS>
-__device__ __forceinline__ float cluster_all_max(ClusterSum<CTAS>& c, float v) {
+__device__ __forceinline__ float cluster_all_max(ClusterSum& c, float v) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     v = warp_max(v);
     if (lane == 0) c.warps[warp] = v;
@@ -410,13 +408,13 @@ __device__ __forceinline__ float cluster_all_max(ClusterSum<CTAS>& c, float v) {
     if (warp == 0) {
         float t = lane < (int)(blockDim.x >> 5) ? c.warps[lane] : -INFINITY;
         t = warp_max(t);
-        if (lane < CTAS)
-            cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(c.parts + c.turn * CTAS + c.rank), lane), t);
+        if (lane < SMPC_CTAS)
+            cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(c.parts + c.turn * SMPC_CTAS + c.rank), lane), t);
     }
     cluster_sync_all();
     float total = -INFINITY;
 #pragma unroll
-    for (int r = 0; r < CTAS; ++r) total = fmaxf(total, c.parts[c.turn * CTAS + r]);
+    for (int r = 0; r < SMPC_CTAS; ++r) total = fmaxf(total, c.parts[c.turn * SMPC_CTAS + r]);
     c.turn ^= 1;
     return total;
 }
@@ -426,9 +424,9 @@ __device__ __forceinline__ float cluster_all_max(ClusterSum<CTAS>& c, float v) {
 // four, a thread's in registers; the bins are added up over warp, CTA and cluster (in an order that the launch shape
 // fixes), and the sums from the top down say which bin holds c.  A pass costs its meeting of the cluster, 2 us, so eight
 // passes of sixteen candidates replace 32 of one
-// (16 rows of 151 936, microseconds: top-p 215 -> 76, top-k 176 -> 58, both 330 -> 107).
-template <int CTAS, typename Element>
-__device__ __forceinline__ uint32_t cluster_descend(ClusterSum<CTAS>& c, float* bins, int n, float limit, bool above, Element element) {
+// (8 rows of 151 936, microseconds: top-p 141 -> 64, top-k 120 -> 49, both 199 -> 91).
+template <typename Element>
+__device__ __forceinline__ uint32_t cluster_descend(ClusterSum& c, float* bins, int n, float limit, bool above, Element element) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t prefix = 0;
     float over = 0.f;           // the sum over the elements whose bits so far are larger than c's
@@ -461,13 +459,13 @@ __device__ __forceinline__ uint32_t cluster_descend(ClusterSum<CTAS>& c, float* 
         __syncthreads();
         if (warp < 16) {        // warp d adds up bin d over the warps and tells every CTA
             const float t = warp_sum(c.table[lane * 17 + warp]);
-            if (lane < CTAS)
-                cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(bins + (c.turn * CTAS + c.rank) * 16 + warp), lane), t);
+            if (lane < SMPC_CTAS)
+                cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(bins + (c.turn * SMPC_CTAS + c.rank) * 16 + warp), lane), t);
         }
         cluster_sync_all();
         float s = 0.f;          // lane d: bin d, then the sum of the bins d and above
 #pragma unroll
-        for (int r = 0; r < CTAS; ++r) s += bins[(c.turn * CTAS + r) * 16 + (lane & 15)];
+        for (int r = 0; r < SMPC_CTAS; ++r) s += bins[(c.turn * SMPC_CTAS + r) * 16 + (lane & 15)];
         c.turn ^= 1;
 #pragma unroll
         for (int h = 1; h < 16; h <<= 1) {
@@ -484,22 +482,21 @@ __device__ __forceinline__ uint32_t cluster_descend(ClusterSum<CTAS>& c, float* 
     return prefix;
 }
 
-template <int CTAS>
 __global__ void __launch_bounds__(SMPC_THREADS)
 sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice, const float* __restrict__ temperature,
                       const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
                       const unsigned long long* __restrict__ seed, const unsigned long long* __restrict__ counter,
                       int* __restrict__ out_token, float* __restrict__ out_logprob) {
     extern __shared__ float sl[];               // this CTA's slice of the scaled logits, and behind it exp(logit - maximum)
-    __shared__ float parts[2 * CTAS], bins[2 * CTAS * 16];
+    __shared__ float parts[2 * SMPC_CTAS], bins[2 * SMPC_CTAS * 16];
     __shared__ float warps[32], table[32 * 17];
     __shared__ float scan[SMPC_THREADS];
-    __shared__ float bestv[2 * CTAS];
+    __shared__ float bestv[2 * SMPC_CTAS];
     __shared__ int owner_s;
     __shared__ float before_s, target_s;
-    ClusterSum<CTAS> cs;
+    ClusterSum cs;
     cs.parts = parts; cs.warps = warps; cs.table = table; cs.turn = 0; cs.rank = cluster_ctarank();
-    const int r = blockIdx.x / CTAS;
+    const int r = blockIdx.x / SMPC_CTAS;
     const float* row = logits + (size_t)r * ld;
     const int lo = (int)cs.rank * slice, hi = min(V, lo + slice), n = max(0, hi - lo);
     const float temp = temperature[r];
@@ -583,21 +580,21 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
         if (warp == 0) {
             float tot = lane < (int)(blockDim.x >> 5) ? warps[lane] : 0.f;
             tot = warp_sum(tot);
-            if (lane < CTAS)
+            if (lane < SMPC_CTAS)
                 cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(bestv + cs.rank), lane), tot);
         }
         cluster_sync_all();
     }
     float run = 0.f;
 #pragma unroll
-    for (int c = 0; c < CTAS; ++c) run += bestv[c];
+    for (int c = 0; c < SMPC_CTAS; ++c) run += bestv[c];
     const float u = philox_uniform(seed[r], counter[r]);
     const float target = u * run;
     // the CTA in which the target falls (the last CTA with anything kept, if rounding leaves the target beyond all)
     int owner_cta = -1, last_cta = 0;
     float acc = 0.f, before_cta = 0.f;
 #pragma unroll
-    for (int c = 0; c < CTAS; ++c) {
+    for (int c = 0; c < SMPC_CTAS; ++c) {
         if (bestv[c] > 0.f) last_cta = c;
         if (owner_cta < 0 && bestv[c] > 0.f && acc + bestv[c] >= target) { owner_cta = c; before_cta = acc; }
         if (owner_cta < 0) acc += bestv[c];
@@ -657,32 +654,22 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
     }
 }
 
-template <int CTAS>
-static int launch_sample_cluster(const float* logits, int ld, int rows, int V, const float* temperature, const int* top_k, const float* top_p,
-                                 const float* min_p, const unsigned long long* seed, const unsigned long long* counter, int* out_token,
-                                 float* out_logprob, cudaStream_t stream) {
-    const int slice = ((V + CTAS - 1) / CTAS + 3) & ~3, smem = 2 * slice * (int)sizeof(float);
-    static AcvSmemConfig smem_config;
-    if (int rc = acv_ensure_smem(smem_config, sample_cluster_kernel<CTAS>, smem)) return rc;
-    acv_launch_cluster(0, dim3(CTAS, 1, 1), sample_cluster_kernel<CTAS>, dim3((unsigned)rows * CTAS), dim3(SMPC_THREADS), (size_t)smem, stream,
-                       logits, ld, V, slice, temperature, top_k, top_p, min_p, seed, counter, out_token, out_logprob);
-    return acv_launch_status();
-}
-
 ACV_API int acv_sample(const float* logits, int ld, int rows, int V, const float* temperature, const int* top_k,
                        const float* top_p, const float* min_p, const unsigned long long* seed,
                        const unsigned long long* counter, int* out_token, float* out_logprob, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (V <= 0) return ACV_ERR_SIZE;
-    // Wide rows: a cluster of CTAs to a row, the row's slices (scaled logits and exponentials) in their shared memory, an SM to
-    // each CTA.  22 clusters of six fit the device at once, 15 of eight: six where the slices fit (16 rows of 151 936, top-p:
-    // 76 us in one wave instead of 122 in two; 64 rows 242 instead of 325; up to 15 rows 76 instead of 64), eight for longer rows.
-    // The choice follows V alone, as the order of the sums does: a draw does not depend on how many rows are drawn.
-    const auto fits = [&](int ctas) { return 2ll * (((V + ctas - 1) / ctas + 3) & ~3) * (int)sizeof(float) <= 203 * 1024; };
-    if (V >= 16384 && V < (1 << 24) && fits(6))
-        return launch_sample_cluster<6>(logits, ld, rows, V, temperature, top_k, top_p, min_p, seed, counter, out_token, out_logprob, stream);
-    if (V >= 16384 && V < (1 << 24) && fits(8))
-        return launch_sample_cluster<8>(logits, ld, rows, V, temperature, top_k, top_p, min_p, seed, counter, out_token, out_logprob, stream);
+    // wide rows: a cluster of CTAs to a row, the row's slices in their shared memory
+    const int slice = ((V + SMPC_CTAS - 1) / SMPC_CTAS + 3) & ~3;
+    const int smem = 2 * slice * (int)sizeof(float);
+    if (V >= 16384 && V < (1 << 24) && smem <= 200 * 1024) {
+        static AcvSmemConfig smem_config;
+        if (int rc = acv_ensure_smem(smem_config, sample_cluster_kernel, smem)) return rc;
+        acv_launch_cluster(0, dim3(SMPC_CTAS, 1, 1), sample_cluster_kernel, dim3((unsigned)rows * SMPC_CTAS), dim3(SMPC_THREADS),
+                           (size_t)smem, stream, logits, ld, V, slice, temperature, top_k, top_p, min_p, seed, counter,
+                           out_token, out_logprob);
+        return acv_launch_status();
+    }
     sample_kernel<<<rows, SMP_THREADS, 0, stream>>>(logits, ld, V, temperature, top_k, top_p, min_p, seed, counter,
                                                     out_token, out_logprob);
     return acv_launch_status();
