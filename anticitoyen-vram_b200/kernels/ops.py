@@ -382,6 +382,9 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
 _gemm_scratch: dict = {}
 
 
+GEMM_WORKSPACE_FLOATS = 1 << 22     # what every plan of a device of up to 256 SMs fits in, so that a capture never meets a larger one
+
+
 def _gemm_buffers(device, ws_floats: int, n_counters: int):
     key = str(device)
     have = _gemm_scratch.get(key)
@@ -389,7 +392,7 @@ def _gemm_buffers(device, ws_floats: int, n_counters: int):
         if torch.cuda.is_current_stream_capturing():
             raise KernelError("gemm_tc: workspace would grow during a graph capture; run the shape once first")
         old = have or (torch.empty(0), torch.empty(0), None)
-        ws = torch.empty(max(ws_floats, 2 * old[0].numel(), 1 << 20), device=device, dtype=torch.float32)
+        ws = torch.empty(max(ws_floats, 2 * old[0].numel(), GEMM_WORKSPACE_FLOATS), device=device, dtype=torch.float32)
         cnt = torch.zeros(max(n_counters, 2 * old[1].numel(), 4096), device=device, dtype=torch.int32)
         status = old[2] if old[2] is not None else torch.zeros(1, device=device, dtype=torch.int32)
         if key in _gemm_scratch:
@@ -508,17 +511,11 @@ def _gemm_tc_plan(M: int, N: int, K: int, sms: int, bn_multiple: int) -> tuple:
         return (1, 128, 2, 6) if wide <= 0.5 * sms else (1, 128, 1, 6)
     if N < 256:
         return 0, (128 if N > 64 else 64), 1, 8
-    if M > 128 and bn_multiple == 16 and n_kb >= 48:
+    if M > 128 and bn_multiple == 16 and n_kb >= 48 and -(-M // 128) * wide <= 0.5 * sms:
         # half of the SMs or fewer would have a tile: two CTAs of a cluster share one (256 tokens, microseconds: 4096 x 12288 63 -> 41,
-        # 2560 x 9728 50 -> 34, 4096 x 4096 24.5 -> 20.6), or with a long K and somewhat more tiles two CTAs through the
-        # workspace share a wider one (256 x 5120 x 17408 91 -> 61, 300 x 4096 x 12288 65 -> 49)
-        rows = -(-M // 128)
-        if rows * wide <= 0.5 * sms:
-            return 1, 128, 2, 6
-        if n_kb >= 128:
-            for bn in (160, 192):
-                if rows * -(-N // bn) <= 0.5 * sms:
-                    return 0, bn, 2, 8
+        # 2560 x 9728 50 -> 34, 4096 x 4096 24.5 -> 20.6).  With a few tiles more two CTAs could share a wider one through the
+        # workspace (256 x 5120 x 17408 91 -> 61), but its counters belong to the device and products of two streams would meet there.
+        return 1, 128, 2, 6
     best, best_cost = 256, None
     for bn in GEMM_TILE_WIDTHS:
         if bn % bn_multiple:

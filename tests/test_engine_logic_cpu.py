@@ -228,6 +228,21 @@ def test_the_plan_of_a_product_follows_its_shape():
     assert len(ops.gemm_tc_plan(2048, 4096, 4096, sms=1)) == 4
 
 
+@pytest.mark.parametrize("sms", [1, 74, 132, 148, 256])
+def test_split_products_share_nothing_between_streams(sms):
+    """Splits of K that a plan asks for are summed inside a cluster (8 CTAs and 100 KB of partial tiles at most), never through
+    the device's one workspace, and the workspace of the first call is large enough for every later one: a capture may
+    meet a shape that never ran before."""
+    from acvram_b200.kernels import ops
+    for M in (1, 16, 17, 32, 33, 64, 65, 128, 129, 256, 300, 512, 513, 1056):
+        for N in list(range(128, 128 * 600, 128 * 7)) + [200, 5120, 4096, 19000]:
+            for K in (64, 1024, 2048, 3072, 4096, 8192, 17408):
+                swap, bn, splits = ops.gemm_tc_plan(M, N, K, sms=sms)[:3]
+                if splits > 1:
+                    assert swap and splits <= 8 and (splits - 1) * bn * 128 * 4 <= 100 * 1024, (M, N, K)
+                    assert -(-N // 128) * -(-M // bn) * splits * bn * 128 <= ops.GEMM_WORKSPACE_FLOATS, (M, N, K)
+
+
 def test_the_splits_of_decode_attention_follow_what_fits_the_device(monkeypatch):
     """How the split-KV kernel cuts the context, for a device that holds 296 of its CTAs at once (stubbed: the real
     figure is asked of the runtime): a few long requests are split so far that a CTA's own streaming is short, many
