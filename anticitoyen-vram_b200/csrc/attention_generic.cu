@@ -163,6 +163,9 @@ __device__ __forceinline__ void ag_put(const AgArgs& a, int t, int h, int e, flo
     if (a.gate) o *= 1.f / (1.f + expf(-to_f32(((const T*)a.gate)[(size_t)t * a.gate_stride + (size_t)h * a.DV + e])));
     ((T*)a.out)[(size_t)t * a.out_stride + (size_t)h * a.DV + e] = from_f32<T>(o);
 }
+// a key's weight against the maximum so far: 0 for a score of -inf, whatever the maximum; a score that is no number (the
+// maximum passes it over) gives a weight that is none, and so does +inf: the sums and the result are none then
+__device__ __forceinline__ float ag_weight(float x, float m) { return x == -INFINITY ? 0.f : expf(x - m); }
 __device__ __forceinline__ float ag_peer(const float* local, int rank) {
     float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_map((uint32_t)__cvta_generic_to_shared(local), rank)) : "memory");
@@ -283,7 +286,7 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
                     const float x = seen ? s[i] - slope[i] * (float)(pos[i] - j) : -INFINITY;
                     const float m_new = fmaxf(m[i], warp_max(x));
                     const float alpha = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);
-                    const float w = seen ? expf(x - m_new) : 0.f;
+                    const float w = ag_weight(x, m_new);
                     l[i] = l[i] * alpha + w;            // a lane's share of the sum
                     m[i] = m_new;
 #pragma unroll
@@ -329,7 +332,7 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
                 f = expf(m[i] - m_new);
                 sum = sum * f + expf(sink - m_new);
             }
-            const float inv = sum > 0.f ? f / sum : 0.f;
+            const float inv = sum == 0.f ? 0.f : f / sum;
 #pragma unroll
             for (int c = 0; c < 4 * VC; ++c) {
                 const int e = (c / 4) * 128 + lane * 4 + c % 4;
@@ -434,7 +437,7 @@ attn_token_kernel(const AgArgs a, int parts, int only_alone) {
                 const float x = row >= 0 ? sm_w[warp][lane][r] - slope * (float)(p - j) : -INFINITY;
                 const float m_new = fmaxf(m[r], warp_max(x));
                 const float alpha = m_new == -INFINITY ? 1.f : expf(m[r] - m_new);
-                const float w = row >= 0 ? expf(x - m_new) : 0.f;
+                const float w = ag_weight(x, m_new);
                 l[r] = l[r] * alpha + w;
                 m[r] = m_new;
 #pragma unroll
@@ -504,10 +507,9 @@ attn_token_kernel(const AgArgs a, int parts, int only_alone) {
                 for (int c = 0; c < parts; ++c) mx = fmaxf(mx, ag_peer(tot_m + r, c));
                 for (int c = 0; c < parts; ++c) {
                     const float pm = ag_peer(tot_m + r, c), pl = ag_peer(tot_l + r, c), po = ag_peer(at_o + e, c);
-                    if (pm == -INFINITY) continue;
-                    const float f = expf(pm - mx);
+                    const float f = pm == -INFINITY ? 0.f : expf(pm - mx);
                     sum = fmaf(pl, f, sum);
-                    o = fmaf(po, f, o);
+                    if (f != 0.f) o = fmaf(po, f, o);
                 }
             }
             if (a.sinks) {
@@ -516,7 +518,7 @@ attn_token_kernel(const AgArgs a, int parts, int only_alone) {
                 sum = sum * f + expf(sink - m_new);
                 o *= f;
             }
-            ag_put<T>(a, t, h0 + r, e % DV, sum > 0.f ? o / sum : 0.f);
+            ag_put<T>(a, t, h0 + r, e % DV, sum == 0.f ? 0.f : o / sum);
         }
         if (parts > 1) cluster_sync_all();      // nobody leaves while its results are read
     }

@@ -262,6 +262,42 @@ def test_attention_generic_options(ops, dtype, q_lens, NH, NKV, D, DV, window, k
     torch.testing.assert_close(out.double(), want, **tol(dtype))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("q_lens,D", [((1, 1, 1), 64), ((1,) * 40, 64), ((70, 2), 64), ((70, 1, 1), 64), ((1, 70), 260)])
+def test_attention_generic_scores_that_are_no_finite_numbers(ops, dtype, q_lens, D):
+    """Infinities and NaN, for tokens one by one, for portions and for the general kernel (head size 260): a query or a key
+    that is no number, or a score of +inf, leaves a result that is none, in its own head and request alone; keys of score
+    -inf weigh nothing, be it one, a whole tile of keys or all of them (a result of zeros)."""
+    page, B, NH, NKV = 16, len(q_lens), 4, 2
+    lens = [100 + n for n in q_lens]
+    per = -(-max(lens) // page)
+    table = torch.arange(B * per, dtype=torch.int32).reshape(B, per).cuda()
+    k, v = rnd(B, per * page, NKV, D, dtype=dtype, seed=70), rnd(B, per * page, NKV, D, dtype=dtype, seed=71)
+    q = rnd(sum(q_lens), NH, D, dtype=dtype, seed=72)
+    q[:, :, 0] = q[:, :, 0].abs() + 0.1                # a key's first element decides the sign of an infinite score
+    first = [sum(q_lens[:b]) for b in range(B)]
+    q[first[0], 1, 5] = float("nan")                    # one query head of one token
+    k[0, 40, 1, 3] = float("nan")                       # one key of the other kv-head: every token behind it
+    k[1, 0:40, 0, 0] = -float("inf")                    # a tile and more
+    k[1, :, 1, 0] = -float("inf")                       # every key
+    if B > 2:
+        k[2, 50, 0, 0] = float("inf")
+        k[2, 64:96, 1, 0] = -float("inf")
+    pages = lambda x: x.reshape(B * per, page, NKV, D).transpose(1, 2).contiguous()
+    pos = torch.cat([torch.arange(l - n, l) for l, n in zip(lens, q_lens)]).to(torch.int32).cuda()
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(q_lens)).to(torch.int32).cuda()
+    out = torch.full((sum(q_lens), NH * D), 7.0, device="cuda", dtype=dtype)
+    ops.attention_generic(q.reshape(-1, NH * D), out, pages(k), pages(v), pos, seq, table, NH, NKV, D, D ** -0.5)
+    for b in range(B):
+        rows = slice(first[b], first[b] + q_lens[b])
+        kk, vv = (x[b].double().repeat_interleave(NH // NKV, 1) for x in (k, v))
+        s = torch.einsum("qhd,khd->hqk", q[rows].double(), kk) * D ** -0.5
+        s = s.masked_fill(torch.arange(per * page, device="cuda") > pos[rows, None], -float("inf"))
+        want = torch.einsum("hqk,khd->qhd", s.softmax(-1), vv)
+        want[(s == -float("inf")).all(-1).T] = 0.0
+        torch.testing.assert_close(out[rows].double(), want.reshape(-1, NH * D), equal_nan=True, **tol(dtype))
+
+
 @pytest.mark.parametrize("in_dtype,out_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32),
                                                 (torch.bfloat16, torch.bfloat16)])
 @pytest.mark.parametrize("M,N,K", [(1, 331, 80), (7, 100, 72), (65, 130, 200), (3, 1000, 4096), (128, 64, 16)])
