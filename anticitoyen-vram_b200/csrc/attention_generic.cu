@@ -19,8 +19,9 @@
 // attn_token_kernel: the query heads of one token and kv-head against its keys, which 8 warps and up to 8 CTAs share, for
 // requests that bring one token and for steps of a few tokens.  attn_generic_kernel: one warp per (token, head), for head
 // sizes over 256 or of no 4-element pieces.  In a step of many tokens the first two run one after the other and each
-// leaves the other's tokens alone.  Measured in float32 with 16 heads on 8 kv-heads of 128 (microseconds, one warp per
-// (token, head) before -> now): 696 tokens of three portions 825 -> 130, 3 tokens at contexts of 300-500 429 -> 22.
+// leaves the other's tokens alone.  Both have one order of sums (below), so a token's result does not depend on the rest of
+// the step.  Measured in float32 with 16 heads on 8 kv-heads of 128 (microseconds, one warp per
+// (token, head) before -> now): 696 tokens of three portions 831 -> 119, 3 tokens at contexts of 300-500 256 -> 20.
 #include "common.cuh"
 #include <type_traits>
 
@@ -132,12 +133,25 @@ __global__ void attn_generic_kernel(const T* __restrict__ q, int q_stride, T* __
 }
 
 // ----------------------------------------------------------------------------- shared by the two tiled kernels
+// One order of sums.  What a (token, head) comes to depends on its position, its options and its keys alone: not on the
+// other tokens of the step, on how a prompt was cut into portions, or on which of the two kernels, how many warps or how many
+// CTAs computed it.  The keys lie in tiles of 32 at absolute positions (key % 32 is the lane), of which a token visits
+// those with a key that it may see (AgTiles), in ascending order; what it does not see in them weighs 0 and leaves every
+// number as it is.  A score is eight chains of multiply-adds (elements whose number / 4 is the same modulo 8, ascending)
+// added one by one, ascending.  Up to AgArgs::chunks chunks of consecutive tiles (as even as whole tiles allow, by the number of
+// tiles alone) each have a running maximum, a sum per lane and a value sum of their own, ascending over the keys
+// (ag_weight), and are added to the total one by one, ascending, rescaled to the larger maximum (ag_fold).  So the rows of
+// a portion add a chunk to their totals when it ends, and a token's warps keep theirs until the last is there: 64 chunks
+// where two CTAs' worth of them fits an SM beside each other, else 32 (more than one long context's 64 warps could share
+// are no use; three tokens at 8000 keys take 140 us with 64, 272 with 32).
+#define AG_CHUNKS(rg, vc) ((rg) * (vc) <= 2 ? 64 : 32)
+
 struct AgArgs {
     const void *q, *k_pages, *v_pages, *gate;
     void* out;
     const int *positions, *seq_of_token, *block_table, *bt_rows;
     const float *sinks, *slopes;
-    int q_stride, out_stride, gate_stride, bt_stride, T, NH, NKV, D, DV, page_size, num_pages, window, keep_first, v_row;
+    int q_stride, out_stride, gate_stride, bt_stride, T, NH, NKV, D, DV, page_size, num_pages, window, keep_first, v_row, chunks;
     float scale;
 };
 
@@ -146,6 +160,10 @@ __device__ __forceinline__ float4 ag_load4(const bf16* p) {
     const uint2 u = *reinterpret_cast<const uint2*>(p);
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
 }
+__device__ __forceinline__ float4 ag_scale4(float4 v, float f) {
+    return make_float4(__fmul_rn(v.x, f), __fmul_rn(v.y, f), __fmul_rn(v.z, f), __fmul_rn(v.w, f));
+}
+__device__ __forceinline__ float ag_dot4(float4 q, float4 k, float s) { return fmaf(q.w, k.w, fmaf(q.z, k.z, fmaf(q.y, k.y, fmaf(q.x, k.x, s)))); }
 // a token whose neighbours in the batch belong to other requests
 __device__ __forceinline__ bool ag_alone(const int* seq, int t, int T) {
     return (t == 0 || seq[t - 1] != seq[t]) && (t + 1 >= T || seq[t + 1] != seq[t]);
@@ -166,6 +184,34 @@ __device__ __forceinline__ void ag_put(const AgArgs& a, int t, int h, int e, flo
 // a key's weight against the maximum so far: 0 for a score of -inf, whatever the maximum; a score that is no number (the
 // maximum passes it over) gives a weight that is none, and so does +inf: the sums and the result are none then
 __device__ __forceinline__ float ag_weight(float x, float m) { return x == -INFINITY ? 0.f : expf(x - m); }
+__device__ __forceinline__ float ag_rescale(float from, float to) { return to == -INFINITY ? 1.f : expf(from - to); }
+// total + chunk under the factors of their maxima (a factor of 0 must not meet a sum that is no finite number)
+__device__ __forceinline__ float ag_fold(float total, float fa, float chunk, float fb) {
+    return fmaf(fa == 0.f ? 0.f : total, fa, fb == 0.f ? 0.f : __fmul_rn(chunk, fb));
+}
+// what the total is multiplied by: a sink is a score without key or value, it takes its share of the weights and adds nothing
+__device__ __forceinline__ float ag_inverse(const AgArgs& a, int h, float m, float sum) {
+    float f = 1.f;
+    if (a.sinks) {
+        const float sink = a.sinks[h], m_new = fmaxf(m, sink);
+        f = expf(m - m_new);
+        sum = fmaf(sum, f, expf(sink - m_new));
+    }
+    return sum == 0.f ? 0.f : f / sum;
+}
+// the tiles of a token at position p: [0, kept) for the first keys that stay visible, then [from, last], n in all
+struct AgTiles { int kept, from, last, n; };
+__device__ __forceinline__ AgTiles ag_tiles(const AgArgs& a, int p) {
+    AgTiles t = {0, 0, -1, 0};
+    if (p < 0) return t;
+    const int lo = a.window > 0 ? max(0, p - a.window + 1) : 0;
+    t.kept = a.window > 0 ? (min(max(a.keep_first, 0), lo) + 31) / 32 : 0;
+    t.from = max(lo / 32, t.kept);
+    t.last = p / 32;
+    t.kept = min(t.kept, t.last + 1);
+    t.n = t.kept + max(0, t.last - t.from + 1);
+    return t;
+}
 __device__ __forceinline__ float ag_peer(const float* local, int rank) {
     float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_map((uint32_t)__cvta_generic_to_shared(local), rank)) : "memory");
@@ -175,14 +221,33 @@ __device__ __forceinline__ float ag_peer(const float* local, int rank) {
 // ----------------------------------------------------------------------------- rows of a portion
 // A CTA: 64 / (NH/NKV) tokens of the flat batch times the heads of one kv-head, eight rows to a warp; the requests among
 // the tokens one after the other (a tile of a portion has one).  Scores: a lane a key, so a 16-byte read of 32 key rows
-// moves 512 different bytes and a row's queries are one address; values: a lane four columns.  Bound by the chains of
+// moves 512 different bytes and a row's queries are one address; values: a lane four columns.  What belongs to a row (its
+// tiles, maximum and total) lies in the lanes 4 i to 4 i + 3 for row i of the warp, so that eight rows' maxima and sums over
+// the lanes take nine exchanges instead of forty.  Bound by the chains of
 // shared-memory reads (9 to 32 multiply-adds of a warp for the scores), hence eight rows a warp and not fewer: 32 rows and
-// four warps to a CTA were slower (156 against 125 us, 696 tokens of three portions), and so was bringing the next tile
-// under this one's arithmetic (144 us: its registers are what the reads are hidden with).
+// four warps to a CTA were slower (156 against 125 us in the form before this one, 696 tokens of three portions), and so was
+// bringing the next tile under this one's arithmetic (144 us: its registers are what the reads are hidden with).  The one
+// order of sums (eight chains to a score, totals in shared memory, tiles at absolute positions) costs 4 % behind 3000 keys
+// (1453 -> 1505 us for 1000 tokens) and one more tile behind a window; shorter prompts are none the worse (130 -> 119).
 #define AR_ROWS 64
 #define AR_KEYS 32
 #define AR_WARP_ROWS 8
 #define AR_THREADS 256
+
+// eight values a lane -> lane l: value l / 4 over all lanes, pairs of lanes 16 apart first, then 8, 4, 2, 1 (warp_sum's order)
+template <bool MAX>
+__device__ __forceinline__ float ar_over_lanes(const float (&v)[AR_WARP_ROWS], int lane) {
+    auto join = [](float x, float y) { return MAX ? fmaxf(x, y) : x + y; };
+    float w[4];
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = join(h16 ? v[i + 4] : v[i], __shfl_xor_sync(0xffffffffu, h16 ? v[i] : v[i + 4], 16));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) w[i] = join(h8 ? w[i + 2] : w[i], __shfl_xor_sync(0xffffffffu, h8 ? w[i] : w[i + 2], 8));
+    float x = join(h4 ? w[1] : w[0], __shfl_xor_sync(0xffffffffu, h4 ? w[0] : w[1], 4));
+    x = join(x, __shfl_xor_sync(0xffffffffu, x, 2));
+    return join(x, __shfl_xor_sync(0xffffffffu, x, 1));
+}
 
 template <typename T, int VC>       // VC: runs of 128 value columns
 __global__ void __launch_bounds__(AR_THREADS, VC == 1 ? 2 : 1)
@@ -194,6 +259,7 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
     float* ks = qs + AR_ROWS * ldk;                 // [32][D + 4]
     float* vs = ks + AR_KEYS * ldk;                 // [32][DV]
     float* ps = vs + AR_KEYS * DV;                  // [8 warps][32 keys][8 rows]
+    float* ts = ps + AR_ROWS * AR_KEYS;             // [64][DV]: the rows' totals
     pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int kvh = blockIdx.y, h0 = kvh * G + blockIdx.z * heads, n_heads = min(heads, G - (int)blockIdx.z * heads);
@@ -211,132 +277,198 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
         for (int i = tid; i < AR_ROWS * (D / 4); i += AR_THREADS) {
             const int r = i / (D / 4), c = (i % (D / 4)) * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < rows) {
-                v = ag_load4((const T*)a.q + (size_t)(t0 + r / n_heads) * a.q_stride + (size_t)(h0 + r % n_heads) * D + c);
-                v.x *= a.scale; v.y *= a.scale; v.z *= a.scale; v.w *= a.scale;
-            }
+            if (r < rows) v = ag_scale4(ag_load4((const T*)a.q + (size_t)(t0 + r / n_heads) * a.q_stride + (size_t)(h0 + r % n_heads) * D + c), a.scale);
             *reinterpret_cast<float4*>(qs + r * ldk + c) = v;
         }
-        int lo = 0x7fffffff, last = -1, hi_lo = 0;      // keys any row sees: [lo, last], and the kept first ones before lo
+        // the tiles that any row visits
+        int kept_tiles = 0, from = 0x7fffffff, last = -1, last_key = -1;
         for (int t = t0; t < t1; ++t) {
-            const int p = a.positions[t], l = a.window > 0 ? max(0, p - a.window + 1) : 0;
-            lo = min(lo, l); last = max(last, p); hi_lo = max(hi_lo, l);
+            const int p = a.positions[t];
+            const AgTiles u = ag_tiles(a, p);
+            if (u.n == 0) continue;
+            kept_tiles = max(kept_tiles, u.kept);
+            from = min(from, u.from);
+            last = max(last, u.last);
+            last_key = max(last_key, p);
         }
-        const int kept = a.window > 0 ? min(min(max(a.keep_first, 0), hi_lo), lo) : 0;
+        from = max(min(from, last + 1), kept_tiles);
         const int r0 = warp * AR_WARP_ROWS;
         int pos[AR_WARP_ROWS];
-        float slope[AR_WARP_ROWS], m[AR_WARP_ROWS], l[AR_WARP_ROWS];
-        float acc[AR_WARP_ROWS][4 * VC];
+        float l[AR_WARP_ROWS], acc[AR_WARP_ROWS][4 * VC];
 #pragma unroll
         for (int i = 0; i < AR_WARP_ROWS; ++i) {
-            const bool in = r0 + i < rows;
-            pos[i] = in ? a.positions[t0 + (r0 + i) / n_heads] : -1;
-            slope[i] = in && a.slopes ? a.slopes[h0 + (r0 + i) % n_heads] : 0.f;
-            m[i] = -INFINITY; l[i] = 0.f;
+            pos[i] = r0 + i < rows ? a.positions[t0 + (r0 + i) / n_heads] : -1;
+            l[i] = 0.f;
 #pragma unroll
             for (int c = 0; c < 4 * VC; ++c) acc[i][c] = 0.f;
+#pragma unroll
+            for (int c = 0; c < VC; ++c)
+                if (c * 128 + lane * 4 < DV) *reinterpret_cast<float4*>(ts + (r0 + i) * DV + c * 128 + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        for (int run = kept > 0 ? 0 : 1; run < 2; ++run) {
-            const int j_end = run == 0 ? kept : last + 1;
-            for (int j0 = run == 0 ? 0 : lo; j0 < j_end; j0 += AR_KEYS) {
-                const int nk = min(AR_KEYS, j_end - j0);
-                // a lane looks up one key's row; a warp brings every eighth key, all of its loads on their way together
-                const long long my_row = lane < nk ? ag_row(a, bt, kvh, j0 + lane) : -1;
-                float4 kx[AR_KEYS / 8][VC], vx[AR_KEYS / 8][VC];
-                bool odd = false;       // a value that is no finite number: a weight of 0 must not meet it
+        // this lane's row
+        const int my = r0 + lane / 4;
+        const AgTiles mt = ag_tiles(a, my < rows ? a.positions[t0 + my / n_heads] : -1);
+        float m = -INFINITY, total_m = -INFINITY, total_l = 0.f;
+        int filled = 0;             // a.chunks times the tiles of the chunk so far, modulo n
+
+        // a lane looks up one key's row, a tile ahead of its use
+        auto look_up = [&](int tile) {
+            const int j = tile * AR_KEYS + lane;
+            return tile <= last && j <= last_key ? ag_row(a, bt, kvh, j) : -1ll;
+        };
+        long long next_row = look_up(kept_tiles > 0 ? 0 : from);
+        for (int tile = kept_tiles > 0 ? 0 : from; tile <= last; tile = tile + 1 == kept_tiles ? from : tile + 1) {
+            const int j0 = tile * AR_KEYS, nk = min(AR_KEYS, last_key + 1 - j0);
+            // a warp brings every eighth key, all of its loads on their way together
+            const long long my_row = next_row;
+            next_row = look_up(tile + 1 == kept_tiles ? from : tile + 1);
+            float4 kx[AR_KEYS / 8][VC], vx[AR_KEYS / 8][VC];
+            bool odd = false;       // a value that is no finite number: a weight of 0 must not meet it
 #pragma unroll
-                for (int i = 0; i < AR_KEYS / 8; ++i) {
-                    const long long row = __shfl_sync(0xffffffffu, my_row, i * 8 + warp);
+            for (int i = 0; i < AR_KEYS / 8; ++i) {
+                const long long row = __shfl_sync(0xffffffffu, my_row, i * 8 + warp);
 #pragma unroll
-                    for (int c = 0; c < VC; ++c) {
-                        const int e = c * 128 + lane * 4;
-                        kx[i][c] = row >= 0 && e < D ? ag_load4((const T*)a.k_pages + row * D + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        vx[i][c] = row >= 0 && e < DV ? ag_load4((const T*)a.v_pages + row * a.v_row + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
+                for (int c = 0; c < VC; ++c) {
+                    const int e = c * 128 + lane * 4;
+                    kx[i][c] = row >= 0 && e < D ? ag_load4((const T*)a.k_pages + row * D + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    vx[i][c] = row >= 0 && e < DV ? ag_load4((const T*)a.v_pages + row * a.v_row + e) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
-                __syncthreads();        // the tile before is done with
+            }
+            __syncthreads();        // the tile before is done with
 #pragma unroll
-                for (int i = 0; i < AR_KEYS / 8; ++i)
+            for (int i = 0; i < AR_KEYS / 8; ++i)
 #pragma unroll
-                    for (int c = 0; c < VC; ++c) {
-                        const int e = c * 128 + lane * 4;
-                        const float4 v = vx[i][c];
-                        odd |= !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY);
-                        if (e < D) *reinterpret_cast<float4*>(ks + (i * 8 + warp) * ldk + e) = kx[i][c];
-                        if (e < DV) *reinterpret_cast<float4*>(vs + (i * 8 + warp) * DV + e) = v;
-                    }
-                odd = __syncthreads_or(odd);
-                float s[AR_WARP_ROWS];
-#pragma unroll
-                for (int i = 0; i < AR_WARP_ROWS; ++i) s[i] = 0.f;
-#pragma unroll 4
-                for (int d = 0; d < D; d += 4) {
-                    const float4 k = *reinterpret_cast<const float4*>(ks + lane * ldk + d);
-#pragma unroll
-                    for (int i = 0; i < AR_WARP_ROWS; ++i) {
-                        const float4 q = *reinterpret_cast<const float4*>(qs + (r0 + i) * ldk + d);
-                        s[i] = fmaf(q.x, k.x, s[i]); s[i] = fmaf(q.y, k.y, s[i]);
-                        s[i] = fmaf(q.z, k.z, s[i]); s[i] = fmaf(q.w, k.w, s[i]);
-                    }
+                for (int c = 0; c < VC; ++c) {
+                    const int e = c * 128 + lane * 4;
+                    const float4 v = vx[i][c];
+                    odd |= !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY);
+                    if (e < D) *reinterpret_cast<float4*>(ks + (i * 8 + warp) * ldk + e) = kx[i][c];
+                    if (e < DV) *reinterpret_cast<float4*>(vs + (i * 8 + warp) * DV + e) = v;
                 }
-                const int j = j0 + lane;
+            odd = __syncthreads_or(odd);
+            if (r0 >= rows) continue;           // (a warp without rows brings its keys and no more)
+            float s[AR_WARP_ROWS];
+#pragma unroll
+            for (int i = 0; i < AR_WARP_ROWS; ++i) s[i] = 0.f;
+            auto score = [&](auto pieces) {     // a row's pieces of 32 elements, or 0: as many as there are, the last not whole
+#pragma unroll 1
+                for (int chain = 0; chain < 32; chain += 4) {
+                    float x[AR_WARP_ROWS];
+#pragma unroll
+                    for (int i = 0; i < AR_WARP_ROWS; ++i) x[i] = 0.f;
+                    auto piece = [&](int d) {
+                        const float4 k = *reinterpret_cast<const float4*>(ks + lane * ldk + d);
+#pragma unroll
+                        for (int i = 0; i < AR_WARP_ROWS; ++i) x[i] = ag_dot4(*reinterpret_cast<const float4*>(qs + (r0 + i) * ldk + d), k, x[i]);
+                    };
+                    if constexpr (decltype(pieces)::value > 0) {
+#pragma unroll
+                        for (int c = 0; c < decltype(pieces)::value; ++c) piece(chain + c * 32);
+                    } else {
+                        for (int d = chain; d < D; d += 32) piece(d);
+                    }
+#pragma unroll
+                    for (int i = 0; i < AR_WARP_ROWS; ++i) s[i] += x[i];
+                }
+            };
+            if (D == 128 * VC) score(std::integral_constant<int, 4 * VC>());
+            else if (D == 64) score(std::integral_constant<int, 2>());
+            else score(std::integral_constant<int, 0>());
+            const int j = j0 + lane;
+#pragma unroll
+            for (int i = 0; i < AR_WARP_ROWS; ++i) {
+                if (a.slopes && r0 + i < rows) s[i] = fmaf(-a.slopes[h0 + (r0 + i) % n_heads], (float)(pos[i] - j), s[i]);
+                if (my_row < 0 || !ag_sees(a, pos[i], j)) s[i] = -INFINITY;
+            }
+            const float m_new = fmaxf(m, ar_over_lanes<true>(s, lane)), alpha = ag_rescale(m, m_new);
+            if (__any_sync(0xffffffffu, alpha != 1.f && m != -INFINITY)) {     // (a chunk's first tile finds sums of 0)
 #pragma unroll
                 for (int i = 0; i < AR_WARP_ROWS; ++i) {
-                    const bool seen = my_row >= 0 && ag_sees(a, pos[i], j);
-                    const float x = seen ? s[i] - slope[i] * (float)(pos[i] - j) : -INFINITY;
-                    const float m_new = fmaxf(m[i], warp_max(x));
-                    const float alpha = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);
-                    const float w = ag_weight(x, m_new);
-                    l[i] = l[i] * alpha + w;            // a lane's share of the sum
-                    m[i] = m_new;
+                    const float f = __shfl_sync(0xffffffffu, alpha, i * 4);
+                    l[i] = __fmul_rn(l[i], f);
 #pragma unroll
-                    for (int c = 0; c < 4 * VC; ++c) acc[i][c] *= alpha;
-                    s[i] = w;
+                    for (int c = 0; c < 4 * VC; ++c) acc[i][c] *= f;
                 }
-                *reinterpret_cast<float4*>(pw + lane * 8) = make_float4(s[0], s[1], s[2], s[3]);
-                *reinterpret_cast<float4*>(pw + lane * 8 + 4) = make_float4(s[4], s[5], s[6], s[7]);
-                __syncwarp();
-                auto weigh = [&](auto guard) {
+            }
+            m = m_new;
 #pragma unroll
-                    for (int c = 0; c < VC; ++c) {
-                        const int col = c * 128 + lane * 4;
-                        if (col >= DV) continue;
+            for (int i = 0; i < AR_WARP_ROWS; ++i) {
+                s[i] = ag_weight(s[i], __shfl_sync(0xffffffffu, m_new, i * 4));
+                l[i] = __fadd_rn(l[i], s[i]);             // a lane's share of the sum
+            }
+            *reinterpret_cast<float4*>(pw + lane * 8) = make_float4(s[0], s[1], s[2], s[3]);
+            *reinterpret_cast<float4*>(pw + lane * 8 + 4) = make_float4(s[4], s[5], s[6], s[7]);
+            __syncwarp();
+            auto weigh = [&](auto guard) {
+#pragma unroll
+                for (int c = 0; c < VC; ++c) {
+                    const int col = c * 128 + lane * 4;
+                    if (col >= DV) continue;
 #pragma unroll 4
-                        for (int k = 0; k < nk; ++k) {
-                            const float4 v = *reinterpret_cast<const float4*>(vs + k * DV + col);
-                            const float4 w0 = *reinterpret_cast<const float4*>(pw + k * 8), w1 = *reinterpret_cast<const float4*>(pw + k * 8 + 4);
-                            const float w[AR_WARP_ROWS] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                    for (int k = 0; k < nk; ++k) {
+                        const float4 v = *reinterpret_cast<const float4*>(vs + k * DV + col);
+                        const float4 w0 = *reinterpret_cast<const float4*>(pw + k * 8), w1 = *reinterpret_cast<const float4*>(pw + k * 8 + 4);
+                        const float w[AR_WARP_ROWS] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-                            for (int i = 0; i < AR_WARP_ROWS; ++i) {
-                                if (decltype(guard)::value && w[i] == 0.f) continue;
-                                acc[i][c * 4 + 0] = fmaf(w[i], v.x, acc[i][c * 4 + 0]);
-                                acc[i][c * 4 + 1] = fmaf(w[i], v.y, acc[i][c * 4 + 1]);
-                                acc[i][c * 4 + 2] = fmaf(w[i], v.z, acc[i][c * 4 + 2]);
-                                acc[i][c * 4 + 3] = fmaf(w[i], v.w, acc[i][c * 4 + 3]);
-                            }
+                        for (int i = 0; i < AR_WARP_ROWS; ++i) {
+                            if (decltype(guard)::value && w[i] == 0.f) continue;
+                            acc[i][c * 4 + 0] = fmaf(w[i], v.x, acc[i][c * 4 + 0]);
+                            acc[i][c * 4 + 1] = fmaf(w[i], v.y, acc[i][c * 4 + 1]);
+                            acc[i][c * 4 + 2] = fmaf(w[i], v.z, acc[i][c * 4 + 2]);
+                            acc[i][c * 4 + 3] = fmaf(w[i], v.w, acc[i][c * 4 + 3]);
                         }
                     }
-                };
-                if (odd) weigh(std::true_type()); else weigh(std::false_type());
-                __syncwarp();
+                }
+            };
+            if (odd) weigh(std::true_type()); else weigh(std::false_type());
+            __syncwarp();
+            // rows whose chunk this tile ends
+            bool ends = false;
+            if (tile < mt.kept || (tile >= mt.from && tile <= mt.last)) {
+                filled += a.chunks;
+                ends = filled >= mt.n;
+                if (ends) filled -= mt.n;
+            }
+            const uint32_t ending = __ballot_sync(0xffffffffu, ends);
+            if (ending) {
+                const float sum = ar_over_lanes<false>(l, lane), both = fmaxf(total_m, m);
+                const float fa = ag_rescale(total_m, both), fb = ag_rescale(m, both);
+                if (ends) { total_l = fmaf(total_l, fa, __fmul_rn(sum, fb)); total_m = both; m = -INFINITY; }
+#pragma unroll
+                for (int i = 0; i < AR_WARP_ROWS; ++i) {
+                    const float ga = __shfl_sync(0xffffffffu, fa, i * 4), gb = __shfl_sync(0xffffffffu, fb, i * 4);
+                    if (!(ending >> (i * 4) & 1)) continue;
+                    l[i] = 0.f;
+#pragma unroll
+                    for (int c = 0; c < VC; ++c) {
+                        float4* at = reinterpret_cast<float4*>(ts + (r0 + i) * DV + c * 128 + lane * 4);
+                        const bool in = c * 128 + lane * 4 < DV;
+                        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (ga != 0.f && in) o = *at;       // (ag_fold's ways, one at a time; the first chunk's ga is 0)
+                        if (gb == 0.f) acc[i][c * 4] = acc[i][c * 4 + 1] = acc[i][c * 4 + 2] = acc[i][c * 4 + 3] = 0.f;
+                        o.x = fmaf(o.x, ga, __fmul_rn(acc[i][c * 4], gb)); o.y = fmaf(o.y, ga, __fmul_rn(acc[i][c * 4 + 1], gb));
+                        o.z = fmaf(o.z, ga, __fmul_rn(acc[i][c * 4 + 2], gb)); o.w = fmaf(o.w, ga, __fmul_rn(acc[i][c * 4 + 3], gb));
+                        if (in) *at = o;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[i][c * 4 + e] = 0.f;
+                    }
+                }
             }
         }
+        const float my_inv = my < rows ? ag_inverse(a, h0 + my % n_heads, total_m, total_l) : 0.f;
 #pragma unroll
         for (int i = 0; i < AR_WARP_ROWS; ++i) {
+            const float inv = __shfl_sync(0xffffffffu, my_inv, i * 4);
             const int r = r0 + i;
-            float sum = warp_sum(l[i]), f = 1.f;
             if (r >= rows) continue;
-            const int t = t0 + r / n_heads, h = h0 + r % n_heads;
-            if (a.sinks) {      // a score without key or value: it takes its share of the weights and adds nothing
-                const float sink = a.sinks[h], m_new = fmaxf(m[i], sink);
-                f = expf(m[i] - m_new);
-                sum = sum * f + expf(sink - m_new);
-            }
-            const float inv = sum == 0.f ? 0.f : f / sum;
 #pragma unroll
-            for (int c = 0; c < 4 * VC; ++c) {
-                const int e = (c / 4) * 128 + lane * 4 + c % 4;
-                if (e < DV) ag_put<T>(a, t, h, e, acc[i][c] * inv);
+            for (int c = 0; c < VC; ++c) {
+                const int e = c * 128 + lane * 4;
+                if (e >= DV) continue;
+                const float4 o = *reinterpret_cast<const float4*>(ts + r * DV + e);
+                const int t = t0 + r / n_heads, h = h0 + r % n_heads;
+                ag_put<T>(a, t, h, e, __fmul_rn(o.x, inv)); ag_put<T>(a, t, h, e + 1, __fmul_rn(o.y, inv));
+                ag_put<T>(a, t, h, e + 2, __fmul_rn(o.z, inv)); ag_put<T>(a, t, h, e + 3, __fmul_rn(o.w, inv));
             }
         }
         t0 = t1;
@@ -345,19 +477,22 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
 }
 
 // ----------------------------------------------------------------------------- one token
-// A cluster of CTAs shares the keys of one token and kv-head, its 8 warps take batches of 32 keys in turn: eight lanes to a
-// key for the scores (four keys a load), a lane four columns for the values; RG query heads ride on each key and value
-// that is read.  Bound by the pages' stream and its latency.  The warps' partial results meet in shared memory, the CTAs'
-// in rank order through the cluster's.
+// A cluster of CTAs shares the chunks of one token and kv-head, each of its warps consecutive ones: eight lanes to a key for
+// the scores (four keys a load), a lane four columns for the values; RG query heads ride on each key and value
+// that is read.  Bound by the pages' stream and its latency.  The chunks' results wait in the CTAs' shared memory; each CTA
+// then adds up its share of the columns over all of them.
 #define AT1_WARPS 8
 #define AG_STRIDE 8      // tokens that a CTA looks at in a step of many tokens
 
 template <typename T, int RG, int VC>
-__global__ void __launch_bounds__(AT1_WARPS * 32)
+__global__ void __launch_bounds__(AT1_WARPS * 32, RG * VC == 1 ? 3 : 2)
 attn_token_kernel(const AgArgs a, int parts, int only_alone) {
-    __shared__ float sm_m[AT1_WARPS][RG], sm_l[AT1_WARPS][RG], tot_m[RG], tot_l[RG];
-    __shared__ __align__(16) float sm_w[AT1_WARPS][32][RG];
-    extern __shared__ __align__(16) float at_o[];      // [8 warps][RG][DV], then [RG][DV] of the CTA in front
+    constexpr int CHUNKS = AG_CHUNKS(RG, VC);
+    __shared__ float sm_m[CHUNKS][RG], sm_l[CHUNKS][RG];                        // this CTA's chunks
+    __shared__ float fac_a[RG][CHUNKS], fac_b[RG][CHUNKS], head_inv[RG];        // all chunks' factors, once all are there
+    __shared__ uint32_t chunk_at[CHUNKS];                                       // and where their value sums lie
+    __shared__ __align__(16) float sm_w[AT1_WARPS][32][RG], sm_s[AT1_WARPS][RG][32 * 8];
+    extern __shared__ __align__(16) float at_o[];      // [CHUNKS / parts][RG][DV]
     pdl_launch_dependents();
     pdl_wait();
     const int D = a.D, DV = a.DV, G = a.NH / a.NKV;
@@ -377,9 +512,11 @@ attn_token_kernel(const AgArgs a, int parts, int only_alone) {
         if (only_alone) __syncthreads();        // the token before is done with the shared memory
         const int p = a.positions[t], seq = a.seq_of_token[t];
         const int* bt = a.block_table + (size_t)(a.bt_rows ? a.bt_rows[seq] : seq) * a.bt_stride;
-        const int lo = a.window > 0 ? max(0, p - a.window + 1) : 0;
-        const int kept = a.window > 0 ? min(max(a.keep_first, 0), lo) : 0;
-        const int total = kept + p + 1 - lo;        // visible keys: the kept first ones, then [lo, p]
+        const AgTiles mt = ag_tiles(a, p);
+        // chunk c: the tiles whose number among the visited ones lies in [c n / n_chunks, (c + 1) n / n_chunks)
+        const int n_chunks = min(mt.n, CHUNKS);
+        const int gw = part * AT1_WARPS + warp, GW = parts * AT1_WARPS;
+        const int c_begin = gw * n_chunks / GW, c_end = (gw + 1) * n_chunks / GW, c_base = part * n_chunks / parts;
 
         // queries: lane `sub` of a key's eight holds elements sub*4 + 32 c
         constexpr int QC = VC * 4;
@@ -390,135 +527,144 @@ attn_token_kernel(const AgArgs a, int parts, int only_alone) {
             for (int c = 0; c < QC; ++c) {
                 const int e = sub * 4 + 32 * c;
                 q[r][c] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (r < n_heads && e < D) {
-                    q[r][c] = ag_load4((const T*)a.q + (size_t)t * a.q_stride + (size_t)(h0 + r) * D + e);
-                    q[r][c].x *= a.scale; q[r][c].y *= a.scale; q[r][c].z *= a.scale; q[r][c].w *= a.scale;
-                }
+                if (r < n_heads && e < D) q[r][c] = ag_scale4(ag_load4((const T*)a.q + (size_t)t * a.q_stride + (size_t)(h0 + r) * D + e), a.scale);
             }
         float m[RG], l[RG], acc[RG][4 * VC];
-#pragma unroll
-        for (int r = 0; r < RG; ++r) {
-            m[r] = -INFINITY; l[r] = 0.f;
-#pragma unroll
-            for (int c = 0; c < 4 * VC; ++c) acc[r][c] = 0.f;
-        }
-        for (int b = (part * AT1_WARPS + warp) * 32; b < total; b += parts * AT1_WARPS * 32) {
-            const int i = b + lane, j = i < kept ? i : lo + i - kept;
-            const long long row = i < total ? ag_row(a, bt, kvh, j) : -1;
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {           // keys g*4 .. g*4 + 3 of the batch, eight lanes each
-                const long long kr_row = __shfl_sync(0xffffffffu, row, g * 4 + grp);
-                const T* kr = (const T*)a.k_pages + kr_row * D;
-                float s[RG];
-#pragma unroll
-                for (int r = 0; r < RG; ++r) s[r] = 0.f;
-#pragma unroll
-                for (int c = 0; c < QC; ++c) {
-                    const int e = sub * 4 + 32 * c;
-                    const float4 k = kr_row >= 0 && e < D ? ag_load4(kr + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (int r = 0; r < RG; ++r) {
-                        s[r] = fmaf(q[r][c].x, k.x, s[r]); s[r] = fmaf(q[r][c].y, k.y, s[r]);
-                        s[r] = fmaf(q[r][c].z, k.z, s[r]); s[r] = fmaf(q[r][c].w, k.w, s[r]);
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < RG; ++r) {
-                    s[r] += __shfl_xor_sync(0xffffffffu, s[r], 1);
-                    s[r] += __shfl_xor_sync(0xffffffffu, s[r], 2);
-                    s[r] += __shfl_xor_sync(0xffffffffu, s[r], 4);
-                    if (sub == 0) sm_w[warp][g * 4 + grp][r] = s[r];
-                }
-            }
-            __syncwarp();
+        auto tile_begin = [&](int o) { return (o < mt.kept ? o : mt.from + o - mt.kept) * 32; };
+        for (int chunk = c_begin; chunk < c_end; ++chunk) {
 #pragma unroll
             for (int r = 0; r < RG; ++r) {
-                const float slope = a.slopes && r < n_heads ? a.slopes[h0 + r] : 0.f;
-                const float x = row >= 0 ? sm_w[warp][lane][r] - slope * (float)(p - j) : -INFINITY;
-                const float m_new = fmaxf(m[r], warp_max(x));
-                const float alpha = m_new == -INFINITY ? 1.f : expf(m[r] - m_new);
-                const float w = ag_weight(x, m_new);
-                l[r] = l[r] * alpha + w;
-                m[r] = m_new;
+                m[r] = -INFINITY; l[r] = 0.f;
 #pragma unroll
-                for (int c = 0; c < 4 * VC; ++c) acc[r][c] *= alpha;
-                sm_w[warp][lane][r] = w;
+                for (int c = 0; c < 4 * VC; ++c) acc[r][c] = 0.f;
             }
-            __syncwarp();
-            const int nk = min(32, total - b);
+            const int o_end = ((chunk + 1) * mt.n + n_chunks - 1) / n_chunks;
+            for (int o = (chunk * mt.n + n_chunks - 1) / n_chunks; o < o_end; ++o) {
+                const int j0 = tile_begin(o), j = j0 + lane;
+                const long long row = ag_sees(a, p, j) ? ag_row(a, bt, kvh, j) : -1;
 #pragma unroll
-            for (int c = 0; c < VC; ++c) {
-                const int col = c * 128 + lane * 4;
+                for (int g = 0; g < 8; ++g) {           // keys g*4 .. g*4 + 3 of the tile, eight lanes each
+                    const long long kr_row = __shfl_sync(0xffffffffu, row, g * 4 + grp);
+                    const T* kr = (const T*)a.k_pages + kr_row * D;
+                    float s[RG];
+#pragma unroll
+                    for (int r = 0; r < RG; ++r) s[r] = 0.f;
+#pragma unroll
+                    for (int c = 0; c < QC; ++c) {
+                        const int e = sub * 4 + 32 * c;
+                        const float4 k = kr_row >= 0 && e < D ? ag_load4(kr + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                        for (int r = 0; r < RG; ++r) s[r] = ag_dot4(q[r][c], k, s[r]);
+                    }
+#pragma unroll
+                    for (int r = 0; r < RG; ++r) sm_s[warp][r][(g * 4 + grp) * 8 + (sub ^ (g & 1) * 4)] = s[r];     // (halves swapped: no bank met twice)
+                }
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < RG; ++r) {
+                    const float slope = a.slopes && r < n_heads ? a.slopes[h0 + r] : 0.f;
+                    const float4* mine = reinterpret_cast<const float4*>(sm_s[warp][r] + lane * 8);
+                    const float4 x0 = mine[lane >> 2 & 1], x1 = mine[(lane >> 2 & 1) ^ 1];
+                    const float dot = ((((((x0.x + x0.y) + x0.z) + x0.w) + x1.x) + x1.y) + x1.z) + x1.w;
+                    const float x = row >= 0 ? fmaf(-slope, (float)(p - j), dot) : -INFINITY;
+                    const float m_new = fmaxf(m[r], warp_max(x)), alpha = ag_rescale(m[r], m_new);
+                    const float w = ag_weight(x, m_new);
+                    l[r] = __fadd_rn(__fmul_rn(l[r], alpha), w);
+                    m[r] = m_new;
+#pragma unroll
+                    for (int c = 0; c < 4 * VC; ++c) acc[r][c] *= alpha;
+                    sm_w[warp][lane][r] = w;
+                }
+                __syncwarp();
+                const int nk = min(32, p + 1 - j0);
+#pragma unroll
+                for (int c = 0; c < VC; ++c) {
+                    const int col = c * 128 + lane * 4;
 #pragma unroll 8
-                for (int k = 0; k < nk; ++k) {
-                    const long long vr_row = __shfl_sync(0xffffffffu, row, k);
-                    const float4 v = vr_row >= 0 && col < DV ? ag_load4((const T*)a.v_pages + vr_row * a.v_row + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int k = 0; k < nk; ++k) {
+                        const long long vr_row = __shfl_sync(0xffffffffu, row, k);
+                        const float4 v = vr_row >= 0 && col < DV ? ag_load4((const T*)a.v_pages + vr_row * a.v_row + col) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                    for (int r = 0; r < RG; ++r) {
-                        const float w = sm_w[warp][k][r];
-                        if (w == 0.f) continue;     // (a weight of 0 must not meet a value that is no finite number)
-                        acc[r][c * 4 + 0] = fmaf(w, v.x, acc[r][c * 4 + 0]);
-                        acc[r][c * 4 + 1] = fmaf(w, v.y, acc[r][c * 4 + 1]);
-                        acc[r][c * 4 + 2] = fmaf(w, v.z, acc[r][c * 4 + 2]);
-                        acc[r][c * 4 + 3] = fmaf(w, v.w, acc[r][c * 4 + 3]);
+                        for (int r = 0; r < RG; ++r) {
+                            const float w = sm_w[warp][k][r];
+                            if (w == 0.f) continue;     // (a weight of 0 must not meet a value that is no finite number)
+                            acc[r][c * 4 + 0] = fmaf(w, v.x, acc[r][c * 4 + 0]);
+                            acc[r][c * 4 + 1] = fmaf(w, v.y, acc[r][c * 4 + 1]);
+                            acc[r][c * 4 + 2] = fmaf(w, v.z, acc[r][c * 4 + 2]);
+                            acc[r][c * 4 + 3] = fmaf(w, v.w, acc[r][c * 4 + 3]);
+                        }
                     }
                 }
+                __syncwarp();
             }
-            __syncwarp();
-        }
+            const int slot = chunk - c_base;
 #pragma unroll
-        for (int r = 0; r < RG; ++r) {
-            const float sum = warp_sum(l[r]);
-            if (lane == 0) { sm_m[warp][r] = m[r]; sm_l[warp][r] = sum; }
+            for (int r = 0; r < RG; ++r) {
+                const float sum = warp_sum(l[r]);
+                if (lane == 0) { sm_m[slot][r] = m[r]; sm_l[slot][r] = sum; }
 #pragma unroll
-            for (int c = 0; c < VC; ++c)
-                if (c * 128 + lane * 4 < DV)
-                    *reinterpret_cast<float4*>(at_o + (warp * RG + r) * DV + c * 128 + lane * 4) =
-                        make_float4(acc[r][c * 4], acc[r][c * 4 + 1], acc[r][c * 4 + 2], acc[r][c * 4 + 3]);
-        }
-        __syncthreads();
-        if (tid < RG) {
-            float mx = -INFINITY, sum = 0.f;
-            for (int w = 0; w < AT1_WARPS; ++w) mx = fmaxf(mx, sm_m[w][tid]);
-            for (int w = 0; w < AT1_WARPS; ++w) {
-                const float f = sm_m[w][tid] == -INFINITY ? 0.f : expf(sm_m[w][tid] - mx);
-                sum += sm_l[w][tid] * f;
-                sm_m[w][tid] = f;       // from here on the warp's factor
+                for (int c = 0; c < VC; ++c)
+                    if (c * 128 + lane * 4 < DV)
+                        *reinterpret_cast<float4*>(at_o + (slot * RG + r) * DV + c * 128 + lane * 4) =
+                            make_float4(acc[r][c * 4], acc[r][c * 4 + 1], acc[r][c * 4 + 2], acc[r][c * 4 + 3]);
             }
-            tot_m[tid] = mx; tot_l[tid] = sum;
-        }
-        __syncthreads();
-        for (int e = tid; e < RG * DV; e += AT1_WARPS * 32) {
-            float o = 0.f;
-            for (int w = 0; w < AT1_WARPS; ++w) {
-                const float f = sm_m[w][e / DV];
-                if (f != 0.f) o = fmaf(f, at_o[w * RG * DV + e], o);
-            }
-            at_o[e] = o;                // (the thread alone reads and writes column e of the warps' rows)
         }
         if (parts > 1) cluster_sync_all(); else __syncthreads();
+        // chunk c lies with the CTA whose range of them, [b n_chunks / parts, (b + 1) n_chunks / parts), holds it
+        auto owner = [&](int c) { return ((c + 1) * parts - 1) / n_chunks; };
+        if (warp < RG) {            // a warp a head, a lane a chunk: the total's maximum in front of it and with it
+            float front_all = -INFINITY, sum = 0.f;
+#pragma unroll
+            for (int c0 = 0; c0 < CHUNKS; c0 += 32) {
+                if (c0 >= n_chunks) break;
+                const int c = c0 + lane;
+                float cm = -INFINITY, cl = 0.f;
+                if (c < n_chunks) {
+                    const int b = owner(c), slot = c - b * n_chunks / parts;
+                    cm = ag_peer(&sm_m[slot][warp], b);
+                    cl = ag_peer(&sm_l[slot][warp], b);
+                }
+                float with = cm;
+#pragma unroll
+                for (int h = 1; h < 32; h <<= 1) {
+                    const float up = __shfl_up_sync(0xffffffffu, with, h);
+                    if (lane >= h) with = fmaxf(with, up);
+                }
+                with = fmaxf(with, front_all);
+                const float front = __shfl_up_sync(0xffffffffu, with, 1);
+                const float fa = ag_rescale(lane ? front : front_all, with), fb = ag_rescale(cm, with), add = __fmul_rn(cl, fb);
+                fac_a[warp][c] = fa;
+                fac_b[warp][c] = fb;
+#pragma unroll
+                for (int i = 0; i < 32; ++i)        // (behind the last chunk: times 1, plus 0)
+                    sum = fmaf(sum, __shfl_sync(0xffffffffu, fa, i), __shfl_sync(0xffffffffu, add, i));
+                front_all = __shfl_sync(0xffffffffu, with, 31);
+            }
+            if (lane == 0) head_inv[warp] = warp < n_heads ? ag_inverse(a, h0 + warp, front_all, sum) : 0.f;
+        } else if (warp == RG) {
+            for (int c = lane; c < n_chunks; c += 32) {
+                const int b = owner(c);
+                chunk_at[c] = cluster_map((uint32_t)__cvta_generic_to_shared(at_o + (c - b * n_chunks / parts) * RG * DV), b);
+            }
+        }
+        __syncthreads();
         const int share = (RG * DV + parts - 1) / parts;
         for (int e = part * share + tid; e < min(RG * DV, (part + 1) * share); e += AT1_WARPS * 32) {
             const int r = e / DV;
             if (r >= n_heads) continue;
-            float mx = tot_m[r], sum = tot_l[r], o = at_o[e];
-            if (parts > 1) {
-                mx = -INFINITY; sum = 0.f; o = 0.f;
-                for (int c = 0; c < parts; ++c) mx = fmaxf(mx, ag_peer(tot_m + r, c));
-                for (int c = 0; c < parts; ++c) {
-                    const float pm = ag_peer(tot_m + r, c), pl = ag_peer(tot_l + r, c), po = ag_peer(at_o + e, c);
-                    const float f = pm == -INFINITY ? 0.f : expf(pm - mx);
-                    sum = fmaf(pl, f, sum);
-                    if (f != 0.f) o = fmaf(po, f, o);
+            float o = 0.f;
+            for (int c0 = 0; c0 < n_chunks; c0 += 16) {         // sixteen on their way together
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    v[i] = 0.f;
+                    if (c0 + i < n_chunks) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[i]) : "r"(chunk_at[c0 + i] + e * 4) : "memory");
                 }
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (c0 + i < n_chunks) o = ag_fold(o, fac_a[r][c0 + i], v[i], fac_b[r][c0 + i]);
             }
-            if (a.sinks) {
-                const float sink = a.sinks[h0 + r], m_new = fmaxf(mx, sink);
-                const float f = expf(mx - m_new);
-                sum = sum * f + expf(sink - m_new);
-                o *= f;
-            }
-            ag_put<T>(a, t, h0 + r, e % DV, sum == 0.f ? 0.f : o / sum);
+            ag_put<T>(a, t, h0 + r, e % DV, __fmul_rn(o, head_inv[r]));
         }
         if (parts > 1) cluster_sync_all();      // nobody leaves while its results are read
     }
@@ -527,7 +673,7 @@ attn_token_kernel(const AgArgs a, int parts, int only_alone) {
 template <typename T, int RG, int VC>
 static int launch_token(const AgArgs& a, int parts, int only_alone, cudaStream_t stream) {
     auto kernel = attn_token_kernel<T, RG, VC>;
-    const int smem = AT1_WARPS * RG * a.DV * 4;
+    const int smem = AG_CHUNKS(RG, VC) / parts * RG * a.DV * 4;
     static AcvSmemConfig cfg;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
     const int G = a.NH / a.NKV, x = only_alone ? (a.T + AG_STRIDE - 1) / AG_STRIDE : a.T * parts;
@@ -538,7 +684,7 @@ static int launch_token(const AgArgs& a, int parts, int only_alone, cudaStream_t
 template <typename T, int VC>
 static int launch_rows(const AgArgs& a, int skip_alone, cudaStream_t stream) {
     auto kernel = attn_rows_kernel<T, VC>;
-    const int smem = ((AR_ROWS + AR_KEYS) * (a.D + 4) + AR_KEYS * a.DV + AR_ROWS * AR_KEYS) * 4;
+    const int smem = ((AR_ROWS + AR_KEYS) * (a.D + 4) + (AR_KEYS + AR_ROWS) * a.DV + AR_ROWS * AR_KEYS) * 4;
     static AcvSmemConfig cfg;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
     const int G = a.NH / a.NKV, tokens = AR_ROWS / G > 0 ? AR_ROWS / G : 1, heads = G < AR_ROWS ? G : AR_ROWS;
@@ -551,14 +697,15 @@ static int launch_rows(const AgArgs& a, int skip_alone, cudaStream_t stream) {
 // (a portion's 64 rows read each key once for all of them, one token's warps once for its own heads).
 #define AG_FEW 64
 template <typename T>
-static int launch_tiled(const AgArgs& a, cudaStream_t stream) {
+static int launch_tiled(AgArgs& a, cudaStream_t stream) {
     const int G = a.NH / a.NKV, wide = (a.D > 128 || a.DV > 128) ? 2 : 1;
+    const int rg = G == 1 ? 1 : G == 2 || wide == 2 ? 2 : 4;
+    a.chunks = AG_CHUNKS(rg, wide);
     const bool few = a.T <= AG_FEW;
     if (!few) {
         const int e = wide == 1 ? launch_rows<T, 1>(a, 1, stream) : launch_rows<T, 2>(a, 1, stream);
         if (e) return e;
     }
-    const int rg = G == 1 ? 1 : G == 2 || wide == 2 ? 2 : 4;
     const long long ctas = (long long)a.T * a.NKV * ((G + rg - 1) / rg);
     int parts = 1;
     while (few && parts < 8 && ctas * parts < 296) parts *= 2;
@@ -609,8 +756,8 @@ ACV_API int acv_attention_generic(const void* q, int q_stride, void* out, int ou
     const int piece = dtype == ACV_F32 ? 16 : 8;
     if (D <= 256 && DV <= 256 && (D | DV | q_stride) % 4 == 0 && ((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) % piece == 0 &&
         (dtype == ACV_F32 || dtype == ACV_BF16)) {
-        const AgArgs a = {q, k_pages, v_pages, gate, out, positions, seq_of_token, block_table, bt_rows, sinks, slopes,
-                          q_stride, out_stride, gate_stride, bt_stride, T_tokens, NH, NKV, D, DV, page_size, num_pages, window, keep_first, v_row, scale};
+        AgArgs a = {q, k_pages, v_pages, gate, out, positions, seq_of_token, block_table, bt_rows, sinks, slopes,
+                          q_stride, out_stride, gate_stride, bt_stride, T_tokens, NH, NKV, D, DV, page_size, num_pages, window, keep_first, v_row, 0, scale};
         return dtype == ACV_F32 ? launch_tiled<float>(a, stream) : launch_tiled<bf16>(a, stream);
     }
     if (dtype == ACV_F32)

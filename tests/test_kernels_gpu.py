@@ -263,6 +263,43 @@ def test_attention_generic_options(ops, dtype, q_lens, NH, NKV, D, DV, window, k
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("NH,NKV,D,DV,window,keep", [(4, 2, 64, 64, 0, 0), (3, 3, 20, 36, 0, 0), (9, 3, 128, 128, 0, 0), (8, 1, 136, 132, 0, 0),
+                                                    (4, 2, 128, 64, 300, 45), (6, 6, 64, 64, 33, 0), (16, 2, 32, 256, 40, 70)])
+def test_attention_generic_one_order_of_sums(ops, dtype, NH, NKV, D, DV, window, keep):
+    """A token's result has the same bits whatever else is in the step and however its prompt was cut: as part of one
+    portion, of portions of odd lengths beside other requests, as one token among a few (where several CTAs share its keys) or
+    among many."""
+    page, lens = 8, [1300, 70, 33, 1, 400]
+    B, per = len(lens) + 80, 1304 // page
+    g = torch.Generator(device="cuda").manual_seed(4)
+    table = torch.randperm(len(lens) * per, device="cuda", generator=g).to(torch.int32).reshape(-1, per)
+    table = torch.cat([table, table[3:4].expand(80, per)])          # 80 further requests of one key to fill a step with
+    kp, vp = rnd(len(lens) * per, NKV, page, D, dtype=dtype, seed=73), rnd(len(lens) * per, NKV, page, DV, dtype=dtype, seed=74)
+    sinks, slopes = rnd(NH, seed=75), rnd(NH, seed=76).abs() * 0.05
+    lens += [1] * 80
+    qs = {b: rnd(lens[b], NH * D, dtype=dtype, seed=80 + b) for b in range(B)}
+    gates = {b: rnd(lens[b], NH * DV, dtype=dtype, seed=200 + b) for b in range(B)}
+
+    def step(parts):        # (request, first token, end) of each portion
+        cat = lambda x: torch.cat([x[b][i:j] for b, i, j in parts])
+        pos = torch.cat([torch.arange(i, j) for _, i, j in parts]).to(torch.int32).cuda()
+        seq = torch.repeat_interleave(torch.tensor([b for b, _, _ in parts]), torch.tensor([j - i for _, i, j in parts])).to(torch.int32).cuda()
+        out = torch.full((len(pos), NH * DV), float("nan"), device="cuda", dtype=dtype)
+        ops.attention_generic(cat(qs), out, kp, vp, pos, seq, table, NH, NKV, D, D ** -0.5, window, value_dim=DV if DV != D else 0,
+                              keep_first=keep, sinks=sinks, slopes=slopes, gate=cat(gates))
+        return dict(zip(parts, out.split([j - i for _, i, j in parts])))
+
+    few, many = [(b, 0, 1) for b in range(5, 8)], [(b, 0, 1) for b in range(5, 85)]
+    whole = {b: step([(b, 0, lens[b])] + many)[(b, 0, lens[b])] for b in range(5)}
+    assert not any(w.isnan().any() for w in whole.values())
+    for b, cuts in ((0, [0, 1, 2, 5, 64, 131, 700, 701, 1299, 1300]), (1, [0, 1, 35, 69, 70]), (2, [0, 32, 33]), (4, [0, 3, 80, 399, 400])):
+        for i, j in zip(cuts, cuts[1:]):
+            for others in ([], few, many, [(3, 0, 1), ((b + 1) % 5, 0, min(66, lens[(b + 1) % 5]))]):
+                got = step(others[:1] + [(b, i, j)] + others[1:])[(b, i, j)]
+                assert torch.equal(got, whole[b][i:j]), (b, i, j, len(others))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("q_lens,D", [((1, 1, 1), 64), ((1,) * 40, 64), ((70, 2), 64), ((70, 1, 1), 64), ((1, 70), 260)])
 def test_attention_generic_scores_that_are_no_finite_numbers(ops, dtype, q_lens, D):
     """Infinities and NaN, for tokens one by one, for portions and for the general kernel (head size 260): a query or a key
