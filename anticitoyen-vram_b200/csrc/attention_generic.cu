@@ -482,11 +482,10 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
 // that is read.  Bound by the pages' stream and its latency.  The chunks' results wait in the CTAs' shared memory; each CTA
 // then adds up its share of the columns over all of them.
 #define AT1_WARPS 8
-#define AG_STRIDE 8      // tokens that a CTA looks at in a step of many tokens
 
 template <typename T, int RG, int VC>
 __global__ void __launch_bounds__(AT1_WARPS * 32, RG * VC == 1 ? 3 : 2)
-attn_token_kernel(const AgArgs a, int parts, int only_alone) {
+attn_token_kernel(const AgArgs a, int parts, int stride) {
     constexpr int CHUNKS = AG_CHUNKS(RG, VC);
     __shared__ float sm_m[CHUNKS][RG], sm_l[CHUNKS][RG];                        // this CTA's chunks
     __shared__ float fac_a[RG][CHUNKS], fac_b[RG][CHUNKS], head_inv[RG];        // all chunks' factors, once all are there
@@ -500,16 +499,16 @@ attn_token_kernel(const AgArgs a, int parts, int only_alone) {
     const int part = blockIdx.x % parts;
     const int chunks = (G + RG - 1) / RG, kvh = blockIdx.y / chunks, h0 = kvh * G + (blockIdx.y % chunks) * RG;
     const int n_heads = min(RG, (kvh + 1) * G - h0);
-    // one token a cluster; in a step of many tokens, without clusters, those of the tokens x, x + gridDim.x .. that are alone
+    // one token a cluster; with a stride, without clusters, those of the `stride` tokens x, x + gridDim.x .. that are alone
     // (bit i: token x + i gridDim.x; all asked for at once, since a look is a round trip to memory)
     uint32_t mine = 1;
-    if (only_alone) {
+    if (stride) {
         const int cand = blockIdx.x + lane * gridDim.x;
-        mine = __ballot_sync(0xffffffffu, lane < AG_STRIDE && cand < a.T && ag_alone(a.seq_of_token, cand, a.T));
+        mine = __ballot_sync(0xffffffffu, lane < stride && cand < a.T && ag_alone(a.seq_of_token, cand, a.T));
     }
     for (; mine; mine &= mine - 1) {
-        const int t = only_alone ? blockIdx.x + (__ffs(mine) - 1) * gridDim.x : blockIdx.x / parts;
-        if (only_alone) __syncthreads();        // the token before is done with the shared memory
+        const int t = stride ? blockIdx.x + (__ffs(mine) - 1) * gridDim.x : blockIdx.x / parts;
+        if (stride) __syncthreads();        // the token before is done with the shared memory
         const int p = a.positions[t], seq = a.seq_of_token[t];
         const int* bt = a.block_table + (size_t)(a.bt_rows ? a.bt_rows[seq] : seq) * a.bt_stride;
         const AgTiles mt = ag_tiles(a, p);
@@ -671,13 +670,13 @@ attn_token_kernel(const AgArgs a, int parts, int only_alone) {
 }
 
 template <typename T, int RG, int VC>
-static int launch_token(const AgArgs& a, int parts, int only_alone, cudaStream_t stream) {
+static int launch_token(const AgArgs& a, int parts, int stride, cudaStream_t stream) {
     auto kernel = attn_token_kernel<T, RG, VC>;
     const int smem = AG_CHUNKS(RG, VC) / parts * RG * a.DV * 4;
     static AcvSmemConfig cfg;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
-    const int G = a.NH / a.NKV, x = only_alone ? (a.T + AG_STRIDE - 1) / AG_STRIDE : a.T * parts;
-    acv_launch_cluster(PDL_ATTN, dim3(parts, 1, 1), kernel, dim3(x, a.NKV * ((G + RG - 1) / RG)), dim3(AT1_WARPS * 32), smem, stream, a, parts, only_alone);
+    const int G = a.NH / a.NKV, x = stride ? (a.T + stride - 1) / stride : a.T * parts;
+    acv_launch_cluster(PDL_ATTN, dim3(parts, 1, 1), kernel, dim3(x, a.NKV * ((G + RG - 1) / RG)), dim3(AT1_WARPS * 32), smem, stream, a, parts, stride);
     return acv_launch_status();
 }
 
@@ -692,12 +691,20 @@ static int launch_rows(const AgArgs& a, int skip_alone, cudaStream_t stream) {
     return acv_launch_status();
 }
 
-// Steps of up to AG_FEW tokens: every token by itself, with as many CTAs to a token and kv-head as put the SMs to work
-// (a short context's CTAs without keys leave at the merge).  More tokens: rows of portions, then the tokens that are alone
-// (a portion's 64 rows read each key once for all of them, one token's warps once for its own heads).
+// Steps of up to AG_FEW tokens: every token by itself, with as many CTAs to a token and kv-head as come in one wave (two to
+// an SM; 16 requests of 1500 keys, 16 heads on 8, with 1, 2, 4, 8: 206, 110, 150, 165 us).  More tokens: rows of portions, then the
+// tokens that are alone
+// (a portion's 64 rows read each key once for all of them, one token's warps once for its own heads).  A CTA looks at as
+// many tokens as leave eight CTAs to an SM, at most AG_STRIDE: all of them may be alone, and one behind the other took 65
+// requests of 500 keys 532 us where 64 take 144 (150 with a CTA each); of a portion's thousands none are.
 #define AG_FEW 64
+#define AG_STRIDE 8
 template <typename T>
 static int launch_tiled(AgArgs& a, cudaStream_t stream) {
+    int device = 0, sms = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (err != cudaSuccess) return (int)err;
     const int G = a.NH / a.NKV, wide = (a.D > 128 || a.DV > 128) ? 2 : 1;
     const int rg = G == 1 ? 1 : G == 2 || wide == 2 ? 2 : 4;
     a.chunks = AG_CHUNKS(rg, wide);
@@ -708,11 +715,11 @@ static int launch_tiled(AgArgs& a, cudaStream_t stream) {
     }
     const long long ctas = (long long)a.T * a.NKV * ((G + rg - 1) / rg);
     int parts = 1;
-    while (few && parts < 8 && ctas * parts < 296) parts *= 2;
-    const int alone = few ? 0 : 1;
-    if (wide == 2) return rg == 1 ? launch_token<T, 1, 2>(a, parts, alone, stream) : launch_token<T, 2, 2>(a, parts, alone, stream);
-    return rg == 1 ? launch_token<T, 1, 1>(a, parts, alone, stream) : rg == 2 ? launch_token<T, 2, 1>(a, parts, alone, stream)
-                                                                         : launch_token<T, 4, 1>(a, parts, alone, stream);
+    while (few && parts < 8 && ctas * parts <= sms) parts *= 2;
+    const int stride = few ? 0 : (int)max(1ll, min((long long)AG_STRIDE, ctas / (8 * sms)));
+    if (wide == 2) return rg == 1 ? launch_token<T, 1, 2>(a, parts, stride, stream) : launch_token<T, 2, 2>(a, parts, stride, stream);
+    return rg == 1 ? launch_token<T, 1, 1>(a, parts, stride, stream) : rg == 2 ? launch_token<T, 2, 1>(a, parts, stride, stream)
+                                                                          : launch_token<T, 4, 1>(a, parts, stride, stream);
 }
 
 template <typename T>

@@ -335,6 +335,34 @@ def test_attention_generic_scores_that_are_no_finite_numbers(ops, dtype, q_lens,
         torch.testing.assert_close(out[rows].double(), want.reshape(-1, NH * D), equal_nan=True, **tol(dtype))
 
 
+def _attention_generic_us(ops, q_lens, NH=16, NKV=8, D=128, keys=500, page=16):
+    """Microseconds of a float32 step of portions that end at `keys` keys each."""
+    B, T, per = len(q_lens), sum(q_lens), -(-keys // page)
+    kp, vp = rnd(B * per, NKV, page, D, seed=77), rnd(B * per, NKV, page, D, seed=78)
+    table = torch.arange(B * per, device="cuda", dtype=torch.int32).reshape(B, per)
+    q, out = rnd(T, NH * D, seed=79), torch.empty(T, NH * D, device="cuda")
+    pos = torch.cat([torch.arange(keys - n, keys) for n in q_lens]).to(torch.int32).cuda()
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(q_lens)).to(torch.int32).cuda()
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    best = float("inf")
+    for _ in range(6):          # (the first pass warms up; the shortest of the others)
+        torch.cuda.synchronize()
+        start.record()
+        for _ in range(10):
+            ops.attention_generic(q, out, kp, vp, pos, seq, table, NH, NKV, D, D ** -0.5)
+        end.record()
+        torch.cuda.synchronize()
+        best = min(best, start.elapsed_time(end) * 100.0)
+    return best
+
+
+@pytest.mark.parametrize("q_lens,times", [([1] * 65, 2.0)])
+def test_attention_generic_has_no_cliff_past_64_tokens(ops, q_lens, times):
+    """A step a little over the size where the kernels change hands costs about what one a little under it does (65
+    requests: 1.1 times the 64; four times when a CTA walked eight of them)."""
+    assert _attention_generic_us(ops, q_lens) < times * _attention_generic_us(ops, [1] * 64)
+
+
 @pytest.mark.parametrize("in_dtype,out_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32),
                                                 (torch.bfloat16, torch.bfloat16)])
 @pytest.mark.parametrize("M,N,K", [(1, 331, 80), (7, 100, 72), (65, 130, 200), (3, 1000, 4096), (128, 64, 16)])
