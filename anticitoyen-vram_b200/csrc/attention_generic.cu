@@ -219,8 +219,11 @@ __device__ __forceinline__ float ag_peer(const float* local, int rank) {
 }
 
 // ----------------------------------------------------------------------------- rows of a portion
-// A CTA: 64 / (NH/NKV) tokens of the flat batch times the heads of one kv-head, eight rows to a warp; the requests among
-// the tokens one after the other (a tile of a portion has one).  Scores: a lane a key, so a 16-byte read of 32 key rows
+// A stretch: up to 64 / (NH/NKV) tokens of one request, within a block of that many tokens of the flat batch, times the heads of one
+// kv-head, eight rows to a warp.  A CTA takes the stretches that begin among its AR_OWN tokens: a portion leaves most
+// CTAs without one (they return at once), and a block of two-token portions has work for as many CTAs as it has (33 requests of two tokens
+// and 500 keys, 16 heads on 8: one CTA a block 1620 us, looking at 8, 4, 2 tokens 471, 257, 146; prompts of 696 tokens 119 with 8
+// and 4, 122 with 2).  Scores: a lane a key, so a 16-byte read of 32 key rows
 // moves 512 different bytes and a row's queries are one address; values: a lane four columns.  What belongs to a row (its
 // tiles, maximum and total) lies in the lanes 4 i to 4 i + 3 for row i of the warp, so that eight rows' maxima and sums over
 // the lanes take nine exchanges instead of forty.  Bound by the chains of
@@ -233,6 +236,7 @@ __device__ __forceinline__ float ag_peer(const float* local, int rank) {
 #define AR_KEYS 32
 #define AR_WARP_ROWS 8
 #define AR_THREADS 256
+#define AR_OWN 4          // tokens among which a CTA looks for stretches to take; under 32
 
 // eight values a lane -> lane l: value l / 4 over all lanes, pairs of lanes 16 apart first, then 8, 4, 2, 1 (warp_sum's order)
 template <bool MAX>
@@ -263,14 +267,24 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
     pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int kvh = blockIdx.y, h0 = kvh * G + blockIdx.z * heads, n_heads = min(heads, G - (int)blockIdx.z * heads);
-    const int t_begin = blockIdx.x * tokens, t_end = min(a.T, t_begin + tokens);
     float* pw = ps + warp * AR_KEYS * AR_WARP_ROWS;
 
-    for (int t0 = t_begin; t0 < t_end;) {
-        const int seq = a.seq_of_token[t0];
-        int t1 = t0 + 1;
-        while (t1 < t_end && a.seq_of_token[t1] == seq) ++t1;
-        if (skip_alone && t1 == t0 + 1 && ag_alone(a.seq_of_token, t0, a.T)) { t0 = t1; continue; }
+    // the stretches that begin among this CTA's AR_OWN tokens: where a request begins, or a multiple of `tokens`
+    const int t_mine = blockIdx.x * AR_OWN;
+    uint32_t begins;
+    {
+        const int t = t_mine + lane, before = t > 0 && t <= a.T ? a.seq_of_token[t - 1] : -1;
+        const int own = __shfl_down_sync(0xffffffffu, before, 1);
+        begins = __ballot_sync(0xffffffffu, lane < AR_OWN && t < a.T && (t % tokens == 0 || own != before));
+    }
+    for (; begins; begins &= begins - 1) {
+        const int t0 = t_mine + __ffs(begins) - 1, seq = a.seq_of_token[t0];
+        int t1 = min(a.T, (t0 / tokens + 1) * tokens);
+        for (int t = t0 + 1; t < t1; t += 32) {         // where the request ends, 32 tokens a look
+            const uint32_t other = __ballot_sync(0xffffffffu, t + lane < t1 && a.seq_of_token[t + lane] != seq);
+            if (other) t1 = t + __ffs(other) - 1;
+        }
+        if (skip_alone && t1 == t0 + 1 && ag_alone(a.seq_of_token, t0, a.T)) continue;
         const int n = t1 - t0, rows = n * n_heads;      // row r: token t0 + r / n_heads, head h0 + r % n_heads
         const int* bt = a.block_table + (size_t)(a.bt_rows ? a.bt_rows[seq] : seq) * a.bt_stride;
         __syncthreads();
@@ -282,7 +296,7 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
         }
         // the tiles that any row visits
         int kept_tiles = 0, from = 0x7fffffff, last = -1, last_key = -1;
-        for (int t = t0; t < t1; ++t) {
+        for (int t = t0 + lane; t < t1; t += 32) {
             const int p = a.positions[t];
             const AgTiles u = ag_tiles(a, p);
             if (u.n == 0) continue;
@@ -291,7 +305,10 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
             last = max(last, u.last);
             last_key = max(last_key, p);
         }
-        from = max(min(from, last + 1), kept_tiles);
+        kept_tiles = __reduce_max_sync(0xffffffffu, kept_tiles);
+        last = __reduce_max_sync(0xffffffffu, last);
+        last_key = __reduce_max_sync(0xffffffffu, last_key);
+        from = max(min(__reduce_min_sync(0xffffffffu, from), last + 1), kept_tiles);
         const int r0 = warp * AR_WARP_ROWS;
         int pos[AR_WARP_ROWS];
         float l[AR_WARP_ROWS], acc[AR_WARP_ROWS][4 * VC];
@@ -471,7 +488,6 @@ attn_rows_kernel(const AgArgs a, int skip_alone) {
                 ag_put<T>(a, t, h, e + 2, __fmul_rn(o.z, inv)); ag_put<T>(a, t, h, e + 3, __fmul_rn(o.w, inv));
             }
         }
-        t0 = t1;
     }
     pdl_launch_dependents();
 }
@@ -686,8 +702,8 @@ static int launch_rows(const AgArgs& a, int skip_alone, cudaStream_t stream) {
     const int smem = ((AR_ROWS + AR_KEYS) * (a.D + 4) + (AR_KEYS + AR_ROWS) * a.DV + AR_ROWS * AR_KEYS) * 4;
     static AcvSmemConfig cfg;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
-    const int G = a.NH / a.NKV, tokens = AR_ROWS / G > 0 ? AR_ROWS / G : 1, heads = G < AR_ROWS ? G : AR_ROWS;
-    acv_launch(PDL_ATTN, kernel, dim3((a.T + tokens - 1) / tokens, a.NKV, (G + heads - 1) / heads), dim3(AR_THREADS), smem, stream, a, skip_alone);
+    const int G = a.NH / a.NKV, heads = G < AR_ROWS ? G : AR_ROWS;
+    acv_launch(PDL_ATTN, kernel, dim3((a.T + AR_OWN - 1) / AR_OWN, a.NKV, (G + heads - 1) / heads), dim3(AR_THREADS), smem, stream, a, skip_alone);
     return acv_launch_status();
 }
 

@@ -356,10 +356,11 @@ def _attention_generic_us(ops, q_lens, NH=16, NKV=8, D=128, keys=500, page=16):
     return best
 
 
-@pytest.mark.parametrize("q_lens,times", [([1] * 65, 2.0)])
+@pytest.mark.parametrize("q_lens,times", [([1] * 65, 2.0), ([2] * 33, 4.0), ([5] * 14, 4.0)])
 def test_attention_generic_has_no_cliff_past_64_tokens(ops, q_lens, times):
     """A step a little over the size where the kernels change hands costs about what one a little under it does (65
-    requests: 1.1 times the 64; four times when a CTA walked eight of them)."""
+    requests: 1.1 times the 64, four times when a CTA walked eight of them; 33 portions of two tokens 1.8 times, eleven
+    times when a CTA walked sixteen of them)."""
     assert _attention_generic_us(ops, q_lens) < times * _attention_generic_us(ops, [1] * 64)
 
 
