@@ -1406,9 +1406,9 @@ def linear_bf16_glu(x: torch.Tensor, w_pairs: torch.Tensor, out: torch.Tensor, l
     N = w_pairs.shape[0]
     if out.shape != (M, N // 2) or out.dtype != torch.bfloat16 or out.stride(1) != 1 or w_pairs.shape[1] != K:
         raise KernelError(f"linear_bf16_glu: shapes {tuple(x.shape)} x {tuple(w_pairs.shape)} -> {tuple(out.shape)} do not fit")
-    plan = gemm_tc_plan(M, N, K, bn_multiple=32)        # (an epilogue for tokens on the rows, without splits of K)
-    if plan[0]:
+    if M <= 128:
         raise KernelError("linear_bf16_glu: tokens must lie on the rows (more than 128 of them)")
+    plan = gemm_tc_plan(M, N, K, bn_multiple=32)        # (an epilogue for tokens on the rows, without splits of K)
     bn, stages = plan[1], plan[3] if len(plan) > 3 else 8
     mode = plan[4] if len(plan) > 4 else 0
     _, _, status = _gemm_buffers(x.device, 0, 0)

@@ -228,6 +228,32 @@ def test_the_plan_of_a_product_follows_its_shape():
     assert len(ops.gemm_tc_plan(2048, 4096, 4096, sms=1)) == 4
 
 
+@pytest.mark.parametrize("M,refused", [(1, True), (65, True), (128, True), (129, False)])
+def test_the_clamped_unit_refuses_what_its_documentation_refuses(monkeypatch, M, refused):
+    """128 tokens and fewer, also where the plan of a plain product puts them on the rows (a weight of more tiles than SMs)."""
+    from acvram_b200.kernels import ops
+    launched = []
+
+    class Library:
+        def acv_gemm_tc_glu(self, *args):
+            launched.append(args)
+            return 0
+
+    monkeypatch.setattr(ops, "library", Library)
+    monkeypatch.setattr(ops, "_need_cuda", lambda *a: None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "sm_count", lambda *a: 148)
+    monkeypatch.setattr(ops, "_gemm_buffers", lambda *a: (None, None, None))
+    N, K = 128 * 160, 64
+    x, w, out = (torch.empty(*s, dtype=torch.bfloat16) for s in ((M, K), (N, K), (M, N // 2)))
+    if refused:
+        with pytest.raises(ops.KernelError, match="more than 128"):
+            ops.linear_bf16_glu(x, w, out, 7.0, 1.7)
+    else:
+        ops.linear_bf16_glu(x, w, out, 7.0, 1.7)
+    assert len(launched) == (0 if refused else 1)
+
+
 @pytest.mark.parametrize("sms", [1, 74, 132, 148, 256])
 def test_split_products_share_nothing_between_streams(sms):
     """Splits of K that a plan asks for are summed inside a cluster (8 CTAs and 100 KB of partial tiles at most), never through
