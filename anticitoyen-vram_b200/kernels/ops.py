@@ -472,7 +472,7 @@ GEMM_PAIR_ROUND = 0.905
 GEMM_PAIR = 4               # fifth element of a plan: the flag that asks for the pair kernel
 
 
-def gemm_tc_plan(M: int, N: int, K: int, sms: int | None = None, bn_multiple: int = 16) -> tuple:
+def gemm_tc_plan(M: int, N: int, K: int, sms: int | None = None, bn_multiple: int = 16, rows: bool = False) -> tuple:
     """(swap, bn, splits, stages[, mode]) for x[M,K] @ w[N,K]^T on a device of ``sms`` multiprocessors.
 
     Up to 128 tokens the weight rows fill the tensor core's M = 128 and the tokens are the narrow
@@ -480,14 +480,14 @@ def gemm_tc_plan(M: int, N: int, K: int, sms: int | None = None, bn_multiple: in
     one wave of the SMs (``GEMM_FEW_TOKENS_RULES``).  Above, and where 65 tokens or more meet more tiles of weight rows
     than SMs, tokens are the M side and a tile is 128
     tokens by 128..256 features: the width that needs the least rounds x width (``GEMM_TILE_WIDTHS``;
-    ``bn_multiple``: widths that are multiples of this only, for an epilogue that wants whole heads; over 128 tokens any
-    but 16 also means tokens on the rows and no split of K),
-    or, where that comes out cheaper, 256 x 256 on a pair of CTAs (``mode`` = ``GEMM_PAIR``)."""
-    return _gemm_tc_plan(M, N, K, sms or sm_count(), bn_multiple)
+    ``bn_multiple``: widths that are multiples of this only, for an epilogue that wants whole heads),
+    or, where that comes out cheaper, 256 x 256 on a pair of CTAs (``mode`` = ``GEMM_PAIR``).  ``rows``: for an epilogue
+    that exists for tokens on the rows without a split of K only; over 128 tokens the plan is one of those then."""
+    return _gemm_tc_plan(M, N, K, sms or sm_count(), bn_multiple, rows)
 
 
 @functools.lru_cache(maxsize=4096)      # (a step asks for the same few shapes layer after layer)
-def _gemm_tc_plan(M: int, N: int, K: int, sms: int, bn_multiple: int) -> tuple:
+def _gemm_tc_plan(M: int, N: int, K: int, sms: int, bn_multiple: int, rows: bool) -> tuple:
     n_kb = -(-K // 64)
     wide = -(-N // 128)
     if M <= 64:
@@ -511,7 +511,7 @@ def _gemm_tc_plan(M: int, N: int, K: int, sms: int, bn_multiple: int) -> tuple:
         return (1, 128, 2, 6) if wide <= 0.5 * sms else (1, 128, 1, 6)
     if N < 256:
         return 0, (128 if N > 64 else 64), 1, 8
-    if M > 128 and bn_multiple == 16 and n_kb >= 48 and -(-M // 128) * wide <= 0.5 * sms:
+    if M > 128 and not rows and n_kb >= 48 and -(-M // 128) * wide <= 0.5 * sms:
         # half of the SMs or fewer would have a tile: two CTAs of a cluster share one (256 tokens, microseconds: 4096 x 12288 63 -> 41,
         # 2560 x 9728 50 -> 34, 4096 x 4096 24.5 -> 20.6).  With a few tiles more two CTAs could share a wider one through the
         # workspace (256 x 5120 x 17408 91 -> 61), but its counters belong to the device and products of two streams would meet there.
@@ -588,7 +588,7 @@ def gemm_tc_qkv_takes(x: torch.Tensor, w: torch.Tensor, head_dim: int, cos_sin: 
         return False
     M, K = x.shape
     N = w.shape[0]
-    swap, bn, splits = gemm_tc_plan(M, N, K, bn_multiple=head_dim if M > 128 else 16)[:3]
+    swap, bn, splits = gemm_tc_plan(M, N, K, bn_multiple=head_dim if M > 128 else 16, rows=M > 128)[:3]
     if not swap:            # tokens on M (one CTA or a pair to a tile): a thread of the epilogue holds whole heads of one token
         return splits == 1 and bn >= head_dim and bn % head_dim == 0
     tiles = -(-N // 128) * -(-M // bn)
@@ -606,7 +606,7 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, num_heads: 
     _need_cuda(x, w, out, k_pages, v_pages)
     M, K = x.shape
     N = w.shape[0]
-    plan = plan or gemm_tc_plan(M, N, K, bn_multiple=head_dim if M > 128 else 16)
+    plan = plan or gemm_tc_plan(M, N, K, bn_multiple=head_dim if M > 128 else 16, rows=M > 128)
     swap, bn, splits, stages = plan[:4]
     cluster = plan[4] if len(plan) > 4 else (1 if swap and 1 < splits <= 8 else 0)
     tiles = (-(-N // 128) * -(-M // bn)) if swap else (-(-M // 128) * -(-N // bn))
@@ -1408,7 +1408,7 @@ def linear_bf16_glu(x: torch.Tensor, w_pairs: torch.Tensor, out: torch.Tensor, l
         raise KernelError(f"linear_bf16_glu: shapes {tuple(x.shape)} x {tuple(w_pairs.shape)} -> {tuple(out.shape)} do not fit")
     if M <= 128:
         raise KernelError("linear_bf16_glu: tokens must lie on the rows (more than 128 of them)")
-    plan = gemm_tc_plan(M, N, K, bn_multiple=32)        # (an epilogue for tokens on the rows, without splits of K)
+    plan = gemm_tc_plan(M, N, K, rows=True)
     bn, stages = plan[1], plan[3] if len(plan) > 3 else 8
     mode = plan[4] if len(plan) > 4 else 0
     _, _, status = _gemm_buffers(x.device, 0, 0)

@@ -665,7 +665,7 @@ def test_gemm_tc_as_planned(ops, M, N, K, form):
 @pytest.mark.parametrize("M,N,K", [(129, 3072, 4096), (200, 512, 4096), (256, 4608, 8192)])
 def test_clamped_unit_keeps_its_tokens_on_the_rows(ops, M, N, K):
     """The product with the clamped gated unit has no form for shared tiles: sizes for which a plain product takes one."""
-    assert ops.gemm_tc_plan(M, N, K, 148)[:3] != ops.gemm_tc_plan(M, N, K, 148, bn_multiple=32)[:3]
+    assert ops.gemm_tc_plan(M, N, K, 148)[:3] != ops.gemm_tc_plan(M, N, K, 148, rows=True)[:3]
     x, w = rnd(M, K, dtype=torch.bfloat16, seed=61), rnd(N, K, dtype=torch.bfloat16, scale=0.02, seed=62)
     out = ops.linear_bf16_glu(x, w, torch.empty(M, N // 2, device="cuda", dtype=torch.bfloat16), 2.0, 1.7)
     z = x.double() @ w.double().T
