@@ -65,22 +65,24 @@ __device__ __forceinline__ at_f2 at_mul(at_f2 a, at_f2 b) {
 __device__ __forceinline__ at_f2 at_both(float x) { return at_pack(x, x); }
 
 // 2^y for two y on the multiply-add pipes: y = n + f, n the nearest whole number (the low bits of y + 1.5 2^23), f in
-// [-1/2, 1/2], 2^f by a polynomial of degree five fitted here for the least largest relative error (7.5e-8 in exact
-// arithmetic; the special-function unit's is 1.2e-7), times 2^n.  y below -126 counts as -126 (1.2e-38 where the exact
-// value is smaller still); a y that is no number stays none.
+// [-1/2, 1/2], 2^f by a minimax polynomial of degree six fitted here for the relative error on that range, its constant held
+// at 1, times 2^n.  Over every float in [-126, 8], against 64 bits: relative error at most 7.0e-8, 2.6e-8 in the mean square;
+// the special-function unit's 1.46e-7 and 5.8e-8 (degree five: 1.56e-7 and 6.5e-8).  Below -126.5, -inf (a key that
+// is not seen) included, it is 0; a y that is no number stays none.
 __device__ __forceinline__ at_f2 at_exp2_poly(at_f2 y) {
     float a, b;
     at_split(y, a, b);
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(-126.f));
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(b) : "f"(-126.f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(-127.f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(b) : "f"(-127.f));
     y = at_pack(a, b);
     const at_f2 z = at_add(y, at_both(12582912.f));
     const at_f2 f = at_fma(at_add(z, at_both(-12582912.f)), at_both(-1.f), y);
-    at_f2 q = at_fma(at_both(1.32764701e-3f), f, at_both(9.67554096e-3f));
-    q = at_fma(q, f, at_both(5.55071346e-2f));
-    q = at_fma(q, f, at_both(2.40221202e-1f));
-    q = at_fma(q, f, at_both(6.93146944e-1f));
-    q = at_fma(q, f, at_both(1.00000012f));
+    at_f2 q = at_fma(at_both(1.53533605e-4f), f, at_both(1.33988610e-3f));
+    q = at_fma(q, f, at_both(9.61843878e-3f));
+    q = at_fma(q, f, at_both(5.55034392e-2f));
+    q = at_fma(q, f, at_both(2.40226477e-1f));
+    q = at_fma(q, f, at_both(6.93147182e-1f));
+    q = at_fma(q, f, at_both(1.f));
     at_split(z, a, b);
     const float s0 = __uint_as_float((__float_as_uint(a) << 23) + 0x3f800000u), s1 = __uint_as_float((__float_as_uint(b) << 23) + 0x3f800000u);
     return at_mul(q, at_pack(s0, s1));
@@ -88,11 +90,11 @@ __device__ __forceinline__ at_f2 at_exp2_poly(at_f2 y) {
 
 // Of eight pairs of columns the first AT_POLY take their exponentials on the multiply-add pipes, the others on the
 // special-function unit (4 lanes a clock and sub-partition: a half tile's 64 columns of the two warps there take it 1024
-// clocks, as long as the half's products take the tensor core).  A pair costs ten packed instructions (20 clocks of the
-// multiply-add pipe, which the rest leaves three quarters idle) in place of 16 clocks of that unit, so three of eight
-// come out even.  Measured, microseconds with one exponential at a time, then 0, 2, 3, 4 of eight pairs: 2048 tokens 49.7, 47.9,
-// 46.5, 45.8, 47.0 (32 heads on 8); 2048 behind 6144 263, 252, 240, 232, 246; 1000 behind 5000 (40 heads) 188, 180, 172, 174, 178.
-#define AT_POLY 3
+// clocks, as long as the half's products take the tensor core).  A pair costs eleven packed instructions (22 clocks of the
+// multiply-add pipe) in place of 16 clocks of that unit, beside what the rest of the softmax asks of that pipe.
+// Measured, microseconds with none, 1, 2, 3, 4 of eight pairs: 2048 tokens 48.2, 47.5, 46.4, 46.5,
+// 48.7 (32 heads on 8); 2048 behind 6144 243, 237, 227, 230, 245; 1000 behind 5000 (40 heads) 172, 168, 168, 172, 179.
+#define AT_POLY 2
 
 struct AttnTcParams {
     bf16* out;
@@ -418,7 +420,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (!failed && !abort_s && mbar_wait(o_full + 8 * hs, 0, &abort_s)) {
             tc_fence_after();
             if (p.sinks && m_run != -INFINITY) l_run += exp2f(p.sinks[head] * AT_LOG2E - m_run);
-            const float inv = l_run > 0.f && m_run != -INFINITY ? 1.f / l_run : 0.f;      // (a row that sees no key: zeros)
+            const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
             bf16* dst = p.out + (size_t)(tok0 + r) * p.out_stride + (size_t)(h0 + hs) * D;
 #pragma unroll
             for (int c0 = 0; c0 < D; c0 += 32) {

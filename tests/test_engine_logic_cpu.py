@@ -299,3 +299,24 @@ def test_the_splits_of_decode_attention_follow_what_fits_the_device(monkeypatch)
     one = ops.decode_splits_cost(2, 8, 8192, 8, True, 296, 512)
     assert ops.decode_splits_cost(2, 8, 8192, 8, True, 64, 512) > 1.3 * one
     assert ops.decode_splits_cost(2, 8, 8192, 8, False, 296, 512) > one
+
+
+def test_the_exponentials_polynomial_is_as_exact_as_the_unit_beside_it():
+    """The constants of csrc/attention_tc.cu's 2^f, evaluated in float as the kernel does: over [-1/2, 1/2] the relative
+    error stays under 1.3e-7, the least that the special-function unit's largest comes to on any part of the range
+    (1.31e-7 to 1.46e-7 over all floats in [-126, 8]), and 2^0 is 1."""
+    import os
+    import re
+    import numpy as np
+    import acvram_b200.kernels.build as kbuild
+    with open(os.path.join(kbuild.CSRC, "attention_tc.cu")) as f:
+        body = f.read().split("at_f2 at_exp2_poly(at_f2 y) {")[1].split("at_split(z, a, b);")[0].split("at_f2 q = ")[1]
+    coefficients = [np.float32(c) for c in re.findall(r"at_both\(([-+.0-9e]+)f\)", body)]
+    assert len(coefficients) > 4 and coefficients[-1] == 1.0
+    f = np.linspace(-0.5, 0.5, 400001).astype(np.float32)
+    q = np.full_like(f, coefficients[0])
+    for c in coefficients[1:]:          # a fused multiply-add: exact in 64 bits, rounded once
+        q = (q.astype(np.float64) * f + np.float64(c)).astype(np.float32)
+    exact = 2.0 ** f.astype(np.float64)
+    assert (np.abs(q - exact) / exact).max() < 1.3e-7
+    assert q[200000] == 1.0 and f[200000] == 0.0

@@ -496,6 +496,26 @@ def test_prompt_attention_exponentials_of_every_size(ops, D, spread):
     assert bad[70, :D].all() and int(bad.sum()) == D
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("window", [0, 20])
+def test_prompt_attention_gives_no_weight_to_keys_that_are_not_seen(ops, D, window):
+    """Values of 1e38 at tokens behind a query, or in front of its window, in the same tile: a weight of the smallest float
+    instead of 0 would show."""
+    NH, NKV, page, n = 2, 1, 64, 256
+    kp, vp = rnd(4, NKV, page, D, dtype=torch.bfloat16, seed=65), rnd(4, NKV, page, D, dtype=torch.bfloat16, seed=66)
+    q = rnd(n, (NH + 2 * NKV) * D, dtype=torch.bfloat16, seed=67)
+    vp[1, :, 36:] = 1e38            # tokens 100 to 127
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    out = torch.full((n, NH * D), 7.0, device="cuda", dtype=torch.bfloat16)
+    ops.attention_tc(q, out, kp, vp, i32([0, 0]), i32([128, 0]), 2, i32([0, n]), i32([n]), i32([[0, 1, 2, 3]]), NH, NKV, D, D ** -0.5, window)
+    d = torch.arange(n, device="cuda")[:, None] - torch.arange(n, device="cuda")
+    s = torch.einsum("qhd,kd->hqk", q[:, :NH * D].double().view(n, NH, D), kp[:, 0].reshape(n, D).double()) * D ** -0.5
+    s = s.masked_fill((d < 0) | ((d >= window) if window else torch.zeros_like(d, dtype=torch.bool)), -float("inf"))
+    want = torch.einsum("hqk,kd->qhd", s.softmax(-1), vp[:, 0].reshape(n, D).double()).reshape(n, NH * D)
+    rows = (torch.arange(n) < 100) | ((torch.arange(n) >= 127 + window) if window else torch.zeros(n, dtype=torch.bool))
+    torch.testing.assert_close(out[rows].double(), want[rows], **tol(torch.bfloat16))
+
+
 @pytest.mark.parametrize("window", [1, 7, 64, 100])
 def test_tensor_core_attention_window_and_mixed_batch(ops, window):
     o1, o2 = _tc_case(ops, 8, 2, 128, 16, lens=[150, 90, 300, 17, 64], q_lens=[150, 1, 70, 1, 2], window=window, seed=62)
