@@ -617,8 +617,8 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
             const float up = __shfl_up_sync(0xffffffffu, upto, h);
             if (lane >= h) upto += up;
         }
-        const uint32_t reached = __ballot_sync(0xffffffffu, mine > 0.f && before_cta + upto >= target);
-        const uint32_t kept = __ballot_sync(0xffffffffu, mine > 0.f);
+        const uint32_t reached = __ballot_sync(0xffffffffu, last >= 0 && before_cta + upto >= target);
+        const uint32_t kept = __ballot_sync(0xffffffffu, last >= 0);     // (a sum that is no number hides no range that is one)
         const int at = reached ? __ffs(reached) - 1 : kept ? 31 - __clz(kept) : 0;      // (rounding may leave the target beyond all)
         const float front = __shfl_up_sync(0xffffffffu, upto, 1);
         if (lane == at) {

@@ -77,6 +77,15 @@ def test_wide_rows_cut_where_the_plain_sampler_cuts(V, kind):
         assert before - 1e-4 <= u <= float(cdf[got[i]]) + 1e-4, f"case {i}"
 
 
+@pytest.mark.parametrize("at", [(100, 104), (104, 100), (100, 2040), (0, 63)])
+def test_a_wide_row_with_a_logit_that_is_no_number_gives_a_kept_token(at):
+    """Top-k 2 of a row whose largest entries are NaN and a number, in the same part of the row: the number is drawn."""
+    row = torch.zeros(16384)
+    row[at[0]], row[at[1]] = float("nan"), 5.0
+    got, _ = run_sample(row[None].cuda(), [1.0], [2], [1.0], [0.0], [7], [3])
+    assert list(got) == [at[1]]
+
+
 def test_draws_follow_the_distribution():
     """Many counters on one row: the empirical frequencies approach the kept probabilities."""
     V = 50
