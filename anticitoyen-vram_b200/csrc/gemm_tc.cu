@@ -720,15 +720,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }
 
 // ----------------------------------------------------------------------------- host side
+#define GT_PARTS_BYTES (100 * 1024)
 template <int BN>
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, int sm_count, int stages,
                        cudaStream_t stream) {
     using S = GemmShape<BN>;
     if (stages < 2) stages = 2;
     if (stages > S::MAX_STAGES) stages = S::MAX_STAGES;
-    // cluster mode needs room for the peers' partial tiles beside the pipeline; else the global workspace serves
-    int parts = p.cluster && p.splits > 1 ? p.splits - 1 : 0;
-    if (parts && (p.splits > 8 || parts * S::PART_BYTES > 100 * 1024)) { p.cluster = 0; parts = 0; }
+    const int parts = p.cluster ? p.splits - 1 : 0;
     const int aux_bytes = p.qkv && p.swap ? BN * 8 + BN * p.head_dim * 4 : 0;
     while ((parts || aux_bytes) && stages > 2 && S::smem_bytes(stages, parts, aux_bytes) > 226 * 1024) --stages;
     p.stages = stages;
@@ -815,7 +814,9 @@ ACV_API void acv_gemm_tc_test_fault(int wait_limit, int skip_kb) {
 
 // x [M,K] (row stride ldx), w [N,K] (row stride ldw), C [M,N] (row stride ldc) bf16 or float.
 // bn: rows of the B operand per tile (16, 32, 64, 128, 160, 192, 224 or 256); swap: the weight is the A operand.
-// splits > 1 needs workspace of tiles*splits*bn*128 floats and `tiles` zeroed counters.
+// splits > 1: summed inside a cluster (flags bit 0, up to 8 splits, the peers' partial tiles of bn*128 floats within
+// GT_PARTS_BYTES); else needs a workspace of tiles*splits*bn*128 floats and `tiles` zeroed counters that no other product uses
+// until this one is done.
 // status: one int, 0 unless a bounded wait inside the kernel ran out.
 static int gemm_tc_run(GemmParams& p, const void* x, int ldx, const void* w, int ldw, void* C, int ldc, int M, int N, int K,
                        int out_f32, int act, int swap, int bn, int splits, float* workspace, long long workspace_floats,
@@ -847,12 +848,14 @@ static int gemm_tc_run(GemmParams& p, const void* x, int ldx, const void* w, int
     if (splits > p.n_kb) splits = p.n_kb;
     p.kb_per_split = (p.n_kb + splits - 1) / splits;
     p.splits = (p.n_kb + p.kb_per_split - 1) / p.kb_per_split;
+    // cluster mode needs room for the peers' partial tiles beside the pipeline; else the global workspace serves
+    if (p.splits < 2 || p.splits > 8 || (p.splits - 1) * bn * GT_BM * 4 > GT_PARTS_BYTES) p.cluster = 0;
     p.C = C; p.workspace = workspace; p.counters = counters; p.status = status;
     p.wait_limit = g_test_wait_limit ? g_test_wait_limit : GT_WAIT_LIMIT;
     p.skip_kb = g_test_skip_kb;
     g_test_wait_limit = 0; g_test_skip_kb = -1;      // one launch only
     const long long tiles = (long long)p.tiles_a * p.tiles_b;
-    if (p.splits > 1 && (tiles * p.splits * bn * GT_BM > workspace_floats || tiles > n_counters)) return ACV_ERR_SCRATCH;
+    if (p.splits > 1 && !p.cluster && (tiles * p.splits * bn * GT_BM > workspace_floats || tiles > n_counters)) return ACV_ERR_SCRATCH;
     if (tiles * p.splits > 0x7fffffff) return ACV_ERR_SIZE;
     CUtensorMap ma, mb;
     int rc = make_map(&ma, a_ptr, p.RA, K, swap ? ldw : ldx, GT_BM);

@@ -382,9 +382,6 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
 _gemm_scratch: dict = {}
 
 
-GEMM_WORKSPACE_FLOATS = 1 << 22     # what every plan of a device of up to 256 SMs fits in, so that a capture never meets a larger one
-
-
 def _gemm_buffers(device, ws_floats: int, n_counters: int):
     key = str(device)
     have = _gemm_scratch.get(key)
@@ -392,7 +389,7 @@ def _gemm_buffers(device, ws_floats: int, n_counters: int):
         if torch.cuda.is_current_stream_capturing():
             raise KernelError("gemm_tc: workspace would grow during a graph capture; run the shape once first")
         old = have or (torch.empty(0), torch.empty(0), None)
-        ws = torch.empty(max(ws_floats, 2 * old[0].numel(), GEMM_WORKSPACE_FLOATS), device=device, dtype=torch.float32)
+        ws = torch.empty(max(ws_floats, 2 * old[0].numel(), 1 << 20), device=device, dtype=torch.float32)
         cnt = torch.zeros(max(n_counters, 2 * old[1].numel(), 4096), device=device, dtype=torch.int32)
         status = old[2] if old[2] is not None else torch.zeros(1, device=device, dtype=torch.int32)
         if key in _gemm_scratch:
@@ -400,6 +397,20 @@ def _gemm_buffers(device, ws_floats: int, n_counters: int):
         have = (ws, cnt, status)
         _gemm_scratch[key] = have
     return have
+
+
+GEMM_CLUSTER_BYTES = 100 * 1024     # of peers' partial tiles that fit beside a split's pipeline (csrc/gemm_tc.cu)
+
+
+def _split_buffers(device, tiles: int, splits: int, bn: int, cluster: int):
+    """(workspace, counters, status word) of a product: the first two are None where a cluster sums the splits in its shared
+    memory, else they belong to this one call (the allocator hands them out in the order of the current stream, inside a
+    capture from the graph's own memory), so products on several streams share the status word and nothing else."""
+    status = _gemm_buffers(device, 0, 0)[2]
+    if splits <= 1 or (cluster & 1 and splits <= 8 and (splits - 1) * bn * 128 * 4 <= GEMM_CLUSTER_BYTES):
+        return None, None, status
+    return (torch.empty(tiles * splits * bn * 128, device=device, dtype=torch.float32),
+            torch.zeros(tiles, device=device, dtype=torch.int32), status)
 
 
 _sm_counts: dict = {}
@@ -562,12 +573,11 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: tuple | N
     stages = plan[3] if len(plan) > 3 else 8
     cluster = plan[4] if len(plan) > 4 else (1 if swap and 1 < splits <= 8 else 0)
     tiles = (-(-N // 128) * -(-M // bn)) if swap else (-(-M // 128) * -(-N // bn))
-    ws, cnt, status = _gemm_buffers(x.device, tiles * splits * bn * 128 if splits > 1 else 0, tiles)
+    ws, cnt, status = _split_buffers(x.device, tiles, splits, bn, cluster)
     args = (_p(x), x.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K,
             1 if out.dtype == torch.float32 else 0,
             (1 | (int(gate_fn) << 4)) if swiglu_pairs else ((ACTIVATIONS[unary] << 4) if unary else 0), swap, bn, splits, _p(ws),
-            ws.numel(), _p(cnt),
-            cnt.numel(), _p(status), sm_count(x.device), stages, cluster | (2 if static_weights else 0))
+            0 if ws is None else ws.numel(), _p(cnt), 0 if cnt is None else cnt.numel(), _p(status), sm_count(x.device), stages, cluster | (2 if static_weights else 0))
     if bias is not None or (swiglu_pairs and gate_fn == 2):
         if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N or not bias.is_contiguous()):
             raise KernelError("gemm_tc: the bias is a contiguous float32 vector with one entry for each row of the weight")
@@ -610,10 +620,10 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, num_heads: 
     swap, bn, splits, stages = plan[:4]
     cluster = plan[4] if len(plan) > 4 else (1 if swap and 1 < splits <= 8 else 0)
     tiles = (-(-N // 128) * -(-M // bn)) if swap else (-(-M // 128) * -(-N // bn))
-    ws, cnt, status = _gemm_buffers(x.device, tiles * splits * bn * 128 if splits > 1 else 0, tiles)
+    ws, cnt, status = _split_buffers(x.device, tiles, splits, bn, cluster)
     _check(library().acv_gemm_tc_qkv(
-        _p(x), x.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K, swap, bn, splits, _p(ws), ws.numel(),
-        _p(cnt), cnt.numel(), _p(status), sm_count(x.device), stages, cluster | (2 if static_weights else 0), num_heads,
+        _p(x), x.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K, swap, bn, splits, _p(ws),
+        0 if ws is None else ws.numel(), _p(cnt), 0 if cnt is None else cnt.numel(), _p(status), sm_count(x.device), stages, cluster | (2 if static_weights else 0), num_heads,
         num_kv_heads, head_dim, _p(q_weight), _p(k_weight), eps, _p(cos_sin),
         cos_sin.shape[0] if cos_sin is not None else 0, _p(positions), _p(seq_of_token), _p(block_table),
         block_table.stride(0), _p(table_rows), _p(k_pages), _p(v_pages), k_pages.shape[2], k_pages.shape[0], _stream()),
@@ -638,7 +648,8 @@ def status_word(device) -> torch.Tensor:
 
 def reset_after_failure() -> None:
     """After a step whose kernels gave up a wait: the status word back to 0, and the arrival counters of the
-    split products and of the split attention back to 0 (a CTA that gave up never arrived at its tile)."""
+    persistent layer and of the split attention back to 0 (a CTA that gave up never arrived at its tile; a split product's
+    belong to its one call)."""
     for _, cnt, status in _gemm_scratch.values():
         status.zero_()
         cnt.zero_()

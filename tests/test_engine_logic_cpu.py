@@ -256,9 +256,8 @@ def test_the_clamped_unit_refuses_what_its_documentation_refuses(monkeypatch, M,
 
 @pytest.mark.parametrize("sms", [1, 74, 132, 148, 256])
 def test_split_products_share_nothing_between_streams(sms):
-    """Splits of K that a plan asks for are summed inside a cluster (8 CTAs and 100 KB of partial tiles at most), never through
-    the device's one workspace, and the workspace of the first call is large enough for every later one: a capture may
-    meet a shape that never ran before."""
+    """Splits of K that ``gemm_tc_plan`` asks for are summed inside a cluster (8 CTAs and 100 KB of partial tiles at most),
+    through no workspace at all."""
     from acvram_b200.kernels import ops
     for M in (1, 16, 17, 32, 33, 64, 65, 128, 129, 256, 300, 512, 513, 1056):
         for N in list(range(128, 128 * 600, 128 * 7)) + [200, 5120, 4096, 19000]:
@@ -266,7 +265,43 @@ def test_split_products_share_nothing_between_streams(sms):
                 swap, bn, splits = ops.gemm_tc_plan(M, N, K, sms=sms)[:3]
                 if splits > 1:
                     assert swap and splits <= 8 and (splits - 1) * bn * 128 * 4 <= 100 * 1024, (M, N, K)
-                    assert -(-N // 128) * -(-M // bn) * splits * bn * 128 <= ops.GEMM_WORKSPACE_FLOATS, (M, N, K)
+
+
+def test_products_that_split_through_a_workspace_have_one_each(monkeypatch):
+    """The plan by which the experts' router and the wkv decay split a long product has no cluster: each call brings a
+    workspace and counters of its own, of the size that the kernel asks for, inside a capture too, whatever ran before."""
+    from acvram_b200.kernels import ops
+    calls = []
+
+    class Library:
+        def acv_gemm_tc(self, *args):
+            calls.append(args)
+            return 0
+
+    kept = []
+    for name in ("empty", "zeros"):         # (kept, so that no address comes twice)
+        monkeypatch.setattr(torch, name, lambda *a, make=getattr(torch, name), **k: kept.append(make(*a, **k)) or kept[-1])
+    monkeypatch.setattr(ops, "library", Library)
+    monkeypatch.setattr(ops, "_need_cuda", lambda *a: None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "sm_count", lambda *a: 148)
+    monkeypatch.setattr(ops, "_gemm_scratch", {})
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    ops.gemm_tc(torch.zeros(4, 64).bfloat16(), torch.zeros(128, 64).bfloat16(), torch.zeros(4, 128))       # (a product ran before)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    w = torch.zeros(64, 2048).bfloat16()
+    seen = set()
+    for T in (512, 4096, 8192, 8192):
+        ops.gemm_tc(torch.zeros(T, 2048).bfloat16(), w, torch.zeros(T, 64), plan=(0, 128, 8, 4, 0))
+        workspace, floats, counters, n_counters = calls[-1][14:18]
+        tiles = T // 128
+        assert floats >= tiles * 8 * 128 * 128 and n_counters >= tiles
+        for address, size in ((workspace, 4 * floats), (counters, 4 * n_counters)):
+            address = getattr(address, "value", address)
+            assert address and not any(a < address + size and address < b for a, b in seen)
+            seen.add((address, address + size))
+    ops.gemm_tc(torch.zeros(8, 2048).bfloat16(), w, torch.zeros(8, 64), plan=(1, 16, 8, 8))
+    assert calls[-1][15] == 0 and calls[-1][17] == 0, "a cluster needs neither"
 
 
 def test_the_splits_of_decode_attention_follow_what_fits_the_device(monkeypatch):

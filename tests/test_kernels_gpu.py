@@ -682,6 +682,27 @@ def test_gemm_tc_as_planned(ops, M, N, K, form):
     assert ops.gemm_status() == 0
 
 
+def test_a_split_product_of_many_tokens_inside_a_capture(ops):
+    """The router's plan for long steps, in a graph that nothing of its size ran before, twice in a row: the first product's
+    counters and partial sums are not the second's."""
+    x, w = rnd(8200, 2048, dtype=torch.bfloat16, seed=63), rnd(64, 2048, dtype=torch.bfloat16, scale=0.05, seed=64)
+    one, two = (torch.full((8200, 64), 7.0, device="cuda") for _ in range(2))
+    ops.gemm_tc(x[:4], w, one[:4])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.gemm_tc(x, w, one, plan=(0, 128, 8, 4, 0))
+        ops.gemm_tc(x[:600], w, two[:600], plan=(0, 128, 8, 4, 0))
+    for _ in range(3):
+        one.fill_(7.0)
+        two.fill_(7.0)
+        graph.replay()
+        want = x.double() @ w.double().T
+        torch.testing.assert_close(one.double(), want, rtol=1e-4, atol=1e-3)
+        torch.testing.assert_close(two[:600].double(), want[:600], rtol=1e-4, atol=1e-3)
+    assert ops.gemm_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(129, 3072, 4096), (200, 512, 4096), (256, 4608, 8192)])
 def test_clamped_unit_keeps_its_tokens_on_the_rows(ops, M, N, K):
     """The product with the clamped gated unit has no form for shared tiles: sizes for which a plain product takes one."""
