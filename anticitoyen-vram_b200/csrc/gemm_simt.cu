@@ -59,6 +59,7 @@ struct GsTile {
     static constexpr int SMEM = (STAGES * STAGE > BM * BN ? STAGES * STAGE : BM * BN) * 4;
     static constexpr int RESIDENT = RESIDENT_;           // CTAs that share an SM
     static constexpr int M_WARPS = WM, ROWS = MI, COLS = NJ, THREADS = NW * 32, KS = KS_;
+    static_assert(RESIDENT * (SMEM + 1024) <= 228 * 1024, "RESIDENT CTAs of this tile do not fit an SM's shared memory");
 };
 
 struct GsArgs {
@@ -242,7 +243,7 @@ static int gs_launch(const GsArgs& p, int parts, int batches, cudaStream_t strea
 
 typedef GsTile<2, 1, 1, 1, 1, 6, 4, 4> GsRow1Narrow;       // 1 x 64
 typedef GsTile<4, 1, 1, 1, 1, 5, 2, 4> GsRow1;             // 1 x 128
-typedef GsTile<2, 1, 1, 4, 1, 6, 4, 4> GsRow4Narrow;       // 4 x 64
+typedef GsTile<2, 1, 1, 4, 1, 6, 3, 4> GsRow4Narrow;       // 4 x 64
 typedef GsTile<4, 1, 1, 4, 1, 5, 2, 4> GsRow4;             // 4 x 128
 typedef GsTile<4, 1, 1, 8, 1, 4, 2, 4> GsRow8;             // 8 x 128
 typedef GsTile<4, 1, 2, 8, 2, 4, 2, 4> GsRow16;            // 16 x 128
@@ -255,7 +256,7 @@ typedef GsTile<8, 4, 2, 8, 4, 3, 2, 2> GsWide64;           // 64 x 128
 // weights' bytes at the memory's speed).  Rows of a tile that hold nothing cost what full ones do, so the narrowest tile
 // that holds all rows is the only one asked for up to 16 of them.
 struct GsWay { int bm, bn, resident, one, full; };
-static const GsWay GS_WAYS[9] = {{1, 64, 4, 400, 1420}, {1, 128, 2, 760, 1420}, {4, 64, 4, 420, 1700}, {4, 128, 2, 800, 1480},
+static const GsWay GS_WAYS[9] = {{1, 64, 4, 400, 1420}, {1, 128, 2, 760, 1420}, {4, 64, 3, 420, 1275}, {4, 128, 2, 800, 1480},
                                  {8, 128, 2, 1100, 1900}, {16, 128, 2, 1700, 2750}, {32, 64, 3, 1800, 3400}, {64, 64, 3, 2400, 5850},
                                  {64, 128, 2, 4100, 6500}};
 
