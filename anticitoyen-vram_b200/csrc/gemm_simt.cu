@@ -277,11 +277,16 @@ static void gs_plan(int M, int N, int K, int batches, int sms, int* way, int* pa
     }
 }
 
-static int gs_run_async(const GsArgs& p, int batches, cudaStream_t stream) {
-    int device = 0, sms = 0;
+static int gs_multiprocessors(int* sms) {
+    int device = 0;
     cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e != cudaSuccess) return (int)e;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device);
+    return (int)e;
+}
+
+static int gs_run_async(const GsArgs& p, int batches, cudaStream_t stream) {
+    int sms = 0;
+    if (const int e = gs_multiprocessors(&sms)) return e;
     int way = 0, parts = 1;
     gs_plan(p.M, p.N, p.K, batches, sms, &way, &parts);
     switch (way) {
@@ -300,10 +305,12 @@ static int gs_run_async(const GsArgs& p, int batches, cudaStream_t stream) {
 // operands without 16-byte pieces, or bfloat16 (a fallback of odd sizes): two tiles, a cluster where there are few of them
 template <typename TI, typename TO>
 static int gs_run_any(const GsArgs& p, int batches, cudaStream_t stream) {
+    int sms = 0;
+    if (const int e = gs_multiprocessors(&sms)) return e;
     const long long tiles = p.M <= 4 ? (p.N + 127) / 128 : (long long)((p.M + 63) / 64) * ((p.N + 63) / 64);
     const int gl = gs_group_length(p.K), filled = (p.K + gl - 1) / gl;
     int parts = 1;
-    while (parts < GS_GROUPS && parts < filled && tiles * batches * parts < 148) parts *= 2;
+    while (parts < GS_GROUPS && parts < filled && tiles * batches * parts < sms) parts *= 2;
     return p.M <= 4 ? gs_launch<TI, TO, false, GsRow4>(p, parts, batches, stream) : gs_launch<TI, TO, false, GsSquare64>(p, parts, batches, stream);
 }
 
