@@ -515,15 +515,16 @@ attn_token_kernel(const AgArgs a, int parts, int stride) {
     const int part = blockIdx.x % parts;
     const int chunks = (G + RG - 1) / RG, kvh = blockIdx.y / chunks, h0 = kvh * G + (blockIdx.y % chunks) * RG;
     const int n_heads = min(RG, (kvh + 1) * G - h0);
-    // one token a cluster; with a stride, without clusters, those of the `stride` tokens x, x + gridDim.x .. that are alone
-    // (bit i: token x + i gridDim.x; all asked for at once, since a look is a round trip to memory)
+    // one token a cluster; with a stride those of the `stride` tokens x, x + X .. that are alone, X clusters in a row of the grid
+    // (bit i: token x + i X; all asked for at once, since a look is a round trip to memory)
+    const int x = blockIdx.x / parts, X = gridDim.x / parts;
     uint32_t mine = 1;
     if (stride) {
-        const int cand = blockIdx.x + lane * gridDim.x;
+        const int cand = x + lane * X;
         mine = __ballot_sync(0xffffffffu, lane < stride && cand < a.T && ag_alone(a.seq_of_token, cand, a.T));
     }
     for (; mine; mine &= mine - 1) {
-        const int t = stride ? blockIdx.x + (__ffs(mine) - 1) * gridDim.x : blockIdx.x / parts;
+        const int t = x + (__ffs(mine) - 1) * X;
         if (stride) __syncthreads();        // the token before is done with the shared memory
         const int p = a.positions[t], seq = a.seq_of_token[t];
         const int* bt = a.block_table + (size_t)(a.bt_rows ? a.bt_rows[seq] : seq) * a.bt_stride;
@@ -581,9 +582,9 @@ attn_token_kernel(const AgArgs a, int parts, int stride) {
                     const float4* mine = reinterpret_cast<const float4*>(sm_s[warp][r] + lane * 8);
                     const float4 x0 = mine[lane >> 2 & 1], x1 = mine[(lane >> 2 & 1) ^ 1];
                     const float dot = ((((((x0.x + x0.y) + x0.z) + x0.w) + x1.x) + x1.y) + x1.z) + x1.w;
-                    const float x = row >= 0 ? fmaf(-slope, (float)(p - j), dot) : -INFINITY;
-                    const float m_new = fmaxf(m[r], warp_max(x)), alpha = ag_rescale(m[r], m_new);
-                    const float w = ag_weight(x, m_new);
+                    const float score = row >= 0 ? fmaf(-slope, (float)(p - j), dot) : -INFINITY;
+                    const float m_new = fmaxf(m[r], warp_max(score)), alpha = ag_rescale(m[r], m_new);
+                    const float w = ag_weight(score, m_new);
                     l[r] = __fadd_rn(__fmul_rn(l[r], alpha), w);
                     m[r] = m_new;
 #pragma unroll
@@ -691,7 +692,7 @@ static int launch_token(const AgArgs& a, int parts, int stride, cudaStream_t str
     const int smem = AG_CHUNKS(RG, VC) / parts * RG * a.DV * 4;
     static AcvSmemConfig cfg;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
-    const int G = a.NH / a.NKV, x = stride ? (a.T + stride - 1) / stride : a.T * parts;
+    const int G = a.NH / a.NKV, x = (stride ? (a.T + stride - 1) / stride : a.T) * parts;
     acv_launch_cluster(PDL_ATTN, dim3(parts, 1, 1), kernel, dim3(x, a.NKV * ((G + RG - 1) / RG)), dim3(AT1_WARPS * 32), smem, stream, a, parts, stride);
     return acv_launch_status();
 }
@@ -707,16 +708,21 @@ static int launch_rows(const AgArgs& a, int skip_alone, cudaStream_t stream) {
     return acv_launch_status();
 }
 
-// Steps of up to AG_FEW tokens: every token by itself, with as many CTAs to a token and kv-head as come in one wave (two to
-// an SM; 16 requests of 1500 keys, 16 heads on 8, with 1, 2, 4, 8: 206, 110, 150, 165 us).  More tokens: rows of portions, then the
-// tokens that are alone
-// (a portion's 64 rows read each key once for all of them, one token's warps once for its own heads).  A CTA looks at as
+// Steps of requests that bring one token each (the caller says so; the results are the same whether it does), and of up to
+// AG_FEW tokens and AG_FEW_ROWS (token, head) rows: every token by itself.  Others: rows of portions, then the tokens that are
+// alone (a portion's 64 rows read each key once for all of them, one token's warps once for its own heads).  Below the line
+// lie tokens that fill half a wave (bfloat16, portions of 20, 17 and 9 tokens, every token by itself against both kernels: 8 heads on 8 of 64 11.4
+// and 15.2 us, 14 on 2 15.7 and 25.8, 5 on 1 of 256 24.4 and 41.7), above it those that take several (32 on 8 of 128 27.9 and
+// 18.7, 40 on 8 39.9 and 29.9; one portion of 64 tokens: 16 on 8 36.6 and 29.6, 40 on 8 77.2 and 31.5).  As many CTAs to a
+// token and kv-head as come in one wave (two to
+// an SM; 16 requests of 1500 keys, 16 heads on 8, with 1, 2, 4, 8: 206, 110, 150, 165 us).  A CTA looks at as
 // many tokens as leave eight CTAs to an SM, at most AG_STRIDE: all of them may be alone, and one behind the other took 65
 // requests of 500 keys 532 us where 64 take 144 (150 with a CTA each); of a portion's thousands none are.
 #define AG_FEW 64
+#define AG_FEW_ROWS 700
 #define AG_STRIDE 8
 template <typename T>
-static int launch_tiled(AgArgs& a, cudaStream_t stream) {
+static int launch_tiled(AgArgs& a, bool singles, cudaStream_t stream) {
     int device = 0, sms = 0;
     cudaError_t err = cudaGetDevice(&device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -724,15 +730,15 @@ static int launch_tiled(AgArgs& a, cudaStream_t stream) {
     const int G = a.NH / a.NKV, wide = (a.D > 128 || a.DV > 128) ? 2 : 1;
     const int rg = G == 1 ? 1 : G == 2 || wide == 2 ? 2 : 4;
     a.chunks = AG_CHUNKS(rg, wide);
-    const bool few = a.T <= AG_FEW;
-    if (!few) {
+    const bool each = singles || (a.T <= AG_FEW && a.T * a.NH <= AG_FEW_ROWS);
+    if (!each) {
         const int e = wide == 1 ? launch_rows<T, 1>(a, 1, stream) : launch_rows<T, 2>(a, 1, stream);
         if (e) return e;
     }
     const long long ctas = (long long)a.T * a.NKV * ((G + rg - 1) / rg);
     int parts = 1;
-    while (few && parts < 8 && ctas * parts <= sms) parts *= 2;
-    const int stride = few ? 0 : (int)max(1ll, min((long long)AG_STRIDE, ctas / (8 * sms)));
+    while (parts < 8 && ctas * parts <= sms) parts *= 2;
+    const int stride = each ? 0 : parts > 1 ? 1 : (int)max(1ll, min((long long)AG_STRIDE, ctas / (8 * sms)));
     if (wide == 2) return rg == 1 ? launch_token<T, 1, 2>(a, parts, stride, stream) : launch_token<T, 2, 2>(a, parts, stride, stream);
     return rg == 1 ? launch_token<T, 1, 1>(a, parts, stride, stream) : rg == 2 ? launch_token<T, 2, 1>(a, parts, stride, stream)
                                                                           : launch_token<T, 4, 1>(a, parts, stride, stream);
@@ -763,12 +769,13 @@ static int launch_generic(const void* q, int q_stride, void* out, int out_stride
     return acv_launch_status();
 }
 
+// singles: no request brings more than one token (a hint for the choice of kernels).
 ACV_API int acv_attention_generic(const void* q, int q_stride, void* out, int out_stride, const void* k_pages,
                                   const void* v_pages, const int* positions, const int* seq_of_token,
                                   const int* block_table, int bt_stride, const int* bt_rows, int T_tokens, int NH, int NKV, int D,
                                   int page_size, int num_pages, float scale, int window, int dtype,
                                   int value_dim, int keep_first, const float* sinks, const float* slopes, const void* gate,
-                                  int gate_stride, cudaStream_t stream) {
+                                  int gate_stride, int singles, cudaStream_t stream) {
     if (T_tokens <= 0) return 0;
     const int DV = value_dim > 0 ? value_dim : D;
     if (D <= 0 || D > 1024 || DV > 512 || NKV <= 0 || NH % NKV) return ACV_ERR_SIZE;
@@ -781,7 +788,7 @@ ACV_API int acv_attention_generic(const void* q, int q_stride, void* out, int ou
         (dtype == ACV_F32 || dtype == ACV_BF16)) {
         AgArgs a = {q, k_pages, v_pages, gate, out, positions, seq_of_token, block_table, bt_rows, sinks, slopes,
                           q_stride, out_stride, gate_stride, bt_stride, T_tokens, NH, NKV, D, DV, page_size, num_pages, window, keep_first, v_row, 0, scale};
-        return dtype == ACV_F32 ? launch_tiled<float>(a, stream) : launch_tiled<bf16>(a, stream);
+        return dtype == ACV_F32 ? launch_tiled<float>(a, singles != 0, stream) : launch_tiled<bf16>(a, singles != 0, stream);
     }
     if (dtype == ACV_F32)
         return launch_generic<float>(q, q_stride, out, out_stride, k_pages, v_pages, positions, seq_of_token,

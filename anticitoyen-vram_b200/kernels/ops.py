@@ -71,7 +71,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "acv_swiglu": [P, P, I, I, I, P],
         "acv_add_bias": [P, I, P, I, I, I, P],
         "acv_qk_norm_rope_append": [P, I, I, I, I, I, P, P, F, P, I, I, P, P, P, I, P, P, P, I, I, I, I, F, I, P],
-        "acv_attention_generic": [P, I, P, I, P, P, P, P, P, I, P, I, I, I, I, I, I, F, I, I, I, I, P, P, P, I, P],
+        "acv_attention_generic": [P, I, P, I, P, P, P, P, P, I, P, I, I, I, I, I, I, F, I, I, I, I, P, P, P, I, I, P],
         "acv_add_group_rmsnorm": [P, P, F, P, P, P, I, I, I, F, I, I, P],
         "acv_input_conv": [P, P, P, P, P, P, P, I, I, I, I, P, P],
         "acv_add_group_rmsnorm_conv": [P, P, F, P, P, P, P, P, I, I, I, F, I, I, I, P],
@@ -346,12 +346,13 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor,
                       num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
                       table_rows: torch.Tensor | None = None, value_dim: int = 0, keep_first: int = 0,
                       sinks: torch.Tensor | None = None, slopes: torch.Tensor | None = None,
-                      gate: torch.Tensor | None = None) -> torch.Tensor:
+                      gate: torch.Tensor | None = None, singles: bool = False) -> torch.Tensor:
     """Paged causal attention for every token of the step.  q: rows of num_heads*head_dim (row stride free).
     ``value_dim`` > 0: value rows (and the result's heads) of that size; ``keep_first``: the first keys of a request
     that stay visible behind the window.  ``sinks`` (float32 [num_heads]): exp(sink_h) joins the softmax's denominator
     (a score with no key and no value); ``slopes`` (float32 [num_heads]): slope_h * (i - j) is taken off the score of
-    query i and key j.  ``gate`` (a view like ``out``): the result is multiplied by sigmoid(gate) in float."""
+    query i and key j.  ``gate`` (a view like ``out``): the result is multiplied by sigmoid(gate) in float.
+    ``singles``: no request of the step brings more than one token (spares the kernel for portions; the results are the same)."""
     _need_cuda(q, out, k_pages)
     _head_vectors(num_heads, sinks, slopes)
     T = q.shape[0]
@@ -359,7 +360,7 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor,
         _p(q), q.stride(0), _p(out), out.stride(0), _p(k_pages), _p(v_pages), _p(positions), _p(seq_of_token),
         _p(block_table), block_table.stride(0), _p(table_rows), T, num_heads, num_kv_heads, head_dim, k_pages.shape[2],
         k_pages.shape[0], scale, window, dtype_code(q.dtype), int(value_dim), int(keep_first), _p(sinks), _p(slopes), *_gate_args(gate, out),
-        _stream()), "attention_generic")
+        int(singles), _stream()), "attention_generic")
     return out
 
 
@@ -986,7 +987,8 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pag
             raise KernelError("attention: the chunked mask is built for the tensor-core kernels' sizes only")
         return attention_generic(qkv, out, k_pages, v_pages, ctx.positions, ctx.seq_of_token, block_table, num_heads,
                                  num_kv_heads, head_dim, scale, window, table_rows=rows, value_dim=value_dim,
-                                 keep_first=keep_first, sinks=sinks, slopes=slopes, gate=gate)
+                                 keep_first=keep_first, sinks=sinks, slopes=slopes, gate=gate,
+                                 singles=getattr(ctx, "num_seqs", 0) == qkv.shape[0])
     if w["n_dec"]:
         kv = min(w["max_dec_kv"], window + keep_first) if window > 0 else w["max_dec_kv"]
         kv = min(kv, chunk) if chunk > 0 else kv
@@ -1846,7 +1848,7 @@ def attention_latent(q: torch.Tensor, out: torch.Tensor, pages: torch.Tensor, ct
             float(scale), int(window), n_split, _p(acc), _p(ml), _p(sinks), _p(status_word(q.device)), _stream()), "attention_latent_tc")
         return out
     return attention_generic(q, out, pages, pages, ctx.positions, ctx.seq_of_token, block_table, num_heads, 1, row, scale,
-                             window, table_rows=rows, value_dim=rank, sinks=sinks)
+                             window, table_rows=rows, value_dim=rank, sinks=sinks, singles=getattr(ctx, "num_seqs", 0) == q.shape[0])
 
 
 LATENT_SPLIT_KEYS = 128         # no share of a one-token request's kept rows is shorter than this

@@ -280,13 +280,13 @@ def test_attention_generic_one_order_of_sums(ops, dtype, NH, NKV, D, DV, window,
     qs = {b: rnd(lens[b], NH * D, dtype=dtype, seed=80 + b) for b in range(B)}
     gates = {b: rnd(lens[b], NH * DV, dtype=dtype, seed=200 + b) for b in range(B)}
 
-    def step(parts):        # (request, first token, end) of each portion
+    def step(parts, singles=False):        # (request, first token, end) of each portion
         cat = lambda x: torch.cat([x[b][i:j] for b, i, j in parts])
         pos = torch.cat([torch.arange(i, j) for _, i, j in parts]).to(torch.int32).cuda()
         seq = torch.repeat_interleave(torch.tensor([b for b, _, _ in parts]), torch.tensor([j - i for _, i, j in parts])).to(torch.int32).cuda()
         out = torch.full((len(pos), NH * DV), float("nan"), device="cuda", dtype=dtype)
         ops.attention_generic(cat(qs), out, kp, vp, pos, seq, table, NH, NKV, D, D ** -0.5, window, value_dim=DV if DV != D else 0,
-                              keep_first=keep, sinks=sinks, slopes=slopes, gate=cat(gates))
+                              keep_first=keep, sinks=sinks, slopes=slopes, gate=cat(gates), singles=singles)
         return dict(zip(parts, out.split([j - i for _, i, j in parts])))
 
     few, many = [(b, 0, 1) for b in range(5, 8)], [(b, 0, 1) for b in range(5, 85)]
@@ -297,6 +297,7 @@ def test_attention_generic_one_order_of_sums(ops, dtype, NH, NKV, D, DV, window,
             for others in ([], few, many, [(3, 0, 1), ((b + 1) % 5, 0, min(66, lens[(b + 1) % 5]))]):
                 got = step(others[:1] + [(b, i, j)] + others[1:])[(b, i, j)]
                 assert torch.equal(got, whole[b][i:j]), (b, i, j, len(others))
+            assert torch.equal(step([(b, i, j)], singles=True)[(b, i, j)], whole[b][i:j]), (b, i, j)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
