@@ -82,9 +82,12 @@ gemm_simt_kernel(const GsArgs p, int parts) {
     const int row0 = (warp % T::M_WARPS) * TY * MI + ty, col0 = (warp / T::M_WARPS) * TX * NJ + tx;     // in the tile
     const int part = blockIdx.x % parts;
     const int m0 = blockIdx.y * BM, n0 = (blockIdx.x / parts) * BN;
-    const int gl = gs_group_length(p.K), groups = GS_GROUPS / parts;
-    const int k_begin = part * groups * gl;
-    const int k_end = min(p.K, k_begin + groups * gl);
+    const int gl = gs_group_length(p.K), share_of_k = GS_GROUPS / parts * gl;
+    const int k_begin = part * share_of_k;
+    const int k_end = min(p.K, k_begin + share_of_k);
+    // (as many groups as K reaches, rounded up to a whole subtree: the others would add nothing)
+    int groups = 1;
+    while (groups * parts < GS_GROUPS && k_begin + groups * gl < k_end) groups *= 2;
     const int iters = k_end > k_begin ? (k_end - k_begin + GS_BK - 1) / GS_BK : 0;
 
     float acc[MI][NJ];
@@ -250,31 +253,35 @@ typedef GsTile<4, 1, 2, 8, 2, 4, 2, 4> GsRow16;            // 16 x 128
 typedef GsTile<4, 2, 4, 4, 4, 4, 3, 4> GsRow32;            // 32 x 64
 typedef GsTile<8, 4, 2, 8, 2, 3, 3, 2> GsSquare64;         // 64 x 64
 typedef GsTile<8, 4, 2, 8, 4, 3, 2, 2> GsWide64;           // 64 x 128
+// 64 x 64 with rows by way of registers, which three CTAs to an SM have not enough of
+typedef GsTile<8, 4, 2, 8, 2, 2, 2, 2> GsSquare64Loads;
 
 // Which tile and how many CTAs to a tile: the way whose busiest SM is done first.  `one` and `full`: cycles for 32 k of a
 // CTA that has its SM to itself and of as many as fit beside each other, measured (a tile's cycles for few rows are its
 // weights' bytes at the memory's speed).  Rows of a tile that hold nothing cost what full ones do, so the narrowest tile
 // that holds all rows is the only one asked for up to 16 of them.
 struct GsWay { int bm, bn, resident, one, full; };
-static const GsWay GS_WAYS[9] = {{1, 64, 4, 400, 1420}, {1, 128, 2, 760, 1420}, {4, 64, 3, 420, 1275}, {4, 128, 2, 800, 1480},
+static const GsWay GS_WAYS[10] = {{1, 64, 4, 400, 1420}, {1, 128, 2, 760, 1420}, {4, 64, 3, 420, 1275}, {4, 128, 2, 800, 1480},
                                  {8, 128, 2, 1100, 1900}, {16, 128, 2, 1700, 2750}, {32, 64, 3, 1800, 3400}, {64, 64, 3, 2400, 5850},
-                                 {64, 128, 2, 4100, 6500}};
+                                 {64, 128, 2, 4100, 6500}, {64, 64, 2, 2400, 4125}};
 
-static void gs_plan(int M, int N, int K, int batches, int sms, int* way, int* parts) {
-    const int gl = gs_group_length(K), filled = (K + gl - 1) / gl;
-    const int first = M <= 1 ? 0 : M <= 4 ? 2 : M <= 8 ? 4 : M <= 16 ? 5 : 6, last = M <= 1 ? 1 : M <= 4 ? 3 : M <= 8 ? 4 : M <= 16 ? 5 : 8;
+// What is counted of K: the stages of the CTA that has most of them (groups behind K have none, and a cluster that K does not
+// reach is no help: 64 rows of 64 x 64 took 11 us as two CTAs of which one was empty, 5 as one).
+static double gs_cost(const GsWay& g, int c, int M, int N, int K, int batches, int sms) {
+    const int gl = gs_group_length(K), stages = min((K + GS_BK - 1) / GS_BK, GS_GROUPS / c * (gl / GS_BK));
+    const long long tiles = (long long)((M + g.bm - 1) / g.bm) * ((N + g.bn - 1) / g.bn) * batches;
+    const long long each = (tiles * c + sms - 1) / sms, rounds = each / g.resident, rest = each % g.resident;
+    const double iter = rounds * (double)g.full + (rest ? g.one + (rest - 1) * (double)(g.full - g.one) / (g.resident - 1) : 0.);
+    return iter * stages + (rounds + (rest > 0)) * 2500.;         // a CTA's first stages and its way out
+}
+
+static void gs_plan(int M, int N, int K, int batches, int sms, int first, int last, int* way, int* parts) {
     double best = -1.;
-    for (int w = first; w <= last; ++w) {
-        const GsWay& g = GS_WAYS[w];
-        const long long tiles = (long long)((M + g.bm - 1) / g.bm) * ((N + g.bn - 1) / g.bn) * batches;
-        for (int c = 1; c <= GS_GROUPS && c < 2 * filled; c *= 2) {
-            const long long each = (tiles * c + sms - 1) / sms, rounds = each / g.resident, rest = each % g.resident;
-            const double iter = rounds * (double)g.full + (rest ? g.one + (rest - 1) * (double)(g.full - g.one) / (g.resident - 1) : 0.);
-            // a CTA's first stages and its way out
-            const double t = iter * (GS_GROUPS / c) * (gl / GS_BK) + (rounds + (rest > 0)) * 2500.;
+    for (int w = first; w <= last; ++w)
+        for (int c = 1; c <= GS_GROUPS; c *= 2) {
+            const double t = gs_cost(GS_WAYS[w], c, M, N, K, batches, sms);
             if (best < 0. || t < best) { best = t; *way = w; *parts = c; }
         }
-    }
 }
 
 static int gs_multiprocessors(int* sms) {
@@ -288,7 +295,8 @@ static int gs_run_async(const GsArgs& p, int batches, cudaStream_t stream) {
     int sms = 0;
     if (const int e = gs_multiprocessors(&sms)) return e;
     int way = 0, parts = 1;
-    gs_plan(p.M, p.N, p.K, batches, sms, &way, &parts);
+    const int M = p.M, first = M <= 1 ? 0 : M <= 4 ? 2 : M <= 8 ? 4 : M <= 16 ? 5 : 6, last = M <= 1 ? 1 : M <= 4 ? 3 : M <= 8 ? 4 : M <= 16 ? 5 : 8;
+    gs_plan(M, p.N, p.K, batches, sms, first, last, &way, &parts);
     switch (way) {
         case 0: return gs_launch<float, float, true, GsRow1Narrow>(p, parts, batches, stream);
         case 1: return gs_launch<float, float, true, GsRow1>(p, parts, batches, stream);
@@ -302,16 +310,14 @@ static int gs_run_async(const GsArgs& p, int batches, cudaStream_t stream) {
     }
 }
 
-// operands without 16-byte pieces, or bfloat16 (a fallback of odd sizes): two tiles, a cluster where there are few of them
+// operands without 16-byte pieces, or bfloat16 (a fallback of odd sizes): two tiles
 template <typename TI, typename TO>
 static int gs_run_any(const GsArgs& p, int batches, cudaStream_t stream) {
     int sms = 0;
     if (const int e = gs_multiprocessors(&sms)) return e;
-    const long long tiles = p.M <= 4 ? (p.N + 127) / 128 : (long long)((p.M + 63) / 64) * ((p.N + 63) / 64);
-    const int gl = gs_group_length(p.K), filled = (p.K + gl - 1) / gl;
-    int parts = 1;
-    while (parts < GS_GROUPS && parts < filled && tiles * batches * parts < sms) parts *= 2;
-    return p.M <= 4 ? gs_launch<TI, TO, false, GsRow4>(p, parts, batches, stream) : gs_launch<TI, TO, false, GsSquare64>(p, parts, batches, stream);
+    int way = 0, parts = 1;
+    gs_plan(p.M, p.N, p.K, batches, sms, p.M <= 4 ? 3 : 9, p.M <= 4 ? 3 : 9, &way, &parts);
+    return p.M <= 4 ? gs_launch<TI, TO, false, GsRow4>(p, parts, batches, stream) : gs_launch<TI, TO, false, GsSquare64Loads>(p, parts, batches, stream);
 }
 
 // in_dtype: type of A and W; out_dtype: type of C.  `batches` products side by side (a head's own matrix for each
