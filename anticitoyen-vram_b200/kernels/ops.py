@@ -438,11 +438,16 @@ def sm_count(device=None) -> int:
 #   6 instead of 4, three feed-forwards of 5 tokens 102.5 -> 94.5 us; 40 tiles (5120 x 17408) 3 instead of 4, two of
 #   32 tokens 211 -> 178.  Between a half and one tile per SM two shallower CTAs share an SM (the 96 tiles of 12288 x 2048:
 #   six feed-forwards of 12 tokens 154 -> 132 us with 3 splits of 3 stages, of 64 tokens 258 -> 188 unsplit), and from 1.5
-#   tiles on one CTA a tile with 3 or 4 stages, as many to an SM as its share of the tiles.
+#   tiles on one CTA a tile with 4 stages, as many to an SM as its share of the tiles (330 to 440 tiles of 16 tokens with
+#   3, 4, 8 stages: 18.2, 17.4, 21.7 to 73.3, 71.5, 74.4 us).
+#   Where K is short the hand-over of a split outweighs the k-blocks that it saves, and that is where the borders in K lie: 7 splits
+#   instead of 4 from 32 k-blocks on (a split has 4 to 5 of them; 15 tiles of 16 tokens 6.1 -> 5.7 us), with the larger partial tiles of 32
+#   tokens from 48 (at 32 k-blocks 7.2 both, at 48 8.6 -> 8.1); 5 splits instead of the 6 that fit for 32 tokens under 64 k-blocks (16 to 22
+#   tiles: 7.4 -> 7.0 to 8.2 -> 7.5 us at 32 k-blocks, 8.6 -> 8.2 at 48, equal from 64 on).
 INF = float("inf")
 GEMM_FEW_TOKENS_RULES = (
-    (2.2,    3.0,    0,   INF, 16, 16,  1, 3),
-    (2.0,    2.2,    0,   INF, 16, 64,  1, 4),
+    (2.0,    3.0,    0,   INF, 16, 16,  1, 4),
+    (2.0,    2.2,    0,   INF, 32, 64,  1, 4),
     (2.0,    INF,    0,   INF, 16, 64,  1, 8),
     (1.5,    2.0,    0,   INF, 16, 16,  1, 4),
     (1.0,    2.0,    0,   INF, 16, 16,  2, 3),
@@ -451,8 +456,8 @@ GEMM_FEW_TOKENS_RULES = (
     (0.0,    0.1014, 32,  INF, 16, 16,  7, 6),
     (0.0,    0.1014, 48,  INF, 32, 32,  7, 6),
     (0.1014, 0.149,  32,  INF, 16, 16,  6, 8),
-    (0.1014, 0.1149, 32,  INF, 32, 32,  5, 6),
-    (0.1149, 0.149,  32,  INF, 32, 32,  6, 6),
+    (0.1014, 0.149,  32,  64,  32, 32,  5, 6),
+    (0.1014, 0.149,  64,  INF, 32, 32,  6, 6),
     (0.149,  0.176,  128, INF, 32, 32,  5, 8),
     (0.0,    0.2231, 48,  INF, 64, 64,  4, 6),
     (0.2231, 0.3041, 128, INF, 16, 64,  3, 8),

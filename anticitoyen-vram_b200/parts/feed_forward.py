@@ -285,7 +285,8 @@ class RoutedExperts(FeedForward):
         if self.router_linear is not None:
             # many tokens against a few dozen router rows: one column of tiles, so the reduction is split eight ways
             # to put more than a ninth of the SMs to work
-            # (a few tokens: that column is one tile, whose k-blocks a cluster of eight shares instead of four)
+            # (a few tokens: that column is one tile, whose k-blocks a cluster of eight shares; the general rule's seven take
+            # 6.6-7.1 us instead of 6.3-6.9, 64 rows of width 4096, 4 and 16 tokens)
             plan = None
             if h.dtype == torch.bfloat16 and H >= 2048 and self.router_linear.out_features <= 128:
                 plan = (0, 128, 8, 4, 0) if T >= 512 else (1, 16, 8, 8) if T <= 16 else None
