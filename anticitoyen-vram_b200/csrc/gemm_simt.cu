@@ -1,11 +1,12 @@
 // C[M,N] = A[M,K] . W[N,K]^T on the CUDA cores, accumulated in true 32-bit
 // (FFMA; no tensor-core mode, hence no TF32 anywhere).  It is the matrix product
-// of the 32-bit path of the model, and it computes logits in float from bfloat16
+// of the 32-bit path of the model for K under GF_MIN_K (longer float sums are made of exact parts on the
+// tensor cores, gemm_split_tc.cu; the entry points here choose), and it computes logits in float from bfloat16
 // operands (the reference upcasts the head's input and accumulates and returns
 // float32, acvram/engine/model.py:369-410; products of bfloat16 values are exact
 // in float, so float accumulation of bfloat16 operands is that computation).
 //
-// The order of a sum is a property of K alone, so a row's result does not depend on
+// The order of a sum is a property of K alone (and so is which of the two makes it), so a row's result does not depend on
 // the other rows, on M, N or the tile that computes it: K is cut into eight groups of
 // gs_group_length(K) consecutive elements; a group is one chain of fused multiply-adds in
 // ascending order; the groups are added as a balanced tree,
@@ -22,6 +23,7 @@
 // stage; operands that are bfloat16 or not made of 16-byte pieces go through registers
 // instead (ASYNC = false).
 #include "common.cuh"
+#include "gemm_split_tc.h"
 
 #define GS_BK 32
 #define GS_LD (GS_BK + 4)
@@ -325,13 +327,20 @@ static int gs_run_any(const GsArgs& p, int batches, cudaStream_t stream) {
 // in_dtype, C's shape, or null): C is multiplied by its sigmoid, in float.
 ACV_API int acv_gemm_simt_batched(const void* A, int lda, long long a_batch, const void* W, int ldw, long long w_batch,
                                   void* C, int ldc, long long c_batch, int M, int N, int K, int batches, int in_dtype,
-                                  int out_dtype, const void* gate, int ldg, long long g_batch, cudaStream_t stream) {
+                                  int out_dtype, const void* gate, int ldg, long long g_batch, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batches <= 0) return 0;
     if (K <= 0 || batches > 65535) return ACV_ERR_SIZE;
     const GsArgs p = {A, W, gate, C, lda, ldw, ldc, ldg, M, N, K, a_batch, w_batch, c_batch, g_batch};
     if (in_dtype == ACV_F32 && out_dtype == ACV_F32) {
         // 16-byte copies: both operands' starts, rows and batches on 16-byte boundaries (a row's end need not be one)
         const bool pieces = ((uintptr_t)A | (uintptr_t)W) % 16 == 0 && (lda | ldw) % 4 == 0 && (a_batch | w_batch) % 4 == 0;
+        if (K >= GF_MIN_K) {
+            int sms = 0;
+            if (const int e = gs_multiprocessors(&sms)) return e;
+            const GfArgs q = {(const float*)A, (const float*)W, (const float*)gate, (float*)C, status, lda, ldw, ldc, ldg, M, N, K,
+                              a_batch, w_batch, c_batch, g_batch};
+            return gf_run(q, pieces, batches, sms, stream);
+        }
         return pieces ? gs_run_async(p, batches, stream) : gs_run_any<float, float>(p, batches, stream);
     }
     if (in_dtype == ACV_BF16 && out_dtype == ACV_F32) return gs_run_any<bf16, float>(p, batches, stream);
@@ -340,6 +349,6 @@ ACV_API int acv_gemm_simt_batched(const void* A, int lda, long long a_batch, con
 }
 
 ACV_API int acv_gemm_simt(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N, int K,
-                          int in_dtype, int out_dtype, cudaStream_t stream) {
-    return acv_gemm_simt_batched(A, lda, 0, W, ldw, 0, C, ldc, 0, M, N, K, 1, in_dtype, out_dtype, nullptr, 0, 0, stream);
+                          int in_dtype, int out_dtype, int* status, cudaStream_t stream) {
+    return acv_gemm_simt_batched(A, lda, 0, W, ldw, 0, C, ldc, 0, M, N, K, 1, in_dtype, out_dtype, nullptr, 0, 0, status, stream);
 }

@@ -99,8 +99,8 @@ def _declare(lib: ctypes.CDLL) -> None:
         "acv_gated_delta_blocks": [P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
         "acv_gated_delta_step_takes": [I, I],
         "acv_gated_delta_step": [P, I, P, P, P, P, F, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
-        "acv_gemm_simt": [P, I, P, I, P, I, I, I, I, I, I, P],
-        "acv_gemm_simt_batched": [P, I, LL, P, I, LL, P, I, LL, I, I, I, I, I, I, P, I, LL, P],
+        "acv_gemm_simt": [P, I, P, I, P, I, I, I, I, I, I, P, P],
+        "acv_gemm_simt_batched": [P, I, LL, P, I, LL, P, I, LL, I, I, I, I, I, I, P, I, LL, P, P],
         "acv_gemm_mma_batched_takes": [P, I, LL, P, I, LL, P, I, LL, I, I],
         "acv_gemm_mma_batched": [P, I, LL, P, I, LL, P, I, LL, I, I, I, I, P, I, LL, P],
         "acv_attention_mixed": [P, I, P, I, P, P, P, P, P, I, P, I, I, I, I, I, I, I, F, I, P, F, P, P, I, I, P, I, P],
@@ -366,7 +366,8 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor,
 
 # ----------------------------------------------------------------------------- matrix products
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    """out[M,N] = a[M,K] @ w[N,K]^T with 32-bit accumulation on the CUDA cores."""
+    """out[M,N] = a[M,K] @ w[N,K]^T with 32-bit accumulation: on the CUDA cores, or (float operands, K from 1024 on) of exact
+    bfloat16 parts on the tensor cores with a smaller error (csrc/gemm_split_tc.cu)."""
     _need_cuda(a, w, out)
     M, K = a.shape
     N = w.shape[0]
@@ -375,7 +376,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
     if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("gemm_simt: innermost strides must be 1")
     _check(library().acv_gemm_simt(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K,
-                                   dtype_code(a.dtype), dtype_code(out.dtype), _stream()), "gemm_simt")
+                                   dtype_code(a.dtype), dtype_code(out.dtype), _status_pointer(a), _stream()), "gemm_simt")
     return out
 
 
@@ -650,6 +651,17 @@ def status_word(device) -> torch.Tensor:
     if device.type == "cuda" and device.index is None:
         device = torch.device("cuda", torch.cuda.current_device())
     return _gemm_buffers(device, 0, 0)[2]
+
+
+_status_at: dict = {}       # device index -> address of its status word, which stays where it is
+
+
+def _status_pointer(t: torch.Tensor):
+    """The status word's address on t's device; none where it is not there yet and a capture forbids to make it."""
+    at = _status_at.get(t.get_device())
+    if at is None and not (str(t.device) not in _gemm_scratch and torch.cuda.is_current_stream_capturing()):
+        at = _status_at[t.get_device()] = _gemm_buffers(t.device, 0, 0)[2].data_ptr()
+    return at
 
 
 def reset_after_failure() -> None:
@@ -1787,7 +1799,8 @@ def gemm_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate: torc
                                         out.stride(1), M, N, K, B, *g, _stream()), "gemm_mma_batched")
         return out
     _check(library().acv_gemm_simt_batched(_p(a), a.stride(0), a.stride(1), _p(w), K, N * K, _p(out), out.stride(0),
-                                           out.stride(1), M, N, K, B, dtype_code(a.dtype), dtype_code(out.dtype), *g, _stream()),
+                                           out.stride(1), M, N, K, B, dtype_code(a.dtype), dtype_code(out.dtype), *g,
+                                           _status_pointer(a), _stream()),
            "gemm_batched")
     return out
 

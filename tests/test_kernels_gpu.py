@@ -386,6 +386,50 @@ def test_gemm_simt_rows_independent(ops):
     assert torch.equal(whole[5:6], one)
 
 
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 32, 33, 64, 65, 129, 700])
+@pytest.mark.parametrize("N,K", [(1, 1024), (129, 1029), (1030, 1100), (2500, 2080), (130, 9220)])
+def test_gemm_split_one_order_of_sums(ops, M, N, K):
+    """Float sums from K = 1024 on are made of bfloat16 parts: the kernel for few tokens (mma.sync) and every tile and
+    sharing of K of the other (tcgen05) give a row the same bits, whatever its alignment.  Its error: a chunk of 32 k loses at most
+    two cut-off additions (2^-23 of its absolute sum each), 2^-24 for the parts' products left out and for the small ones' sums;
+    chunks and groups are added to nearest, no more than K / 256 + 2 chunks to a group and eight groups."""
+    a = rnd(700, K, seed=46)
+    w = rnd(N, K, scale=0.05, seed=47)
+    one = ops.gemm_simt(a[:1], w, torch.empty(1, N, device="cuda"))
+    got = ops.gemm_simt(a[:M], w, torch.full((M, N), float("nan"), device="cuda"))
+    assert torch.equal(got[:1], one)
+    # the same rows at strides of 16-byte pieces (which K may end within) and of none
+    for pad in (-K % 4, -K % 4 + 1):
+        x, y = torch.zeros(M, K + pad, device="cuda"), torch.zeros(N, K + pad, device="cuda")
+        x[:, :K], y[:, :K] = a[:M], w
+        assert torch.equal(ops.gemm_simt(x[:, :K], y[:, :K], torch.empty(M, N, device="cuda")), got)
+    size = a[:M].double().abs() @ w.double().abs().T
+    assert ((got.double() - a[:M].double() @ w.double().T).abs() <= (6 + K / 256 + 2 + 8) * 2.0 ** -24 * size).all()
+    assert ops.gemm_status() == 0
+
+
+@pytest.mark.parametrize("M", [3, 16, 40, 200])
+def test_gemm_split_infinities_and_gate(ops, M):
+    """Infinities, NaN and values near the largest have no finite parts: those outputs are what a chain of multiply-adds gives,
+    the others keep their bits; the gate of the batched form."""
+    K, N = 1030, 140
+    a, w = rnd(M, K, seed=48), rnd(N, K, scale=0.05, seed=49)
+    clean = ops.gemm_simt(a, w, torch.empty(M, N, device="cuda"))
+    a[0, 5], a[1, 1029], w[7, 3], w[9, 1028], a[2, 17] = float("inf"), float("nan"), -float("inf"), float("nan"), 3.4e38
+    w[:, 17] = 0.01
+    got = ops.gemm_simt(a, w, torch.empty(M, N, device="cuda"))
+    want = a.double() @ w.double().T
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()].double(), want[got.isinf()])
+    torch.testing.assert_close(got[2, 10:].double(), want[2, 10:], rtol=1e-6, atol=0)
+    w2, gate = rnd(2, N, K, scale=0.05, seed=50), rnd(M, 2, N, seed=51)
+    x = rnd(M, 2, K, seed=52)
+    out = ops.gemm_batched(x, w2, torch.empty(M, 2, N, device="cuda"), gate)
+    want = torch.einsum("mbk,bnk->mbn", x.double(), w2.double()) * torch.sigmoid(gate.double())
+    torch.testing.assert_close(out.double(), want, rtol=1e-5, atol=1e-5)
+    assert clean.isfinite().all()
+
+
 @pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 16, 17, 33, 65, 129, 700])
 @pytest.mark.parametrize("N,K", [(1, 4), (65, 33), (129, 256), (200, 2052), (1030, 260)])
 def test_gemm_simt_one_order_of_sums(ops, M, N, K):
