@@ -400,6 +400,31 @@ __device__ __forceinline__ float cluster_all_sum(ClusterSum& c, float v) {
     c.turn ^= 1;
     return total;
 }
+// the maximum over the cluster of `v`, and the mean over its threads of those `v` that are finite (0 where there are none)
+__device__ __forceinline__ float cluster_max_and_mean(ClusterSum& c, float* sums, float v, float& mean) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool finite = fabsf(v) <= 3.402823466e38f;
+    const float top = warp_max(v), sum = warp_sum(finite ? v : 0.f), count = (float)__popc(__ballot_sync(0xffffffffu, finite));
+    if (lane == 0) { c.table[warp] = top; c.table[32 + warp] = sum; c.table[64 + warp] = count; }
+    __syncthreads();
+    if (warp < 3) {
+        float t = c.table[warp * 32 + lane];
+        t = warp == 0 ? warp_max(t) : warp_sum(t);
+        float* to = warp == 0 ? c.parts + c.turn * SMPC_CTAS : sums + (warp - 1) * SMPC_CTAS;
+        if (lane < SMPC_CTAS) cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(to + c.rank), lane), t);
+    }
+    cluster_sync_all();
+    float total = -INFINITY, all = 0.f, n = 0.f;
+#pragma unroll
+    for (int r = 0; r < SMPC_CTAS; ++r) {
+        total = fmaxf(total, c.parts[c.turn * SMPC_CTAS + r]);
+        all += sums[r];
+        n += sums[SMPC_CTAS + r];
+    }
+    c.turn ^= 1;
+    mean = n > 0.f ? all / n : 0.f;
+    return total;
+}
 __device__ __forceinline__ float cluster_all_max(ClusterSum& c, float v) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     v = warp_max(v);
@@ -419,19 +444,68 @@ __device__ __forceinline__ float cluster_all_max(ClusterSum& c, float v) {
     return total;
 }
 
+// What a pass of sixteen bins finds: v[d] is this thread's sum over its elements of digit d, `seen` how many of its elements took
+// part.  The bins are added up over warp, CTA and cluster (in an order that the launch shape fixes), and the sums from the top
+// down say which bin the wanted key lies in: the largest d for which over + (bins d and above) reaches `limit` (above: exceeds
+// it), 0 if none does (found: whether one did).  `over` takes the bins above d.  Returns d; seen: the cluster's count.
+__device__ __forceinline__ uint32_t cluster_bins(ClusterSum& c, float* bins, float (&v)[16], float& seen, float limit, bool above,
+                                                 float& over, bool& found) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // over the warp: a lane gives away half of what it carries at each exchange and ends with bin `lane % 16`
+#pragma unroll
+    for (int h = 8; h > 0; h >>= 1) {
+        const bool high = lane & h;
+#pragma unroll
+        for (int d = 0; d < 8; ++d)
+            if (d < h) {
+                const float give = high ? v[d] : v[d + h], keep = high ? v[d + h] : v[d];
+                v[d] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+            }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+    seen = warp_sum(seen);
+    if (lane < 16) c.table[warp * 17 + lane] = v[0];
+    if (lane == 16) c.table[warp * 17 + 16] = seen;
+    __syncthreads();
+    if (warp < 17) {        // warp d adds up bin d over the warps and tells every CTA
+        const float t = warp_sum(c.table[lane * 17 + warp]);
+        if (lane < SMPC_CTAS)
+            cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(bins + (c.turn * SMPC_CTAS + c.rank) * 17 + warp), lane), t);
+    }
+    cluster_sync_all();
+    float s = 0.f;          // lane d: bin d, then the sum of the bins d and above
+    seen = 0.f;
+#pragma unroll
+    for (int r = 0; r < SMPC_CTAS; ++r) {
+        s += bins[(c.turn * SMPC_CTAS + r) * 17 + (lane & 15)];
+        seen += bins[(c.turn * SMPC_CTAS + r) * 17 + 16];
+    }
+    c.turn ^= 1;
+#pragma unroll
+    for (int h = 1; h < 16; h <<= 1) {
+        const float up = __shfl_down_sync(0xffffffffu, s, h, 16);
+        if ((lane & 15) + h < 16) s += up;
+    }
+    const float at = over + s;
+    const uint32_t good = __ballot_sync(0xffffffffu, above ? at > limit : at >= limit) & 0xffffu;
+    const int d = good ? 31 - __clz(good) : 0;
+    const float beyond = __shfl_sync(0xffffffffu, s, (d + 1) & 15, 16);
+    if (d < 15) over += beyond;
+    found = good != 0;
+    return (uint32_t)d;
+}
+
 // The largest c for which the sum of w over the elements with key >= c reaches `limit` (above: exceeds it), 0 if none
 // does.  Four bits a pass, from the top: the elements that share the bits found so far fall into 16 bins by their next
-// four, a thread's in registers; the bins are added up over warp, CTA and cluster (in an order that the launch shape
-// fixes), and the sums from the top down say which bin holds c.  A pass costs its meeting of the cluster, 2 us, so eight
+// four, a thread's in registers.  A pass costs its meeting of the cluster, 2 us, so eight
 // passes of sixteen candidates replace 32 of one
 // (8 rows of 151 936, microseconds: top-p 141 -> 64, top-k 120 -> 49, both 199 -> 91).
 template <typename Element>
 __device__ __forceinline__ uint32_t cluster_descend(ClusterSum& c, float* bins, int n, float limit, bool above, Element element) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t prefix = 0;
     float over = 0.f;           // the sum over the elements whose bits so far are larger than c's
     for (int shift = 28; shift >= 0; shift -= 4) {
-        float v[16];
+        float v[16], seen = 0.f;
 #pragma unroll
         for (int d = 0; d < 16; ++d) v[d] = 0.f;
         for (int i = threadIdx.x; i < n; i += SMPC_THREADS) {
@@ -443,43 +517,129 @@ __device__ __forceinline__ uint32_t cluster_descend(ClusterSum& c, float* bins, 
 #pragma unroll
             for (uint32_t d = 0; d < 16; ++d) v[d] += digit == d ? w : 0.f;
         }
-        // over the warp: a lane gives away half of what it carries at each exchange and ends with bin `lane % 16`
-#pragma unroll
-        for (int h = 8; h > 0; h >>= 1) {
-            const bool high = lane & h;
-#pragma unroll
-            for (int d = 0; d < 8; ++d)
-                if (d < h) {
-                    const float give = high ? v[d] : v[d + h], keep = high ? v[d + h] : v[d];
-                    v[d] = keep + __shfl_xor_sync(0xffffffffu, give, h);
-                }
-        }
-        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
-        if (lane < 16) c.table[warp * 17 + lane] = v[0];
-        __syncthreads();
-        if (warp < 16) {        // warp d adds up bin d over the warps and tells every CTA
-            const float t = warp_sum(c.table[lane * 17 + warp]);
-            if (lane < SMPC_CTAS)
-                cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(bins + (c.turn * SMPC_CTAS + c.rank) * 16 + warp), lane), t);
-        }
-        cluster_sync_all();
-        float s = 0.f;          // lane d: bin d, then the sum of the bins d and above
-#pragma unroll
-        for (int r = 0; r < SMPC_CTAS; ++r) s += bins[(c.turn * SMPC_CTAS + r) * 16 + (lane & 15)];
-        c.turn ^= 1;
-#pragma unroll
-        for (int h = 1; h < 16; h <<= 1) {
-            const float up = __shfl_down_sync(0xffffffffu, s, h, 16);
-            if ((lane & 15) + h < 16) s += up;
-        }
-        const float at = over + s;
-        const uint32_t good = __ballot_sync(0xffffffffu, above ? at > limit : at >= limit) & 0xffffu;
-        const int d = good ? 31 - __clz(good) : 0;
-        const float beyond = __shfl_sync(0xffffffffu, s, (d + 1) & 15, 16);
-        if (d < 15) over += beyond;
-        prefix |= (uint32_t)d << shift;
+        bool found;
+        prefix |= cluster_bins(c, bins, v, seen, limit, above, over, found) << shift;
     }
     return prefix;
+}
+
+// The same answer in fewer passes where the row's values are spread as a vocabulary's logits are.  The first passes sort by the
+// distance from the maximum in units of 1/scale, then 16ths and 256ths of them (a step function of the logit, so its bins
+// follow the keys' order; what lies 16 units and further shares the lowest bin).  The unit is a sixth of what lies between the
+// maximum and the mean of the threads' own maxima: two fifths of a standard deviation or so, whatever the temperature, and few
+// entries at the lowest value of the type do not move it.  As soon as few enough elements took part in a pass, those of
+// the bin it chose, a few hundred of the row at most, go to every CTA of the cluster, and each finds c among them by itself:
+// the largest key whose sum (over + the candidates of its key and above) reaches the limit.  False: there are too many of
+// them, none reaches the limit, or an element's distance is no number; the caller then searches bit by bit.
+// Two or three passes and the lists instead of eight passes (8 rows of 151 936, microseconds: top-p 66 -> 41, top-k 51 -> 34, both 92 -> 53).
+#define SMPC_NEAR 64            // candidates that a CTA may bring
+struct NearList {
+    float2 got[SMPC_CTAS * SMPC_NEAR], list[SMPC_CTAS * SMPC_NEAR];     // key (as bits) and w
+    int counts[SMPC_CTAS], scan[32];
+    uint32_t best[32];
+};
+
+template <typename Element>
+__device__ __forceinline__ bool cluster_near(ClusterSum& c, float* bins, NearList& nl, const float* sl, float mx, float scale, int n, float limit,
+                                             bool above, Element element, uint32_t& answer) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!(scale > 0.f && scale <= 1e30f)) return false;
+    auto place = [&](int i) { return 4095 - min((int)((mx - sl[i]) * scale), 4095); };
+    uint32_t prefix = 0;
+    float over = 0.f;
+    int all = 0;
+    for (int shift = 8;; shift -= 4) {
+        if (shift < 0) return false;
+        float v[16], seen = 0.f;
+#pragma unroll
+        for (int d = 0; d < 16; ++d) v[d] = 0.f;
+        for (int i = threadIdx.x; i < n; i += SMPC_THREADS) {
+            const uint32_t at = (uint32_t)place(i);
+            if (shift == 8) {
+                if (!(mx - sl[i] >= 0.f)) seen += 1e9f;         // (no number: a count that no list is made for)
+            } else if ((at ^ prefix) >> (shift + 4)) {
+                continue;
+            }
+            seen += 1.f;
+            uint32_t key;
+            float w;
+            element(i, key, w);
+            const uint32_t digit = at >> shift & 15u;
+#pragma unroll
+            for (uint32_t d = 0; d < 16; ++d) v[d] += digit == d ? w : 0.f;
+        }
+        bool found;
+        prefix |= cluster_bins(c, bins, v, seen, limit, above, over, found) << shift;
+        if (!found || seen >= 1e9f || !(prefix >> 8)) return false;     // (or it lies in the bin of all that is far)
+        if (seen > 8.f * SMPC_CTAS * SMPC_NEAR) continue;       // (spread evenly over the bins: half of the lists)
+        // this CTA's candidates, thread by thread, then index by index
+        int mine = 0;
+        for (int i = threadIdx.x; i < n; i += SMPC_THREADS) mine += (uint32_t)place(i) >> shift == prefix >> shift;
+        int upto = mine;
+#pragma unroll
+        for (int h = 1; h < 32; h <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, upto, h);
+            if (lane >= h) upto += up;
+        }
+        if (lane == 31) nl.scan[warp] = upto;
+        __syncthreads();
+        int total = 0, before = upto - mine;
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            if (q == warp) before += total;
+            total += nl.scan[q];
+        }
+        if (mine && total <= SMPC_NEAR)
+            for (int i = threadIdx.x; i < n; i += SMPC_THREADS) {
+                if ((uint32_t)place(i) >> shift != prefix >> shift) continue;
+                uint32_t key;
+                float w;
+                element(i, key, w);
+                const uint32_t to = (uint32_t)__cvta_generic_to_shared(&nl.got[c.rank * SMPC_NEAR + before++]);
+#pragma unroll
+                for (int r = 0; r < SMPC_CTAS; ++r) {
+                    const uint32_t at = cluster_map(to, r);
+                    cluster_store_f32(at, __uint_as_float(key));
+                    cluster_store_f32(at + 4, w);
+                }
+            }
+        if (threadIdx.x < SMPC_CTAS)
+            cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(&nl.counts[c.rank]), threadIdx.x), __int_as_float(total));
+        cluster_sync_all();
+        int my_off = 0;
+        bool fits = true;
+        const int of = threadIdx.x / SMPC_NEAR;
+        all = 0;
+#pragma unroll
+        for (int r = 0; r < SMPC_CTAS; ++r) {
+            const int k = nl.counts[r];
+            if (r == of) my_off = all;
+            all += k;
+            fits = fits && k <= SMPC_NEAR;
+        }
+        if (!fits) continue;        // (the next pass meets before anybody writes a list or a count again)
+        if (of < SMPC_CTAS && (int)(threadIdx.x % SMPC_NEAR) < nl.counts[of]) nl.list[my_off + threadIdx.x % SMPC_NEAR] = nl.got[threadIdx.x];
+        __syncthreads();
+        break;
+    }
+    uint32_t best = 0;
+    for (int q = warp; q < all; q += SMPC_THREADS / 32) {
+        const uint32_t key = __float_as_uint(nl.list[q].x);
+        float sum = 0.f;
+        for (int j = lane; j < all; j += 32) {
+            const float2 e = nl.list[j];
+            sum += __float_as_uint(e.x) >= key ? e.y : 0.f;
+        }
+        const float at = over + warp_sum(sum);
+        if (above ? at > limit : at >= limit) best = max(best, key);
+    }
+    if (lane == 0) nl.best[warp] = best;
+    __syncthreads();
+    best = nl.best[lane];
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, h));
+    answer = best;
+    return best != 0;
 }
 
 __global__ void __launch_bounds__(SMPC_THREADS)
@@ -488,7 +648,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
                       const unsigned long long* __restrict__ seed, const unsigned long long* __restrict__ counter,
                       int* __restrict__ out_token, float* __restrict__ out_logprob) {
     extern __shared__ float sl[];               // this CTA's slice of the scaled logits, and behind it exp(logit - maximum)
-    __shared__ float parts[2 * SMPC_CTAS], bins[2 * SMPC_CTAS * 16];
+    __shared__ float parts[2 * SMPC_CTAS], bins[2 * SMPC_CTAS * 17];
+    __shared__ NearList near;
+    __shared__ float sums[2 * SMPC_CTAS];
     __shared__ float warps[32], table[32 * 17];
     __shared__ float scan[SMPC_THREADS];
     __shared__ float bestv[2 * SMPC_CTAS];
@@ -508,7 +670,16 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
         sl[i] = v;
         mx = fmaxf(mx, v);
     }
-    mx = cluster_all_max(cs, mx);           // (its barriers also make the slice visible to the CTA's threads)
+    const int k = top_k[r];
+    const float tp = top_p[r];
+    float scale = 0.f;                      // (either meeting's barriers also make the slice visible to the CTA's threads)
+    if (!greedy && ((k > 0 && k < V) || (tp > 0.f && tp < 1.f))) {
+        float mean;                         // of the threads' maxima
+        mx = cluster_max_and_mean(cs, sums, mx, mean);
+        scale = 1536.f / (mx - mean);
+    } else {
+        mx = cluster_all_max(cs, mx);
+    }
 
     if (greedy) {
         // the lowest index that holds the maximum: the smallest of the CTAs' candidates (slices are in index order)
@@ -536,12 +707,13 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
     for (int i = threadIdx.x; i < n; i += blockDim.x) se[i] = expf(sl[i] - mx);
     __syncthreads();
     uint32_t cut = 0;  // keys >= cut are kept
-    const int k = top_k[r];
-    if (k > 0 && k < V)     // the largest c with count(key >= c) >= k
-        cut = cluster_descend(cs, bins, n, (float)k, false, [&](int i, uint32_t& key, float& w) { key = order_key(sl[i]); w = 1.f; });
+    if (k > 0 && k < V) {   // the largest c with count(key >= c) >= k
+        auto element = [&](int i, uint32_t& key, float& w) { key = order_key(sl[i]); w = 1.f; };
+        if (!cluster_near(cs, bins, near, sl, mx, scale, n, (float)k, false, element, cut))
+            cut = cluster_descend(cs, bins, n, (float)k, false, element);
+    }
     const float mp = min_p[r];
     const bool use_minp = mp > 0.f;
-    const float tp = top_p[r];
     if (tp > 0.f && tp < 1.f) {
         float z = 0.f;
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -552,12 +724,15 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
         z = cluster_all_sum(cs, z);
         // the largest t with mass(key > t) > limit, that is with mass(key - 1 >= t) > limit
         const uint32_t kept_from = cut;
-        const uint32_t t = cluster_descend(cs, bins, n, tp * z, true, [&](int i, uint32_t& key, float& w) {
+        auto element = [&](int i, uint32_t& key, float& w) {
             const uint32_t full = order_key(sl[i]);
             const float e = se[i];
             key = full - 1u;
             w = full >= kept_from && full != 0u && !(use_minp && e < mp) ? e : 0.f;
-        });
+        };
+        uint32_t t;
+        if (!cluster_near(cs, bins, near, sl, mx, scale, n, tp * z, true, element, t))
+            t = cluster_descend(cs, bins, n, tp * z, true, element);
         cut = t + 1u > cut ? t + 1u : cut;
     }
 

@@ -77,6 +77,36 @@ def test_wide_rows_cut_where_the_plain_sampler_cuts(V, kind):
         assert before - 1e-4 <= u <= float(cdf[got[i]]) + 1e-4, f"case {i}"
 
 
+@pytest.mark.parametrize("V", [16384, 151936])
+@pytest.mark.parametrize("kind", ["cold", "hot", "crowded", "far", "lowest"])
+def test_wide_rows_whose_cut_is_searched_near_the_maximum(V, kind):
+    """The search by distance from the maximum: two passes and the lists, three, more candidates than a list holds, a cut in the
+    bin of all that is far, half of the row at the type's lowest value; a draw just inside the kept mass, whatever the seed."""
+    g = torch.Generator().manual_seed(V + 1)
+    x = torch.randn(V, generator=g)
+    row = {"cold": lambda: x * 9, "hot": lambda: x * 0.01, "crowded": lambda: (x * 40).round() / 40,
+           "far": lambda: torch.cat([x[: V // 2], x[V // 2:] * 1e-3 - 60.0]), "lowest": lambda: torch.where(x < 0, torch.finfo(torch.float32).min, x)}[kind]()
+    cases = [(1.0, 50, 1.0, 0.0), (1.0, 0, 0.9, 0.0), (1.0, V // 2 + 1000, 1.0, 0.0), (1.0, V - 3, 0.9995, 0.0), (1.0, 300, 0.95, 0.01), (1.0, 64, 1.0, 0.0)]
+    R = len(cases)
+    for counter in range(3):
+        got, _ = run_sample(row.repeat(R, 1).cuda(), *[[c[j] for c in cases] for j in (0, 1, 2, 3)], list(range(R)), [counter] * R)
+        for i, (_, k, p, mp) in enumerate(cases):
+            z = row.double()
+            weight = (z - z.max()).exp()
+            keep = z >= z.topk(k).values[-1] if 0 < k < V else torch.ones(V, dtype=torch.bool)
+            keep &= weight >= mp
+            if p < 1.0:
+                values, at = torch.unique(z[keep], return_inverse=True)
+                mass = torch.zeros(len(values), dtype=torch.float64).index_add_(0, at, weight[keep])
+                above = mass.flip(0).cumsum(0).flip(0) - mass
+                keep &= z >= values[above <= p * mass.sum() * (1 + 1e-6)][0]
+            assert keep[got[i]], f"case {i}: a dropped token was drawn"
+            cdf = torch.where(keep, weight, 0.0).cumsum(0) / weight[keep].sum()
+            u = plain_qwen3.philox_uniform(i, counter)
+            before = float(cdf[got[i]] - weight[got[i]] / weight[keep].sum())
+            assert before - 1e-4 <= u <= float(cdf[got[i]]) + 1e-4, f"case {i}"
+
+
 @pytest.mark.parametrize("at", [(100, 104), (104, 100), (100, 2040), (0, 63)])
 def test_a_wide_row_with_a_logit_that_is_no_number_gives_a_kept_token(at):
     """Top-k 2 of a row whose largest entries are NaN and a number, in the same part of the row: the number is drawn."""
