@@ -531,7 +531,7 @@ __device__ __forceinline__ uint32_t cluster_descend(ClusterSum& c, float* bins, 
 // the bin it chose, a few hundred of the row at most, go to every CTA of the cluster, and each finds c among them by itself:
 // the largest key whose sum (over + the candidates of its key and above) reaches the limit.  False: there are too many of
 // them, none reaches the limit, or an element's distance is no number; the caller then searches bit by bit.
-// Two or three passes and the lists instead of eight passes (8 rows of 151 936, microseconds: top-p 66 -> 41, top-k 51 -> 34, both 92 -> 53).
+// Two or three passes and the lists instead of eight passes (8 rows of 151 936, microseconds: top-p 66 -> 43, top-k 51 -> 34, both 92 -> 53).
 #define SMPC_NEAR 64            // candidates that a CTA may bring
 struct NearList {
     float2 got[SMPC_CTAS * SMPC_NEAR], list[SMPC_CTAS * SMPC_NEAR];     // key (as bits) and w

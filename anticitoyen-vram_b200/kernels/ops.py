@@ -99,6 +99,8 @@ def _declare(lib: ctypes.CDLL) -> None:
         "acv_gated_delta_blocks": [P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
         "acv_gated_delta_step_takes": [I, I],
         "acv_gated_delta_step": [P, I, P, P, P, P, F, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
+        "acv_gemm_rows": [P, I, P, I, P, I, I, I, I, I, I, I, I, P],
+        "acv_gemm_rows_qkv": [P, I, P, I, P, I, I, I, I, I, I, I, I, I, P, P, F, P, I, P, P, P, I, P, P, P, I, I, P],
         "acv_gemm_simt": [P, I, P, I, P, I, I, I, I, I, I, P, P],
         "acv_gemm_simt_batched": [P, I, LL, P, I, LL, P, I, LL, I, I, I, I, I, I, P, I, LL, P, P],
         "acv_gemm_mma_batched_takes": [P, I, LL, P, I, LL, P, I, LL, I, I],
@@ -549,6 +551,22 @@ def _gemm_tc_plan(M: int, N: int, K: int, sms: int, bn_multiple: int, rows: bool
     return 0, best, 1, 8
 
 
+@functools.lru_cache(maxsize=4096)
+def gemm_rows_pays(M: int, N: int, K: int, sms: int) -> bool:
+    """Whether a product of up to 16 tokens is faster without a tile of 128 weight rows (csrc/gemm_rows.cu) than with one:
+    up to 8 tokens where the weights stay under 128 MB (12288 x 4096 20.1 us against 22.0; 24576 x 4096 35.5 against 34.9,
+    5120 x 17408 37 against 34) and for a vocabulary (151936 x 1024 57.6 against 56.5, x 4096 193 against 206); up to 16, whose
+    rows each block reads, under 50 MB (12288 x 2048 11.9 us against 12.7; 5120 x 5120 15.3 against 14.0, 19456 x 2560 22.1 against 21.4)."""
+    if K % 64 or N % 16 or M > 16:
+        return False
+    return N * K <= 1 << 26 or N >= 1 << 16 if M <= 8 else N * K <= 25_500_000
+
+
+def _gemm_rows_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
+    return (x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and gemm_rows_pays(x.shape[0], w.shape[0], x.shape[1], sm_count(x.device)))
+
+
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: tuple | None = None,
             swiglu_pairs: bool = False, static_weights: bool = False, bias: torch.Tensor | None = None,
             gate_fn: int = 0, unary: str | None = None, limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
@@ -556,7 +574,8 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: tuple | N
     added in the epilogue to the float accumulator (before the activation of the paired form).
 
     ``static_weights``: w was written long before this call (a model's weights), so the kernel may
-    read its first tiles while the kernel before it in the stream is still running.
+    read its first tiles while the kernel before it in the stream is still running.  Without a plan, a bias or another
+    activation, up to 16 tokens then go to ``csrc/gemm_rows.cu`` where that is faster (``gemm_rows_pays``).
 
     With ``swiglu_pairs`` the rows of w come in (gate, up) pairs and out is [M, N/2]:
     out[:, i] = silu(x . w[2i]) * (x . w[2i+1]), rounded as the separate kernels round; with ``gate_fn`` 1 the gate
@@ -575,6 +594,10 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: tuple | N
         raise KernelError("gemm_tc: the paired SwiGLU output needs an even number of weight rows and a bfloat16 output")
     if w.shape[1] != K or out.shape != (M, n_out) or x.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError(f"gemm_tc: shapes {tuple(x.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
+    if plan is None and static_weights and bias is None and unary is None and gate_fn == 0 and _gemm_rows_takes(x, w):
+        _check(library().acv_gemm_rows(_p(x), x.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K,
+                                       1 if out.dtype == torch.float32 else 0, int(swiglu_pairs), 1, sm_count(x.device), _stream()), "gemm_rows")
+        return out
     plan = plan or gemm_tc_plan(M, N, K)
     swap, bn, splits = plan[:3]
     stages = plan[3] if len(plan) > 3 else 8
@@ -623,6 +646,17 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, num_heads: 
     _need_cuda(x, w, out, k_pages, v_pages)
     M, K = x.shape
     N = w.shape[0]
+    # A head is a cluster of two or four blocks: as long as all heads' clusters come in one wave, up to 8 tokens with two blocks to
+    # an SM (48 heads of 128, K 4096: 13.3 us against 14.1; 16 tokens, where two do not fit, 18.0 against 15.0; 32 heads, K 1024: 4.2
+    # and 4.8 against 6.1 and 6.7).
+    if plan is None and static_weights and M <= 16 and _gemm_rows_takes(x, w) \
+            and N // head_dim <= (33 if head_dim == 128 else 74) * (2 if M <= 8 else 1) * sm_count(x.device) // 148:
+        _check(library().acv_gemm_rows_qkv(
+            _p(x), x.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K, 1, sm_count(x.device), num_heads, num_kv_heads,
+            head_dim, _p(q_weight), _p(k_weight), eps, _p(cos_sin), cos_sin.shape[0] if cos_sin is not None else 0, _p(positions),
+            _p(seq_of_token), _p(block_table), block_table.stride(0), _p(table_rows), _p(k_pages), _p(v_pages), k_pages.shape[2],
+            k_pages.shape[0], _stream()), "gemm_rows_qkv")
+        return out
     plan = plan or gemm_tc_plan(M, N, K, bn_multiple=head_dim if M > 128 else 16, rows=M > 128)
     swap, bn, splits, stages = plan[:4]
     cluster = plan[4] if len(plan) > 4 else (1 if swap and 1 < splits <= 8 else 0)

@@ -824,6 +824,56 @@ def test_gemm_tc_fused_swiglu(ops, plan, M, I, K):
                                                torch.zeros(M, I, device="cuda", dtype=torch.bfloat16)), **tol(torch.bfloat16))
 
 
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(16, 64), (48, 192), (4096, 1024), (80, 4160), (96, 4096), (19456, 640), (6144, 2560), (66000, 512)])
+def test_gemm_rows(ops, M, N, K):
+    """Products of up to 16 tokens with weights written long before: sixteen or 32 rows to a block, one round of blocks and
+    several, K that leaves warps without a chunk and K that their rings go round in; plain in both types, and (gate, up) pairs."""
+    wide = rnd(M, K + 64, dtype=torch.bfloat16, seed=260)
+    x = wide[:, 64:]
+    w = rnd(N, K, dtype=torch.bfloat16, scale=0.05, seed=261)
+    want = x.double() @ w.double().T
+    out = ops.gemm_tc(x, w, torch.full((M, N), 3.0, device="cuda"), static_weights=True)
+    torch.testing.assert_close(out.double(), want, rtol=1e-4, atol=1e-4)
+    # (more than a rounding to bfloat16 apart only where a float sum lies at a boundary: one unit in the last place)
+    out = ops.gemm_tc(x, w, torch.full((M, N), 3.0, device="cuda", dtype=torch.bfloat16), static_weights=True)
+    torch.testing.assert_close(out.double(), want, rtol=2.0 ** -8, atol=1e-4)
+    got = ops.gemm_tc(x, w, torch.full((M, N // 2), 3.0, device="cuda", dtype=torch.bfloat16), swiglu_pairs=True, static_weights=True)
+    gate, up = out.double()[:, 0::2], out.double()[:, 1::2]
+    torch.testing.assert_close(got.double(), gate * torch.sigmoid(gate) * up, rtol=2.0 ** -6, atol=1e-4)
+    assert not ops.gemm_rows_pays(17, N, K, 148) and ops.gemm_rows_pays(M, N, K, 148) == (M <= 8 or N * K <= 25_500_000)
+
+
+@pytest.mark.parametrize("NH,NKV,D,T,K", [(16, 8, 128, 8, 1024), (32, 8, 128, 5, 640), (4, 4, 128, 1, 512), (6, 2, 64, 16, 128), (5, 1, 64, 9, 2112), (3, 1, 128, 13, 192)])
+@pytest.mark.parametrize("normed,rotated", [(True, True), (False, True), (True, False)])
+def test_gemm_rows_qkv(ops, NH, NKV, D, T, K, normed, rotated):
+    """The projection of few tokens whose blocks share a head's norm through their cluster, against the product followed by
+    the rotation kernel (sums in another order: a rounding may move here and there)."""
+    page, per_request, N = 16, 10, (NH + 2 * NKV) * D
+    x = rnd(T, K, dtype=torch.bfloat16, seed=262)
+    w = rnd(N, K, dtype=torch.bfloat16, scale=0.05, seed=263)
+    qw = (1.0 + 0.1 * rnd(D, seed=264)) if normed else None
+    kw = (1.0 + 0.1 * rnd(D, seed=265)) if normed else None
+    ang = torch.rand(200, D // 2, device="cuda") * 6.28
+    cos_sin = torch.cat([ang.cos(), ang.sin()], dim=1).contiguous() if rotated else None
+    seq = torch.tensor([i % 3 for i in range(T)], dtype=torch.int32, device="cuda")
+    pos = torch.tensor([(7 * i + 3) % 150 for i in range(T)], dtype=torch.int32, device="cuda")
+    table = torch.randperm(32, device="cuda").to(torch.int32)[:3 * per_request].view(3, per_request).contiguous()
+    if T > 2:
+        table[int(seq[2]), int(pos[2]) // page] = -1
+    kp1 = torch.zeros(32, NKV, page, D, device="cuda", dtype=torch.bfloat16)
+    vp1, kp2, vp2 = torch.zeros_like(kp1), torch.zeros_like(kp1), torch.zeros_like(kp1)
+    assert ops.gemm_rows_pays(T, N, K, 148)
+    want = ops.gemm_tc(x, w, torch.zeros(T, N, device="cuda", dtype=torch.bfloat16), static_weights=True)
+    ops.qk_norm_rope_append(want, NH, NKV, D, qw, kw, 1e-6, cos_sin, pos, seq, table, kp1, vp1)
+    got = torch.zeros(T, N, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_tc_qkv(x, w, got, NH, NKV, D, qw, kw, 1e-6, cos_sin, pos, seq, table, kp2, vp2, static_weights=True)
+    for a, b in ((got[:, :NH * D], want[:, :NH * D]), (kp2, kp1), (vp2, vp1)):
+        torch.testing.assert_close(a, b, **tol(torch.bfloat16))
+        assert (a != b).float().mean() < 0.02
+    assert not got[:, NH * D:].any()
+
+
 @pytest.mark.parametrize("M,N,K", [(2100, 2304, 200), (5000, 520, 136), (257, 256, 64), (256, 4104, 72), (9000, 264, 4096)])
 def test_gemm_tc_pairs_of_ctas(ops, M, N, K):
     """Tiles of 256 x 256 on pairs of CTAs (tcgen05 cta_group::2): more tiles than pairs (a pair walks several, the
