@@ -28,6 +28,10 @@
 // portion may start anywhere in its prompt (acvram/engine/layers.py:1020-1041); the reference runs this
 // case through SDPA on a gathered dense copy (acvram/engine/attention.py:519-584).
 // Every wait is bounded; a wait that runs out is recorded in `status` and the kernel returns.
+//
+// Where there are fewer CTAs than SMs, or a last round of them that leaves most SMs idle, the key tiles of a CTA are shared out over
+// a cluster (`parts`, two to eight): each works through its share as above and leaves its O, maxima and sums in its shared memory;
+// each then makes its share of the columns, the parts' O weighted by 2^(their maximum - the row's).
 #include "tc_ptx.cuh"
 #include "tensor_map.h"
 
@@ -115,9 +119,12 @@ struct AttnTcParams {
     const bf16* gate;       // or null: rows like the result's, 16-byte pieces: the result is multiplied by sigmoid(gate) in float
     int gate_stride;
     const float* slopes;    // [NH] or null: the score of query i and key j loses slope_h (i - j)
+    int parts;              // CTAs that share a tile's keys, a cluster
+    int pair0, pairs;       // the pairs of a group's heads that this launch takes: their first and how many
 };
 
-template <int D>
+// SHARED: a cluster's CTAs share a tile's keys (a kernel of its own: the loop beside the merge's code took 1 % longer)
+template <int D, bool SHARED>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, AttnTcParams p) {
@@ -140,9 +147,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     ACV_TL(TL_ATTN_TC, 64);
     // the CTA's heads, from its number alone (the barriers' counts depend on it)
-    const int n_rep = p.NH / p.NKV, pairs = (n_rep + 1) >> 1;
-    const int tile = blockIdx.x / (p.NKV * pairs), hp = blockIdx.x - tile * (p.NKV * pairs);
-    const int kvh = hp / pairs, pair = hp - kvh * pairs;
+    const int n_rep = p.NH / p.NKV, pairs = p.pairs;
+    const int parts = SHARED ? p.parts : 1, unit = (int)blockIdx.x / parts, part = (int)blockIdx.x - unit * parts;
+    const int tile = unit / (p.NKV * pairs), hp = unit - tile * (p.NKV * pairs);
+    const int kvh = hp / pairs, pair = p.pair0 + hp - kvh * pairs;
     const int h0 = kvh * n_rep + 2 * pair;                  // the CTA's first head; the second is h0 + 1
     const int n_heads = 2 * pair + 1 < n_rep ? 2 : 1;
     if (threadIdx.x == 0) {
@@ -195,8 +203,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const int j_first = lo & ~(AT_BN - 1);
     // key tiles in front of the window that hold kept first keys come first; tile t begins at key tile_j0(t)
     const int n_sink = p.keep_first > 0 ? min(j_first / AT_BN, (p.keep_first + AT_BN - 1) / AT_BN) : 0;
-    const int n_tiles = n_sink + (hi - j_first) / AT_BN + 1;
-    auto tile_j0 = [&](int t) { return t < n_sink ? t * AT_BN : j_first + (t - n_sink) * AT_BN; };
+    const int all_tiles = n_sink + (hi - j_first) / AT_BN + 1;
+    const int t_first = all_tiles * part / parts, n_tiles = all_tiles * (part + 1) / parts - t_first;     // this CTA's share
+    auto tile_j0 = [&](int t) { t += t_first; return t < n_sink ? t * AT_BN : j_first + (t - n_sink) * AT_BN; };
     const int* bt = p.block_table + (size_t)(p.bt_rows ? p.bt_rows[seq] : seq) * p.bt_stride;
     pdl_wait();             // queries, and the keys and values of this step's tokens, are the projection's output
 
@@ -260,6 +269,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             };
             bool ok = mbar_wait(q_full, 0, &abort_s);
             if (!ok) { abort_s = 1; atomicExch(p.status, 12); }
+            if (n_tiles == 0) ok = false;           // (more CTAs than key tiles)
             if (ok && !mbar_wait(k_full, 0, &abort_s)) { ok = false; abort_s = 1; atomicExch(p.status, 13); }
             if (ok) {
                 tc_fence_after();
@@ -417,7 +427,24 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             acv_tl_marks[7] = (unsigned long long)(2 * n_tiles);
         }
 #endif
-        if (!failed && !abort_s && mbar_wait(o_full + 8 * hs, 0, &abort_s)) {
+        const bool whole = !failed && !abort_s && mbar_wait(o_full + 8 * hs, 0, &abort_s);
+        if (SHARED) {
+            // both heads' products are complete: O goes where the tiles were, 16 bytes of a row beside the next row's
+            asm volatile("bar.sync 1, %0;" ::"r"(n_heads * 128) : "memory");
+            tc_fence_after();
+            float4* left = reinterpret_cast<float4*>(base) + hs * (D / 4 * 128) + r;
+#pragma unroll
+            for (int c0 = 0; c0 < D; c0 += 32) {
+                uint32_t o[32];
+                if (n_tiles > 0) tc_ld32(tmem_o + c0, o);
+#pragma unroll
+                for (int c = 0; c < 32; c += 4)
+                    left[((c0 + c) >> 2) * 128] = n_tiles > 0 ? make_float4(__uint_as_float(o[c]), __uint_as_float(o[c + 1]),
+                                                                            __uint_as_float(o[c + 2]), __uint_as_float(o[c + 3]))
+                                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            reinterpret_cast<float2*>(base + 2 * D * 512)[hs * 128 + r] = make_float2(m_run, l_run);
+        } else if (whole) {
             tc_fence_after();
             if (p.sinks && m_run != -INFINITY) l_run += exp2f(p.sinks[head] * AT_LOG2E - m_run);
             const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
@@ -455,10 +482,96 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     }
                 }
             }
-        } else if (!failed && !abort_s) {
+        }
+        if (!whole && !failed && !abort_s) {
             abort_s = 1;
             atomicExch(p.status, 16);
         }
+    }
+    if constexpr (SHARED) {
+        __syncwarp();
+        cluster_sync_all();
+        const int hs = (warp - 2) >> 2;
+        if (warp >= 2 && warp != 10 && hs < n_heads) {
+            const int r = (warp & 3) * 32 + lane, head = h0 + hs;
+            float m = -INFINITY, mp[8], lp[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                mp[q] = -INFINITY;
+                lp[q] = 0.f;
+                if (q < parts)
+                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(mp[q]), "=f"(lp[q])
+                                 : "r"(cluster_map(gt_smem(base) + 2 * D * 512 + (hs * 128 + r) * 8, q)) : "memory");
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) m = fmaxf(m, mp[q]);
+            float l = 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                mp[q] = mp[q] == -INFINITY ? -1.f : exp2f(mp[q] - m);       // now the part's weight; below 0: it saw no key
+                if (mp[q] >= 0.f) l += lp[q] * mp[q];
+            }
+            if (p.sinks && m != -INFINITY) l += exp2f(p.sinks[head] * AT_LOG2E - m);
+            const float inv = l > 0.f ? 1.f / l : 0.f;
+            const size_t row = (size_t)(tok0 + r);
+            const int c_end = D / 8 * (part + 1) / parts;
+            for (int c0 = D / 8 * part / parts; c0 < c_end; c0 += 2) {      // twice eight columns, all parts' asked for at once
+                float o[2][8];
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) o[i][e] = 0.f;
+#pragma unroll
+                for (int q0 = 0; q0 < 8; q0 += 4) {
+                    if (q0 >= parts) break;
+                    float v[4][2][8];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            if (q0 + q < parts && c0 + i < c_end) {
+                                const uint32_t at = cluster_map(gt_smem(base) + ((hs * (D / 4) + 2 * (c0 + i)) * 128 + r) * 16, q0 + q);
+                                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                             : "=f"(v[q][i][0]), "=f"(v[q][i][1]), "=f"(v[q][i][2]), "=f"(v[q][i][3]) : "r"(at));
+                                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                             : "=f"(v[q][i][4]), "=f"(v[q][i][5]), "=f"(v[q][i][6]), "=f"(v[q][i][7]) : "r"(at + 2048));
+                            }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (q0 + q < parts && mp[q0 + q] >= 0.f) {
+#pragma unroll
+                            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) o[i][e] = fmaf(v[q][i][e], mp[q0 + q], o[i][e]);
+                        }
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int c = c0 + i;
+                    if (r >= rows || c >= c_end) continue;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) o[i][e] *= inv;
+                    if (p.out_f32) {
+                        float* dst = reinterpret_cast<float*>(p.out) + row * p.out_stride + (size_t)head * D + c * 8;
+                        *reinterpret_cast<float4*>(dst) = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
+                        *reinterpret_cast<float4*>(dst + 4) = make_float4(o[i][4], o[i][5], o[i][6], o[i][7]);
+                        continue;
+                    }
+                    if (p.gate) {
+                        const uint4 g = *reinterpret_cast<const uint4*>(p.gate + row * p.gate_stride + (size_t)head * D + c * 8);
+                        const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            o[i][2 * e] *= __fdividef(1.f, 1.f + __expf(-__uint_as_float(gw[e] << 16)));
+                            o[i][2 * e + 1] *= __fdividef(1.f, 1.f + __expf(-__uint_as_float(gw[e] & 0xffff0000u)));
+                        }
+                    }
+                    *reinterpret_cast<uint4*>(p.out + row * p.out_stride + (size_t)head * D + c * 8) =
+                        make_uint4(pack_bf16x2(o[i][0], o[i][1]), pack_bf16x2(o[i][2], o[i][3]), pack_bf16x2(o[i][4], o[i][5]), pack_bf16x2(o[i][6], o[i][7]));
+                }
+            }
+        }
+        cluster_sync_all();         // nobody leaves while its O is read
     }
 
     tc_fence_before();
@@ -469,29 +582,36 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
 }
 
-template <int D>
-static int launch_attn_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcParams& p,
+template <int D, bool SHARED>
+static int launch_attn_tc_as(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcParams& p,
                           int n_tiles, cudaStream_t stream) {
     constexpr int SMEM = 2 * (D / 64) * AT_ATOM /*Q of two heads*/ + 4 * (D / 64) * AT_ATOM /*K,V x2*/ + 1024 + 256;
     static AcvSmemConfig smem_config;          // per kernel instance and device
-    if (int rc = acv_ensure_smem(smem_config, attn_tc_kernel<D>, SMEM)) return rc;
-    const int n_rep = p.NH / p.NKV;
-    acv_launch(PDL_MISC, attn_tc_kernel<D>, dim3((unsigned)(n_tiles * (p.NKV * ((n_rep + 1) / 2)))), AT_THREADS, SMEM, stream, mq, mk, mv, p);
+    if (int rc = acv_ensure_smem(smem_config, attn_tc_kernel<D, SHARED>, SMEM)) return rc;
+    acv_launch_cluster(PDL_MISC, dim3(p.parts, 1, 1), attn_tc_kernel<D, SHARED>, dim3((unsigned)(n_tiles * p.NKV * p.pairs * p.parts)),
+                       dim3(AT_THREADS), SMEM, stream, mq, mk, mv, p);
     return acv_launch_status();
+}
+
+template <int D>
+static int launch_attn_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcParams& p, int n_tiles, cudaStream_t stream) {
+    return p.parts > 1 ? launch_attn_tc_as<D, true>(mq, mk, mv, p, n_tiles, stream) : launch_attn_tc_as<D, false>(mq, mk, mv, p, n_tiles, stream);
 }
 
 // q: the step's stacked projection [T, q_width] (queries are its first NH*D columns, row stride q_stride);
 // pages [num_pages, NKV, page_size, D]; tile lists as for the tiled kernel, with tiles of 128 query tokens.
-// Takes head sizes 64 and 128 and page sizes that are powers of two from 8 to 128.
+// Takes head sizes 64 and 128 and page sizes that are powers of two from 8 to 128.  parts: CTAs that share a tile's keys (1 to 8);
+// parts_odd > 0: the odd heads of the groups by a launch of their own, with so many.
 ACV_API int acv_attention_tc(const void* q, int q_stride, int T, void* out, int out_stride, const void* k_pages,
                              const void* v_pages, const int* tile_seq, const int* tile_q0, int n_tiles, const int* cu_q,
                              const int* kv_len, const int* block_table, int bt_stride, const int* bt_rows, int NH, int NKV,
                              int D, int page_size, int num_pages, float scale, int window, int chunk, int out_f32, int* status,
                              int keep_first, const float* sinks, const float* slopes, const void* gate, int gate_stride,
-                             cudaStream_t stream) {
+                             int parts, int parts_odd, cudaStream_t stream) {
     if (n_tiles <= 0) return 0;
     if (NKV <= 0 || NH % NKV || NH > 65535 || (D != 64 && D != 128)) return ACV_ERR_SIZE;
-    if ((long long)n_tiles * NH > 0x7fffffffLL) return ACV_ERR_SIZE;
+    if (parts < 1 || parts > 8 || parts_odd < 0 || parts_odd > 8 || (parts_odd && (NH / NKV % 2 == 0 || NH / NKV < 3))) return ACV_ERR_SIZE;
+    if ((long long)n_tiles * NH * 8 > 0x7fffffffLL) return ACV_ERR_SIZE;
     int page_shift = -1;
     for (int b = 3; b <= 7; ++b)
         if ((1 << b) == page_size) page_shift = b;
@@ -520,8 +640,15 @@ ACV_API int acv_attention_tc(const void* q, int q_stride, int T, void* out, int 
     if (gate && out_f32) return ACV_ERR_SIZE;
     if (slopes && !(scale > 0.f)) return ACV_ERR_SIZE;
     p.status = status;
-    if (D == 64) return launch_attn_tc<64>(mq, mk, mv, p, n_tiles, stream);
-    return launch_attn_tc<128>(mq, mk, mv, p, n_tiles, stream);
+    p.parts = parts;
+    p.pair0 = 0;
+    p.pairs = parts_odd ? NH / NKV / 2 : (NH / NKV + 1) / 2;
+    if (const int e = D == 64 ? launch_attn_tc<64>(mq, mk, mv, p, n_tiles, stream) : launch_attn_tc<128>(mq, mk, mv, p, n_tiles, stream)) return e;
+    if (!parts_odd) return 0;
+    p.parts = parts_odd;
+    p.pair0 = p.pairs;
+    p.pairs = 1;
+    return D == 64 ? launch_attn_tc<64>(mq, mk, mv, p, n_tiles, stream) : launch_attn_tc<128>(mq, mk, mv, p, n_tiles, stream);
 }
 
 ACV_TL_EXPORT(attention_tc)

@@ -124,7 +124,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "acv_gemm_tc": [P, I, P, I, P, I, I, I, I, I, I, I, I, I, P, LL, P, LL, P, I, I, I, P],
         "acv_gemm_tc_bias": [P, I, P, I, P, I, I, I, I, I, I, I, I, I, P, LL, P, LL, P, I, I, I, P, F, F, P],
         "acv_attention_decode": [P, I, P, I, P, P, P, P, I, P, P, I, P, I, I, I, I, I, F, I, I, I, P, P, P, LL, LL, LL, I, I, I, I, P, P, P, I, P],
-        "acv_attention_tc": [P, I, I, P, I, P, P, P, P, I, P, P, P, I, P, I, I, I, I, I, F, I, I, I, P, I, P, P, P, I, P],
+        "acv_attention_tc": [P, I, I, P, I, P, P, P, P, I, P, P, P, I, P, I, I, I, I, I, F, I, I, I, P, I, P, P, P, I, I, I, P],
         "acv_attention_chunk": [P, I, P, I, P, P, P, P, I, P, P, P, I, P, I, I, I, I, I, F, I, I, I, I, P],
         "acv_table_update": [P, I, I, P, I, P],
         "acv_embed_scaled": [P, P, P, I, I, I, F, I, P],
@@ -932,16 +932,18 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pa
                  block_table: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim: int, scale: float,
                  window: int, table_rows: torch.Tensor | None = None, chunk: int = 0, keep_first: int = 0,
                  sinks: torch.Tensor | None = None, slopes: torch.Tensor | None = None,
-                 gate: torch.Tensor | None = None) -> torch.Tensor:
+                 gate: torch.Tensor | None = None, parts: tuple = (1, 0)) -> torch.Tensor:
     """Causal attention of portions of prompts on tcgen05 (tiles of QUERY_TILE query tokens, pages by TMA).
-    ``sinks``, ``slopes`` (float32 [heads]), ``gate``: as in ``attention_generic``."""
+    ``sinks``, ``slopes`` (float32 [heads]), ``gate``: as in ``attention_generic``.  ``parts``: how many thread blocks, a
+    cluster, share a tile's keys, and where the second is not 0 the same for the groups' odd heads, by a launch of their own
+    (``attention_tc_parts``)."""
     _head_vectors(num_heads, sinks, slopes)
     _, _, status = _gemm_buffers(q.device, 0, 0)
     _check(library().acv_attention_tc(
         _p(q), q.stride(0), q.shape[0], _p(out), out.stride(0), _p(k_pages), _p(v_pages), _p(tile_seq), _p(tile_q0),
         n_tiles, _p(cu_q), _p(kv_len), _p(block_table), block_table.stride(0), _p(table_rows), num_heads, num_kv_heads,
         head_dim, k_pages.shape[2], k_pages.shape[0], scale, window, chunk, 1 if out.dtype == torch.float32 else 0, _p(status),
-        int(keep_first), _p(sinks), _p(slopes), *_gate_args(gate, out), _stream()), "attention_tc")
+        int(keep_first), _p(sinks), _p(slopes), *_gate_args(gate, out), *parts, _stream()), "attention_tc")
     return out
 
 
@@ -985,7 +987,57 @@ def attention_work(q_lens, kv_lens, cu_q) -> tuple[dict, dict]:
     values = {"n_dec": int(dec.size), "n_tiles": int(sum(t.size for t in tile_seq)),
               "max_dec_kv": max((k for k, q in zip(kv_lens, q_lens) if q == 1), default=0),
               "max_tile_kv": max((k for k, q in zip(kv_lens, q_lens) if q > 1), default=0)}
+    if tile_keys:           # key tiles of all tiles, of the longest and of the shortest
+        blocks = -(-np.concatenate(tile_keys) // QUERY_TILE)
+        values["tile_blocks"] = (int(blocks.sum()), int(blocks.max()), int(blocks.min()))
     return arrays, values
+
+
+# Clusters of 1..8 thread blocks, an SM to each, that a B200's parts hold at once.
+CLUSTERS_AT_ONCE = (0, 148, 74, 45, 33, 26, 22, 15, 15)
+
+
+# Microseconds in ``attention_tc``: a round of blocks, a round that merges its clusters' parts, a tile of 128 keys of two heads;
+# and what a head without a partner takes of that.
+TC_PARTS_FIXED, TC_PARTS_MERGE, TC_PARTS_BLOCK, TC_PARTS_ODD = 4.0, 12.0, 2.1, 0.6
+
+
+def _tc_parts(units: int, work: float, longest: float, shortest: float, sms: int, rounds_of: int) -> tuple:
+    """(least microseconds, parts) for ``units`` of blocks with ``work`` key tiles in all."""
+    best = None
+    for parts in range(1, max(1, min(8, rounds_of)) + 1):
+        at_once = max(1, CLUSTERS_AT_ONCE[parts] * sms // 148)
+        span = longest if parts == 1 else longest / rounds_of * -(-rounds_of // parts)
+        if units > at_once:
+            span = max(span, work / (parts * at_once) + shortest / parts)
+        cost = -(-units // at_once) * (TC_PARTS_FIXED if parts == 1 else TC_PARTS_MERGE) + span * TC_PARTS_BLOCK
+        if best is None or cost < (0.95 * best[0] if best[1] == 1 else best[0]):
+            best = (cost, parts)
+    return best
+
+
+@functools.lru_cache(maxsize=4096)
+def attention_tc_parts(n_tiles: int, blocks: tuple, num_heads: int, num_kv_heads: int, limit: int, sms: int) -> tuple:
+    """How many blocks share the keys of a tile of queries in ``attention_tc`` (``parts`` there), by the time of the rounds of
+    blocks that come one after the other.  ``blocks``: key tiles of all tiles of queries, of the longest and of the shortest;
+    ``limit`` > 0: none sees more.  Microseconds with one block and with the parts chosen: 16 heads on 8, 1000 tokens behind 5000
+    101 -> 62, 64 behind 2000 40 -> 19; 32 on 8, 500 behind 5000 94 -> 58, 2048 in front of nothing (256 blocks) 48 either way;
+    40 on 8, 1000 behind 5000, pairs by one block and the fifth heads by two, 169 -> 150."""
+    total, longest, shortest = blocks
+    if limit and limit < longest:
+        total, longest, shortest = min(total, n_tiles * limit), limit, min(shortest, limit)
+    n_rep, each = num_heads // num_kv_heads, n_tiles * num_kv_heads
+    if n_rep == 1:          # one head to a block throughout
+        return _tc_parts(each, total * num_kv_heads * TC_PARTS_ODD, longest * TC_PARTS_ODD, shortest * TC_PARTS_ODD, sms, longest)[1], 0
+    pairs, odd = n_rep // 2, n_rep % 2
+    cost, parts = _tc_parts(each * (pairs + odd), total * num_kv_heads * (pairs + TC_PARTS_ODD * odd), longest,
+                            shortest * (TC_PARTS_ODD if odd else 1.0), sms, longest)
+    if odd:
+        a = _tc_parts(each * pairs, total * num_kv_heads * pairs, longest, shortest, sms, longest)
+        b = _tc_parts(each, total * num_kv_heads * TC_PARTS_ODD, longest * TC_PARTS_ODD, shortest * TC_PARTS_ODD, sms, longest)
+        if a[0] + b[0] + 3.0 < 0.95 * cost:
+            return a[1], b[1]
+    return parts, 0
 
 
 def attention_work_decode(padded: int, max_kv: int) -> tuple[dict, dict]:
@@ -994,6 +1046,14 @@ def attention_work_decode(padded: int, max_kv: int) -> tuple[dict, dict]:
     ar = np.arange(padded, dtype=np.int32)
     return ({"dec_tokens": ar, "dec_seqs": ar, "tile_seq": np.zeros(0, np.int32), "tile_q0": np.zeros(0, np.int32)},
             {"n_dec": padded, "n_tiles": 0, "max_dec_kv": max_kv, "max_tile_kv": 0})
+
+
+def _tile_parts(work: dict, num_heads: int, num_kv_heads: int, window: int, keep_first: int, chunk: int, device) -> tuple:
+    if "tile_blocks" not in work:
+        return 1, 0
+    seen = min((n for n in (window + keep_first if window > 0 else 0, chunk) if n > 0), default=0)
+    return attention_tc_parts(work["n_tiles"], work["tile_blocks"], num_heads, num_kv_heads, -(-seen // QUERY_TILE) + 1 if seen else 0,
+                              sm_count(device))
 
 
 def attention(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, ctx,
@@ -1052,7 +1112,8 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pag
     if w["n_tiles"] and attention_tc_takes(qkv, out, k_pages, head_dim):
         attention_tc(qkv, out, k_pages, v_pages, w["tile_seq"], w["tile_q0"], w["n_tiles"], ctx.cu_q, ctx.kv_len,
                      block_table, num_heads, num_kv_heads, head_dim, scale, window, table_rows=rows, chunk=chunk,
-                     keep_first=keep_first, sinks=sinks, slopes=slopes, gate=gate)
+                     keep_first=keep_first, sinks=sinks, slopes=slopes, gate=gate, parts=_tile_parts(w, num_heads, num_kv_heads, window,
+                     keep_first, chunk, qkv.device))
     elif w["n_tiles"]:
         attention_chunk(qkv, out, k_pages, v_pages, w["tile_seq"], w["tile_q0"], w["n_tiles"], ctx.cu_q, ctx.kv_len,
                         block_table, num_heads, num_kv_heads, head_dim, scale, window, table_rows=rows,

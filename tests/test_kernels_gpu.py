@@ -900,6 +900,43 @@ def test_tensor_core_attention_growing_scores(ops):
         torch.testing.assert_close(o1, o2, **tol(torch.bfloat16))
 
 
+@pytest.mark.parametrize("parts", [(2, 0), (3, 0), (8, 0), (1, 2), (2, 3)])
+@pytest.mark.parametrize("NH,NKV,D,window,keep,extra", [(10, 2, 128, 0, 0, ""), (4, 2, 64, 0, 0, "sinks"), (6, 2, 128, 300, 0, "gate"), (3, 3, 64, 200, 70, "float"), (10, 2, 64, 0, 0, "slopes")])
+def test_tensor_core_attention_with_keys_shared_out(ops, parts, NH, NKV, D, window, keep, extra):
+    """A tile's key tiles over a cluster's blocks (more blocks than key tiles among them, pairs of heads and heads without a
+    partner, the odd heads by a launch of their own) against one block: the same softmax with its weights taken relative to
+    another maximum, so a weight's rounding to bfloat16 may fall differently."""
+    if parts[1] and (NH // NKV % 2 == 0 or NH // NKV < 3):
+        pytest.skip("no odd heads beside pairs")
+    import numpy as np
+    q_lens, lens, page = [300, 2, 129, 40], [1100, 2, 129, 900], 16
+    cu = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    arrays, values = ops.attention_work(q_lens, lens, cu)
+    T, per = int(cu[-1]), max(lens) // page + 1
+    d = lambda a: torch.as_tensor(np.asarray(a, dtype=np.int32), device="cuda")
+    q = rnd(T, (NH + 2 * NKV) * D, dtype=torch.bfloat16, seed=270)
+    kp, vp = (rnd(4 * per, NKV, page, D, dtype=torch.bfloat16, seed=s) for s in (271, 272))
+    table = torch.randperm(4 * per, device="cuda").to(torch.int32).view(4, per).contiguous()
+    table[3, 3] = -1            # a page that is not held
+    more = {"sinks": {"sinks": rnd(NH, seed=273)}, "slopes": {"slopes": rnd(NH, seed=274).abs() * 0.01},
+            "gate": {"gate": rnd(T, NH * D, dtype=torch.bfloat16, seed=275)}}.get(extra, {})
+    run = lambda p: ops.attention_tc(q, torch.full((T, NH * D), 7.0, device="cuda", dtype=torch.float32 if extra == "float" else torch.bfloat16),
+                                     kp, vp, d(arrays["tile_seq"]), d(arrays["tile_q0"]), values["n_tiles"], d(cu), d(lens), table, NH, NKV, D,
+                                     D ** -0.5, window, keep_first=keep, parts=p, **more)
+    torch.testing.assert_close(run(parts), run((1, 0)), **tol(torch.bfloat16))
+    assert ops.gemm_status() == 0
+
+
+def test_attention_tc_parts():
+    """One block where the SMs have enough of them, more where they have not, never more than key tiles."""
+    from acvram_b200.kernels.ops import attention_tc_parts
+    assert attention_tc_parts(16, (136, 16, 1), 32, 8, 0, 148) == (1, 0)
+    assert attention_tc_parts(8, (355, 47, 41), 40, 8, 0, 148) == (1, 2)
+    assert attention_tc_parts(8, (355, 47, 41), 16, 8, 0, 148)[0] > 1
+    assert attention_tc_parts(8, (355, 47, 41), 16, 8, 2, 148) == (1, 0)
+    assert attention_tc_parts(1, (3, 3, 3), 2, 2, 0, 148)[0] <= 3
+
+
 @pytest.mark.parametrize("NH,NKV,D,T,K", [(32, 8, 128, 8, 4096), (6, 2, 64, 5, 264), (5, 1, 64, 17, 128), (4, 4, 128, 1, 512),
                                           (3, 1, 128, 32, 136),
                                           # many tokens: tokens on the tensor-memory lanes, whole heads inside a thread's row
