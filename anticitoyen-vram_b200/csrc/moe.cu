@@ -11,37 +11,15 @@
 //   acv_moe_route    one warp per token: router logits, scores, choice; also the shared expert's gate
 //   acv_moe_group    one block: rows (token, choice) counted per expert, each expert's rows padded to
 //                    whole tiles of MOE_TILE rows; a tile belongs to one expert
-//   acv_moe_gemm_*   tiles x column blocks: rows gathered by the grouping, the expert's weights by tile
+//   acv_moe_gemm_*   tiles x column blocks: rows gathered by the grouping, the expert's weights by tile (few rows to an expert:
+//                    acv_moe_rows, csrc/moe_rows.cu)
 //   acv_moe_combine  per token: the chosen experts' outputs in the order of the choice, plus the
 //                    shared expert's output times its gate, summed in 32-bit
 #include "common.cuh"
 #include "mma_tiles.cuh"
+#include "moe_act.cuh"
 
 #define MOE_TILE 64          // rows of a tile of the grouped products (ops.MOE_TILE)
-
-// gated activation of an expert (ops.GLU_*)
-#define GLU_SWISH_CLAMPED 0  // g = min(a, limit), u = clamp(b, -limit, limit): g * sigmoid(alpha g) * (u + shift), shift 1
-// (silu(a) * b is the same unit without limits, alpha 1 and shift 0)
-// acv_glu also takes 1, 2, 3: act(a) * b with act the plain activation of that number (gelu_tanh, silu, gelu)
-
-template <typename T> __device__ __forceinline__ float sigmoid_f32(float x);
-template <> __device__ __forceinline__ float sigmoid_f32<float>(float x) { return 1.f / (1.f + expf(-x)); }
-template <> __device__ __forceinline__ float sigmoid_f32<bf16>(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-
-template <typename T>
-__device__ __forceinline__ float glu_act(float a, float b, float limit, float alpha, float shift = 1.f) {
-    const float g = fminf(a, limit);
-    const float u = fminf(fmaxf(b, -limit), limit);
-    return g * sigmoid_f32<T>(alpha * g) * (u + shift);
-}
-
-// activation of an expert that has no gate: y = act(W_up x), out = W_down y  (ops.ACTIVATIONS)
-__device__ __forceinline__ float plain_act(float z, int kind) {
-    if (kind == 1) return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-    if (kind == 2) return z / (1.f + expf(-z));
-    if (kind == 3) return 0.5f * z * (1.f + erff(z * 0.7071067811865476f));
-    return z;
-}
 
 // ----------------------------------------------------------------------------- routing
 #define MR_WARPS 4

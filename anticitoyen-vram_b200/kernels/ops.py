@@ -99,6 +99,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "acv_gated_delta_blocks": [P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
         "acv_gated_delta_step_takes": [I, I],
         "acv_gated_delta_step": [P, I, P, P, P, P, F, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
+        "acv_moe_rows": [P, I, P, LL, I, P, I, P, P, P, I, P, I, I, I, I, I, F, F, F, I, I, P],
         "acv_gemm_rows": [P, I, P, I, P, I, I, I, I, I, I, I, I, P],
         "acv_gemm_rows_qkv": [P, I, P, I, P, I, I, I, I, I, I, I, I, I, P, P, F, P, I, P, P, P, I, P, P, P, I, I, P],
         "acv_gemm_simt": [P, I, P, I, P, I, I, I, I, I, I, P, P],
@@ -1474,6 +1475,40 @@ def moe_gemm_mma(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, grouped: t
                                       _p(grouped), _p(tile_expert), _p(row_weight), top, tile_expert.numel(), N, K,
                                       which, limit, alpha, shift, int(pairs), _stream()), "moe_gemm_mma")
     return out
+
+
+def moe_rows(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, grouped: torch.Tensor, tile_expert: torch.Tensor,
+             tiles_used: torch.Tensor, tile: int, row_weight: torch.Tensor | None, top: int, glu: bool, limit: float = 0.0,
+             alpha: float = 0.0, pairs: bool = False, plain_act: str | None = None, shift: float = 1.0) -> torch.Tensor:
+    """``moe_gemm_mma`` for tiles of 8 or 16 rows (``moe_rows_tile``): the arguments of that, the rows of ``out`` in the order of
+    ``grouped``."""
+    _need_cuda(a, w, out, grouped, tile_expert, tiles_used)
+    E, NW, K = w.shape
+    N = NW // 2 if glu else NW
+    which, pairs = _moe_which(glu, plain_act, pairs)
+    if a.shape[1] != K or out.shape[1] != N or out.stride(1) != 1 or out.dtype != (torch.bfloat16 if which != 1 else torch.float32) or \
+            out.shape[0] < tile_expert.numel() * tile or grouped.numel() < tile_expert.numel() * tile:
+        raise KernelError(f"moe_rows: shapes {tuple(a.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
+    _check(library().acv_moe_rows(_p(a), a.stride(0), _p(w), w.stride(0), w.stride(1), _p(out), out.stride(0), _p(grouped),
+                                  _p(tile_expert), _p(tiles_used), tile, _p(row_weight), top, tile_expert.numel(), N, K, which, limit,
+                                  alpha, shift, int(pairs), sm_count(a.device), _stream()), "moe_rows")
+    return out
+
+
+def moe_rows_tile(rows: int, experts: int, h: torch.Tensor, up: torch.Tensor, down: torch.Tensor) -> int:
+    """Rows of a tile (8 or 16) where the experts' products are made by ``moe_rows``, 0 where they are not."""
+    tile = 8 if rows <= MOE_ROWS_8 * experts else 16
+    if rows > MOE_ROWS_16 * experts or h.shape[1] % 64 or down.shape[2] % 64 or up.shape[1] % 32 or down.shape[1] % 32 \
+            or not moe_gemm_mma_takes(h, up):
+        return 0
+    tiles = moe_max_tiles(rows, experts, tile)
+    return tile if tiles <= 512 and tiles * tile <= 2048 else 0
+
+
+# Rows to an expert up to which tiles of 8 and of 16 rows are used.  A layer's microseconds with tiles of 64 (moe_gemm_mma), 8 and 16
+# rows: 64 experts of 1024 at width 4096 at 0.1 rows an expert 102, 57, 60; 1.5: 273, 229, 246; 6: 360, 302, 304; 9.4: 369, 344, 320;
+# 32 experts of 768 at width 2048 at 8: 99, 96, 96; 12.5: 106, 122, 113.
+MOE_ROWS_8, MOE_ROWS_16 = 7, 10
 
 
 def moe_experts_up(h: torch.Tensor, gate_up: torch.Tensor, act: torch.Tensor, grouped: torch.Tensor, tile_expert: torch.Tensor,

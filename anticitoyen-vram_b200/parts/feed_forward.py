@@ -333,6 +333,19 @@ class RoutedExperts(FeedForward):
             # the experts' outputs leave the product as bfloat16 (as every projection's do); their sum is 32-bit
             parts = torch.empty((tiles * tile, H), device=dev, dtype=h.dtype)
             ops.gemm_tc_grouped(act, self.down, parts, tile_expert, used, row_scale=scale if w_out is not None else None)
+        elif tile := ops.moe_rows_tile(rows, E, h, self.gate_up, self.down):
+            # few rows to an expert: the weights' stream is all
+            tiles = ops.moe_max_tiles(rows, E, tile)
+            grouped = torch.empty(tiles * tile, device=dev, dtype=torch.int32)
+            tile_expert = torch.empty(tiles, device=dev, dtype=torch.int32)
+            used = torch.empty(1, device=dev, dtype=torch.int32)
+            ops.moe_group(ids, E, grouped, place, tile_expert, tile, used)
+            act = torch.empty((tiles * tile, F), device=dev, dtype=h.dtype)
+            limit, alpha, shift = self.unit
+            ops.moe_rows(h, self.gate_up, act, grouped, tile_expert, used, tile, w_in, top, not self.plain, limit, alpha, self.pairs,
+                         plain_act=self.activation if self.plain else None, shift=shift)
+            parts = torch.empty((tiles * tile, H), device=dev, dtype=torch.float32)
+            ops.moe_rows(act, self.down, parts, grouped, tile_expert, used, tile, w_out, top, False)
         else:
             grouped = torch.empty(tiles * ops.MOE_TILE, device=dev, dtype=torch.int32)
             tile_expert = torch.empty(tiles, device=dev, dtype=torch.int32)

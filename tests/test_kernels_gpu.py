@@ -980,3 +980,37 @@ def test_gemm_tc_qkv_epilogue(ops, NH, NKV, D, T, K, normed, rotated, pair):
     torch.testing.assert_close(kp2, kp1, **tol(torch.bfloat16))
     assert torch.equal(vp2, vp1)
     assert (q2 != q1).float().mean() < 0.02 and (kp2 != kp1).float().mean() < 0.02
+
+
+@pytest.mark.parametrize("tile", [8, 16])
+@pytest.mark.parametrize("form", ["gated", "pairs", "plain", "down"])
+@pytest.mark.parametrize("T,E,top,N,K", [(1, 4, 2, 64, 64), (13, 6, 3, 96, 640), (40, 3, 2, 32, 2112)])
+def test_moe_rows(ops, tile, form, T, E, top, N, K):
+    """The experts' products in tiles of 8 and 16 rows against the tiled form, row by row: experts without a row, with a part of a
+    tile and with several tiles; K that leaves warps without a chunk and K that their rings go round in."""
+    rows = T * top
+    g = torch.Generator(device="cuda").manual_seed(280)
+    ids = torch.randint(0, max(1, E - 1), (rows,), device="cuda", generator=g, dtype=torch.int32)      # (the last expert has none)
+    weight = torch.rand(rows, device="cuda", generator=g) + 0.5
+    glu, plain = form in ("gated", "pairs"), "silu" if form == "plain" else None
+    w = rnd(E, 2 * N if glu else N, K, dtype=torch.bfloat16, scale=0.05, seed=281)
+    outs = []
+    for t in (ops.MOE_TILE, tile):
+        tiles = ops.moe_max_tiles(rows, E, t)
+        grouped, te, place = (torch.empty(n, device="cuda", dtype=torch.int32) for n in (tiles * t, tiles, rows))
+        used = torch.empty(1, device="cuda", dtype=torch.int32)
+        ops.moe_group(ids, E, grouped, place, te, t, used)
+        x = rnd(T, K, dtype=torch.bfloat16, seed=282)
+        if form == "down":
+            by_row = rnd(rows, K, dtype=torch.bfloat16, seed=283)
+            x = torch.zeros(tiles * t, K, device="cuda", dtype=torch.bfloat16)
+            x[place.long()] = by_row
+        out = torch.zeros(tiles * t, N, device="cuda", dtype=torch.float32 if form == "down" else torch.bfloat16)
+        more = dict(limit=7.0, alpha=1.702, pairs=form == "pairs", plain_act=plain)
+        if t == ops.MOE_TILE:
+            ops.moe_gemm_mma(x, w, out, grouped, te, weight, top, glu, **more)
+        else:
+            ops.moe_rows(x, w, out, grouped, te, used, t, weight, top, glu, **more)
+        outs.append(out[place.long()])
+    torch.testing.assert_close(outs[1], outs[0], **(dict(rtol=1e-4, atol=1e-4) if form == "down" else tol(torch.bfloat16)))
+    assert outs[0].abs().max() > 0
