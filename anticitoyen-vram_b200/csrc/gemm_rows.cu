@@ -1,4 +1,4 @@
-// C[M,N] = X[M,K] . W[N,K]^T in bfloat16 for up to 16 tokens, float accumulators: the products of a decode step.
+// C[M,N] = X[M,K] . W[N,K]^T in bfloat16 for up to 32 tokens, float accumulators: the products of a decode step.
 //
 // What bounds such a product beside its weights' stream is what comes before the first and after the last of it: of the 5 us that
 // a product of a few MB took on tcgen05 (128 weight rows to a tile, K split over a cluster, the splits' tiles sent to one CTA, the
@@ -272,7 +272,7 @@ static bool rw_wide(int N, int K, int sms) {
 }
 
 static int rw_checks(const RowsParams& p) {
-    if (p.M > 16 || p.K <= 0 || p.K % 64 || p.N % 16) return ACV_ERR_SIZE;
+    if (p.M > 32 || p.K <= 0 || p.K % 64 || p.N % 16) return ACV_ERR_SIZE;
     if (((uintptr_t)p.x | (uintptr_t)p.w) % 16 || p.ldx % 8 || p.ldw % 8) return ACV_ERR_ALIGN;
     return 0;
 }
@@ -288,6 +288,7 @@ ACV_API int acv_gemm_rows(const void* x, int ldx, const void* w, int ldw, void* 
     p.out_f32 = out_f32; p.swiglu = swiglu; p.early_w = flags & 1;
     if (const int e = rw_checks(p)) return e;
     if (swiglu && out_f32) return ACV_ERR_DTYPE;
+    if (M > 16) return rw_launch<2, 4, 3, false>(p, sms, stream);
     const bool wide = rw_wide(N, K, sms);
     if (M > 8) return wide ? rw_launch<4, 2, 3, false>(p, sms, stream) : rw_launch<2, 2, 6, false>(p, sms, stream);
     if (!wide) return K <= 1024 ? rw_launch<2, 1, 3, false>(p, sms, stream) : rw_launch<2, 1, 6, false>(p, sms, stream);
@@ -307,7 +308,7 @@ ACV_API int acv_gemm_rows_qkv(const void* x, int ldx, const void* w, int ldw, vo
     p.positions = positions; p.seq_of_token = seq_of_token; p.block_table = block_table; p.bt_stride = bt_stride; p.bt_rows = bt_rows;
     p.k_pages = (bf16*)k_pages; p.v_pages = (bf16*)v_pages; p.page_size = page_size; p.num_pages = num_pages;
     if (const int e = rw_checks(p)) return e;
-    if ((D != 64 && D != 128) || N != (NH + 2 * NKV) * D || page_size <= 0) return ACV_ERR_SIZE;
+    if (M > 16 || (D != 64 && D != 128) || N != (NH + 2 * NKV) * D || page_size <= 0) return ACV_ERR_SIZE;
     if (M > 8) return rw_launch<4, 2, 3, true>(p, sms, stream);
     // more heads than come at once with an SM to a block: a shallow ring, two blocks to an SM
     if (N / D > (D == 128 ? 33 : 74) * sms / 148) return rw_launch<4, 1, 2, true>(p, sms, stream);

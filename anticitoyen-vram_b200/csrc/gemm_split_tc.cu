@@ -15,9 +15,9 @@
 // Converter warps read float rows straight into registers (a stage ahead), cut them into parts and leave those in shared
 // memory as swizzled K-major tiles; one thread issues the products; other warps add up the chunks.
 //
-// What bounds it: the converters' instructions (five an element and operand) and a stage's hand-overs; the tensor cores are
-// busy 40 % of the time.  Microseconds, eight chains of multiply-adds on the CUDA cores (gemm_simt.cu) and now: 696 tokens
-// 4096 x 1024 212 -> 75, 1024 x 2048 101 -> 50, 1024 x 3072 143 -> 65, 2048 tokens 4096 x 4096 1750 -> 518 (133 TFLOP/s),
+// What bounds it: shared memory (a stage of 128 tokens takes it some 2300 clocks, 96 KB of parts written and what the products read
+// of them, the tensor cores 1536) and the stages' hand-overs; the tensor cores are busy 50 % of the time.  Microseconds, eight chains of multiply-adds on the CUDA cores (gemm_simt.cu) and now: 696 tokens
+// 4096 x 1024 212 -> 71, 1024 x 2048 101 -> 49, 1024 x 3072 143 -> 62, 2048 tokens 4096 x 4096 1750 -> 479 (143 TFLOP/s),
 // 64 tokens 4096 x 1024 22 -> 14, 17 tokens 151936 x 1024 355 -> 214.  Error against 64 bits (2-norm): K 1024 2.1e-7 ->
 // 0.94e-7, 4096 4.1e-7 -> 1.1e-7, 12288 6.8e-7 -> 1.5e-7.
 #include "tc_ptx.cuh"
@@ -35,6 +35,9 @@ struct GfTile {
     // (registers are given out to warps by fours, so the one warp that issues the products comes with three that do nothing)
     static constexpr int THREADS = (GF_CONV + EPI + 4) * 32;
     static constexpr int COLS = BT / (EPI / 4);                 // tokens of an epilogue thread
+    // the next stage's rows asked for once this one is handed over, not row by row as their registers come free: 2048 tokens
+    // 4096 x 4096 518 -> 479 us in tiles of 128 tokens, whose converters are short of registers, no change in the others
+    static constexpr bool LATE = EPI == 8;
     static constexpr int PIECE = EPI == 8 ? 16 : 32;            // columns read at a time (96 registers a thread, or 128)
     static constexpr int TMEM = 4 * BT < 32 ? 32 : 4 * BT;      // three chunks | the groups' sum
     static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
@@ -201,12 +204,20 @@ gemm_split_tc_kernel(const GfArgs p, int parts, int per) {
                 if (!mine(i)) break;
                 gf_store_parts(at + (i < W_ROUNDS ? i : i - W_ROUNDS) * (GF_CONV * 4 * 128) + (i < W_ROUNDS ? 0 : 3 * T::W_PART),
                                i < W_ROUNDS ? T::W_PART : T::T_PART, x[i]);
-                if (whole) gf_load8<PIECES>(row_of(i) + next, x[i]);
+                if (!T::LATE && whole) gf_load8<PIECES>(row_of(i) + next, x[i]);
             }
-            if (!whole && it + 1 < iters) ragged(next);
+            if (!T::LATE && !whole && it + 1 < iters) ragged(next);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(full0 + 8 * s);
+            if constexpr (T::LATE) {
+                if (whole) {
+#pragma unroll
+                    for (int i = 0; i < ROUNDS; ++i) gf_load8<PIECES>(row_of(i) + next, x[i]);
+                } else if (it + 1 < iters) {
+                    ragged(next);
+                }
+            }
         }
     } else if (warp < GF_CONV + T::EPI) {
         // ------------------------------------------------------------------ chunks and groups added up
@@ -346,9 +357,9 @@ int gf_run_as(const GfArgs& p, bool pieces, int batches, int way, int per, cudaS
 // Which tile and how the groups are shared out: the way whose rounds of the device take least.  A round is as many CTAs as
 // have an SM each, with clusters as many as fit the device's parts; its time in nanoseconds is a stage's times the stages of a CTA
 // and what comes before and after them, measured (4096 x 1024, microseconds: 64 tokens as 64 x all / 64 x 2 / 64 x 1 groups
-// 30 / 14 / 28; 696 tokens as 128 x all / 128 x 2 / 64 x all 75 / 107 / 82).
+// 30 / 14 / 28; 696 tokens as 128 x all / 128 x 2 / 64 x all 71 / 104 / 82).
 struct GfWay { int bt, stage, rest; };
-static const GfWay GF_WAYS[3] = {{32, 1200, 5200}, {64, 1350, 6800}, {128, 1850, 10000}};
+static const GfWay GF_WAYS[3] = {{32, 1200, 5200}, {64, 1350, 6800}, {128, 1700, 10000}};
 static const int GF_CLUSTERS[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};      // of 1..8 CTAs that 148 SMs hold at once
 
 int gf_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stream) {

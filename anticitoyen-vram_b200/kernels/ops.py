@@ -554,12 +554,15 @@ def _gemm_tc_plan(M: int, N: int, K: int, sms: int, bn_multiple: int, rows: bool
 
 @functools.lru_cache(maxsize=4096)
 def gemm_rows_pays(M: int, N: int, K: int, sms: int) -> bool:
-    """Whether a product of up to 16 tokens is faster without a tile of 128 weight rows (csrc/gemm_rows.cu) than with one:
+    """Whether a product of up to 32 tokens is faster without a tile of 128 weight rows (csrc/gemm_rows.cu) than with one:
     up to 8 tokens where the weights stay under 128 MB (12288 x 4096 20.1 us against 22.0; 24576 x 4096 35.5 against 34.9,
     5120 x 17408 37 against 34) and for a vocabulary (151936 x 1024 57.6 against 56.5, x 4096 193 against 206); up to 16, whose
-    rows each block reads, under 50 MB (12288 x 2048 11.9 us against 12.7; 5120 x 5120 15.3 against 14.0, 19456 x 2560 22.1 against 21.4)."""
-    if K % 64 or N % 16 or M > 16:
+    rows each block reads, under 50 MB (12288 x 2048 11.9 us against 12.7; 5120 x 5120 15.3 against 14.0, 19456 x 2560 22.1 against 21.4); up to 32 under 17 MB, or 26
+    where each SM has one block (4096 x 2048 7.4 us against 8.3, 2048 x 6144 9.4 against 11.6; 2560 x 4096 11.4 against 9.7)."""
+    if K % 64 or N % 16 or M > 32:
         return False
+    if M > 16:
+        return N * K <= 8_500_000 or N <= 16 * sms and N * K <= 13_000_000
     return N * K <= 1 << 26 or N >= 1 << 16 if M <= 8 else N * K <= 25_500_000
 
 
@@ -576,7 +579,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: tuple | N
 
     ``static_weights``: w was written long before this call (a model's weights), so the kernel may
     read its first tiles while the kernel before it in the stream is still running.  Without a plan, a bias or another
-    activation, up to 16 tokens then go to ``csrc/gemm_rows.cu`` where that is faster (``gemm_rows_pays``).
+    activation, up to 32 tokens then go to ``csrc/gemm_rows.cu`` where that is faster (``gemm_rows_pays``).
 
     With ``swiglu_pairs`` the rows of w come in (gate, up) pairs and out is [M, N/2]:
     out[:, i] = silu(x . w[2i]) * (x . w[2i+1]), rounded as the separate kernels round; with ``gate_fn`` 1 the gate
