@@ -448,8 +448,9 @@ __device__ __forceinline__ float cluster_all_max(ClusterSum& c, float v) {
 // part.  The bins are added up over warp, CTA and cluster (in an order that the launch shape fixes), and the sums from the top
 // down say which bin the wanted key lies in: the largest d for which over + (bins d and above) reaches `limit` (above: exceeds
 // it), 0 if none does (found: whether one did).  `over` takes the bins above d.  Returns d; seen: the cluster's count.
-__device__ __forceinline__ uint32_t cluster_bins(ClusterSum& c, float* bins, float (&v)[16], float& seen, float limit, bool above,
-                                                 float& over, bool& found) {
+// share > 0: the limit is that share of the sum of all bins.
+__device__ __forceinline__ uint32_t cluster_bins(ClusterSum& c, float* bins, float (&v)[16], float& seen, float& limit, bool above,
+                                                 float& over, bool& found, float share = 0.f) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // over the warp: a lane gives away half of what it carries at each exchange and ends with bin `lane % 16`
 #pragma unroll
@@ -486,6 +487,7 @@ __device__ __forceinline__ uint32_t cluster_bins(ClusterSum& c, float* bins, flo
         const float up = __shfl_down_sync(0xffffffffu, s, h, 16);
         if ((lane & 15) + h < 16) s += up;
     }
+    if (share > 0.f) limit = share * __shfl_sync(0xffffffffu, s, 0, 16);
     const float at = over + s;
     const uint32_t good = __ballot_sync(0xffffffffu, above ? at > limit : at >= limit) & 0xffffu;
     const int d = good ? 31 - __clz(good) : 0;
@@ -529,19 +531,22 @@ __device__ __forceinline__ uint32_t cluster_descend(ClusterSum& c, float* bins, 
 // maximum and the mean of the threads' own maxima: two fifths of a standard deviation or so, whatever the temperature, and few
 // entries at the lowest value of the type do not move it.  As soon as few enough elements took part in a pass, those of
 // the bin it chose, a few hundred of the row at most, go to every CTA of the cluster, and each finds c among them by itself:
-// the largest key whose sum (over + the candidates of its key and above) reaches the limit.  False: there are too many of
-// them, none reaches the limit, or an element's distance is no number; the caller then searches bit by bit.
-// Two or three passes and the lists instead of eight passes (8 rows of 151 936, microseconds: top-p 66 -> 43, top-k 51 -> 34, both 92 -> 53).
+// the largest key whose sum (over + the candidates of its key and above) reaches the limit.  share > 0: the limit is that share
+// of the sum of all w, which the first pass finds.  False: there are too many candidates, none reaches the limit, or an
+// element's distance is no number; the caller then searches bit by bit.
+// Two or three passes and the lists instead of eight passes (8 rows of 151 936, microseconds: top-p 66 -> 41, top-k 51 -> 34).
 #define SMPC_NEAR 64            // candidates that a CTA may bring
 struct NearList {
     float2 got[SMPC_CTAS * SMPC_NEAR], list[SMPC_CTAS * SMPC_NEAR];     // key (as bits) and w
     int counts[SMPC_CTAS], scan[32];
     uint32_t best[32];
+    float2 kept[SMPC_CTAS * SMPC_NEAR];     // of the cluster's first CTA: what is left of the row (index as bits, logit).  Its own
+    int kept_counts[SMPC_CTAS];             // place: no meeting parts it from the reading of the lists above
 };
 
 template <typename Element>
 __device__ __forceinline__ bool cluster_near(ClusterSum& c, float* bins, NearList& nl, const float* sl, float mx, float scale, int n, float limit,
-                                             bool above, Element element, uint32_t& answer) {
+                                             float share, bool above, Element element, uint32_t& answer) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (!(scale > 0.f && scale <= 1e30f)) return false;
     auto place = [&](int i) { return 4095 - min((int)((mx - sl[i]) * scale), 4095); };
@@ -569,7 +574,7 @@ __device__ __forceinline__ bool cluster_near(ClusterSum& c, float* bins, NearLis
             for (uint32_t d = 0; d < 16; ++d) v[d] += digit == d ? w : 0.f;
         }
         bool found;
-        prefix |= cluster_bins(c, bins, v, seen, limit, above, over, found) << shift;
+        prefix |= cluster_bins(c, bins, v, seen, limit, above, over, found, shift == 8 ? share : 0.f) << shift;
         if (!found || seen >= 1e9f || !(prefix >> 8)) return false;     // (or it lies in the bin of all that is far)
         if (seen > 8.f * SMPC_CTAS * SMPC_NEAR) continue;       // (spread evenly over the bins: half of the lists)
         // this CTA's candidates, thread by thread, then index by index
@@ -642,6 +647,120 @@ __device__ __forceinline__ bool cluster_near(ClusterSum& c, float* bins, NearLis
     return best != 0;
 }
 
+// What is left of a row after a top-k of a few dozen: each CTA's kept entries go to the cluster's first, in index order, which
+// makes the top-p cut and the draw alone: one meeting and no pass over the row instead of five and four (8 rows of 151 936 with
+// both rules: 53 -> 34 us, 92 with all cuts bit by bit).  The rules are the whole row's.  False: a CTA has more than a list's
+// share; the row goes on whole.
+#define SMPC_FEW 256            // top-k up to which it is tried: half of what the lists hold, as a row's best may lie unevenly
+__device__ __forceinline__ bool sample_few(ClusterSum& c, NearList& nl, float* table, const float* sl, const float* se, float mx, int lo, int n,
+                                           uint32_t cut, float mp, float tp, uint64_t seed, uint64_t counter, int* out_token, float* out_logprob) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // a thread's share is a run of neighbours, so the lists are in index order
+    const int chunk = (n + SMPC_THREADS - 1) / SMPC_THREADS, c_lo = min(n, (int)threadIdx.x * chunk), c_hi = min(n, c_lo + chunk);
+    auto kept = [&](int i) { return order_key(sl[i]) >= cut && !(mp > 0.f && se[i] < mp); };
+    int mine = 0;
+    for (int i = c_lo; i < c_hi; ++i) mine += kept(i);
+    int upto = mine;
+#pragma unroll
+    for (int h = 1; h < 32; h <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, upto, h);
+        if (lane >= h) upto += up;
+    }
+    __syncthreads();
+    if (lane == 31) nl.scan[warp] = upto;
+    __syncthreads();
+    int total = 0, at = upto - mine;
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+        if (q == warp) at += total;
+        total += nl.scan[q];
+    }
+    if (mine && total <= SMPC_NEAR)
+        for (int i = c_lo; i < c_hi; ++i) {
+            if (!kept(i)) continue;
+            const uint32_t to = cluster_map((uint32_t)__cvta_generic_to_shared(&nl.kept[c.rank * SMPC_NEAR + at++]), 0);
+            cluster_store_f32(to, __int_as_float(lo + i));
+            cluster_store_f32(to + 4, sl[i]);
+        }
+    if (threadIdx.x < SMPC_CTAS)
+        cluster_store_f32(cluster_map((uint32_t)__cvta_generic_to_shared(&nl.kept_counts[c.rank]), threadIdx.x), __int_as_float(total));
+    cluster_sync_all();
+    int all = 0, my_off = 0;
+    bool fits = true;
+    const int of = threadIdx.x / SMPC_NEAR;
+#pragma unroll
+    for (int r = 0; r < SMPC_CTAS; ++r) {
+        const int k = nl.kept_counts[r];
+        if (r == of) my_off = all;
+        all += k;
+        fits = fits && k <= SMPC_NEAR;
+    }
+    if (!fits || all == 0) return false;
+    if (c.rank != 0) return true;
+    if (of < SMPC_CTAS && (int)(threadIdx.x % SMPC_NEAR) < nl.kept_counts[of])
+        nl.list[my_off + threadIdx.x % SMPC_NEAR] = nl.kept[threadIdx.x];
+    __syncthreads();
+    const bool in = (int)threadIdx.x < all;
+    const float s = in ? nl.list[threadIdx.x].y : 0.f;
+    float e = in ? expf(s - mx) : 0.f;
+    if (tp > 0.f && tp < 1.f) {
+        if (threadIdx.x < SMPC_CTAS * SMPC_NEAR) nl.got[threadIdx.x] = make_float2(__uint_as_float(order_key(s)), e);
+        const float limit = tp * block_sum(e, table);       // (its barriers also make the list the block's)
+        uint32_t best = 0;
+        for (int q = warp; q < all; q += SMPC_THREADS / 32) {
+            const uint32_t key = __float_as_uint(nl.got[q].x);
+            float sum = 0.f;
+            for (int j = lane; j < all; j += 32) {
+                const float2 o = nl.got[j];
+                sum += __float_as_uint(o.x) >= key ? o.y : 0.f;
+            }
+            if (warp_sum(sum) > limit) best = max(best, key);
+        }
+        __syncthreads();
+        if (lane == 0) nl.best[warp] = best;
+        __syncthreads();
+        best = nl.best[lane];
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, h));
+        if (order_key(s) < best) e = 0.f;
+    }
+    // the draw: running sums in index order
+    const bool live = in && e > 0.f;
+    float run = e;
+#pragma unroll
+    for (int h = 1; h < 32; h <<= 1) {
+        const float up = __shfl_up_sync(0xffffffffu, run, h);
+        if (lane >= h) run += up;
+    }
+    __syncthreads();
+    if (lane == 31) table[warp] = run;
+    __syncthreads();
+    float front = 0.f, whole = 0.f;
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+        if (q == warp) front = whole;
+        whole += table[q];
+    }
+    const float target = philox_uniform(seed, counter) * whole;
+    // the first whose running sum reaches the target; the last that is kept, if rounding leaves the target beyond all
+    const uint32_t reached = __ballot_sync(0xffffffffu, live && front + run >= target), alive = __ballot_sync(0xffffffffu, live);
+    __syncthreads();
+    if (lane == 0) {
+        nl.scan[warp] = reached ? warp * 32 + __ffs(reached) - 1 : 0x7fffffff;
+        nl.best[warp] = alive ? warp * 32 + 31 - __clz(alive) + 1 : 0;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const int first = __reduce_min_sync(0xffffffffu, nl.scan[lane]), last = (int)__reduce_max_sync(0xffffffffu, nl.best[lane]) - 1;
+        const int pick = first != 0x7fffffff ? first : max(last, 0);
+        if (lane == 0) {
+            *out_token = __float_as_int(nl.list[pick].x);
+            if (out_logprob) *out_logprob = (nl.list[pick].y - mx) - logf(whole);
+        }
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(SMPC_THREADS)
 sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice, const float* __restrict__ temperature,
                       const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
@@ -707,21 +826,18 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
     for (int i = threadIdx.x; i < n; i += blockDim.x) se[i] = expf(sl[i] - mx);
     __syncthreads();
     uint32_t cut = 0;  // keys >= cut are kept
-    if (k > 0 && k < V) {   // the largest c with count(key >= c) >= k
-        auto element = [&](int i, uint32_t& key, float& w) { key = order_key(sl[i]); w = 1.f; };
-        if (!cluster_near(cs, bins, near, sl, mx, scale, n, (float)k, false, element, cut))
-            cut = cluster_descend(cs, bins, n, (float)k, false, element);
-    }
     const float mp = min_p[r];
     const bool use_minp = mp > 0.f;
+    if (k > 0 && k < V) {   // the largest c with count(key >= c) >= k
+        auto element = [&](int i, uint32_t& key, float& w) { key = order_key(sl[i]); w = 1.f; };
+        const bool few = cluster_near(cs, bins, near, sl, mx, scale, n, (float)k, 0.f, false, element, cut);
+        if (!few) cut = cluster_descend(cs, bins, n, (float)k, false, element);
+        if (few && k <= SMPC_FEW &&
+            sample_few(cs, near, table, sl, se, mx, lo, n, cut, use_minp ? mp : 0.f, tp, seed[r], counter[r], out_token + r,
+                       out_logprob ? out_logprob + r : nullptr))
+            return;
+    }
     if (tp > 0.f && tp < 1.f) {
-        float z = 0.f;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const float s = sl[i];
-            const float e = se[i];
-            if (order_key(s) >= cut && !(use_minp && e < mp)) z += e;
-        }
-        z = cluster_all_sum(cs, z);
         // the largest t with mass(key > t) > limit, that is with mass(key - 1 >= t) > limit
         const uint32_t kept_from = cut;
         auto element = [&](int i, uint32_t& key, float& w) {
@@ -731,8 +847,16 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
             w = full >= kept_from && full != 0u && !(use_minp && e < mp) ? e : 0.f;
         };
         uint32_t t;
-        if (!cluster_near(cs, bins, near, sl, mx, scale, n, tp * z, true, element, t))
+        if (!cluster_near(cs, bins, near, sl, mx, scale, n, 0.f, tp, true, element, t)) {
+            float z = 0.f;
+            for (int i = threadIdx.x; i < n; i += blockDim.x) {
+                const float s = sl[i];
+                const float e = se[i];
+                if (order_key(s) >= cut && !(use_minp && e < mp)) z += e;
+            }
+            z = cluster_all_sum(cs, z);
             t = cluster_descend(cs, bins, n, tp * z, true, element);
+        }
         cut = t + 1u > cut ? t + 1u : cut;
     }
 

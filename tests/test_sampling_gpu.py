@@ -2,6 +2,8 @@
 
 from __future__ import annotations
 
+import math
+
 import pytest
 import torch
 
@@ -105,6 +107,37 @@ def test_wide_rows_whose_cut_is_searched_near_the_maximum(V, kind):
             u = plain_qwen3.philox_uniform(i, counter)
             before = float(cdf[got[i]] - weight[got[i]] / weight[keep].sum())
             assert before - 1e-4 <= u <= float(cdf[got[i]]) + 1e-4, f"case {i}"
+
+
+@pytest.mark.parametrize("kind", ["spread", "ties", "clumped", "below"])
+@pytest.mark.parametrize("V", [16384, 50001])
+def test_wide_rows_of_which_a_top_k_leaves_few(V, kind):
+    """The cut and the draw on the entries that a small top-k leaves: one, a list's share and one more, the most and one more;
+    many of one value; all in one part of the row; a probability floor that leaves the maximum alone.  The draw is the kept
+    mass's at the seed's point (a float sum of at most V weights is good to 1e-4 of it), and its log-probability is the share's."""
+    g = torch.Generator().manual_seed(V + 2)
+    x = torch.randn(V, generator=g)
+    row = {"spread": lambda: x * 2, "ties": lambda: (x * 4).round() / 2, "clumped": lambda: torch.where(torch.arange(V) < 500, x + 6.0, x),
+           "below": lambda: torch.where(torch.arange(V) == V - 1, 30.0, x)}[kind]()
+    cases = [(k, p, mp) for k in (1, 2, 63, 64, 65, 256, 257) for p, mp in ((1.0, 0.0), (0.9, 0.0), (0.3, 0.05))]
+    for counter in range(3):
+        got, logprob = run_sample(row.repeat(len(cases), 1).cuda(), [1.0] * len(cases), *[[c[j] for c in cases] for j in (0, 1, 2)],
+                                  list(range(len(cases))), [counter] * len(cases), logprobs=True)
+        for i, (k, p, mp) in enumerate(cases):
+            z = row.double()
+            weight = (z - z.max()).exp()
+            keep = (z >= z.topk(k).values[-1]) & (weight >= mp)
+            if p < 1.0:
+                values, at = torch.unique(z[keep], return_inverse=True)
+                mass = torch.zeros(len(values), dtype=torch.float64).index_add_(0, at, weight[keep])
+                above = mass.flip(0).cumsum(0).flip(0) - mass
+                keep &= z >= values[above <= p * mass.sum() * (1 + 1e-6)][0]
+            assert keep[got[i]], f"case {cases[i]}: a dropped token was drawn"
+            share = weight / weight[keep].sum()
+            upto = float(torch.where(keep, share, 0.0).cumsum(0)[got[i]])
+            u = plain_qwen3.philox_uniform(i, counter)
+            assert upto - float(share[got[i]]) - 1e-4 <= u <= upto + 1e-4, f"case {cases[i]}"
+            assert abs(float(logprob[i]) - math.log(float(share[got[i]]))) < 1e-4, f"case {cases[i]}"
 
 
 @pytest.mark.parametrize("at", [(100, 104), (104, 100), (100, 2040), (0, 63)])
