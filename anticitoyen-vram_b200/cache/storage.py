@@ -60,6 +60,7 @@ class CacheStorage:
                 sdtype = getattr(torch, g.need.dtype)
                 self.tensors.append(torch.zeros((g.num_slots, g.max_requests + 1, *g.need.shape), device=self.device,
                                                 dtype=sdtype))
+        self._pages: dict[int, tuple[torch.Tensor, torch.Tensor]] = {}      # cache slot -> its views, once asked for
 
     def bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in (*self.tensors, *self.value_tensors.values()))
@@ -71,6 +72,12 @@ class CacheStorage:
 
     def pages(self, cache_slot: int) -> tuple[torch.Tensor, torch.Tensor]:
         """(keys, values) of a cache slot, ``[num_pages, kv_heads, page_size, head_dim]`` (values: ``value_dim``)."""
+        got = self._pages.get(cache_slot)
+        if got is None:
+            got = self._pages[cache_slot] = self._pages_of(cache_slot)
+        return got
+
+    def _pages_of(self, cache_slot: int) -> tuple[torch.Tensor, torch.Tensor]:
         plan = self.manager.plan
         g, i = plan.group_of_slot[cache_slot], plan.index_in_group[cache_slot]
         if g in self.value_tensors:

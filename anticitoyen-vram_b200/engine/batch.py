@@ -255,13 +255,20 @@ class BatchBuilder:
         if max(kv_lens, default=0) > self.max_positions:
             raise ValueError(f"a request would reach {max(kv_lens)} tokens; the model has {self.max_positions} positions")
 
-        tokens = np.concatenate([np.asarray(e.tokens, dtype=np.int64) for e in entries]) if B else np.zeros(0, np.int64)
+        if T == B:          # one token each: a list without an array for every request
+            tokens = np.asarray([e.tokens[0] for e in entries], dtype=np.int64)
+        else:
+            tokens = np.concatenate([np.asarray(e.tokens, dtype=np.int64) for e in entries])
         if T and (tokens.min() < 0 or tokens.max() >= self.vocab_size):
             raise ValueError(f"token id outside the vocabulary of {self.vocab_size}")
-        cu = np.zeros(B + 1, dtype=np.int32)
-        np.cumsum(q_lens, out=cu[1:])
-        seq_of = np.repeat(np.arange(B, dtype=np.int32), q_lens)
-        positions = np.arange(T, dtype=np.int32) - np.repeat(cu[:-1] - np.asarray(starts, dtype=np.int32), q_lens)
+        if T == B:
+            cu = np.arange(B + 1, dtype=np.int32)
+            seq_of, positions = cu[:B], np.asarray(starts, dtype=np.int32)
+        else:
+            cu = np.zeros(B + 1, dtype=np.int32)
+            np.cumsum(q_lens, out=cu[1:])
+            seq_of = np.repeat(np.arange(B, dtype=np.int32), q_lens)
+            positions = np.arange(T, dtype=np.int32) - np.repeat(cu[:-1] - np.asarray(starts, dtype=np.int32), q_lens)
         rows = []
         for i, e in enumerate(entries):
             for w in e.want:
@@ -289,19 +296,24 @@ class BatchBuilder:
         total = sum(_round4(a.size) for _, a in sections)
         host, dev = self._buffers(max(total, 4))
         hnp = host.numpy()
-        offsets = {}
+        sizes, place = [], {}           # of the buffer's pieces, the sections and what rounds them up; each section's piece
         off = 0
         for name, arr in sections:
-            hnp[off:off + arr.size] = arr
-            offsets[name] = (off, arr.size)
-            off += _round4(arr.size)
-        dev[:total].copy_(host[:total], non_blocking=True)
+            n = arr.size
+            hnp[off:off + n] = arr
+            place[name] = len(sizes)
+            sizes.append(n)
+            if n & 3:
+                sizes.append(4 - (n & 3))
+            off += _round4(n)
+        sent = dev[:total]
+        sent.copy_(host[:total], non_blocking=True)
         self.last_h2d_bytes = total * 4
         self._sent()
+        pieces = sent.split_with_sizes(sizes)
 
         def view(name: str) -> torch.Tensor:
-            o, n = offsets[name]
-            return dev[o:o + n]
+            return pieces[place[name]]
 
         self._apply_updates([(gi, view(f"upd{gi}"), len(upd)) for (gi, _), upd in zip(self._paged, updates)])
         ctx = StepContext(

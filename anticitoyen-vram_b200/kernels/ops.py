@@ -213,8 +213,9 @@ def _cuda_error_text(code: int) -> str:
 
 
 def _stream() -> int:
-    """The current stream's handle, without a stream object around it (a launch asks for it; 0.3 us instead of 2)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    """The current stream's handle, without a stream object around it (a launch asks for it; 0.3 us instead of 2).  The device
+    is asked of the binding itself: whoever has a tensor on a device has initialised it."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _p(t: torch.Tensor | None):
@@ -373,12 +374,14 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
     bfloat16 parts on the tensor cores with a smaller error (csrc/gemm_split_tc.cu)."""
     _need_cuda(a, w, out)
     M, K = a.shape
-    N = w.shape[0]
-    if w.shape[1] != K or out.shape[0] != M or out.shape[1] != N or a.dtype != w.dtype:
+    w_shape, out_shape = w.shape, out.shape
+    a_stride, w_stride, out_stride = a.stride(), w.stride(), out.stride()
+    N = w_shape[0]
+    if w_shape[1] != K or out_shape[0] != M or out_shape[1] != N or a.dtype != w.dtype:
         raise KernelError(f"gemm_simt: shapes {tuple(a.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
-    if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
+    if a_stride[1] != 1 or w_stride[1] != 1 or out_stride[1] != 1:
         raise KernelError("gemm_simt: innermost strides must be 1")
-    _check(library().acv_gemm_simt(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K,
+    _check(library().acv_gemm_simt(a.data_ptr(), a_stride[0], w.data_ptr(), w_stride[0], out.data_ptr(), out_stride[0], M, N, K,
                                    dtype_code(a.dtype), dtype_code(out.dtype), _status_pointer(a), _stream()), "gemm_simt")
     return out
 
@@ -387,8 +390,13 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tens
 _gemm_scratch: dict = {}
 
 
+@functools.lru_cache(maxsize=64)
+def _device_key(device) -> str:
+    return str(device)
+
+
 def _gemm_buffers(device, ws_floats: int, n_counters: int):
-    key = str(device)
+    key = _device_key(device)
     have = _gemm_scratch.get(key)
     if have is None or have[0].numel() < ws_floats or have[1].numel() < n_counters:
         if torch.cuda.is_current_stream_capturing():
@@ -425,7 +433,9 @@ def sm_count(device=None) -> int:
     """Streaming multiprocessors of the device (asked once per device; 148, a B200's, where there is no device)."""
     if not _sm_counts and not torch.cuda.is_available():
         return 148
-    index = torch.cuda.current_device() if device is None or torch.device(device).index is None else torch.device(device).index
+    index = None if device is None else torch.device(device).index
+    if index is None:
+        index = torch.cuda.current_device()
     if index not in _sm_counts:
         _sm_counts[index] = torch.cuda.get_device_properties(index).multi_processor_count
     return _sm_counts[index]
@@ -598,7 +608,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: tuple | N
         raise KernelError("gemm_tc: the paired SwiGLU output needs an even number of weight rows and a bfloat16 output")
     if w.shape[1] != K or out.shape != (M, n_out) or x.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError(f"gemm_tc: shapes {tuple(x.shape)} x {tuple(w.shape)} -> {tuple(out.shape)} do not fit")
-    if plan is None and static_weights and bias is None and unary is None and gate_fn == 0 and _gemm_rows_takes(x, w):
+    if M <= 32 and plan is None and static_weights and bias is None and unary is None and gate_fn == 0 and _gemm_rows_takes(x, w):
         _check(library().acv_gemm_rows(_p(x), x.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K,
                                        1 if out.dtype == torch.float32 else 0, int(swiglu_pairs), 1, sm_count(x.device), _stream()), "gemm_rows")
         return out
@@ -971,29 +981,28 @@ def attention_work(q_lens, kv_lens, cu_q) -> tuple[dict, dict]:
     QUERY_TILE tokens of the requests with more (portions of prompts), late tiles first since they see most keys.
     Returns (int32 arrays that the kernels read on the device, counts and maxima for the launches)."""
     import numpy as np
-    ql = np.asarray(q_lens, dtype=np.int32)
-    dec = np.nonzero(ql == 1)[0].astype(np.int32)
-    tile_seq, tile_q0, tile_keys = [], [], []
-    for i in np.nonzero(ql > 1)[0]:
-        starts_i = np.arange(0, q_lens[i], QUERY_TILE, dtype=np.int32)
-        tile_seq.append(np.full(starts_i.size, i, dtype=np.int32))
-        tile_q0.append(starts_i)
-        tile_keys.append(int(kv_lens[i]) - int(q_lens[i]) + np.minimum(starts_i + QUERY_TILE, int(q_lens[i])))   # keys a tile's last query sees
-    empty = np.zeros(0, np.int32)
-    if tile_seq:
-        # the tiles with most keys first, over all requests: the hardware hands out CTAs in this order, and the kernel
-        # that gives a CTA two tiles pairs the list's front with its back
-        order = np.argsort(-np.concatenate(tile_keys), kind="stable")
-        tile_seq, tile_q0 = [np.concatenate(tile_seq)[order]], [np.concatenate(tile_q0)[order]]
+    q_lens, kv_lens = [int(q) for q in q_lens], [int(k) for k in kv_lens]
+    dec = np.asarray([i for i, q in enumerate(q_lens) if q == 1], dtype=np.int32)
+    seq, q0, keys = [], [], []          # of every tile: its request, its first query, the keys its last query sees
+    for i, q in enumerate(q_lens):
+        if q > 1:
+            before = kv_lens[i] - q
+            seq += [i] * -(-q // QUERY_TILE)
+            q0 += range(0, q, QUERY_TILE)
+            keys += range(before + QUERY_TILE, before + q, QUERY_TILE)
+            keys.append(before + q)
+    # the tiles with most keys first, over all requests: the hardware hands out CTAs in this order, and the kernel
+    # that gives a CTA two tiles pairs the list's front with its back
+    order = sorted(range(len(keys)), key=keys.__getitem__, reverse=True)        # (stable: equal ones keep their order)
     arrays = {"dec_tokens": np.asarray(cu_q, dtype=np.int32)[:-1][dec], "dec_seqs": dec,
-              "tile_seq": np.concatenate(tile_seq) if tile_seq else empty,
-              "tile_q0": np.concatenate(tile_q0) if tile_q0 else empty}
-    values = {"n_dec": int(dec.size), "n_tiles": int(sum(t.size for t in tile_seq)),
+              "tile_seq": np.asarray([seq[t] for t in order], dtype=np.int32),
+              "tile_q0": np.asarray([q0[t] for t in order], dtype=np.int32)}
+    values = {"n_dec": len(dec), "n_tiles": len(order),
               "max_dec_kv": max((k for k, q in zip(kv_lens, q_lens) if q == 1), default=0),
               "max_tile_kv": max((k for k, q in zip(kv_lens, q_lens) if q > 1), default=0)}
-    if tile_keys:           # key tiles of all tiles, of the longest and of the shortest
-        blocks = -(-np.concatenate(tile_keys) // QUERY_TILE)
-        values["tile_blocks"] = (int(blocks.sum()), int(blocks.max()), int(blocks.min()))
+    if order:               # key tiles of all tiles, of the longest and of the shortest
+        blocks = [-(-k // QUERY_TILE) for k in keys]
+        values["tile_blocks"] = (sum(blocks), max(blocks), min(blocks))
     return arrays, values
 
 
@@ -1053,10 +1062,13 @@ def attention_work_decode(padded: int, max_kv: int) -> tuple[dict, dict]:
 
 
 def _tile_parts(work: dict, num_heads: int, num_kv_heads: int, window: int, keep_first: int, chunk: int, device) -> tuple:
-    if "tile_blocks" not in work:
+    blocks = work.get("tile_blocks")
+    if blocks is None:
         return 1, 0
-    seen = min((n for n in (window + keep_first if window > 0 else 0, chunk) if n > 0), default=0)
-    return attention_tc_parts(work["n_tiles"], work["tile_blocks"], num_heads, num_kv_heads, -(-seen // QUERY_TILE) + 1 if seen else 0,
+    seen = window + keep_first if window > 0 else chunk
+    if window > 0 and chunk > 0:
+        seen = min(seen, chunk)
+    return attention_tc_parts(work["n_tiles"], blocks, num_heads, num_kv_heads, -(-seen // QUERY_TILE) + 1 if seen > 0 else 0,
                               sm_count(device))
 
 

@@ -109,7 +109,7 @@ class SwiGLU(FeedForward):
                 ops.glu(gu, out, ops.ACTIVATIONS["silu"], 0.0, 0.0)
 
     def forward(self, h, ctx):
-        act = torch.empty((h.shape[0], self.intermediate_size), device=h.device, dtype=h.dtype)
+        act = h.new_empty((h.shape[0], self.intermediate_size))
         self.inner(h, ctx, act)
         return self.down(act)
 

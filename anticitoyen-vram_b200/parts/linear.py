@@ -60,7 +60,7 @@ class Linear:
         output: in the tensor-core product's epilogue where that product runs, by a kernel of its own otherwise."""
         w = self.weight
         out_dtype = out_dtype or x.dtype
-        out = torch.empty((x.shape[0], self.out_features), device=x.device, dtype=out_dtype)
+        out = x.new_empty((x.shape[0], self.out_features), dtype=out_dtype)      # (0.5 us under torch.empty with a device)
         if x.shape[0] == 0:
             return out
         if x.dtype == torch.float32:

@@ -339,7 +339,7 @@ class Attention(Mixer):
         rotary = self.position.rotary_table()
         if rotary is not None and self.qkv.bias is None and ops.gemm_tc_qkv_takes(h, self.qkv.weight, D, rotary, kp):
             # a few tokens: norm, rotation and append ride on the projection's kernel as its tile leaves
-            qkv = torch.empty((h.shape[0], self.qkv.out_features), device=h.device, dtype=h.dtype)
+            qkv = h.new_empty((h.shape[0], self.qkv.out_features))
             ops.gemm_tc_qkv(h, self.qkv.weight, qkv, NH, NKV, D, self.q_norm, self.k_norm, eps, rotary, ctx.positions,
                             ctx.seq_of_token, table, kp, vp, static_weights=True, table_rows=rows)
         elif rotary is not None:
@@ -358,7 +358,7 @@ class Attention(Mixer):
             if kp is not None:
                 ops.qk_norm_rope_append(qkv, NH, NKV, D, None, None, 0.0, None, ctx.positions, ctx.seq_of_token,
                                         table, kp, vp, table_rows=rows)
-        out = torch.empty((qkv.shape[0], self.q_size), device=h.device, dtype=h.dtype)
+        out = h.new_empty((qkv.shape[0], self.q_size))
         ops.attention(qkv, out, cache.k_pages, cache.v_pages, ctx, table, NH, NKV, D, self.scale, self.window,
                       work=ctx.work[self.metadata_key], **({"keep_first": self.keep_first} if self.keep_first else {}))
         return self.o(out)

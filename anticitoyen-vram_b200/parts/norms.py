@@ -53,7 +53,7 @@ class RMSNorm(Norm):
         is rounded once.  ``delta_scale``: x += delta_scale * delta (float32 stream only)."""
         n = rows.shape[0] if rows is not None else x.shape[0]
         out_dtype = out_dtype or (delta.dtype if delta is not None else x.dtype)
-        out = torch.empty((n, x.shape[1]), device=x.device, dtype=out_dtype)
+        out = x.new_empty((n, x.shape[1]), dtype=out_dtype)
         if self.groups > 1 or delta_scale != 1.0 or (x.dtype == torch.float32 and delta is not None and delta.dtype != out_dtype):
             if x.dtype != torch.float32:
                 raise ValueError("a grouped norm or a factor on the residual wants a float32 residual stream (ModelPlan.residual_dtype)")
@@ -97,5 +97,5 @@ class LayerNorm(Norm):
             raise ValueError("the layer norm is built for a float32 residual stream (ModelPlan.residual_dtype)")
         n = rows.shape[0] if rows is not None else x.shape[0]
         out_dtype = out_dtype or (delta.dtype if delta is not None else x.dtype)
-        out = torch.empty((n, x.shape[1]), device=x.device, dtype=out_dtype)
+        out = x.new_empty((n, x.shape[1]), dtype=out_dtype)
         return ops.add_layernorm(x, delta, self.weight, self.bias, self.eps, out, rows, delta_scale)

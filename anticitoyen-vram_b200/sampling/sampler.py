@@ -34,6 +34,7 @@ class Sampler:
         self._hosts: list[torch.Tensor | None] = [None, None]
         self._events: list = [None, None]
         self._devs: list[torch.Tensor | None] = [None, None]
+        self._views: list[tuple | None] = [None, None]
         self._turn = 0
 
     def _stage(self, ints: int) -> tuple[torch.Tensor, torch.Tensor]:
@@ -45,6 +46,7 @@ class Sampler:
             cap = max(1024, 1 << (ints - 1).bit_length())
             self._hosts[i] = torch.empty(cap, dtype=torch.int32, pin_memory=self.device.type == "cuda")
             self._devs[i] = torch.empty(cap, dtype=torch.int32, device=self.device)
+            self._views[i] = None
         return self._hosts[i], self._devs[i]
 
     def _send(self, host: torch.Tensor, dev: torch.Tensor, ints: int) -> None:
@@ -53,6 +55,16 @@ class Sampler:
             if self._events[self._turn] is None:
                 self._events[self._turn] = torch.cuda.Event()
             self._events[self._turn].record()
+
+    def _row_views(self, dev: torch.Tensor, R: int, R4: int) -> tuple[torch.Tensor, ...]:
+        """The rows' parameters in the staging buffer of this turn; the views of the last number of rows are kept."""
+        kept = self._views[self._turn]
+        if kept is None or kept[0] != R:
+            f = dev[:6 * R4].view(torch.float32)
+            d64 = dev[8 * R4:12 * R4].view(torch.int64)
+            kept = self._views[self._turn] = (R, (*(f[j * R4:j * R4 + R] for j in range(6)), dev[6 * R4:6 * R4 + R],
+                                                  d64[:R], d64[R4:R4 + R]))
+        return kept[1]
 
     def __call__(self, logits: torch.Tensor, params: Sequence[SamplingParams], histories: Sequence[Sequence[int]],
                  seeds: Sequence[int], counters: Sequence[int], want_logprobs: bool = False):
@@ -79,26 +91,28 @@ class Sampler:
         host, dev = self._stage(ints)
         h = host.numpy()
         hf = h.view(np.float32)
-        for j, name in enumerate(("temperature", "top_p", "min_p", "repetition_penalty", "presence_penalty",
-                                  "frequency_penalty")):
-            hf[j * R4:j * R4 + R] = [getattr(p, name) for p in params]
+        hf[:R] = [p.temperature for p in params]
+        hf[R4:R4 + R] = [p.top_p for p in params]
+        hf[2 * R4:2 * R4 + R] = [p.min_p for p in params]
         h[o_k:o_k + R] = [p.top_k for p in params]
         h64 = h[o_seed:o_seed + 4 * R4].view(np.int64)
         h64[:R] = [s & 0x7FFFFFFFFFFFFFFF for s in seeds]
         h64[R4:R4 + R] = list(counters)
         if n_pen:
+            hf[3 * R4:3 * R4 + R] = [p.repetition_penalty for p in params]
+            hf[4 * R4:4 * R4 + R] = [p.presence_penalty for p in params]
+            hf[5 * R4:5 * R4 + R] = [p.frequency_penalty for p in params]
             P4 = _round4(n_pen)
             h[o_pen:o_pen + n_pen] = rows
             h[o_pen + P4:o_pen + P4 + n_pen] = toks
             h[o_pen + 2 * P4:o_pen + 2 * P4 + n_pen] = counts
         self._send(host, dev, ints)
-        f = lambda j: dev[j * R4:j * R4 + R].view(torch.float32)
-        d64 = dev[o_seed:o_seed + 4 * R4].view(torch.int64)
+        temperature, top_p, min_p, repetition, presence, frequency, top_k, seed, counter = self._row_views(dev, R, R4)
         if n_pen:
             P4 = _round4(n_pen)
             logits = logits.clone()
             ops.apply_penalties(logits, dev[o_pen:o_pen + n_pen], dev[o_pen + P4:o_pen + P4 + n_pen],
-                                dev[o_pen + 2 * P4:o_pen + 2 * P4 + n_pen], f(3), f(4), f(5))
+                                dev[o_pen + 2 * P4:o_pen + 2 * P4 + n_pen], repetition, presence, frequency)
         logprobs = torch.empty(R, device=self.device, dtype=torch.float32) if want_logprobs else None
-        ops.sample(logits, f(0), dev[o_k:o_k + R], f(1), f(2), d64[:R], d64[R4:R4 + R], tokens, logprobs)
+        ops.sample(logits, temperature, top_k, top_p, min_p, seed, counter, tokens, logprobs)
         return tokens, logprobs

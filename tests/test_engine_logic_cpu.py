@@ -355,3 +355,22 @@ def test_the_exponentials_polynomial_is_as_exact_as_the_unit_beside_it():
     exact = 2.0 ** f.astype(np.float64)
     assert (np.abs(q - exact) / exact).max() < 1.3e-7
     assert q[200000] == 1.0 and f[200000] == 0.0
+
+
+@pytest.mark.parametrize("q_lens,held", [([1], [700]), ([1, 1, 1], [0, 5, 127]), ([128, 1, 129, 2], [0, 40, 255, 126]), ([300, 300, 3], [0, 0, 600]), ([], [])])
+def test_attention_work_lists(q_lens, held):
+    """The requests of one token, the others' tiles with most keys first (equal ones in the batch's order), and the counts."""
+    import numpy as np
+    from acvram_b200.kernels.ops import QUERY_TILE, attention_work
+    kv_lens, cu = [h + q for h, q in zip(held, q_lens)], np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    tiles = [(i, a, held[i] + min(a + QUERY_TILE, q)) for i, q in enumerate(q_lens) if q > 1 for a in range(0, q, QUERY_TILE)]
+    tiles.sort(key=lambda t: -t[2])
+    blocks = [-(-t[2] // QUERY_TILE) for t in tiles]
+    dec = [i for i, q in enumerate(q_lens) if q == 1]
+    arrays, values = attention_work(q_lens, kv_lens, cu)
+    assert all(a.dtype == np.int32 for a in arrays.values())
+    assert {k: a.tolist() for k, a in arrays.items()} == {"dec_tokens": [int(cu[i]) for i in dec], "dec_seqs": dec,
+                                                          "tile_seq": [t[0] for t in tiles], "tile_q0": [t[1] for t in tiles]}
+    assert values == {"n_dec": len(dec), "n_tiles": len(tiles), "max_dec_kv": max((kv_lens[i] for i in dec), default=0),
+                      "max_tile_kv": max((k for k, q in zip(kv_lens, q_lens) if q > 1), default=0),
+                      **({"tile_blocks": (sum(blocks), max(blocks), min(blocks))} if tiles else {})}
