@@ -14,7 +14,8 @@
 // or 8) each take a whole subtree.
 //
 // What bounds it: for many rows the FFMA pipes (of 73 TFLOP/s; three different registers to an instruction leave 60), for few
-// rows the weights' stream.  Measured, microseconds before (tiles of 64 x 64, scalar reads, no split of K) and now: 696 rows
+// rows the weights' stream.  Measured when it made the sums of every K, microseconds before (tiles of 64 x 64, scalar reads, no
+// split of K) and after (gemm_split_tc.cu has what these sizes take there): 696 rows
 // 4096 x 1024 240 -> 209, 1024 x 2048 174 -> 100, 1024 x 3072 258 -> 143, 2048 rows 4096 x 4096 -> 1750 (39 TFLOP/s); 3 rows
 // 4096 x 1024 71 -> 6.5, 1024 x 3072 211 -> 7.7, 151936 x 1024 713 -> 114 (5460 GB/s of weights).  Both
 // operands lie in shared memory as they lie in global memory (K innermost, rows padded to
