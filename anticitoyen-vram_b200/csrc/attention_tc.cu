@@ -582,10 +582,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
 }
 
+// Dynamic shared memory: two heads' Q, K and V in two stages, what aligning takes, the barriers.  CTAs that share keys hold all of
+// tensor memory while they wait for one another, so none of them may wait for columns behind a CTA that waits in turn: they take
+// shared memory enough that no second such CTA fits beside one (heads of 64 would leave half of an SM's 228 KB, of which a CTA's
+// first KB is the system's).
+template <int D, bool SHARED>
+constexpr int attn_tc_smem() {
+    constexpr int needs = 6 * (D / 64) * AT_ATOM + 1024 + 256, alone = 192 * 1024;
+    return SHARED && needs < alone ? alone : needs;
+}
+
 template <int D, bool SHARED>
 static int launch_attn_tc_as(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcParams& p,
                           int n_tiles, cudaStream_t stream) {
-    constexpr int SMEM = 2 * (D / 64) * AT_ATOM /*Q of two heads*/ + 4 * (D / 64) * AT_ATOM /*K,V x2*/ + 1024 + 256;
+    constexpr int SMEM = attn_tc_smem<D, SHARED>();
+    static_assert(!SHARED || 2 * (SMEM + 1024) > 228 * 1024, "one CTA that shares keys to an SM");
     static AcvSmemConfig smem_config;          // per kernel instance and device
     if (int rc = acv_ensure_smem(smem_config, attn_tc_kernel<D, SHARED>, SMEM)) return rc;
     acv_launch_cluster(PDL_MISC, dim3(p.parts, 1, 1), attn_tc_kernel<D, SHARED>, dim3((unsigned)(n_tiles * p.NKV * p.pairs * p.parts)),
@@ -596,6 +607,12 @@ static int launch_attn_tc_as(const CUtensorMap& mq, const CUtensorMap& mk, const
 template <int D>
 static int launch_attn_tc(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcParams& p, int n_tiles, cudaStream_t stream) {
     return p.parts > 1 ? launch_attn_tc_as<D, true>(mq, mk, mv, p, n_tiles, stream) : launch_attn_tc_as<D, false>(mq, mk, mv, p, n_tiles, stream);
+}
+
+// Dynamic shared memory of a CTA for heads of D (64 or 128) whose tile's keys `parts` CTAs share.
+ACV_API int acv_attention_tc_shared_bytes(int D, int parts) {
+    if (D == 64) return parts > 1 ? attn_tc_smem<64, true>() : attn_tc_smem<64, false>();
+    return parts > 1 ? attn_tc_smem<128, true>() : attn_tc_smem<128, false>();
 }
 
 // q: the step's stacked projection [T, q_width] (queries are its first NH*D columns, row stride q_stride);

@@ -374,3 +374,12 @@ def test_attention_work_lists(q_lens, held):
     assert values == {"n_dec": len(dec), "n_tiles": len(tiles), "max_dec_kv": max((kv_lens[i] for i in dec), default=0),
                       "max_tile_kv": max((k for k, q in zip(kv_lens, q_lens) if q > 1), default=0),
                       **({"tile_blocks": (sum(blocks), max(blocks), min(blocks))} if tiles else {})}
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_blocks_that_share_keys_have_an_sm_each(head_dim):
+    """Blocks of a cluster that waits for all of its blocks while each holds all of an SM's tensor memory: two of them on one SM
+    could wait for each other's columns without an end.  Their shared memory alone (228 KB an SM, 1 KB of it to each block's
+    system) keeps them apart, whatever registers the compiler gives them."""
+    from acvram_b200.kernels import ops
+    assert 2 * (ops.library().acv_attention_tc_shared_bytes(head_dim, 2) + 1024) > 228 * 1024
