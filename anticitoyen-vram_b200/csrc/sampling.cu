@@ -775,6 +775,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
     __shared__ float bestv[2 * SMPC_CTAS];
     __shared__ int owner_s;
     __shared__ float before_s, target_s;
+    cluster_arrive();           // (waited for before the first word to a peer)
     ClusterSum cs;
     cs.parts = parts; cs.warps = warps; cs.table = table; cs.turn = 0; cs.rank = cluster_ctarank();
     const int r = blockIdx.x / SMPC_CTAS;
@@ -789,6 +790,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, int slice
         sl[i] = v;
         mx = fmaxf(mx, v);
     }
+    cluster_wait();             // every CTA of the row has started
     const int k = top_k[r];
     const float tp = top_p[r];
     float scale = 0.f;                      // (either meeting's barriers also make the slice visible to the CTA's threads)

@@ -383,3 +383,35 @@ def test_blocks_that_share_keys_have_an_sm_each(head_dim):
     system) keeps them apart, whatever registers the compiler gives them."""
     from acvram_b200.kernels import ops
     assert 2 * (ops.library().acv_attention_tc_shared_bytes(head_dim, 2) + 1024) > 228 * 1024
+
+
+def _device_functions(path):
+    """(name, is it a kernel, body) of the functions of a CUDA source, which begin and end at a line's start."""
+    import re
+    with open(path) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    for head, body in re.findall(r"^((?:template|__global__|__device__|static __device__)[^;{]*?)\{\n(.*?)^\}", text, re.M | re.S):
+        name = re.search(r"(\w+)\s*\(", re.sub(r"__launch_bounds__\([^)]*\)", "", head))
+        if name:            # (not a struct)
+            yield name.group(1), "__global__" in head, body
+
+
+@pytest.mark.parametrize("source", ["sampling.cu", "gemm_rows.cu", "gemm_split_tc.cu", "gemm_simt.cu", "attention_tc.cu", "attention_decode.cu",
+                                    "attention_generic.cu", "gemm_tc.cu"])
+def test_kernels_know_that_their_cluster_has_started_before_they_touch_a_peer(source):
+    """A block's shared memory may be touched by a peer only once the block is known to run: in each kernel a wait of the
+    cluster's barrier stands before the first peer address, also where a function that it calls makes that address."""
+    import os
+    import re
+    import acvram_b200.kernels.build as kbuild
+    functions = list(_device_functions(os.path.join(kbuild.CSRC, source)))
+    touches, kernels = {"cluster_map"}, 0
+    for _ in functions:         # (functions that touch a peer before they have waited for the cluster themselves)
+        for name, kernel, body in functions:
+            peer = re.search(r"\b(" + "|".join(touches) + r")\s*\(", body)
+            waited = re.search(r"\bcluster_(wait|sync_all)\s*\(", body)
+            if peer and not (waited and waited.start() < peer.start()):
+                assert not kernel, f"{source}: {name} touches a peer through {peer.group(1)} before it has waited for its cluster"
+                touches.add(name)
+            kernels += bool(kernel and peer)
+    assert kernels
