@@ -60,11 +60,10 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
         if constexpr (PIECES) {
             const int bytes = left >= 4 ? 16 : left > 0 ? left * 4 : 0;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(bytes ? src : W), "r"(bytes) : "memory");
-        } else {
-            float v[4];
+        } else {            // (rows without 16-byte pieces: float by float)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = i < left ? __ldg(src + i) : 0.f;
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+            for (int i = 0; i < 4; ++i)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * i), "l"(i < left ? src + i : W), "r"(i < left ? 4 : 0) : "memory");
         }
     };
     auto ask = [&]() {

@@ -45,15 +45,16 @@ struct GfTile {
     static_assert(SMEM + 1024 <= 228 * 1024, "a CTA fits an SM's shared memory");
 };
 
-// eight consecutive floats of a row
+// eight consecutive floats of a row (by plain loads: the rows may be the kernel's in front, which runs while this one begins, and the
+// read-only path is not ordered behind the wait for it)
 template <bool PIECES>
 __device__ __forceinline__ void gf_load8(const float* from, float (&x)[8]) {
     if constexpr (PIECES) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(from)), b = __ldg(reinterpret_cast<const float4*>(from) + 1);
+        const float4 a = reinterpret_cast<const float4*>(from)[0], b = reinterpret_cast<const float4*>(from)[1];
         x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
     } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = __ldg(from + i);
+        for (int i = 0; i < 8; ++i) x[i] = from[i];
     }
 }
 
@@ -179,7 +180,7 @@ gemm_split_tc_kernel(const GfArgs p, int parts, int per) {
             for (int j = 0; j < 8; ++j)
 #pragma unroll
                 for (int i = 0; i < ROUNDS; ++i) {
-                    const float v = k + j < k_end && mine(i) ? __ldg(row_of(i) + k + j) : 0.f;
+                    const float v = k + j < k_end && mine(i) ? row_of(i)[k + j] : 0.f;
 #pragma unroll
                     for (int q = 0; q < 8; ++q) x[i][q] = q == j ? v : x[i][q];
                 }

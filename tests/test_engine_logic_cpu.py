@@ -415,3 +415,18 @@ def test_kernels_know_that_their_cluster_has_started_before_they_touch_a_peer(so
                 touches.add(name)
             kernels += bool(kernel and peer)
     assert kernels
+
+
+def test_read_only_loads_are_of_what_no_kernel_in_front_writes():
+    """Kernels begin while the one in front still runs, and ``__ldg`` is for what stays as it is for a kernel's whole life: norm
+    weights and biases, never a row of activations."""
+    import os
+    import re
+    import acvram_b200.kernels.build as kbuild
+    constants = ("w + i0 + c", "w + half + i0 + c", "reinterpret_cast<const float4*>(p.bias + col0")
+    for path in kbuild.sources() + kbuild._headers():
+        with open(path) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        assert "ld.global.nc" not in text, path
+        for found in re.finditer(r"__ldg\(", text):
+            assert text[found.end():].startswith(constants), f"{os.path.basename(path)}: {text[found.start():found.end() + 40]!r}"
