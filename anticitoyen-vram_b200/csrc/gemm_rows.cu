@@ -300,7 +300,12 @@ ACV_API int acv_gemm_rows_qkv(const void* x, int ldx, const void* w, int ldw, vo
                               int NH, int NKV, int D, const float* q_w, const float* k_w, float eps, const float* cos_sin, int table_rows,
                               const int* positions, const int* seq_of_token, const int* block_table, int bt_stride, const int* bt_rows,
                               void* k_pages, void* v_pages, int page_size, int num_pages, cudaStream_t stream) {
-    if (M <= 0 || N <= 0) return 0;
+    // (what acv_gemm_tc_qkv refuses, whose calls of few tokens come here: an empty product is none of it)
+    if ((D != 64 && D != 128) || NH <= 0 || NKV <= 0 || N != (NH + 2 * NKV) * D || !k_pages || !v_pages || !positions || !seq_of_token ||
+        !block_table || page_size <= 0 || ((uintptr_t)k_pages & 15) || ((uintptr_t)v_pages & 15) || (cos_sin && ((uintptr_t)cos_sin & 15)))
+        return ACV_ERR_SIZE;
+    if (M <= 0) return 0;
+    if (((uintptr_t)out & 15) || (ldo & 7)) return ACV_ERR_SIZE;
     RowsParams p = {};
     p.x = (const bf16*)x; p.w = (const bf16*)w; p.out = out;
     p.ldx = ldx; p.ldw = ldw; p.ldo = ldo; p.M = M; p.N = N; p.K = K; p.early_w = flags & 1;
@@ -308,7 +313,7 @@ ACV_API int acv_gemm_rows_qkv(const void* x, int ldx, const void* w, int ldw, vo
     p.positions = positions; p.seq_of_token = seq_of_token; p.block_table = block_table; p.bt_stride = bt_stride; p.bt_rows = bt_rows;
     p.k_pages = (bf16*)k_pages; p.v_pages = (bf16*)v_pages; p.page_size = page_size; p.num_pages = num_pages;
     if (const int e = rw_checks(p)) return e;
-    if (M > 16 || (D != 64 && D != 128) || N != (NH + 2 * NKV) * D || page_size <= 0) return ACV_ERR_SIZE;
+    if (M > 16) return ACV_ERR_SIZE;
     if (M > 8) return rw_launch<4, 2, 3, true>(p, sms, stream);
     // more heads than come at once with an SM to a block: a shallow ring, two blocks to an SM
     if (N / D > (D == 128 ? 33 : 74) * sms / 148) return rw_launch<4, 1, 2, true>(p, sms, stream);

@@ -430,3 +430,25 @@ def test_read_only_loads_are_of_what_no_kernel_in_front_writes():
         assert "ld.global.nc" not in text, path
         for found in re.finditer(r"__ldg\(", text):
             assert text[found.end():].startswith(constants), f"{os.path.basename(path)}: {text[found.start():found.end() + 40]!r}"
+
+
+@pytest.mark.parametrize("wrong", ["positions", "seq_of_token", "block_table", "k_pages", "v_pages", "k_pages + 8", "v_pages + 4", "cos_sin + 4", "out + 2",
+                                   "ldo", "page_size", "N", "D", "NKV"])
+def test_the_projection_of_few_tokens_refuses_what_the_others_refuse(wrong):
+    """A missing array, pages, angles or a result off their 16 bytes, sizes that do not fit: refused on the host by both entry points of
+    the projection with its norm, rotation and append, so that a call does not depend on its number of tokens."""
+    import ctypes
+    from acvram_b200.kernels import ops
+    lib = ops.library()
+    at = 1 << 20            # (an address that nobody reads: the call ends at its checks)
+    a = dict(x=at, ldx=1024, w=at, ldw=1024, out=at, ldo=4096, M=8, N=4096, K=1024, NH=16, NKV=8, D=128, q_w=None, k_w=None, eps=1e-6, cos_sin=at,
+             table_rows=100, positions=at, seq_of_token=at, block_table=at, bt_stride=16, bt_rows=None, k_pages=at, v_pages=at, page_size=16, num_pages=8)
+    name, _, add = wrong.partition(" + ")
+    a[name] = a[name] + int(add) if add else {"ldo": 4100, "page_size": 0, "N": 4224, "D": 96, "NKV": 0}.get(name)
+    tail = [a[k] for k in ("NH", "NKV", "D", "q_w", "k_w")] + [ctypes.c_float(a["eps"])] + [
+        a[k] for k in ("cos_sin", "table_rows", "positions", "seq_of_token", "block_table", "bt_stride", "bt_rows", "k_pages", "v_pages", "page_size", "num_pages")] + [None]
+    head = [a[k] for k in ("x", "ldx", "w", "ldw", "out", "ldo", "M", "N", "K")]
+    size = -3
+    assert lib.acv_gemm_rows_qkv(*head, 1, 148, *tail) == size
+    if name not in ("out", "ldo"):          # (those the other finds out behind its tensor maps, which need a device)
+        assert lib.acv_gemm_tc_qkv(*head, 1, 16, 1, None, 0, None, 0, at, 148, 4, 2, *tail) == size
