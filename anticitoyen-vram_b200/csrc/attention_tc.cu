@@ -506,9 +506,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
             for (int q = 0; q < 8; ++q) m = fmaxf(m, mp[q]);
             float l = 0.f;
+            // now the part's weight; below 0: it saw no key.  (A maximum passes over scores that are no numbers, a sum does not: a part
+            // of them alone has the sum NaN, and its O is added with the weight 0 or 1, either of which leaves NaN in the row; an
+            // infinite maximum has the weight 1, not 2^(inf - inf).)
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                mp[q] = mp[q] == -INFINITY ? -1.f : exp2f(mp[q] - m);       // now the part's weight; below 0: it saw no key
+                mp[q] = mp[q] == -INFINITY && lp[q] == 0.f ? -1.f : mp[q] == m ? 1.f : exp2f(mp[q] - m);
                 if (mp[q] >= 0.f) l += lp[q] * mp[q];
             }
             if (p.sinks && m != -INFINITY) l += exp2f(p.sinks[head] * AT_LOG2E - m);

@@ -929,6 +929,41 @@ def test_tensor_core_attention_with_keys_shared_out(ops, parts, NH, NKV, D, wind
     assert ops.gemm_status() == 0
 
 
+@pytest.mark.parametrize("parts", [(2, 0), (3, 0), (8, 0), (1, 3)])
+@pytest.mark.parametrize("NH,NKV,D", [(6, 2, 128), (5, 1, 64)])
+@pytest.mark.parametrize("what", ["query", "first keys", "last keys", "all keys", "one key", "infinite query", "infinite key", "value"])
+def test_shared_out_keys_keep_what_is_no_number(ops, parts, NH, NKV, D, what):
+    """A query, keys or a value that are NaN or infinite leave the same entries of the result without a number whether one block
+    sees all keys or a cluster shares them (a part whose scores are all NaN has no maximum, but it has a sum); the others are the
+    plain softmax's."""
+    if parts[1] and (NH // NKV % 2 == 0 or NH // NKV < 3):
+        pytest.skip("no odd heads beside pairs")
+    import numpy as np
+    q_len, length, page = 140, 1100, 16
+    arrays, values = ops.attention_work([q_len], [length], [0, q_len])
+    per = length // page + 1
+    d = lambda a: torch.as_tensor(np.asarray(a, dtype=np.int32), device="cuda")
+    q = rnd(q_len, (NH + 2 * NKV) * D, dtype=torch.bfloat16, seed=276)
+    kp, vp = (rnd(per, NKV, page, D, dtype=torch.bfloat16, seed=s) for s in (277, 278))
+    nan, inf = float("nan"), float("inf")
+    at = slice(0, 700 // page) if what == "first keys" else slice(700 // page, per) if what == "last keys" else slice(None)
+    if what in ("query", "infinite query"):
+        q[[0, 77, 139]] = nan if what == "query" else inf
+    elif what in ("first keys", "last keys", "all keys"):
+        kp[at] = nan
+    elif what == "value":
+        vp[3, :, 5] = nan
+    else:
+        kp[30, :, 7, 2] = nan if what == "one key" else inf
+    run = lambda p: ops.attention_tc(q, torch.full((q_len, NH * D), 7.0, device="cuda", dtype=torch.float32), kp, vp, d(arrays["tile_seq"]), d(arrays["tile_q0"]),
+                                     values["n_tiles"], d([0, q_len]), d([length]), d(range(per)).view(1, per), NH, NKV, D, D ** -0.5, 0, parts=p)
+    got, want = run(parts), run((1, 0))
+    assert torch.equal(got.isnan(), want.isnan()) and not want.isinf().any() and not got.isinf().any()
+    assert want.isnan().any()
+    torch.testing.assert_close(got, want, equal_nan=True, **tol(torch.bfloat16))
+    assert ops.gemm_status() == 0
+
+
 def test_attention_tc_parts():
     """One block where the SMs have enough of them, more where they have not, never more than key tiles."""
     from acvram_b200.kernels.ops import attention_tc_parts
