@@ -16,6 +16,7 @@
 
 // two floats into three pairs of bfloat16, each the rounding of what is left
 __device__ __forceinline__ void gr_parts(float a, float b, uint32_t& h1, uint32_t& h2, uint32_t& h3) {
+    gf_scale(a, b);
     h1 = pack_bf16(a, b);
     gf_less(a, b, h1);
     h2 = pack_bf16(a, b);
@@ -182,7 +183,7 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
             for (int j = 1; j < GF_GROUPS; ++j)
                 if (j < groups) x = x + v[j];
             again |= !(fabsf(x) <= 3.402823466e38f);
-            C[(size_t)m * p.ldc + gn] = x;
+            C[(size_t)m * p.ldc + gn] = x * GF_SCALE_BACK;
         }
     }
     cp_async_wait<0>();

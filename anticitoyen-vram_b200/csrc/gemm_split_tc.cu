@@ -61,6 +61,8 @@ __device__ __forceinline__ void gf_load8(const float* from, float (&x)[8]) {
 // the three parts of eight floats into shared memory, `part` bytes apart
 __device__ __forceinline__ void gf_store_parts(uint32_t dst, uint32_t part, float (&x)[8]) {
 #pragma unroll
+    for (int i = 0; i < 4; ++i) gf_scale(x[2 * i], x[2 * i + 1]);
+#pragma unroll
     for (int p = 0; p < 3; ++p) {
         uint32_t h[4];
 #pragma unroll
@@ -151,7 +153,7 @@ gemm_split_tc_kernel(const GfArgs p, int parts, int per) {
     bool again = gate != nullptr;       // this thread's outputs are looked at again: a gate, or one that is no finite number
     auto put = [&](int gm, float x) {
         again |= !(fabsf(x) <= 3.402823466e38f);
-        C[(size_t)gm * p.ldc] = x;
+        C[(size_t)gm * p.ldc] = x * GF_SCALE_BACK;
     };
     auto look_again = [&](int first, int behind, int step) {
 #pragma unroll 1

@@ -10,6 +10,14 @@
 #define GF_GROUPS 8
 #define GF_GROUP 128        // k of a group at least
 
+// Operands are multiplied by 2^24 before they are taken apart and sums by 2^-48 at the end, which changes no bit of either (a
+// result below 2^-126 is rounded, once): a float's lowest bit lies 2^-23 below its first, under the smallest bfloat16 for floats
+// below 2^-110 (relative error of the parts at 1e-34 and 1e-37: 3e-7 and 3e-4); scaled, all parts of all floats are bfloat16
+// values, and normal ones but for those of floats that are subnormal themselves.  What the scale takes out of a float's range,
+// operands from 2^104 and sums from 2^80 on, comes out as no finite number and is made by gf_plain.
+#define GF_SCALE 16777216.f
+#define GF_SCALE_BACK 3.552713678800501e-15f
+
 struct GfArgs {
     const float *A, *W, *gate;
     float* C;
@@ -27,6 +35,11 @@ __host__ __device__ __forceinline__ int gf_group_length(int K) {
 __device__ __forceinline__ void gf_less(float& a, float& b, uint32_t h) {
     asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tsub.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
         : "+f"(a), "+f"(b) : "f"(__uint_as_float(h << 16)), "f"(__uint_as_float(h & 0xffff0000u)));
+}
+
+__device__ __forceinline__ void gf_scale(float& a, float& b) {
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "+f"(a), "+f"(b) : "f"(GF_SCALE));
 }
 
 // an output by itself, in the order of gemm_simt.cu

@@ -408,6 +408,48 @@ def test_gemm_split_one_order_of_sums(ops, M, N, K):
     assert ops.gemm_status() == 0
 
 
+@pytest.mark.parametrize("M", [1, 9, 16, 17, 40, 130])
+@pytest.mark.parametrize("a_size,w_size", [(1e-34, 1.0), (1.0, 1e-36), (1e-38, 1e3), (1e-42, 1.0), (1e-20, 1e-21), (1e-38, 1e30), (1e-44, 1e38), (1e14, 1e13), (1e33, 1e-30), (2e37, 1.0)])
+def test_gemm_split_small_and_large_operands(ops, M, a_size, w_size):
+    """Operands down to the smallest floats keep their 24 bits (their parts are scaled), and those that leave a float's range by
+    the scale or as sums are made by multiply-adds.  The bound of ``test_gemm_split_one_order_of_sums`` (of plain chains of K / 8
+    where those are), and half of the smallest float for a result that is one of the smallest."""
+    K, N = 1030, 140
+    a, w = rnd(M, K, seed=53) * a_size, rnd(N, K, scale=0.05, seed=54) * w_size
+    got = ops.gemm_simt(a, w, torch.full((M, N), float("nan"), device="cuda")).double()
+    size = a.double().abs() @ w.double().abs().T
+    assert ((got - a.double() @ w.double().T).abs() <= (6 + K / 8 + 2 + 8) * 2.0 ** -24 * size + 2.0 ** -150).all()
+    if a_size < 1e13:
+        assert ((got - a.double() @ w.double().T).abs() <= (6 + K / 256 + 2 + 8) * 2.0 ** -24 * size + 2.0 ** -150).all()
+
+
+@pytest.mark.parametrize("M", [16, 33, 64, 129, 700])
+@pytest.mark.parametrize("N,K", [(129, 1029), (1030, 4100)])
+@pytest.mark.parametrize("kind", ["spread", "cancelling", "one sign", "tiny"])
+def test_gemm_split_every_row_by_itself(ops, M, N, K, kind):
+    """Rows among many against the same rows one by one, bit by bit, over both octets of the kernel for few tokens and every part of
+    the tiles of the other, where the units that make the sums could differ: terms of all sizes in one sum, terms that cancel,
+    sums that grow throughout, values at the lower end."""
+    g = torch.Generator(device="cuda").manual_seed(55)
+    a, w = rnd(M, K, seed=56), rnd(N, K, scale=0.05, seed=57)
+    if kind in ("spread", "tiny"):
+        for t in (a, w):
+            t *= 2.0 ** torch.randint(-20, 21, t.shape, device="cuda", generator=g)
+    if kind == "tiny":
+        a *= 2.0 ** -110
+    if kind == "cancelling":            # each term and, somewhere behind it, nearly its opposite
+        a[:, K // 2:2 * (K // 2)] = -a[:, :K // 2].flip(1)
+        w[:, K // 2:2 * (K // 2)] = w[:, :K // 2].flip(1) * (1 + 2.0 ** -12 * rnd(N, K // 2, seed=58))
+    if kind == "one sign":
+        a, w = a.abs(), w.abs()
+    got = ops.gemm_simt(a, w, torch.full((M, N), float("nan"), device="cuda"))
+    for r in sorted({r for r in (0, 3, 7, 8, 11, 15, 16, 31, 32, 63, 64, 95, 96, 127, 128, M - 1) if r < M}):
+        assert torch.equal(ops.gemm_simt(a[r:r + 1], w, torch.empty(1, N, device="cuda"))[0], got[r]), f"row {r}"
+    for n in (2, 8, 9, 16, 17, 40):     # and among other numbers of rows
+        if n < M:
+            assert torch.equal(ops.gemm_simt(a[M - n:], w, torch.empty(n, N, device="cuda")), got[M - n:]), f"{n} rows"
+
+
 @pytest.mark.parametrize("M", [3, 16, 40, 200])
 def test_gemm_split_infinities_and_gate(ops, M):
     """Infinities, NaN and values near the largest have no finite parts: those outputs are what a chain of multiply-adds gives,
