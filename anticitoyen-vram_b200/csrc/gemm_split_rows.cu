@@ -2,13 +2,16 @@
 // mma.sync, whose sums of 16 products are the tcgen05 unit's to the bit (the tests compare the two), so a row's result does not
 // depend on how many rows there are.
 //
-// What bounds it is the weights' stream.  Every lane brings its own operands by 16-byte asynchronous copies into a ring of its
+// What bounds it is the weights' stream.  Every lane brings its own operands by asynchronous copies into a ring of its
 // own (four neighbouring k of a weight row; which k of a step of 16 a lane holds is the same for tokens and weights), so the
 // ring's depth is under way at any time, no registers hold what is on its way and no barrier stands in the loop.  A warp takes
 // one group of K (gf_group_length) for 8 R weight rows, which fill the tensor core's M; the groups of a row meet in shared
 // memory.  A block goes on to its next rows with their first copies already under way.  Microseconds, multiply-adds on the
-// CUDA cores (gemm_simt.cu) and now: 1, 3, 8 and 16 tokens 4096 x 1024 5.6, 6.3, 8.0, 9.8 -> 5.8, 5.9, 6.0, 7.7; 1024 x 3072 6.3,
-// 7.8, 10.3, 12.6 -> 7.0, 7.0, 7.0, 10.9; 151936 x 1024 108, 124, 166, 235 -> 119, 119, 120 (5.2 TB/s of weights), 174.
+// CUDA cores (gemm_simt.cu) and now: 1, 4, 8 and 16 tokens 4096 x 1024 5.6, 6.2, 7.5, 8.9 -> 5.8, 5.7, 6.0, 7.3; 1024 x 3072 6.0,
+// 7.7, 10.1, 12.3 -> 6.3, 6.3, 6.4, 9.4; 12288 x 2048 21.5, 28.6, 36.2, 40.9 -> 19.9, 21.9, 23.4, 31.8; 151936 x 1024 107, 125, 165, 235
+// -> 96 (6.4 TB/s of weights), 98, 104, 152.  One token on few rows is what it makes more slowly: 1024 x 2048 4.6 -> 5.0,
+// 2048 x 2048 5.5 -> 6.0, 4096 x 2048 8.3 -> 8.8, 2048 x 6144 12.1 -> 13.3.  Rows without 16-byte pieces, 50000 x 1026: 127, 128, 317, 317 ->
+// 68, 71, 71, 86.
 #include "mma_tiles.cuh"
 #include "gemm_split_tc.h"
 
@@ -30,30 +33,30 @@ __device__ __forceinline__ void gr_mma(float (&d)[4], const uint32_t (&a)[4], ui
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// R: octets of weight rows of a warp (1 or 2); H: octets of tokens; DEPTH: chunks of 32 k in a warp's ring
-template <int R, int H, int DEPTH, bool PIECES>
-__global__ void __launch_bounds__(GR_WARPS * 32, 2)
-gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
-    constexpr int CHUNK = 2 * (R + H) * 512;        // bytes: two steps' rows, a lane's 16 bytes side by side
+// R: octets of weight rows of a warp (1 or 2); H: octets of tokens; DEPTH: chunks of 32 k in a warp's ring; Q: chunks that are made side
+// by side (a chunk is a chain of twelve products, each behind the one before it).  PARTS: the tokens' parts are made once and stay in
+// shared memory (192 bytes a token and chunk), else the tokens' floats come through the ring and are taken apart for every tile.
+template <int R, int H, int DEPTH, int Q, bool PARTS, bool PIECES>
+__global__ void __launch_bounds__(GR_WARPS * 32, Q > 2 ? 1 : 2)
+gemm_split_rows_kernel(const GfArgs p, int groups) {
+    constexpr int ROWS = R + (PARTS ? 0 : H), CHUNK = 2 * ROWS * 512, COLS = 8 * R;     // CHUNK: two steps' rows, a lane's 16 bytes side by side
     extern __shared__ __align__(16) unsigned char ring[];
-    __shared__ float part[2][GR_WARPS][8 * H][8 * R + 1];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
-    // slots: `groups` rounded up to a power of two; GR_WARPS / slots rows' tiles side by side
-    const int group = warp % slots, set = warp / slots, sets = GR_WARPS / slots, cols = sets * 8 * R, tokens = min(p.M, 8 * H);
+    __shared__ float part[2][GR_WARPS][8 * H][COLS + 1];
+    const int group = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;      // (a warp to a group)
     const float* A = p.A + (size_t)blockIdx.z * p.a_batch;
     const float* W = p.W + (size_t)blockIdx.z * p.w_batch;
     float* C = p.C + (size_t)blockIdx.z * p.c_batch;
     const float* gate = p.gate ? p.gate + (size_t)blockIdx.z * p.g_batch : nullptr;
     bool again = gate != nullptr;
     const int gl = gf_group_length(p.K), k_begin = group * gl, mine = group < groups ? min(gl, p.K - k_begin) : 0;
-    const int chunks = (mine + 31) / 32, tiles = (p.N + cols - 1) / cols;
-    const uint32_t own = smem_u32(ring) + warp * (DEPTH * CHUNK) + lane * 16;
+    const int chunks = (mine + 31) / 32, tiles = (p.N + COLS - 1) / COLS;
+    const uint32_t own = smem_u32(ring) + group * (DEPTH * CHUNK) + lane * 16;
     const float* wr[R];
     const float* ar[H];
     int next_tile = blockIdx.x, next = 0, into = 0;         // the chunk that is asked for next, and its place in the ring
     auto rows = [&]() {         // weight rows that do not exist: the last one that does (their outputs go nowhere); tokens: zeros
 #pragma unroll
-        for (int r = 0; r < R; ++r) wr[r] = W + (size_t)min(next_tile * cols + (set * R + r) * 8 + g, p.N - 1) * p.ldw + k_begin + tq * 4;
+        for (int r = 0; r < R; ++r) wr[r] = W + (size_t)min(next_tile * COLS + r * 8 + g, p.N - 1) * p.ldw + k_begin + tq * 4;
 #pragma unroll
         for (int h = 0; h < H; ++h) ar[h] = A + (size_t)(h * 8 + g) * p.lda + k_begin + tq * 4;
     };
@@ -74,9 +77,11 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
             for (int e = 0; e < 2; ++e) {
                 const int left = mine - next * 32 - e * 16 - tq * 4;
 #pragma unroll
-                for (int r = 0; r < R; ++r) copy(dst + (e * (R + H) + r) * 512, wr[r] + e * 16, left);
+                for (int r = 0; r < R; ++r) copy(dst + (e * ROWS + r) * 512, wr[r] + e * 16, left);
+                if constexpr (!PARTS) {
 #pragma unroll
-                for (int h = 0; h < H; ++h) copy(dst + (e * (R + H) + R + h) * 512, ar[h] + e * 16, h * 8 + g < p.M ? left : 0);
+                    for (int h = 0; h < H; ++h) copy(dst + (e * ROWS + R + h) * 512, ar[h] + e * 16, h * 8 + g < p.M ? left : 0);
+                }
             }
             into = into + 1 == DEPTH ? 0 : into + 1;
             if (++next == chunks) {
@@ -92,11 +97,36 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
         }
         cp_async_commit();
     };
+    // the tokens' parts: of each chunk and token, of each four lanes' k, the parts of the first and of the second step (a lane's 48 bytes)
+    const uint32_t parts_at = smem_u32(ring) + GR_WARPS * DEPTH * CHUNK + group * (gl / 32) * p.M * 192;
     pdl_wait();
     if (chunks) {
         rows();
 #pragma unroll
-        for (int i = 0; i < DEPTH - 1; ++i) ask();
+        for (int i = 0; i < DEPTH - Q; ++i) ask();
+        if constexpr (PARTS) {
+#pragma unroll 4
+            for (int i = lane; i < chunks * p.M * 8; i += 32) {
+                const int q = i & 3, e = i >> 2 & 1, m = (i >> 3) % p.M, c = (i >> 3) / p.M, k = c * 32 + e * 16 + q * 4;
+                const float* src = A + (size_t)m * p.lda + k_begin + k;
+                float4 v;
+                if (PIECES && k + 4 <= mine) {
+                    v = *reinterpret_cast<const float4*>(src);
+                } else {
+                    v.x = k < mine ? src[0] : 0.f;
+                    v.y = k + 1 < mine ? src[1] : 0.f;
+                    v.z = k + 2 < mine ? src[2] : 0.f;
+                    v.w = k + 3 < mine ? src[3] : 0.f;
+                }
+                uint32_t h[3][2];
+                gr_parts(v.x, v.y, h[0][0], h[1][0], h[2][0]);
+                gr_parts(v.z, v.w, h[0][1], h[1][1], h[2][1]);
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(parts_at + ((c * p.M + m) * 4 + q) * 48 + e * 24 + j * 8), "r"(h[j][0]), "r"(h[j][1]) : "memory");
+            }
+            __syncwarp();
+        }
     }
     int from = 0;
     for (int tile = blockIdx.x, turn = 0; tile < tiles; tile += gridDim.x, turn ^= 1) {
@@ -107,44 +137,76 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) sum[h][i] = 0.f;
 #pragma unroll 1
-            for (int n = 0; n < chunks; ++n) {
-                cp_async_wait<DEPTH - 2>();         // (a lane reads what it brought itself)
-                const uint32_t src = own + from * CHUNK;
-                from = from + 1 == DEPTH ? 0 : from + 1;
-                auto read = [&](int at) {
-                    float4 v;
-                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(src + at * 512) : "memory");
-                    return v;
-                };
-                uint32_t w[2][3][4], t[2][3][H][2];             // weights: (g, low k) (g + 8, low) (g, high) (g + 8, high)
+            for (int n = 0; n < chunks; n += Q) {
+                cp_async_wait<DEPTH - 2 * Q>();         // (a lane reads what it brought itself)
+                uint32_t w[Q][2][3][4], t[Q][2][3][H][2];       // weights: (g, low k) (g + 8, low) (g, high) (g + 8, high)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
+                for (int z = 0; z < Q; ++z) {           // (chunks behind the last are made of what there is and not added)
+                    const uint32_t src = own + from * CHUNK;
+                    if (n + z < chunks) from = from + 1 == DEPTH ? 0 : from + 1;
+                    auto read = [&](int at) {
+                        float4 v;
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(src + at * 512) : "memory");
+                        return v;
+                    };
+                    if constexpr (PARTS) {
 #pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const float4 v = read(e * (R + H) + r);
-                        gr_parts(v.x, v.y, w[e][0][r], w[e][1][r], w[e][2][r]);
-                        gr_parts(v.z, v.w, w[e][0][2 + r], w[e][1][2 + r], w[e][2][2 + r]);
+                        for (int h = 0; h < H; ++h) {
+                            uint32_t u[12];
+#pragma unroll
+                            for (int j = 0; j < 12; ++j) u[j] = 0;
+                            if (h * 8 + g < p.M && n + z < chunks) {
+                                const uint32_t at = parts_at + (((n + z) * p.M + h * 8 + g) * 4 + tq) * 48;
+#pragma unroll
+                                for (int j = 0; j < 3; ++j)
+                                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                                                 : "=r"(u[4 * j]), "=r"(u[4 * j + 1]), "=r"(u[4 * j + 2]), "=r"(u[4 * j + 3]) : "r"(at + j * 16));
+                            }
+#pragma unroll
+                            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                                    for (int i = 0; i < 2; ++i) t[z][e][q][h][i] = u[e * 6 + q * 2 + i];
+                        }
                     }
-                    if constexpr (R == 1) {
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) w[e][q][1] = w[e][q][3] = 0;
-                    }
+                    for (int e = 0; e < 2; ++e) {
 #pragma unroll
-                    for (int h = 0; h < H; ++h) {
-                        const float4 v = read(e * (R + H) + R + h);
-                        gr_parts(v.x, v.y, t[e][0][h][0], t[e][1][h][0], t[e][2][h][0]);
-                        gr_parts(v.z, v.w, t[e][0][h][1], t[e][1][h][1], t[e][2][h][1]);
+                        for (int r = 0; r < R; ++r) {
+                            const float4 v = read(e * ROWS + r);
+                            gr_parts(v.x, v.y, w[z][e][0][r], w[z][e][1][r], w[z][e][2][r]);
+                            gr_parts(v.z, v.w, w[z][e][0][2 + r], w[z][e][1][2 + r], w[z][e][2][2 + r]);
+                        }
+                        if constexpr (R == 1) {
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) w[z][e][q][1] = w[z][e][q][3] = 0;
+                        }
+                        if constexpr (!PARTS) {
+#pragma unroll
+                            for (int h = 0; h < H; ++h) {
+                                const float4 v = read(e * ROWS + R + h);
+                                gr_parts(v.x, v.y, t[z][e][0][h][0], t[z][e][1][h][0], t[z][e][2][h][0]);
+                                gr_parts(v.z, v.w, t[z][e][0][h][1], t[z][e][1][h][1], t[z][e][2][h][1]);
+                            }
+                        }
                     }
                 }
-                ask();                              // (into the place that was read in the turn before this one)
-                float c[H][4];
 #pragma unroll
-                for (int h = 0; h < H; ++h)
+                for (int z = 0; z < Q; ++z)
+                    if (n + z < chunks) ask();          // (into the places that were read in the turn before this one)
+                float c[Q][H][4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) c[h][i] = 0.f;
+                for (int z = 0; z < Q; ++z)
+#pragma unroll
+                    for (int h = 0; h < H; ++h)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) c[z][h][i] = 0.f;
                 auto product = [&](int e, int pt, int pw) {
 #pragma unroll
-                    for (int h = 0; h < H; ++h) gr_mma(c[h], w[e][pw], t[e][pt][h][0], t[e][pt][h][1]);
+                    for (int z = 0; z < Q; ++z)
+#pragma unroll
+                        for (int h = 0; h < H; ++h) gr_mma(c[z][h], w[z][e][pw], t[z][e][pt][h][0], t[z][e][pt][h][1]);
                 };
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
@@ -157,9 +219,13 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
                 product(0, 0, 0);
                 product(1, 0, 0);
 #pragma unroll
-                for (int h = 0; h < H; ++h)
+                for (int z = 0; z < Q; ++z)
+                    if (n + z < chunks) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) sum[h][i] += c[h][i];
+                        for (int h = 0; h < H; ++h)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) sum[h][i] += c[z][h][i];
+                    }
             }
             // c: (row g, tokens 2 tq and the next), (row g + 8, the same)
 #pragma unroll
@@ -167,17 +233,17 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) part[turn][warp][h * 8 + 2 * tq + e][r * 8 + g] = sum[h][2 * r + e];
+                    for (int e = 0; e < 2; ++e) part[turn][group][h * 8 + 2 * tq + e][r * 8 + g] = sum[h][2 * r + e];
         }
         __syncthreads();
         if (tile + (int)gridDim.x >= tiles) pdl_launch_dependents();
         // outputs: token by token, weight rows side by side
-        for (int i = threadIdx.x; i < tokens * cols; i += GR_WARPS * 32) {
-            const int m = i / cols, c = i - m * cols, q = c / (8 * R), gn = tile * cols + c;
+        for (int i = threadIdx.x; i < p.M * COLS; i += GR_WARPS * 32) {
+            const int m = i / COLS, c = i - m * COLS, gn = tile * COLS + c;
             if (gn >= p.N) continue;
             float v[GF_GROUPS];
 #pragma unroll
-            for (int j = 0; j < GF_GROUPS; ++j) v[j] = j < groups ? part[turn][q * slots + j][m][c - q * 8 * R] : 0.f;
+            for (int j = 0; j < GF_GROUPS; ++j) v[j] = j < groups ? part[turn][j][m][c] : 0.f;
             float x = v[0];
 #pragma unroll
             for (int j = 1; j < GF_GROUPS; ++j)
@@ -190,8 +256,8 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
     if (!again) return;
     // this thread's outputs once more: a gate, or one that is no finite number
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-        for (int i = threadIdx.x; i < tokens * cols; i += GR_WARPS * 32) {
-            const int m = i / cols, gn = tile * cols + i - m * cols;
+        for (int i = threadIdx.x; i < p.M * COLS; i += GR_WARPS * 32) {
+            const int m = i / COLS, gn = tile * COLS + i - m * COLS;
             if (gn >= p.N) continue;
             float x = C[(size_t)m * p.ldc + gn];
             if (!(fabsf(x) <= 3.402823466e38f)) x = gf_plain(A + (size_t)m * p.lda, W + (size_t)gn * p.ldw, p.K);
@@ -200,36 +266,60 @@ gemm_split_rows_kernel(const GfArgs p, int groups, int slots) {
         }
 }
 
-template <int R, int H, int DEPTH, bool PIECES>
+// Shared memory of a block, and how many blocks of it an SM holds (of 228 KB, 1 KB of it the system's for each block; 200 KB where
+// copies of four bytes go through what is left as its first-level cache).
+template <int R, int H, int DEPTH, bool PARTS>
+static int gr_smem(const GfArgs& p, int groups) {
+    return GR_WARPS * DEPTH * 2 * (R + (PARTS ? 0 : H)) * 512 + (PARTS ? groups * (gf_group_length(p.K) / 32) * p.M * 192 : 0);
+}
+template <int R, int H, int DEPTH, bool PARTS, bool PIECES>
+static int gr_resident(const GfArgs& p, int groups) {
+    return (PIECES ? 228 : 200) * 1024 / (gr_smem<R, H, DEPTH, PARTS>(p, groups) + 2 * GR_WARPS * 8 * H * (8 * R + 1) * 4 + 1024);
+}
+
+template <int R, int H, int DEPTH, int Q, bool PARTS, bool PIECES>
 static int gr_launch(const GfArgs& p, int groups, int batches, int sms, cudaStream_t stream) {
-    constexpr int smem = GR_WARPS * DEPTH * 2 * (R + H) * 512;
+    static_assert(DEPTH >= 2 * Q, "chunks are asked for while as many are made");
+    const int smem = gr_smem<R, H, DEPTH, PARTS>(p, groups), resident = gr_resident<R, H, DEPTH, PARTS, PIECES>(p, groups);
     static AcvSmemConfig cfg;
-    auto kernel = gemm_split_rows_kernel<R, H, DEPTH, PIECES>;
+    auto kernel = gemm_split_rows_kernel<R, H, DEPTH, Q, PARTS, PIECES>;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
-    int slots = 1;
-    while (slots < groups) slots *= 2;
-    const int rows = GR_WARPS / slots * 8 * R;
-    const dim3 grid(min((p.N + rows - 1) / rows, 2 * sms), 1, batches);
     if (batches > 65535) return ACV_ERR_SIZE;
-    acv_launch(PDL_GEMM, kernel, grid, dim3(GR_WARPS * 32), smem, stream, p, groups, slots);
+    const dim3 grid(min((p.N + 8 * R - 1) / (8 * R), max(1, min(resident, Q > 2 ? 1 : 2)) * sms), 1, batches);
+    acv_launch(PDL_GEMM, kernel, grid, dim3(GR_WARPS * 32), smem, stream, p, groups);
     return acv_launch_status();
 }
 
-int gr_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stream) {
+// Eight weight rows to a warp where sixteen would leave half of the SMs without a block, and three chunks side by side there, as a block
+// has its SM to itself and waits for its chains (1 token 1024 x 3072 sixteen rows 7.7, eight 6.7, by threes 6.3; 1024 x 2048 5.7, 4.9,
+// 5.0; 2048 x 2048, 128 blocks of sixteen, 6.0, 7.6, 8.4).
+// The tokens' parts made once pay where a block meets enough tiles with them, the more tokens the more of them, and two blocks still
+// fit an SM (1, 4, 8 tokens, through the ring and made once: 4096 x 1024 5.6, 5.9, 6.0 and 5.7, 6.0, 6.8; 12288 x 2048 22.9, 23.0 and 19.9,
+// 21.7 (8 do not fit); 151936 x 1024 119, 119, 123 and 96, 98, 104; 16 tokens, one block to an SM, 174 and 152, 6144 x 1024 9.7 and 11.4),
+// and wherever they fit for rows that come float by float (4096 x 1025, 1, 4, 8, 16 tokens 12.9, 14.0, 15.7, 19.0 and 8.9, 9.8, 10.2,
+// 13.0).  One token on few long rows: made once and by twos (2048 x 6144 14.0 -> 13.3).
+template <bool PIECES>
+static int gr_run_as(const GfArgs& p, int batches, int sms, cudaStream_t stream) {
     const int gl = gf_group_length(p.K), groups = (p.K + gl - 1) / gl;
-    // eight weight rows to a warp where sixteen would leave half of the SMs without a block (1024 x 3072 8.0 -> 7.0 us; 2048 x 2048,
-    // 128 blocks of sixteen, 6.2 and 8.0)
-    int slots = 1;
-    while (slots < groups) slots *= 2;
-    const int rows = GR_WARPS / slots * 16;
-    const bool few = (long long)((p.N + rows - 1) / rows) * batches * 2 <= sms;
-#define GR_CASE(RR, HH, DD) \
-    return pieces ? gr_launch<RR, HH, DD, true>(p, groups, batches, sms, stream) : gr_launch<RR, HH, DD, false>(p, groups, batches, sms, stream)
+    const long long tiles = (long long)((p.N + 15) / 16) * batches;
+    const bool few = tiles * 2 <= sms;
     if (p.M > 8) {
-        if (few) GR_CASE(1, 2, 4);
-        GR_CASE(2, 2, 3);
+        if (few) return gr_launch<1, 2, 4, 1, false, PIECES>(p, groups, batches, sms, stream);
+        if ((!PIECES || tiles >= 12LL * sms) && gr_resident<2, 2, 4, true, PIECES>(p, groups) >= 1)
+            return gr_launch<2, 2, 4, 1, true, PIECES>(p, groups, batches, sms, stream);
+        return gr_launch<2, 2, 3, 1, false, PIECES>(p, groups, batches, sms, stream);
     }
-    if (few) GR_CASE(1, 1, 6);
-    GR_CASE(2, 1, 4);
-#undef GR_CASE
+    if (few) return gr_launch<1, 1, 9, 3, false, PIECES>(p, groups, batches, sms, stream);
+    if (!PIECES || 2 * tiles >= (2LL + p.M) * sms) {
+        if (PIECES && gr_resident<2, 1, 4, true, PIECES>(p, groups) >= 2) return gr_launch<2, 1, 4, 1, true, PIECES>(p, groups, batches, sms, stream);
+        if (gr_resident<2, 1, 3, true, PIECES>(p, groups) >= 2) return gr_launch<2, 1, 3, 1, true, PIECES>(p, groups, batches, sms, stream);
+        if (!PIECES && gr_resident<2, 1, 4, true, PIECES>(p, groups) >= 1) return gr_launch<2, 1, 4, 1, true, PIECES>(p, groups, batches, sms, stream);
+    }
+    if (PIECES && p.M == 1 && p.K >= 4096 && tiles <= sms && gr_resident<2, 1, 6, true, PIECES>(p, groups) >= 1)
+        return gr_launch<2, 1, 6, 2, true, PIECES>(p, groups, batches, sms, stream);
+    return gr_launch<2, 1, 4, 1, false, PIECES>(p, groups, batches, sms, stream);
+}
+
+int gr_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stream) {
+    return pieces ? gr_run_as<true>(p, batches, sms, stream) : gr_run_as<false>(p, batches, sms, stream);
 }

@@ -16,9 +16,10 @@
 // memory as swizzled K-major tiles; one thread issues the products; other warps add up the chunks.
 //
 // What bounds it: shared memory (a stage of 128 tokens takes it some 2300 clocks, 96 KB of parts written and what the products read
-// of them, the tensor cores 1536) and the stages' hand-overs; the tensor cores are busy 50 % of the time.  Microseconds, eight chains of multiply-adds on the CUDA cores (gemm_simt.cu) and now: 696 tokens
-// 4096 x 1024 212 -> 71, 1024 x 2048 101 -> 49, 1024 x 3072 143 -> 62, 2048 tokens 4096 x 4096 1750 -> 479 (143 TFLOP/s),
-// 64 tokens 4096 x 1024 22 -> 14, 17 tokens 151936 x 1024 355 -> 214.  Error against 64 bits (2-norm): K 1024 2.1e-7 ->
+// of them, the tensor cores 1536) and the stages' hand-overs; the tensor cores are busy 50 % of the time.  Microseconds, eight chains
+// of multiply-adds on the CUDA cores (gemm_simt.cu) and now: 696 tokens
+// 4096 x 1024 212 -> 73, 1024 x 2048 101 -> 51, 1024 x 3072 142 -> 65, 2048 tokens 4096 x 4096 1750 -> 489 (141 TFLOP/s),
+// 64 tokens 4096 x 1024 22 -> 15, 17 tokens 151936 x 1024 354 -> 214.  Error against 64 bits (2-norm): K 1024 2.1e-7 ->
 // 0.94e-7, 4096 4.1e-7 -> 1.1e-7, 12288 6.8e-7 -> 1.5e-7.
 #include "tc_ptx.cuh"
 #include "gemm_split_tc.h"
@@ -36,7 +37,7 @@ struct GfTile {
     static constexpr int THREADS = (GF_CONV + EPI + 4) * 32;
     static constexpr int COLS = BT / (EPI / 4);                 // tokens of an epilogue thread
     // the next stage's rows asked for once this one is handed over, not row by row as their registers come free: 2048 tokens
-    // 4096 x 4096 518 -> 479 us in tiles of 128 tokens, whose converters are short of registers, no change in the others
+    // 4096 x 4096 518 -> 479 us (before operands were scaled) in tiles of 128 tokens, whose converters are short of registers, no change in the others
     static constexpr bool LATE = EPI == 8;
     static constexpr int PIECE = EPI == 8 ? 16 : 32;            // columns read at a time (96 registers a thread, or 128)
     static constexpr int TMEM = 4 * BT < 32 ? 32 : 4 * BT;      // three chunks | the groups' sum

@@ -8,7 +8,6 @@
 #define GF_MIN_K 1024
 #define GF_BK 64            // groups are multiples of it
 #define GF_GROUPS 8
-#define GF_GROUP 128        // k of a group at least
 
 // Operands are multiplied by 2^24 before they are taken apart and sums by 2^-48 at the end, which changes no bit of either (a
 // result below 2^-126 is rounded, once): a float's lowest bit lies 2^-23 below its first, under the smallest bfloat16 for floats
@@ -26,10 +25,8 @@ struct GfArgs {
     long long a_batch, w_batch, c_batch, g_batch;
 };
 
-__host__ __device__ __forceinline__ int gf_group_length(int K) {
-    const int l = ((K + GF_GROUPS - 1) / GF_GROUPS + GF_BK - 1) / GF_BK * GF_BK;
-    return l < GF_GROUP ? GF_GROUP : l;
-}
+// (K from GF_MIN_K on: six to eight groups)
+__host__ __device__ __forceinline__ int gf_group_length(int K) { return ((K + GF_GROUPS - 1) / GF_GROUPS + GF_BK - 1) / GF_BK * GF_BK; }
 
 // (a, b) minus the pair of bfloat16 values packed in h
 __device__ __forceinline__ void gf_less(float& a, float& b, uint32_t h) {

@@ -408,6 +408,19 @@ def test_gemm_split_one_order_of_sums(ops, M, N, K):
     assert ops.gemm_status() == 0
 
 
+@pytest.mark.parametrize("N,K", [(1500, 4100), (3600, 1029), (12000, 1100), (28500, 1024), (500, 1540)])
+@pytest.mark.parametrize("odd", [0, 1])
+def test_gemm_split_few_tokens_every_way(ops, N, K, odd):
+    """Up to 16 tokens, whose parts come through the ring or lie in shared memory, two or three chunks side by side, in rows of
+    16-byte pieces and without: the bits that seventeen have on the tiles' kernel."""
+    pad = -K % 4 + odd
+    x, y = torch.zeros(17, K + pad, device="cuda"), torch.zeros(N, K + pad, device="cuda")
+    x[:, :K], y[:, :K] = rnd(17, K, seed=59), rnd(N, K, scale=0.05, seed=60)
+    want = ops.gemm_simt(x[:, :K], y[:, :K], torch.full((17, N), float("nan"), device="cuda"))
+    for M in (1, 2, 4, 5, 8, 9, 13, 16):
+        assert torch.equal(ops.gemm_simt(x[:M, :K], y[:, :K], torch.full((M, N), float("nan"), device="cuda")), want[:M]), M
+
+
 @pytest.mark.parametrize("M", [1, 9, 16, 17, 40, 130])
 @pytest.mark.parametrize("a_size,w_size", [(1e-34, 1.0), (1.0, 1e-36), (1e-38, 1e3), (1e-42, 1.0), (1e-20, 1e-21), (1e-38, 1e30), (1e-44, 1e38), (1e14, 1e13), (1e33, 1e-30), (2e37, 1.0)])
 def test_gemm_split_small_and_large_operands(ops, M, a_size, w_size):
