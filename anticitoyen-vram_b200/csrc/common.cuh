@@ -159,6 +159,8 @@ static inline void acv_launch(int kernel_class, void (*kernel)(KArgs...), dim3 g
 }
 
 // ----------------------------------------------------------------------------- thread-block clusters
+// Clusters of 1..8 CTAs, an SM to each, that a B200's 148 SMs hold at once.
+static const int ACV_CLUSTERS_AT_ONCE[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

@@ -364,7 +364,6 @@ int gf_run_as(const GfArgs& p, bool pieces, int batches, int way, int per, cudaS
 // 30 / 14 / 28; 696 tokens as 128 x all / 128 x 2 / 64 x all 71 / 104 / 82).
 struct GfWay { int bt, stage, rest; };
 static const GfWay GF_WAYS[3] = {{32, 1200, 5200}, {64, 1350, 6800}, {128, 1700, 10000}};
-static const int GF_CLUSTERS[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};      // of 1..8 CTAs that 148 SMs hold at once
 
 int gf_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stream) {
     if (p.M <= 16) return gr_run(p, pieces, batches, sms, stream);
@@ -376,7 +375,7 @@ int gf_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stre
             const GfWay& g = GF_WAYS[w];
             const int each = q == 2 ? groups : q + 1, parts = (groups + each - 1) / each;
             const long long tiles = (long long)((p.M + g.bt - 1) / g.bt) * ((p.N + GF_ROWS - 1) / GF_ROWS) * batches;
-            const long long at_once = max(1, GF_CLUSTERS[parts] * sms / 148);
+            const long long at_once = max(1, ACV_CLUSTERS_AT_ONCE[parts] * sms / 148);
             const double t = (double)((tiles + at_once - 1) / at_once) * (min(stages, each * group) * (double)g.stage + g.rest);
             if (best < 0. || t < best) { best = t; way = w; per = each; }
         }

@@ -127,6 +127,8 @@ def _declare(lib: ctypes.CDLL) -> None:
         "acv_attention_decode": [P, I, P, I, P, P, P, P, I, P, P, I, P, I, I, I, I, I, F, I, I, I, P, P, P, LL, LL, LL, I, I, I, I, P, P, P, I, P],
         "acv_attention_tc": [P, I, I, P, I, P, P, P, P, I, P, P, P, I, P, I, I, I, I, I, F, I, I, I, P, I, P, P, P, I, I, I, P],
         "acv_attention_tc_shared_bytes": [I, I],
+        "acv_attention_tc_parts": [I, I, I, I, I, I, I, I],
+        "acv_attention_work": [P, P, P, I, I, P, P, P, P, I, P],
         "acv_attention_chunk": [P, I, P, I, P, P, P, P, I, P, P, P, I, P, I, I, I, I, I, F, I, I, I, I, P],
         "acv_table_update": [P, I, I, P, I, P],
         "acv_embed_scaled": [P, P, P, I, I, I, F, I, P],
@@ -982,76 +984,35 @@ def attention_work(q_lens, kv_lens, cu_q) -> tuple[dict, dict]:
     QUERY_TILE tokens of the requests with more (portions of prompts), late tiles first since they see most keys.
     Returns (int32 arrays that the kernels read on the device, counts and maxima for the launches)."""
     import numpy as np
-    q_lens, kv_lens = [int(q) for q in q_lens], [int(k) for k in kv_lens]
-    dec = np.asarray([i for i, q in enumerate(q_lens) if q == 1], dtype=np.int32)
-    seq, q0, keys = [], [], []          # of every tile: its request, its first query, the keys its last query sees
-    for i, q in enumerate(q_lens):
-        if q > 1:
-            before = kv_lens[i] - q
-            seq += [i] * -(-q // QUERY_TILE)
-            q0 += range(0, q, QUERY_TILE)
-            keys += range(before + QUERY_TILE, before + q, QUERY_TILE)
-            keys.append(before + q)
-    # the tiles with most keys first, over all requests: the hardware hands out CTAs in this order, and the kernel
-    # that gives a CTA two tiles pairs the list's front with its back
-    order = sorted(range(len(keys)), key=keys.__getitem__, reverse=True)        # (stable: equal ones keep their order)
-    arrays = {"dec_tokens": np.asarray(cu_q, dtype=np.int32)[:-1][dec], "dec_seqs": dec,
-              "tile_seq": np.asarray([seq[t] for t in order], dtype=np.int32),
-              "tile_q0": np.asarray([q0[t] for t in order], dtype=np.int32)}
-    values = {"n_dec": len(dec), "n_tiles": len(order),
-              "max_dec_kv": max((k for k, q in zip(kv_lens, q_lens) if q == 1), default=0),
-              "max_tile_kv": max((k for k, q in zip(kv_lens, q_lens) if q > 1), default=0)}
-    if order:               # key tiles of all tiles, of the longest and of the shortest
-        blocks = [-(-k // QUERY_TILE) for k in keys]
-        values["tile_blocks"] = (sum(blocks), max(blocks), min(blocks))
+    B = len(q_lens)
+    cap = int(cu_q[-1]) // QUERY_TILE + B if B else 0       # (each request's last tile may be a part of one)
+    buf = np.empty(5 * B + 2 * cap + 8, np.int32)
+    buf[:B], buf[B:2 * B], buf[2 * B:3 * B + 1] = q_lens, kv_lens, cu_q
+    at, dec, til = buf.__array_interface__["data"][0], 3 * B + 1, 5 * B + 1
+    code = library().acv_attention_work(at, at + 4 * B, at + 8 * B, B, QUERY_TILE, at + 4 * dec, at + 4 * (dec + B), at + 4 * til,
+                                        at + 4 * (til + cap), cap, at + 4 * (til + 2 * cap))
+    if code:
+        raise KernelError(f"attention_work: {_ERRORS.get(code, f'refused with code {code}')}")
+    n_dec, n_tiles, max_dec, max_tile, *blocks = buf[til + 2 * cap:].tolist()
+    arrays = {"dec_tokens": buf[dec + B:dec + B + n_dec], "dec_seqs": buf[dec:dec + n_dec],
+              "tile_seq": buf[til:til + n_tiles], "tile_q0": buf[til + cap:til + cap + n_tiles]}
+    values = {"n_dec": n_dec, "n_tiles": n_tiles, "max_dec_kv": max_dec, "max_tile_kv": max_tile}
+    if n_tiles:             # key tiles of all tiles, of the longest and of the shortest
+        values["tile_blocks"] = tuple(blocks)
     return arrays, values
-
-
-# Clusters of 1..8 thread blocks, an SM to each, that a B200's parts hold at once.
-CLUSTERS_AT_ONCE = (0, 148, 74, 45, 33, 26, 22, 15, 15)
-
-
-# Microseconds in ``attention_tc``: a round of blocks, a round that merges its clusters' parts, a tile of 128 keys of two heads;
-# and what a head without a partner takes of that.
-TC_PARTS_FIXED, TC_PARTS_MERGE, TC_PARTS_BLOCK, TC_PARTS_ODD = 4.0, 12.0, 2.1, 0.6
-
-
-def _tc_parts(units: int, work: float, longest: float, shortest: float, sms: int, rounds_of: int) -> tuple:
-    """(least microseconds, parts) for ``units`` of blocks with ``work`` key tiles in all."""
-    best = None
-    for parts in range(1, max(1, min(8, rounds_of)) + 1):
-        at_once = max(1, CLUSTERS_AT_ONCE[parts] * sms // 148)
-        span = longest if parts == 1 else longest / rounds_of * -(-rounds_of // parts)
-        if units > at_once:
-            span = max(span, work / (parts * at_once) + shortest / parts)
-        cost = -(-units // at_once) * (TC_PARTS_FIXED if parts == 1 else TC_PARTS_MERGE) + span * TC_PARTS_BLOCK
-        if best is None or cost < (0.95 * best[0] if best[1] == 1 else best[0]):
-            best = (cost, parts)
-    return best
 
 
 @functools.lru_cache(maxsize=4096)
 def attention_tc_parts(n_tiles: int, blocks: tuple, num_heads: int, num_kv_heads: int, limit: int, sms: int) -> tuple:
     """How many blocks share the keys of a tile of queries in ``attention_tc`` (``parts`` there), by the time of the rounds of
-    blocks that come one after the other.  ``blocks``: key tiles of all tiles of queries, of the longest and of the shortest;
-    ``limit`` > 0: none sees more.  Microseconds with one block and with the parts chosen: 16 heads on 8, 1000 tokens behind 5000
-    101 -> 62, 64 behind 2000 40 -> 19; 32 on 8, 500 behind 5000 94 -> 58, 2048 in front of nothing (256 blocks) 48 either way;
-    40 on 8, 1000 behind 5000, pairs by one block and the fifth heads by two, 169 -> 150."""
-    total, longest, shortest = blocks
-    if limit and limit < longest:
-        total, longest, shortest = min(total, n_tiles * limit), limit, min(shortest, limit)
-    n_rep, each = num_heads // num_kv_heads, n_tiles * num_kv_heads
-    if n_rep == 1:          # one head to a block throughout
-        return _tc_parts(each, total * num_kv_heads * TC_PARTS_ODD, longest * TC_PARTS_ODD, shortest * TC_PARTS_ODD, sms, longest)[1], 0
-    pairs, odd = n_rep // 2, n_rep % 2
-    cost, parts = _tc_parts(each * (pairs + odd), total * num_kv_heads * (pairs + TC_PARTS_ODD * odd), longest,
-                            shortest * (TC_PARTS_ODD if odd else 1.0), sms, longest)
-    if odd:
-        a = _tc_parts(each * pairs, total * num_kv_heads * pairs, longest, shortest, sms, longest)
-        b = _tc_parts(each, total * num_kv_heads * TC_PARTS_ODD, longest * TC_PARTS_ODD, shortest * TC_PARTS_ODD, sms, longest)
-        if a[0] + b[0] + 3.0 < 0.95 * cost:
-            return a[1], b[1]
-    return parts, 0
+    blocks that come one after the other (csrc/attention_plan.cu).  ``blocks``: key tiles of all tiles of queries, of the longest
+    and of the shortest; ``limit`` > 0: none sees more.  Microseconds with one block and with the parts chosen: 16 heads on 8, 1000
+    tokens behind 5000 101 -> 62, 64 behind 2000 40 -> 19; 32 on 8, 500 behind 5000 94 -> 58, 2048 in front of nothing (256 blocks)
+    48 either way; 40 on 8, 1000 behind 5000, pairs by one block and the fifth heads by two, 169 -> 150."""
+    parts = library().acv_attention_tc_parts(n_tiles, *blocks, num_heads, num_kv_heads, limit, sms)
+    if parts < 1:
+        raise KernelError(f"attention_tc_parts: {_ERRORS.get(parts, f'refused with code {parts}')}")
+    return parts % 16, parts // 16
 
 
 def attention_work_decode(padded: int, max_kv: int) -> tuple[dict, dict]:

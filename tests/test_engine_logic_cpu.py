@@ -452,3 +452,67 @@ def test_the_projection_of_few_tokens_refuses_what_the_others_refuse(wrong):
     assert lib.acv_gemm_rows_qkv(*head, 1, 148, *tail) == size
     if name not in ("out", "ldo"):          # (those the other finds out behind its tensor maps, which need a device)
         assert lib.acv_gemm_tc_qkv(*head, 1, 16, 1, None, 0, None, 0, at, 148, 4, 2, *tail) == size
+
+
+def test_attention_work_over_many_batches():
+    """The native lists against a sort in plain Python, over batches of all kinds: one-token requests, portions behind contexts,
+    tiles that see equally many keys, many of each."""
+    import random
+    import numpy as np
+    from acvram_b200.kernels.ops import QUERY_TILE, attention_work
+    r = random.Random(3)
+    for _ in range(300):
+        q_lens = [r.choice([1, 1, 2, 127, 128, 129, 300, r.randrange(1, 3000)]) for _ in range(r.choice([1, 2, 3, 20, 150]))]
+        kv_lens = [q + r.choice([0, 0, 128, r.randrange(5000)]) for q in q_lens]
+        cu = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+        tiles = [(i, a, kv - q + min(a + QUERY_TILE, q)) for i, (q, kv) in enumerate(zip(q_lens, kv_lens)) if q > 1 for a in range(0, q, QUERY_TILE)]
+        tiles.sort(key=lambda t: -t[2])
+        blocks = [-(-t[2] // QUERY_TILE) for t in tiles]
+        dec = [i for i, q in enumerate(q_lens) if q == 1]
+        arrays, values = attention_work(q_lens, kv_lens, cu)
+        assert {k: (a.dtype, a.tolist()) for k, a in arrays.items()} == {
+            k: (np.int32, v) for k, v in {"dec_tokens": [int(cu[i]) for i in dec], "dec_seqs": dec, "tile_seq": [t[0] for t in tiles],
+                                          "tile_q0": [t[1] for t in tiles]}.items()}
+        assert values == {"n_dec": len(dec), "n_tiles": len(tiles), "max_dec_kv": max((kv_lens[i] for i in dec), default=0),
+                          "max_tile_kv": max((k for k, q in zip(kv_lens, q_lens) if q > 1), default=0),
+                          **({"tile_blocks": (sum(blocks), max(blocks), min(blocks))} if tiles else {})}
+
+
+def test_shares_of_a_tile_are_the_cheapest_by_the_model():
+    """The native choice of blocks to a tile's keys against the model in plain Python, over groups of one to nine heads, windows, and
+    few and many tiles."""
+    import random
+    from acvram_b200.kernels.ops import attention_tc_parts
+    at_once_of = (0, 148, 74, 45, 33, 26, 22, 15, 15)
+
+    def cheapest(units, work, longest, shortest, most, sms):
+        best = None
+        for parts in range(1, max(1, min(8, most)) + 1):
+            at_once = max(1, at_once_of[parts] * sms // 148)
+            span = longest if parts == 1 else longest / most * -(-most // parts)
+            if units > at_once:
+                span = max(span, work / (parts * at_once) + shortest / parts)
+            cost = -(-units // at_once) * (4.0 if parts == 1 else 12.0) + span * 2.1
+            if best is None or cost < (0.95 * best[0] if best[1] == 1 else best[0]):
+                best = (cost, parts)
+        return best
+
+    r, seen = random.Random(4), set()
+    for _ in range(2000):
+        blocks = [r.randrange(1, r.choice([2, 9, 70, 300])) for _ in range(r.choice([1, 2, 8, 40]))]
+        n, total, longest, shortest = len(blocks), sum(blocks), max(blocks), min(blocks)
+        kv, rep, limit, sms = r.choice([1, 2, 4, 8]), r.randrange(1, 10), r.choice([0, 0, 1, 5, 40]), r.choice([148, 132])
+        got = attention_tc_parts(n, (total, longest, shortest), kv * rep, kv, limit, sms)
+        if limit and limit < longest:
+            total, longest, shortest = min(total, n * limit), limit, min(shortest, limit)
+        pairs, odd = rep // 2, rep % 2
+        lone = lambda: cheapest(n * kv, total * kv * 0.6, longest * 0.6, shortest * 0.6, longest, sms)
+        if rep == 1:
+            want = lone()[1], 0
+        else:
+            cost, parts = cheapest(n * kv * (pairs + odd), total * kv * (pairs + 0.6 * odd), longest, shortest * (0.6 if odd else 1.0), longest, sms)
+            a, b = cheapest(n * kv * pairs, total * kv * pairs, longest, shortest, longest, sms), lone()
+            want = (a[1], b[1]) if odd and a[0] + b[0] + 3.0 < 0.95 * cost else (parts, 0)
+        assert got == want, (blocks, kv, rep, limit, sms)
+        seen.add(want)
+    assert len(seen) > 12
