@@ -1431,11 +1431,14 @@ def moe_gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, grouped: 
     return out
 
 
+def _moe_mma_weights(w: torch.Tensor) -> bool:
+    return w.dtype == torch.bfloat16 and w.is_contiguous() and (w.shape[1] * w.shape[2]) % 8 == 0 and w.data_ptr() % 16 == 0
+
+
 def moe_gemm_mma_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
     """The tensor-core form of the grouped products wants bfloat16 and rows of 16-byte alignment."""
-    return (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.shape[1] % 8 == 0 and a.stride(0) % 8 == 0
-            and a.stride(1) == 1 and w.is_contiguous() and (w.shape[1] * w.shape[2]) % 8 == 0 and a.data_ptr() % 16 == 0
-            and w.data_ptr() % 16 == 0)
+    return (a.dtype == torch.bfloat16 and a.shape[1] % 8 == 0 and a.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0
+            and _moe_mma_weights(w))
 
 
 def moe_gemm_mma(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, grouped: torch.Tensor, tile_expert: torch.Tensor,
@@ -1476,7 +1479,7 @@ def moe_rows_tile(rows: int, experts: int, h: torch.Tensor, up: torch.Tensor, do
     """Rows of a tile (8 or 16) where the experts' products are made by ``moe_rows``, 0 where they are not."""
     tile = 8 if rows <= MOE_ROWS_8 * experts else 16
     if rows > MOE_ROWS_16 * experts or h.shape[1] % 64 or down.shape[2] % 64 or up.shape[1] % 32 or down.shape[1] % 32 \
-            or not moe_gemm_mma_takes(h, up):
+            or not moe_gemm_mma_takes(h, up) or not _moe_mma_weights(down):
         return 0
     tiles = moe_max_tiles(rows, experts, tile)
     return tile if tiles <= 512 and tiles * tile <= 2048 else 0

@@ -518,3 +518,26 @@ def test_shares_of_a_tile_are_the_cheapest_by_the_model():
         assert got == want, (blocks, kv, rep, limit, sms)
         seen.add(want)
     assert {w[0] for w in seen} >= set(range(1, 9)) and any(w[1] for w in seen)
+
+
+@pytest.mark.parametrize("which", ["neither", "up", "down"])
+@pytest.mark.parametrize("how", ["off its 16 bytes", "every other matrix", "float"])
+def test_experts_of_few_rows_want_both_products_weights_dense_and_aligned(which, how):
+    """Weights that the tiled products on the tensor cores leave to the CUDA cores are not sent to the kernel for few rows, which
+    would refuse them: the first product's and the second's alike."""
+    import torch
+    from acvram_b200.kernels import ops
+    E, H, F = 4, 128, 64
+
+    def weights(rows, cols, odd):
+        if not odd:
+            return torch.zeros(E, rows, cols, dtype=torch.bfloat16)
+        if how == "float":
+            return torch.zeros(E, rows, cols)
+        if how == "every other matrix":
+            return torch.zeros(2 * E, rows, cols, dtype=torch.bfloat16)[::2]
+        return torch.zeros(E * rows * cols + 4, dtype=torch.bfloat16)[4:].view(E, rows, cols)
+
+    h = torch.zeros(3, H, dtype=torch.bfloat16)
+    tile = ops.moe_rows_tile(6, E, h, weights(2 * F, H, which == "up"), weights(H, F, which == "down"))
+    assert (tile == 8) == (which == "neither")
