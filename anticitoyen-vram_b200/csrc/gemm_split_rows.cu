@@ -43,11 +43,12 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
     extern __shared__ __align__(16) unsigned char ring[];
     __shared__ float part[2][GR_WARPS][8 * H][COLS + 1];
     const int group = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;      // (a warp to a group)
-    const float* A = p.A + (size_t)blockIdx.z * p.a_batch;
+    const int m0 = blockIdx.y * 8 * H, M = min(p.M - m0, 8 * H);        // the block's tokens
+    const float* A = p.A + (size_t)blockIdx.z * p.a_batch + (size_t)m0 * p.lda;
     const float* W = p.W + (size_t)blockIdx.z * p.w_batch;
-    float* C = p.C + (size_t)blockIdx.z * p.c_batch;
-    const float* gate = p.gate ? p.gate + (size_t)blockIdx.z * p.g_batch : nullptr;
-    bool again = gate != nullptr;
+    float* C = p.C + (size_t)blockIdx.z * p.c_batch + (size_t)m0 * p.ldc;
+    const float* gate = p.gate ? p.gate + (size_t)blockIdx.z * p.g_batch + (size_t)m0 * p.ldg : nullptr;
+    bool again = false;
     const int gl = gf_group_length(p.K), k_begin = group * gl, mine = group < groups ? min(gl, p.K - k_begin) : 0;
     const int chunks = (mine + 31) / 32, tiles = (p.N + COLS - 1) / COLS;
     const uint32_t own = smem_u32(ring) + group * (DEPTH * CHUNK) + lane * 16;
@@ -80,7 +81,7 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
                 for (int r = 0; r < R; ++r) copy(dst + (e * ROWS + r) * 512, wr[r] + e * 16, left);
                 if constexpr (!PARTS) {
 #pragma unroll
-                    for (int h = 0; h < H; ++h) copy(dst + (e * ROWS + R + h) * 512, ar[h] + e * 16, h * 8 + g < p.M ? left : 0);
+                    for (int h = 0; h < H; ++h) copy(dst + (e * ROWS + R + h) * 512, ar[h] + e * 16, h * 8 + g < M ? left : 0);
                 }
             }
             into = into + 1 == DEPTH ? 0 : into + 1;
@@ -98,7 +99,7 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
         cp_async_commit();
     };
     // the tokens' parts: of each chunk and token, of each four lanes' k, the parts of the first and of the second step (a lane's 48 bytes)
-    const uint32_t parts_at = smem_u32(ring) + GR_WARPS * DEPTH * CHUNK + group * (gl / 32) * p.M * 192;
+    const uint32_t parts_at = smem_u32(ring) + GR_WARPS * DEPTH * CHUNK + group * (gl / 32) * M * 192;
     pdl_wait();
     if (chunks) {
         rows();
@@ -106,8 +107,8 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
         for (int i = 0; i < DEPTH - Q; ++i) ask();
         if constexpr (PARTS) {
 #pragma unroll 4
-            for (int i = lane; i < chunks * p.M * 8; i += 32) {
-                const int q = i & 3, e = i >> 2 & 1, m = (i >> 3) % p.M, c = (i >> 3) / p.M, k = c * 32 + e * 16 + q * 4;
+            for (int i = lane; i < chunks * M * 8; i += 32) {
+                const int q = i & 3, e = i >> 2 & 1, m = (i >> 3) % M, c = (i >> 3) / M, k = c * 32 + e * 16 + q * 4;
                 const float* src = A + (size_t)m * p.lda + k_begin + k;
                 float4 v;
                 if (PIECES && k + 4 <= mine) {
@@ -123,7 +124,7 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
                 gr_parts(v.z, v.w, h[0][1], h[1][1], h[2][1]);
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
-                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(parts_at + ((c * p.M + m) * 4 + q) * 48 + e * 24 + j * 8), "r"(h[j][0]), "r"(h[j][1]) : "memory");
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(parts_at + ((c * M + m) * 4 + q) * 48 + e * 24 + j * 8), "r"(h[j][0]), "r"(h[j][1]) : "memory");
             }
             __syncwarp();
         }
@@ -155,8 +156,8 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
                             uint32_t u[12];
 #pragma unroll
                             for (int j = 0; j < 12; ++j) u[j] = 0;
-                            if (h * 8 + g < p.M && n + z < chunks) {
-                                const uint32_t at = parts_at + (((n + z) * p.M + h * 8 + g) * 4 + tq) * 48;
+                            if (h * 8 + g < M && n + z < chunks) {
+                                const uint32_t at = parts_at + (((n + z) * M + h * 8 + g) * 4 + tq) * 48;
 #pragma unroll
                                 for (int j = 0; j < 3; ++j)
                                     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
@@ -238,7 +239,7 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
         __syncthreads();
         if (tile + (int)gridDim.x >= tiles) pdl_launch_dependents();
         // outputs: token by token, weight rows side by side
-        for (int i = threadIdx.x; i < p.M * COLS; i += GR_WARPS * 32) {
+        for (int i = threadIdx.x; i < M * COLS; i += GR_WARPS * 32) {
             const int m = i / COLS, c = i - m * COLS, gn = tile * COLS + c;
             if (gn >= p.N) continue;
             float v[GF_GROUPS];
@@ -248,19 +249,23 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
 #pragma unroll
             for (int j = 1; j < GF_GROUPS; ++j)
                 if (j < groups) x = x + v[j];
-            again |= !(fabsf(x) <= 3.402823466e38f);
-            C[(size_t)m * p.ldc + gn] = x * GF_SCALE_BACK;
+            const bool number = fabsf(x) <= 3.402823466e38f;
+            again |= !number;
+            x *= GF_SCALE_BACK;
+            if (gate && number) x /= 1.f + expf(-gate[(size_t)m * p.ldg + gn]);
+            C[(size_t)m * p.ldc + gn] = x;
         }
     }
     cp_async_wait<0>();
     if (!again) return;
-    // this thread's outputs once more: a gate, or one that is no finite number
+    // this thread's outputs once more, those that are no finite number (a gate that is none leaves none again)
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-        for (int i = threadIdx.x; i < p.M * COLS; i += GR_WARPS * 32) {
+        for (int i = threadIdx.x; i < M * COLS; i += GR_WARPS * 32) {
             const int m = i / COLS, gn = tile * COLS + i - m * COLS;
             if (gn >= p.N) continue;
             float x = C[(size_t)m * p.ldc + gn];
-            if (!(fabsf(x) <= 3.402823466e38f)) x = gf_plain(A + (size_t)m * p.lda, W + (size_t)gn * p.ldw, p.K);
+            if (fabsf(x) <= 3.402823466e38f) continue;
+            x = gf_plain(A + (size_t)m * p.lda, W + (size_t)gn * p.ldw, p.K);
             if (gate) x /= 1.f + expf(-gate[(size_t)m * p.ldg + gn]);
             C[(size_t)m * p.ldc + gn] = x;
         }
@@ -270,7 +275,7 @@ gemm_split_rows_kernel(const GfArgs p, int groups) {
 // copies of four bytes go through what is left as its first-level cache).
 template <int R, int H, int DEPTH, bool PARTS>
 static int gr_smem(const GfArgs& p, int groups) {
-    return GR_WARPS * DEPTH * 2 * (R + (PARTS ? 0 : H)) * 512 + (PARTS ? groups * (gf_group_length(p.K) / 32) * p.M * 192 : 0);
+    return GR_WARPS * DEPTH * 2 * (R + (PARTS ? 0 : H)) * 512 + (PARTS ? groups * (gf_group_length(p.K) / 32) * min(p.M, 8 * H) * 192 : 0);
 }
 template <int R, int H, int DEPTH, bool PARTS, bool PIECES>
 static int gr_resident(const GfArgs& p, int groups) {
@@ -285,31 +290,39 @@ static int gr_launch(const GfArgs& p, int groups, int batches, int sms, cudaStre
     auto kernel = gemm_split_rows_kernel<R, H, DEPTH, Q, PARTS, PIECES>;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
     if (batches > 65535) return ACV_ERR_SIZE;
-    const dim3 grid(min((p.N + 8 * R - 1) / (8 * R), max(1, min(resident, Q > 2 ? 1 : 2)) * sms), 1, batches);
+    const dim3 grid(min((p.N + 8 * R - 1) / (8 * R), max(1, min(resident, Q > 2 ? 1 : 2)) * sms), (p.M + 8 * H - 1) / (8 * H), batches);
     acv_launch(PDL_GEMM, kernel, grid, dim3(GR_WARPS * 32), smem, stream, p, groups);
     return acv_launch_status();
 }
 
-// Eight weight rows to a warp where sixteen would leave half of the SMs without a block, and three chunks side by side there, as a block
-// has its SM to itself and waits for its chains (1 token 1024 x 3072 sixteen rows 7.7, eight 6.7, by threes 6.3; 1024 x 2048 5.7, 4.9,
-// 5.0; 2048 x 2048, 128 blocks of sixteen, 6.0, 7.6, 8.4).
+// Which way, all measured in microseconds.
+// Few outputs: a block to eight weight rows and eight tokens, whatever the number of tokens, as long as each has an SM to itself (or
+// shares one with one other, up to K = 4096; longer chains take longer than the tiles' kernel there), since what counts is how many
+// chains run side by side.  64 tokens, tiles, and this: 64 x 1024 6.5, 2.9; 64 x 5120 16.2, 9.0; 256 x 1024 (256 blocks) 6.9, 4.4,
+// 256 x 5120 16.7, 17.7; 16 tokens 1024 x 2048 (256 blocks) sixteen tokens to a block 6.9, eight 7.8.  A block that has its SM to
+// itself makes chunks side by side, as it waits for its chains: by threes (1 token 1024 x 3072 one by one 6.7, by twos 6.5, by threes
+// 6.3), by twos where a group is four chunks (8 tokens 256 x 1024 3.4, 2.9).
+// Sixteen weight rows to a warp otherwise (2048 x 2048, 128 blocks, 6.0, with eight rows 7.6).
 // The tokens' parts made once pay where a block meets enough tiles with them, the more tokens the more of them, and two blocks still
 // fit an SM (1, 4, 8 tokens, through the ring and made once: 4096 x 1024 5.6, 5.9, 6.0 and 5.7, 6.0, 6.8; 12288 x 2048 22.9, 23.0 and 19.9,
 // 21.7 (8 do not fit); 151936 x 1024 119, 119, 123 and 96, 98, 104; 16 tokens, one block to an SM, 174 and 152, 6144 x 1024 9.7 and 11.4),
 // and wherever they fit for rows that come float by float (4096 x 1025, 1, 4, 8, 16 tokens 12.9, 14.0, 15.7, 19.0 and 8.9, 9.8, 10.2,
 // 13.0).  One token on few long rows: made once and by twos (2048 x 6144 14.0 -> 13.3).
+static long long gr_octets(const GfArgs& p, int batches) { return (long long)((p.N + 7) / 8) * ((p.M + 7) / 8) * batches; }
+bool gr_takes(const GfArgs& p, int batches, int sms) { return p.M <= 16 || gr_octets(p, batches) <= (p.K <= 4096 ? 2 : 1) * sms; }
+
 template <bool PIECES>
 static int gr_run_as(const GfArgs& p, int batches, int sms, cudaStream_t stream) {
     const int gl = gf_group_length(p.K), groups = (p.K + gl - 1) / gl;
-    const long long tiles = (long long)((p.N + 15) / 16) * batches;
-    const bool few = tiles * 2 <= sms;
+    const long long tiles = (long long)((p.N + 15) / 16) * batches, octets = gr_octets(p, batches);
+    if (octets <= sms && gl > 128) return gr_launch<1, 1, 9, 3, false, PIECES>(p, groups, batches, sms, stream);
+    if (octets <= sms || p.M > 16) return gr_launch<1, 1, 6, 2, false, PIECES>(p, groups, batches, sms, stream);
     if (p.M > 8) {
-        if (few) return gr_launch<1, 2, 4, 1, false, PIECES>(p, groups, batches, sms, stream);
+        if (tiles * 2 <= sms) return gr_launch<1, 2, 4, 1, false, PIECES>(p, groups, batches, sms, stream);
         if ((!PIECES || tiles >= 12LL * sms) && gr_resident<2, 2, 4, true, PIECES>(p, groups) >= 1)
             return gr_launch<2, 2, 4, 1, true, PIECES>(p, groups, batches, sms, stream);
         return gr_launch<2, 2, 3, 1, false, PIECES>(p, groups, batches, sms, stream);
     }
-    if (few) return gr_launch<1, 1, 9, 3, false, PIECES>(p, groups, batches, sms, stream);
     if (!PIECES || 2 * tiles >= (2LL + p.M) * sms) {
         if (PIECES && gr_resident<2, 1, 4, true, PIECES>(p, groups) >= 2) return gr_launch<2, 1, 4, 1, true, PIECES>(p, groups, batches, sms, stream);
         if (gr_resident<2, 1, 3, true, PIECES>(p, groups) >= 2) return gr_launch<2, 1, 3, 1, true, PIECES>(p, groups, batches, sms, stream);

@@ -366,7 +366,7 @@ struct GfWay { int bt, stage, rest; };
 static const GfWay GF_WAYS[3] = {{32, 1200, 5200}, {64, 1350, 6800}, {128, 1700, 10000}};
 
 int gf_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stream) {
-    if (p.M <= 16) return gr_run(p, pieces, batches, sms, stream);
+    if (gr_takes(p, batches, sms)) return gr_run(p, pieces, batches, sms, stream);
     const int gl = gf_group_length(p.K), stages = (p.K + GF_BK - 1) / GF_BK, group = gl / GF_BK, groups = (p.K + gl - 1) / gl;
     int way = 0, per = groups;
     double best = -1.;

@@ -53,4 +53,6 @@ static __device__ __noinline__ float gf_plain(const float* a, const float* w, in
 }
 
 int gf_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stream);
-int gr_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stream);        // up to 16 tokens
+// the kernel for few tokens or few outputs, and whether it is the one for these
+int gr_run(const GfArgs& p, bool pieces, int batches, int sms, cudaStream_t stream);
+bool gr_takes(const GfArgs& p, int batches, int sms);
