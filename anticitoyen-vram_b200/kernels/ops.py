@@ -567,16 +567,31 @@ def _gemm_tc_plan(M: int, N: int, K: int, sms: int, bn_multiple: int, rows: bool
 
 @functools.lru_cache(maxsize=4096)
 def gemm_rows_pays(M: int, N: int, K: int, sms: int) -> bool:
-    """Whether a product of up to 32 tokens is faster without a tile of 128 weight rows (csrc/gemm_rows.cu) than with one:
-    up to 8 tokens where the weights stay under 128 MB (12288 x 4096 20.1 us against 22.0; 24576 x 4096 35.5 against 34.9,
-    5120 x 17408 37 against 34) and for a vocabulary (151936 x 1024 57.6 against 56.5, x 4096 193 against 206); up to 16, whose
-    rows each block reads, under 50 MB (12288 x 2048 11.9 us against 12.7; 5120 x 5120 15.3 against 14.0, 19456 x 2560 22.1 against 21.4); up to 32 under 17 MB, or 26
-    where each SM has one block (4096 x 2048 7.4 us against 8.3, 2048 x 6144 9.4 against 11.6; 2560 x 4096 11.4 against 9.7)."""
+    """Whether a product of up to 32 tokens is faster without a tile of 128 weight rows (csrc/gemm_rows.cu) than with one
+    (microseconds here: without, with).  A block's weight rows cost it a meeting of its warps, and what it reads of them hides that
+    only where K is long, so what decides is how many blocks come one after the other on an SM.
+    Up to 8 tokens: 224 rows an SM in pairs of sixteen (32768 x 512, 8 tokens 7.7, 7.9; 49152 x 512 11.3, 9.3; 168 under K 384, 128 under 128:
+    32768 x 256 5.8, 4.4; 24576 x 64 4.0, 3.3), 112 where a block is sixteen (16400 x 1024, 5 tokens 7.6, 8.4; 32784 x 512 10.5, 7.9; 96 for
+    eight tokens); beyond them K from 896 on, and the last rounds decide: a round is 64 rows an SM here and 128 there, its time here 6 % more up
+    to K 2048 (3 for one token), the same from there on (2 tokens 131072 x 1024 45, 43; 65536 x 1024 23, 26; 151936 x 4096 193, 206).  Weights
+    under 128 MB, or a vocabulary's.
+    Up to 16 tokens, whose rows each block reads: 112 rows an SM for K 384 to 1024, 96 else, 64 where a block is sixteen (16 tokens 16384 x 512
+    5.7, 6.3; 24576 x 512 7.8, 7.1; 16400 x 512 7.5, 6.3), under 50 MB of weights (12288 x 2048 11.9, 12.7; 5120 x 5120 15.3, 14.0).  Up to 32: 48 rows an SM (32 tokens 6144 x 512 4.6, 5.7;
+    8192 x 512 5.8, 5.7; 12288 x 640 10.9, 6.8), under 17 MB, or 26 where each SM has one block (4096 x 2048 7.4, 8.3; 2560 x 4096 11.4, 9.7)."""
     if K % 64 or N % 16 or M > 32:
         return False
+    pairs = N % 32 == 0
     if M > 16:
-        return N * K <= 8_500_000 or N <= 16 * sms and N * K <= 13_000_000
-    return N * K <= 1 << 26 or N >= 1 << 16 if M <= 8 else N * K <= 25_500_000
+        return N <= 48 * sms and (N * K <= 8_500_000 or N <= 16 * sms and N * K <= 13_000_000)
+    if M > 8:
+        return N * K <= 25_500_000 and N <= (64 if not pairs else 112 if 384 <= K <= 1024 else 96) * sms
+    if not pairs or N * K > 1 << 26 and N < 1 << 16:
+        return N <= (112 if M < 8 else 96) * sms and N * K <= 1 << 26
+    if N <= (224 if K >= 384 else 168 if K >= 128 else 128) * sms and N * K <= 1 << 26:
+        return True
+    rows, tiles = N / (64 * sms), N / (128 * sms)
+    here, there = math.ceil(rows) / rows, math.ceil(tiles) / tiles
+    return K >= 896 and here * (1.0 if K >= 2048 else 1.03 if M == 1 else 1.06) < there
 
 
 def _gemm_rows_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -663,11 +678,11 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, num_heads: 
     _need_cuda(x, w, out, k_pages, v_pages)
     M, K = x.shape
     N = w.shape[0]
-    # A head is a cluster of two or four blocks: as long as all heads' clusters come in one wave, up to 8 tokens with two blocks to
-    # an SM (48 heads of 128, K 4096: 13.3 us against 14.1; 16 tokens, where two do not fit, 18.0 against 15.0; 32 heads, K 1024: 4.2
-    # and 4.8 against 6.1 and 6.7).
+    # A head is a cluster of two or four blocks: as long as all heads' clusters come in one wave, up to 8 tokens and K 4096 with two
+    # blocks to an SM and the shallow rings that leaves room for (48 heads of 128, 8 tokens, K 4096: 13.3 us against 14.1, K 5120 15.5
+    # against 14.0; 16 tokens, where two do not fit, 18.0 against 15.0; 32 heads, K 1024: 4.2 and 4.8 against 6.1 and 6.7).
     if plan is None and static_weights and M <= 16 and _gemm_rows_takes(x, w) \
-            and N // head_dim <= (33 if head_dim == 128 else 74) * (2 if M <= 8 else 1) * sm_count(x.device) // 148:
+            and N // head_dim <= (33 if head_dim == 128 else 74) * (2 if M <= 8 and K <= 4096 else 1) * sm_count(x.device) // 148:
         _check(library().acv_gemm_rows_qkv(
             _p(x), x.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), M, N, K, 1, sm_count(x.device), num_heads, num_kv_heads,
             head_dim, _p(q_weight), _p(k_weight), eps, _p(cos_sin), cos_sin.shape[0] if cos_sin is not None else 0, _p(positions),
@@ -1481,13 +1496,16 @@ def moe_rows_tile(rows: int, experts: int, h: torch.Tensor, up: torch.Tensor, do
     if rows > MOE_ROWS_16 * experts or h.shape[1] % 64 or down.shape[2] % 64 or up.shape[1] % 32 or down.shape[1] % 32 \
             or not moe_gemm_mma_takes(h, up) or not _moe_mma_weights(down):
         return 0
+    if tile == 16 and h.shape[1] < 1024 and experts * down.shape[2] > 96 * sm_count(h.device):
+        return 0            # short rows for more than six blocks one after the other on an SM
     tiles = moe_max_tiles(rows, experts, tile)
     return tile if tiles <= 512 and tiles * tile <= 2048 else 0
 
 
 # Rows to an expert up to which tiles of 8 and of 16 rows are used.  A layer's microseconds with tiles of 64 (moe_gemm_mma), 8 and 16
 # rows: 64 experts of 1024 at width 4096 at 0.1 rows an expert 102, 57, 60; 1.5: 273, 229, 246; 6: 360, 302, 304; 9.4: 369, 344, 320;
-# 32 experts of 768 at width 2048 at 8: 99, 96, 96; 12.5: 106, 122, 113.
+# 32 experts of 768 at width 2048 at 8: 99, 96, 96; 12.5: 106, 122, 113.  Where rows are short, a tile's sums take what its loads save: at 8
+# rows an expert with tiles of 64 and 16 rows 64 experts of 384 at width 768 36, 40; of 256 at 512 23, 26; 32 of 256 at 1024 29, 23.
 MOE_ROWS_8, MOE_ROWS_16 = 7, 10
 
 

@@ -541,3 +541,16 @@ def test_experts_of_few_rows_want_both_products_weights_dense_and_aligned(which,
     h = torch.zeros(3, H, dtype=torch.bfloat16)
     tile = ops.moe_rows_tile(6, E, h, weights(2 * F, H, which == "up"), weights(H, F, which == "down"))
     assert (tile == 8) == (which == "neither")
+
+
+@pytest.mark.parametrize("M,N,K,pays", [
+    (1, 6144, 1024, True), (8, 4096, 4096, True), (16, 4096, 1024, True), (32, 6144, 512, True), (8, 32768, 512, True), (1, 151936, 1024, True),
+    (8, 151936, 4096, True), (2, 65536, 1024, True), (5, 16400, 1024, True),
+    # measured slower than with tiles of 128 weight rows: short K behind many blocks, sixteen rows to a block, even last rounds there
+    (32, 32768, 128, False), (16, 49168, 64, False), (8, 49152, 512, False), (8, 49168, 640, False), (4, 32784, 256, False), (8, 32768, 128, False),
+    (8, 24576, 64, False), (16, 24576, 512, False), (16, 16400, 512, False), (32, 12288, 640, False), (2, 131072, 1024, False), (8, 66000, 1024, False),
+    # sizes that the kernel does not take
+    (33, 4096, 1024, False), (8, 4104, 1024, False), (8, 4096, 1000, False)])
+def test_products_of_few_tokens_go_where_they_are_faster(M, N, K, pays):
+    from acvram_b200.kernels import ops
+    assert ops.gemm_rows_pays(M, N, K, 148) == pays
