@@ -572,8 +572,8 @@ def gemm_rows_pays(M: int, N: int, K: int, sms: int) -> bool:
     only where K is long, so what decides is how many blocks come one after the other on an SM.
     Up to 8 tokens: 224 rows an SM in pairs of sixteen (32768 x 512, 8 tokens 7.7, 7.9; 49152 x 512 11.3, 9.3; 168 under K 384, 128 under 128:
     32768 x 256 5.8, 4.4; 24576 x 64 4.0, 3.3), 112 where a block is sixteen (16400 x 1024, 5 tokens 7.6, 8.4; 32784 x 512 10.5, 7.9; 96 for
-    eight tokens); beyond them K from 896 on, and the last rounds decide: a round is 64 rows an SM here and 128 there, its time here 6 % more up
-    to K 2048 (3 for one token), the same from there on (2 tokens 131072 x 1024 45, 43; 65536 x 1024 23, 26; 151936 x 4096 193, 206).  Weights
+    eight tokens); beyond them K from 896 on, and the last rounds decide: a round is 64 rows an SM here and 128 there, its time here 5 % more up
+    to K 2048, the same from there on (2 tokens 131072 x 1024 45, 43; 65536 x 1024 23, 26; 151936 x 4096 193, 206).  Weights
     under 128 MB, or a vocabulary's.
     Up to 16 tokens, whose rows each block reads: 112 rows an SM for K 384 to 1024, 96 else, 64 where a block is sixteen (16 tokens 16384 x 512
     5.7, 6.3; 24576 x 512 7.8, 7.1; 16400 x 512 7.5, 6.3), under 50 MB of weights (12288 x 2048 11.9, 12.7; 5120 x 5120 15.3, 14.0).  Up to 32: 48 rows an SM (32 tokens 6144 x 512 4.6, 5.7;
@@ -591,7 +591,7 @@ def gemm_rows_pays(M: int, N: int, K: int, sms: int) -> bool:
         return True
     rows, tiles = N / (64 * sms), N / (128 * sms)
     here, there = math.ceil(rows) / rows, math.ceil(tiles) / tiles
-    return K >= 896 and here * (1.0 if K >= 2048 else 1.03 if M == 1 else 1.06) < there
+    return K >= 896 and here * (1.0 if K >= 2048 else 1.05) < there
 
 
 def _gemm_rows_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
