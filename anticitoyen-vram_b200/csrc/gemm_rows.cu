@@ -12,9 +12,7 @@
 // 2.7, 12288 x 2048 12.6 -> 9.9, 4096 x 4096 10.2 -> 7.2, 4096 x 12288 22.0 -> 20.1 (4.9 TB/s), 151936 x 4096 206 -> 193 (6.4 TB/s); with the q,k,v way out
 // 32 heads of 128, K 1024, 6.1 -> 4.2, 48 heads, K 4096, 14.1 -> 13.3.
 #include "gemm_epilogue.cuh"
-#include "mma_tiles.cuh"
-
-#define RW_WARPS 8
+#include "rows_ring.cuh"
 
 struct RowsParams {
     const bf16 *x, *w;
@@ -32,17 +30,17 @@ struct RowsParams {
 // QKV: a block holds 32 rows of a head, sixteen of each half, so that an angle's two rows meet in it; the head's blocks are a cluster
 // (two for heads of 64, four for 128) whose blocks tell each other their sums of squares.
 template <int R, int H, int DEPTH, bool QKV>
-__global__ void __launch_bounds__(RW_WARPS * 32, 2)
+__global__ void __launch_bounds__(RR_WARPS * 32, 2)
 gemm_rows_kernel(const RowsParams p) {
-    constexpr int CHUNK = 2 * (R + H) * 512;        // bytes: two blocks of 32 k, a lane's 16 bytes side by side
-    constexpr int COLS = 8 * R;
+    using Chunk = RrChunk<R, H>;
+    constexpr int CHUNK = Chunk::BYTES, COLS = 8 * R;
     extern __shared__ __align__(16) unsigned char ring[];
-    __shared__ float part[2][RW_WARPS][8 * H][COLS + 4];
+    __shared__ float part[2][RR_WARPS][8 * H][COLS + 4];
     __shared__ float squares[QKV ? 4 : 1][8 * H];
     ACV_TL(TL_GEMM, 0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     const int all = p.K / 64, tiles = p.N / COLS;
-    const int c0 = all * warp / RW_WARPS, chunks = all * (warp + 1) / RW_WARPS - c0;       // this warp's chunks of K
+    const int c0 = all * warp / RR_WARPS, chunks = all * (warp + 1) / RR_WARPS - c0;       // this warp's chunks of K
     const uint32_t own = smem_u32(ring) + warp * (DEPTH * CHUNK) + lane * 16;
     // the first row of octet r of a tile
     auto row_of = [&](int tile, int r) {
@@ -56,9 +54,6 @@ gemm_rows_kernel(const RowsParams p) {
     const bf16* xr = p.x + (size_t)g * p.ldx + c0 * 64 + tq * 8;
     const bf16* wr = p.w + (size_t)(row_of(blockIdx.x, 0) + g) * p.ldw + c0 * 64 + tq * 8;
     int w_tile = blockIdx.x, w_next = 0, w_into = 0, x_tile = blockIdx.x, x_next = 0, x_into = 0;
-    auto copy = [](uint32_t dst, const void* src, int bytes) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-    };
     auto ask_w = [&]() {
         if (w_tile >= tiles) return;
         const uint32_t dst = own + w_into * CHUNK;
@@ -66,7 +61,7 @@ gemm_rows_kernel(const RowsParams p) {
         for (int r = 0; r < R; ++r) {
             const int row = QKV ? (r >> 1) * (p.head_dim >> 1) + (r & 1) * 8 : r * 8;
 #pragma unroll
-            for (int b = 0; b < 2; ++b) copy(dst + (b * (R + H) + r) * 512, wr + (size_t)row * p.ldw + b * 32, 16);
+            for (int b = 0; b < 2; ++b) cp_async16(Chunk::weights_at(dst, b, r), wr + (size_t)row * p.ldw + b * 32, true);
         }
         w_into = w_into + 1 == DEPTH ? 0 : w_into + 1;
         if (++w_next == chunks) {
@@ -85,7 +80,7 @@ gemm_rows_kernel(const RowsParams p) {
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const bool in = h * 8 + g < p.M;
-                    copy(dst + (b * (R + H) + R + h) * 512, in ? xr + (size_t)h * 8 * p.ldx + x_next * 64 + b * 32 : p.x, in ? 16 : 0);
+                    cp_async16(Chunk::tokens_at(dst, b, h), in ? xr + (size_t)h * 8 * p.ldx + x_next * 64 + b * 32 : p.x, in);
                 }
             x_into = x_into + 1 == DEPTH ? 0 : x_into + 1;
             if (++x_next == chunks) { x_next = 0; x_tile += gridDim.x; }
@@ -124,63 +119,22 @@ gemm_rows_kernel(const RowsParams p) {
     }
     int from = 0;
     for (int tile = blockIdx.x, turn = 0; tile < tiles; tile += gridDim.x, turn ^= 1) {
-        float c[2][R / 2][H][4];        // (two chains)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int a = 0; a < R / 2; ++a)
-#pragma unroll
-                for (int h = 0; h < H; ++h)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) c[j][a][h][i] = 0.f;
+        RrSums<R, H> sums;
+        sums.clear();
 #pragma unroll 1
         for (int n = 0; n < chunks; ++n) {
             cp_async_wait<DEPTH - 2>();         // (a lane reads what it brought itself)
             const uint32_t src = own + from * CHUNK;
             from = from + 1 == DEPTH ? 0 : from + 1;
-            uint4 wv[2][R], xv[2][H];
-            auto read = [&](int at) {
-                uint4 v;
-                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src + at * 512) : "memory");
-                return v;
-            };
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) wv[b][r] = read(b * (R + H) + r);
-#pragma unroll
-                for (int h = 0; h < H; ++h) xv[b][h] = read(b * (R + H) + R + h);
-            }
+            Chunk chunk;
+            chunk.read(src);
             ask_w();                            // (into the place that the turn before this one read)
             ask_x();
-#pragma unroll
-            for (int b = 0; b < 2; ++b)
-#pragma unroll
-                for (int a = 0; a < R / 2; ++a) {
-                    const uint4 lo = wv[b][2 * a], hi = wv[b][2 * a + 1];
-                    const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
-#pragma unroll
-                    for (int h = 0; h < H; ++h) {
-                        mma_bf16(c[0][a][h], a0, xv[b][h].x, xv[b][h].y);
-                        mma_bf16(c[1][a][h], a1, xv[b][h].z, xv[b][h].w);
-                    }
-                }
+            sums.add(chunk);
         }
-        // c: (row g, tokens 2 tq and the next), (row g + 8, the same)
-#pragma unroll
-        for (int h = 0; h < H; ++h)
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    part[turn][warp][h * 8 + 2 * tq + e][r * 8 + g] = c[0][r / 2][h][2 * (r & 1) + e] + c[1][r / 2][h][2 * (r & 1) + e];
+        sums.leave(part, turn, warp, g, tq);
         __syncthreads();
-        auto sum = [&](int m, int q) {
-            float v = 0.f;
-#pragma unroll
-            for (int j = 0; j < RW_WARPS; ++j) v += part[turn][j][m][q];
-            return v;
-        };
+        auto sum = [&](int m, int q) { return rr_sum(part[turn], m, q); };
         if constexpr (QKV) {
             // (the grid is the tiles: one turn)
             const int head = tile / (p.head_dim / COLS), half = p.head_dim >> 1;
@@ -229,12 +183,12 @@ gemm_rows_kernel(const RowsParams p) {
                 }
             }
         } else if (p.swiglu) {
-            for (int i = threadIdx.x; i < p.M * (COLS / 2); i += RW_WARPS * 32) {
+            for (int i = threadIdx.x; i < p.M * (COLS / 2); i += RR_WARPS * 32) {
                 const int m = i / (COLS / 2), q = i - m * (COLS / 2);
                 ((bf16*)p.out)[(size_t)m * p.ldo + tile * (COLS / 2) + q] = swiglu_pair(sum(m, 2 * q), sum(m, 2 * q + 1));
             }
         } else {
-            for (int i = threadIdx.x; i < p.M * COLS; i += RW_WARPS * 32) {
+            for (int i = threadIdx.x; i < p.M * COLS; i += RR_WARPS * 32) {
                 const int m = i / COLS, q = i - m * COLS;
                 const size_t at = (size_t)m * p.ldo + tile * COLS + q;
                 if (p.out_f32) ((float*)p.out)[at] = sum(m, q);
@@ -247,16 +201,16 @@ gemm_rows_kernel(const RowsParams p) {
 
 template <int R, int H, int DEPTH, bool QKV>
 static int rw_launch(const RowsParams& p, int sms, cudaStream_t stream) {
-    constexpr int smem = RW_WARPS * DEPTH * 2 * (R + H) * 512, fixed = 2 * RW_WARPS * 8 * H * (8 * R + 4) * 4 + 2048;
+    constexpr int smem = RR_WARPS * DEPTH * RrChunk<R, H>::BYTES, fixed = 2 * RR_WARPS * 8 * H * (8 * R + 4) * 4 + 2048;
     constexpr int resident = 228 * 1024 / (smem + fixed) > 2 ? 2 : 228 * 1024 / (smem + fixed);
     static_assert(resident >= 1, "a block fits an SM's shared memory");
     static AcvSmemConfig cfg;
     auto kernel = gemm_rows_kernel<R, H, DEPTH, QKV>;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
     if (QKV)
-        acv_launch_cluster(PDL_GEMM, dim3(p.head_dim / (8 * R), 1, 1), kernel, dim3(p.N / (8 * R)), dim3(RW_WARPS * 32), smem, stream, p);
+        acv_launch_cluster(PDL_GEMM, dim3(p.head_dim / (8 * R), 1, 1), kernel, dim3(p.N / (8 * R)), dim3(RR_WARPS * 32), smem, stream, p);
     else
-        acv_launch(PDL_GEMM, kernel, dim3(min(p.N / (8 * R), resident * sms)), dim3(RW_WARPS * 32), smem, stream, p);
+        acv_launch(PDL_GEMM, kernel, dim3(min(p.N / (8 * R), resident * sms)), dim3(RR_WARPS * 32), smem, stream, p);
     return acv_launch_status();
 }
 

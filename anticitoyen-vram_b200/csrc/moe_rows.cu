@@ -3,14 +3,13 @@
 //
 // What bounds them is the stream of the chosen experts' weights, and the tiled form (moe.cu: 64 columns to a block, K walked
 // through three stages behind a barrier each, a new block for every tile) draws 5.1 to 5.5 TB/s.  Here blocks stay and walk over
-// (tile, columns) as csrc/gemm_rows.cu walks over columns: eight warps take an eighth of K each, a lane brings its own operands
+// (tile, columns) as gemm_rows.cu walks over columns (the inner loop is shared, rows_ring.cuh): eight warps take an eighth of K each, a lane brings its own operands
 // by 16-byte copies into a ring of its own, and the next columns' first copies are under way before the sums of these meet.
 // A layer of 64 experts of 1024 at width 4096, six choices, microseconds, the tiled form and now: 1 token 102 -> 57, 16 tokens 273 -> 229,
 // 64 tokens 360 -> 302; 32 experts of 768 at width 2048, four choices: 1 token 61 -> 29, 16 tokens 86 -> 70.
-#include "mma_tiles.cuh"
+#include "rows_ring.cuh"
 #include "moe_act.cuh"
 
-#define MX_WARPS 8
 #define MX_TILES 512        // tiles, and rows in them, that a block keeps the list of
 #define MX_ROWS 2048
 
@@ -27,29 +26,28 @@ struct MoeRowsParams {
 // H: octets of rows of a tile; DEPTH: chunks of 64 k in a warp's ring.  A block's 32 weight rows are 32 outputs, or the gate and the
 // up rows of sixteen.
 template <int H, int DEPTH, bool GLU>
-__global__ void __launch_bounds__(MX_WARPS * 32, 1)
+__global__ void __launch_bounds__(RR_WARPS * 32, 1)
 moe_rows_kernel(const MoeRowsParams p) {
-    constexpr int R = 4, CHUNK = 2 * (R + H) * 512, COLS = GLU ? 16 : 32, ROWS = 8 * H;
+    constexpr int R = 4, COLS = GLU ? 16 : 32, ROWS = 8 * H;
+    using Chunk = RrChunk<R, H>;
+    constexpr int CHUNK = Chunk::BYTES;
     extern __shared__ __align__(16) unsigned char ring[];
-    __shared__ float part[2][MX_WARPS][ROWS][36];
+    __shared__ float part[2][RR_WARPS][ROWS][36];
     __shared__ int experts[MX_TILES], rows[MX_ROWS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     pdl_launch_dependents();
     pdl_wait();
     const int used = *p.tiles_used;
-    for (int i = threadIdx.x; i < used; i += MX_WARPS * 32) experts[i] = p.tile_expert[i];
-    for (int i = threadIdx.x; i < used * ROWS; i += MX_WARPS * 32) rows[i] = p.grouped[i];
+    for (int i = threadIdx.x; i < used; i += RR_WARPS * 32) experts[i] = p.tile_expert[i];
+    for (int i = threadIdx.x; i < used * ROWS; i += RR_WARPS * 32) rows[i] = p.grouped[i];
     __syncthreads();
     const int all = p.K / 64, across = p.N / COLS, items = used * across;
-    const int c0 = all * warp / MX_WARPS, chunks = all * (warp + 1) / MX_WARPS - c0;       // this warp's chunks of K
+    const int c0 = all * warp / RR_WARPS, chunks = all * (warp + 1) / RR_WARPS - c0;       // this warp's chunks of K
     const uint32_t own = smem_u32(ring) + warp * (DEPTH * CHUNK) + lane * 16;
     const int step_u = GLU ? (p.pairs ? 1 : p.N) : 16;          // from octets 0, 1 to octets 2, 3: the up rows, or the next sixteen
     const int step_n = GLU && p.pairs ? 2 : 1;                  // from an output's weight row to the next one's
     const bf16 *wr = nullptr, *xr[H];
     int next_item = blockIdx.x, next = 0, into = 0;
-    auto copy = [](uint32_t dst, const void* src, int bytes) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-    };
     auto begin = [&]() {
         if (next_item >= items) return;
         const int tile = next_item / across, n0 = (next_item - tile * across) * COLS;
@@ -67,13 +65,13 @@ moe_rows_kernel(const MoeRowsParams p) {
             for (int r = 0; r < R; ++r) {
                 const bf16* from = wr + (size_t)((r >> 1) * step_u + (r & 1) * 8 * step_n) * p.ldw;
 #pragma unroll
-                for (int b = 0; b < 2; ++b) copy(dst + (b * (R + H) + r) * 512, from + b * 32, 16);
+                for (int b = 0; b < 2; ++b) cp_async16(Chunk::weights_at(dst, b, r), from + b * 32, true);
             }
 #pragma unroll
             for (int h = 0; h < H; ++h)
 #pragma unroll
                 for (int b = 0; b < 2; ++b)         // (rows that hold no token are zeros)
-                    copy(dst + (b * (R + H) + R + h) * 512, xr[h] ? xr[h] + next * 64 + b * 32 : p.x, xr[h] ? 16 : 0);
+                    cp_async16(Chunk::tokens_at(dst, b, h), xr[h] ? xr[h] + next * 64 + b * 32 : p.x, xr[h] != nullptr);
             into = into + 1 == DEPTH ? 0 : into + 1;
             if (++next == chunks) {
                 next = 0;
@@ -92,68 +90,29 @@ moe_rows_kernel(const MoeRowsParams p) {
     }
     int from = 0;
     for (int item = blockIdx.x, turn = 0; item < items; item += gridDim.x, turn ^= 1) {
-        float c[2][2][H][4];            // (two chains)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int h = 0; h < H; ++h)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) c[j][a][h][i] = 0.f;
+        RrSums<R, H> sums;
+        sums.clear();
 #pragma unroll 1
         for (int n = 0; n < chunks; ++n) {
             cp_async_wait<DEPTH - 2>();         // (a lane reads what it brought itself)
             const uint32_t src = own + from * CHUNK;
             from = from + 1 == DEPTH ? 0 : from + 1;
-            uint4 wv[2][R], xv[2][H];
-            auto read = [&](int at) {
-                uint4 v;
-                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src + at * 512) : "memory");
-                return v;
-            };
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) wv[b][r] = read(b * (R + H) + r);
-#pragma unroll
-                for (int h = 0; h < H; ++h) xv[b][h] = read(b * (R + H) + R + h);
-            }
+            Chunk chunk;
+            chunk.read(src);
             ask();                              // (into the place that the turn before this one read)
-#pragma unroll
-            for (int b = 0; b < 2; ++b)
-#pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    const uint4 lo = wv[b][2 * a], hi = wv[b][2 * a + 1];
-                    const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
-#pragma unroll
-                    for (int h = 0; h < H; ++h) {
-                        mma_bf16(c[0][a][h], a0, xv[b][h].x, xv[b][h].y);
-                        mma_bf16(c[1][a][h], a1, xv[b][h].z, xv[b][h].w);
-                    }
-                }
+            sums.add(chunk);
         }
-        // c: (weight row g, tokens 2 tq and the next), (weight row g + 8, the same)
-#pragma unroll
-        for (int h = 0; h < H; ++h)
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    part[turn][warp][h * 8 + 2 * tq + e][r * 8 + g] = c[0][r / 2][h][2 * (r & 1) + e] + c[1][r / 2][h][2 * (r & 1) + e];
+        sums.leave(part, turn, warp, g, tq);
         __syncthreads();
         const int tile = item / across, n0 = (item - tile * across) * COLS;
-        for (int i = threadIdx.x; i < ROWS * COLS; i += MX_WARPS * 32) {
+        for (int i = threadIdx.x; i < ROWS * COLS; i += RR_WARPS * 32) {
             const int m = i / COLS, q = i - m * COLS, s = rows[tile * ROWS + m];
             if (s < 0) continue;
             const float w = p.row_weight ? p.row_weight[s] : 1.f;
             const size_t at = (size_t)(tile * ROWS + m) * p.ldo + n0 + q;
-            float v = 0.f, u = 0.f;
-#pragma unroll
-            for (int j = 0; j < MX_WARPS; ++j) v += part[turn][j][m][q];
+            const float v = rr_sum(part[turn], m, q);
             if constexpr (GLU) {
-#pragma unroll
-                for (int j = 0; j < MX_WARPS; ++j) u += part[turn][j][m][16 + q];
+                const float u = rr_sum(part[turn], m, 16 + q);
                 ((bf16*)p.out)[at] = __float2bfloat16_rn(glu_act<bf16>(v * w, u * w, p.limit, p.alpha, p.shift));
             } else if (p.which == 2) {
                 ((bf16*)p.out)[at] = __float2bfloat16_rn(plain_act(v * w, p.pairs));
@@ -167,11 +126,11 @@ moe_rows_kernel(const MoeRowsParams p) {
 
 template <int H, int DEPTH, bool GLU>
 static int mx_launch(const MoeRowsParams& p, int blocks, cudaStream_t stream) {
-    constexpr int smem = MX_WARPS * DEPTH * 2 * (4 + H) * 512;
+    constexpr int smem = RR_WARPS * DEPTH * RrChunk<4, H>::BYTES;
     static AcvSmemConfig cfg;
     auto kernel = moe_rows_kernel<H, DEPTH, GLU>;
     if (const int e = acv_ensure_smem(cfg, kernel, smem)) return e;
-    acv_launch(PDL_GEMM, kernel, dim3(blocks), dim3(MX_WARPS * 32), smem, stream, p);
+    acv_launch(PDL_GEMM, kernel, dim3(blocks), dim3(RR_WARPS * 32), smem, stream, p);
     return acv_launch_status();
 }
 
