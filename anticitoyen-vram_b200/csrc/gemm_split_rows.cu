@@ -1,6 +1,7 @@
-// The 32-bit product of gemm_split_tc.cu for up to 16 tokens: the same parts, the same products in the same order, on
-// mma.sync, whose sums of 16 products are the tcgen05 unit's to the bit (the tests compare the two), so a row's result does not
-// depend on how many rows there are.
+// The 32-bit product of gemm_split_tc.cu for up to 16 tokens, and for few outputs: the same parts, the same products in the same order,
+// on mma.sync, whose sums of 16 products are the tcgen05 unit's to the bit, so a row's result does not depend on how many rows
+// there are.  No document says that the two units sum alike: it is measured, and the tests compare them over terms of all sizes, terms
+// that cancel, sums that grow throughout, and operands at both ends of a float's range.
 //
 // What bounds it is the weights' stream.  Every lane brings its own operands by asynchronous copies into a ring of its
 // own (four neighbouring k of a weight row; which k of a step of 16 a lane holds is the same for tokens and weights), so the
@@ -9,8 +10,9 @@
 // memory.  A block goes on to its next rows with their first copies already under way.  Microseconds, multiply-adds on the
 // CUDA cores (gemm_simt.cu) and now: 1, 4, 8 and 16 tokens 4096 x 1024 5.6, 6.2, 7.5, 8.9 -> 5.8, 5.7, 6.0, 7.3; 1024 x 3072 6.0,
 // 7.7, 10.1, 12.3 -> 6.3, 6.3, 6.4, 9.4; 12288 x 2048 21.5, 28.6, 36.2, 40.9 -> 19.9, 21.9, 23.4, 31.8; 151936 x 1024 107, 125, 165, 235
-// -> 96 (6.4 TB/s of weights), 98, 104, 152.  One token on few rows is what it makes more slowly: 1024 x 2048 4.6 -> 5.0,
-// 2048 x 2048 5.5 -> 6.0, 4096 x 2048 8.3 -> 8.8, 2048 x 6144 12.1 -> 13.3.  Rows without 16-byte pieces, 50000 x 1026: 127, 128, 317, 317 ->
+// -> 96 (6.4 TB/s of weights), 98, 104, 152.  One token on few or long rows is what it makes more slowly: 1024 x 2048 4.6 -> 5.0,
+// 2048 x 2048 5.5 -> 6.0, 2048 x 6144 12.1 -> 13.3, 512 x 4096 6.9 -> 8.1, 1024 x 12288 19 -> 22; and K just above 1024, whose groups are
+// six (3000 x 1100, 2 tokens 6.1 -> 7.8).  Rows without 16-byte pieces, 50000 x 1026: 127, 128, 317, 317 ->
 // 68, 71, 71, 86.
 #include "mma_tiles.cuh"
 #include "gemm_split_tc.h"

@@ -1,15 +1,16 @@
 // C[M,N] = A[M,K] . W[N,K]^T in 32-bit precision on the fifth-generation tensor cores.
 //
-// A float is the exact sum of three bfloat16 values, x = x1 + x2 + x3 (each the rounding of what the ones before it leave:
-// 8 + 8 + 8 bits), and products of bfloat16 values are exact in the tensor core's float accumulators.  Of the nine products
-// of parts the six above 2^-24 of the result are made: over a chunk of GF_CHUNK k the accumulator takes w1 a2, w2 a1, w1 a3,
+// A float, times 2^24 so that the smallest ones are among them (gemm_split_tc.h), is the exact sum of three bfloat16 values,
+// x = x1 + x2 + x3 (each the rounding of what the ones before it leave: 8 + 8 + 8 bits), and products of bfloat16 values are exact
+// in the tensor core's float accumulators.  Of the nine products of parts the six above 2^-24 of the result are made: over a chunk of GF_CHUNK k the accumulator takes w1 a2, w2 a1, w1 a3,
 // w2 a2, w3 a1 (2^-8 of the result and less) and at last w1 a1.  The tensor core's additions cut off instead of rounding, so
 // no more than the two of w1 a1 follow one another at full size; the chunks are added in registers, to nearest.
 //
 // The order of a sum is a property of K alone, as in gemm_simt.cu: K is cut into up to eight groups of gf_group_length(K), a
 // group is its chunks in ascending order, groups are added in ascending order.  So a row's result does not depend
 // on the other rows, on M, N or the tile.  An output that is no finite number this way (an infinity among the operands has no
-// three parts) is made again by a plain chain of multiply-adds, with the order of gemm_simt.cu.
+// three parts; operands from 2^104 and sums from 2^80 on leave a float's range by the scale) is made again by a plain chain of
+// multiply-adds, with the order of gemm_simt.cu.
 //
 // Weight rows fill the tensor core's M = 128, tokens are its N (BT of them): weights are read once for up to 128 tokens.
 // Converter warps read float rows straight into registers (a stage ahead), cut them into parts and leave those in shared

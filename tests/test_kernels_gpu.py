@@ -485,6 +485,21 @@ def test_gemm_split_infinities_and_gate(ops, M):
     assert clean.isfinite().all()
 
 
+@pytest.mark.parametrize("M", [3, 16, 40, 500])
+def test_gemm_split_gate_beside_infinities(ops, M):
+    """The batched form's gate on results that leave with it and on those that are made again: infinities, a NaN, a sum out of the
+    scale's range, a gate that closes and one that is none."""
+    K, N = 1030, 140
+    w, gate, x = rnd(2, N, K, scale=0.05, seed=61), rnd(M, 2, N, seed=62), rnd(M, 2, K, seed=63)
+    x[0, 0, 5], x[1, 1, 1029], w[1, 7, 3], x[2, 0, 17] = float("inf"), float("nan"), -float("inf"), 3e30
+    gate[0, 0, 3], gate[2, 0, 9], gate[2, 1, 11] = -float("inf"), float("inf"), float("nan")
+    out = ops.gemm_batched(x, w, torch.full((M, 2, N), 7.0, device="cuda"), gate)
+    want = torch.einsum("mbk,bnk->mbn", x.double(), w.double()) / (1 + torch.exp(-gate.double()))
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.isinf())
+    ok = want.isfinite()
+    torch.testing.assert_close(out[ok].double(), want[ok], rtol=1e-5, atol=1e-5)
+
+
 @pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 16, 17, 33, 65, 129, 700])
 @pytest.mark.parametrize("N,K", [(1, 4), (65, 33), (129, 256), (200, 2052), (1030, 260)])
 def test_gemm_simt_one_order_of_sums(ops, M, N, K):
