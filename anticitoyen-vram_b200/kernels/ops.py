@@ -1492,21 +1492,26 @@ def moe_rows(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, grouped: torch
 
 def moe_rows_tile(rows: int, experts: int, h: torch.Tensor, up: torch.Tensor, down: torch.Tensor) -> int:
     """Rows of a tile (8 or 16) where the experts' products are made by ``moe_rows``, 0 where they are not."""
-    tile = 8 if rows <= MOE_ROWS_8 * experts else 16
-    if rows > MOE_ROWS_16 * experts or h.shape[1] % 64 or down.shape[2] % 64 or up.shape[1] % 32 or down.shape[1] % 32 \
-            or not moe_gemm_mma_takes(h, up) or not _moe_mma_weights(down):
+    if rows > MOE_ROWS_16 * experts or h.shape[0] > MOE_ROWS_TOKENS_16 or h.shape[1] % 64 or down.shape[2] % 64 or up.shape[1] % 32 \
+            or down.shape[1] % 32 or not moe_gemm_mma_takes(h, up) or not _moe_mma_weights(down):
         return 0
-    if tile == 16 and h.shape[1] < 1024 and experts * down.shape[2] > 96 * sm_count(h.device):
+    fits = lambda tile: moe_max_tiles(rows, experts, tile) <= min(512, 2048 // tile)
+    if rows <= MOE_ROWS_8 * experts and (h.shape[0] <= MOE_ROWS_TOKENS_8 or not fits(16)):
+        return 8 if fits(8) else 0
+    if h.shape[1] < 1024 and experts * down.shape[2] > 96 * sm_count(h.device):
         return 0            # short rows for more than six blocks one after the other on an SM
-    tiles = moe_max_tiles(rows, experts, tile)
-    return tile if tiles <= 512 and tiles * tile <= 2048 else 0
+    return 16 if fits(16) else 0
 
 
 # Rows to an expert up to which tiles of 8 and of 16 rows are used.  A layer's microseconds with tiles of 64 (moe_gemm_mma), 8 and 16
 # rows: 64 experts of 1024 at width 4096 at 0.1 rows an expert 102, 57, 60; 1.5: 273, 229, 246; 6: 360, 302, 304; 9.4: 369, 344, 320;
 # 32 experts of 768 at width 2048 at 8: 99, 96, 96; 12.5: 106, 122, 113.  Where rows are short, a tile's sums take what its loads save: at 8
 # rows an expert with tiles of 64 and 16 rows 64 experts of 384 at width 768 36, 40; of 256 at 512 23, 26; 32 of 256 at 1024 29, 23.
+# An expert's tiles read its weights once each, and where many tokens choose the same few experts the tiles are many, so tiles of 8 are
+# for up to 40 tokens and of 16 for up to 112 (64 experts of 768 at width 4096, 64 tokens, as evenly as they come, and all on six
+# experts: tiles of 64 232, 120; of 8 211, 116; of 16 224, 88; experts of 1024 323, 111; 271, 139; 273, 106; 100 tokens 336, 150; 309, 217; 291, 175).
 MOE_ROWS_8, MOE_ROWS_16 = 7, 10
+MOE_ROWS_TOKENS_8, MOE_ROWS_TOKENS_16 = 40, 112
 
 
 def moe_experts_up(h: torch.Tensor, gate_up: torch.Tensor, act: torch.Tensor, grouped: torch.Tensor, tile_expert: torch.Tensor,

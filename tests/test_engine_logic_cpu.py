@@ -554,3 +554,16 @@ def test_experts_of_few_rows_want_both_products_weights_dense_and_aligned(which,
 def test_products_of_few_tokens_go_where_they_are_faster(M, N, K, pays):
     from acvram_b200.kernels import ops
     assert ops.gemm_rows_pays(M, N, K, 148) == pays
+
+
+@pytest.mark.parametrize("T,E,top,W,F,tile", [
+    (1, 64, 6, 4096, 1024, 8), (40, 64, 6, 4096, 1024, 8), (41, 64, 6, 4096, 1024, 16), (64, 64, 6, 4096, 1024, 16), (106, 64, 6, 4096, 1024, 16),
+    (107, 64, 6, 4096, 1024, 0), (64, 128, 8, 2048, 768, 8), (56, 32, 4, 2048, 768, 16), (113, 32, 2, 2048, 768, 0), (64, 64, 8, 768, 384, 0),
+    (32, 64, 8, 768, 384, 8), (64, 32, 4, 1024, 256, 16), (4, 8, 2, 96, 64, 0), (4, 8, 2, 128, 96, 0)])
+def test_tiles_of_experts_of_few_rows(T, E, top, W, F, tile):
+    """Eight or sixteen rows by the rows to an expert and the tokens, which bound how often an expert's weights are read, however
+    unevenly they choose; none for short rows behind many blocks and for sizes that the kernel does not take."""
+    import torch
+    from acvram_b200.kernels import ops
+    weights = lambda rows, cols: torch.empty(E, rows, cols, dtype=torch.bfloat16)
+    assert ops.moe_rows_tile(T * top, E, torch.zeros(T, W, dtype=torch.bfloat16), weights(2 * F, W), weights(W, F)) == tile
